@@ -40,6 +40,10 @@ unsigned long long qw_gpu_launch_count(const qw_gpu *g);
 /* Replay identical batches as CUDA graphs (default off; QW_GRAPH=1 in the environment turns it on). */
 void qw_gpu_set_graphs(qw_gpu *g, bool on);
 
+/* This batch is launched directly even while graphs are on: for work whose sizes do not come again (recording and
+ * instantiating a graph costs more than launching it once). */
+void qw_batch_plain(qw_batch *b);
+
 /* Programmatic dependent launch for the kernels of later batches (default on; QW_PDL=0 in the environment turns it
  * off): each kernel may start while its predecessor drains and waits on the device for the predecessor's results. */
 void qw_gpu_set_pdl(qw_gpu *g, bool on);

@@ -123,6 +123,7 @@ struct qw_batch {
     cudaEvent_t e0, e1;
     std::vector<cudaEvent_t> pev;  // profiling: 2 per dispatch
     bool submitted, failed;
+    bool plain;  // launched directly even when graphs are on: it is not going to be replayed
 };
 
 static void graph_cache_clear(qw_gpu *g) {
@@ -471,7 +472,7 @@ extern "C" qw_batch *qw_batch_begin(qw_gpu *g, bool /*concurrent*/) {
     memset(b->cur_b, 0, sizeof b->cur_b);
     b->cur_tg = 0;
     b->e0 = b->e1 = nullptr;
-    b->submitted = b->failed = false;
+    b->submitted = b->failed = b->plain = false;
     b->recs.reserve(1024);
     return b;
 }
@@ -527,6 +528,9 @@ extern "C" void qw_batch_dispatch(qw_batch *b, unsigned gx, unsigned gy, unsigne
     b->recs.push_back(r);
 }
 
+extern "C" void qw_batch_plain(qw_batch *b) {
+    if (b) b->plain = true;
+}
 extern "C" void qw_batch_barrier(qw_batch *) {}
 extern "C" void qw_batch_flush(qw_batch *) {}
 
@@ -585,7 +589,7 @@ extern "C" void qw_batch_submit(qw_batch *b) {
         return;
     }
     cudaEventRecord(b->e0, b->stream);
-    if (g->graphs && !g->profile && b->recs.size() > 1) {
+    if (g->graphs && !b->plain && !g->profile && b->recs.size() > 1) {
         std::vector<uint8_t> key;
         key.reserve(b->recs.size() * 320);
         auto put = [&](const void *p, size_t n) { key.insert(key.end(), (const uint8_t *)p, (const uint8_t *)p + n); };

@@ -17,6 +17,7 @@
 using namespace qw;
 
 #define GDN_EPS 1e-6f
+#define GDN_SEQ_MAX 64  // tokens of one gdn_seq launch (their normalised q and k sit in shared memory)
 
 // proj row layout (fp16, stride PS): [q: HK*DK | k: HK*DK | v: HV*DV | z: HV*DV | a: HV | b: HV]
 struct dn_epi_args {
@@ -75,6 +76,50 @@ static cudaError_t launch_dn_epi(const QwLaunch &L) {
     return cudaGetLastError();
 }
 QW_FAMILY(dn_epi, launch_dn_epi, 256)
+
+// The same epilogue for nb consecutive tokens of ONE slot (a piece of a prompt), newest token first: row r is the token at
+// sequence position nb - 1 - r of the piece.  A token's three predecessors are rows of the same projection (the state holds
+// exactly those fp16 values as fp32) or, for the first three tokens, the slot's conv state, which this kernel only reads:
+// gdn_seq, the next launch, writes the piece's last three inputs into it.
+// binds as dn_epi (2 is not written).  grid (ceil((C + 2 HV)/256), nb) x 256
+__global__ void __launch_bounds__(256) dn_epi_seq_k(const __half *proj, const float *cw, const float *pool, const float *An, const float *dtb, __half *cv,
+                                                    float *la, float *be, const int32_t *sids, dn_epi_args a, uint32_t C, uint32_t HV) {
+    pdl_sync();
+    const uint32_t g = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
+    const int tau = (int)(a.nb - 1 - t);  // position in the piece
+    const __half *pr = proj + (size_t)t * a.proj_stride;
+    if (g < C) {
+        const float *st = pool + ((size_t)sids[0] * a.nlayers + a.layer) * 3 * C + g;
+        auto at = [&](int k) { return k >= 0 ? __half2float(pr[(size_t)(tau - k) * a.proj_stride + g]) : st[(size_t)(3 + k) * C]; };
+        const float s0 = at(tau - 3), s1 = at(tau - 2), s2 = at(tau - 1), s3 = __half2float(pr[g]);
+        const float4 w = *(const float4 *)(cw + 4 * (size_t)g);
+        const float y = w.x * s0 + w.y * s1 + w.z * s2 + w.w * s3;
+        cv[(size_t)t * C + g] = __float2half_rn(y / (1.0f + expf(-y)));
+    } else if (g < C + HV) {
+        const uint32_t j = g - C;
+        const float xa = __half2float(pr[C + HV * 128 + j]) + dtb[j];
+        const float sp = xa > 20.0f ? xa : logf(1.0f + expf(xa));
+        la[t * HV + j] = An[j] * sp;
+    } else if (g < C + 2 * HV) {
+        const uint32_t j = g - C - HV;
+        be[t * HV + j] = 1.0f / (1.0f + expf(-__half2float(pr[C + HV * 128 + HV + j])));
+    }
+}
+
+static cudaError_t launch_dn_epi_seq(const QwLaunch &L) {
+    const uint32_t HK = (uint32_t)L.def("HK", 16), HV = (uint32_t)L.def("HV", 32), DK = (uint32_t)L.def("DK", 128), DV = (uint32_t)L.def("DV", 128);
+    const uint32_t C = 2 * HK * DK + HV * DV;
+    dn_epi_args a = L.bytes<dn_epi_args>(9);
+    QW_CHECK_ARG(DV == 128 && DK == 128 && L.has_bytes(9, 16) && a.nb >= 1 && a.nb <= GDN_SEQ_MAX && a.layer < a.nlayers);
+    QW_CHECK_ARG(a.proj_stride >= C + HV * DV + 2 * HV);
+    for (int i = 0; i <= 8; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+    QW_CHECK_ARG(L.avail(0) >= ((size_t)(a.nb - 1) * a.proj_stride + C + HV * DV + 2 * HV) * 2 && L.avail(1) >= (size_t)C * 16 &&
+                 L.avail(5) >= (size_t)a.nb * C * 2 && L.avail(6) >= (size_t)a.nb * HV * 4 && L.avail(7) >= (size_t)a.nb * HV * 4 && L.avail(8) >= 4);
+    qw_launch(dn_epi_seq_k, dim3((C + 2 * HV + 255) / 256, a.nb), 256, 0, L.stream, L.buf<__half>(0), L.buf<float>(1), L.buf<float>(2), L.buf<float>(3),
+              L.buf<float>(4), L.buf<__half>(5), L.buf<float>(6), L.buf<float>(7), L.buf<int32_t>(8), a, C, HV);
+    return cudaGetLastError();
+}
+QW_FAMILY(dn_epi_seq, launch_dn_epi_seq, 256)
 
 // ------------------------------------------------------------------------------------------------ recurrent step
 struct gdn_args {
@@ -212,3 +257,168 @@ static cudaError_t launch_gdn_fstep(const QwLaunch &L) {
     return cudaGetLastError();
 }
 QW_FAMILY(gdn_fstep, launch_gdn_fstep, 512)
+
+// ------------------------------------------------------------------------------------------------ recurrence over a piece of a prompt
+// nb consecutive tokens of ONE slot (row r = token nb - 1 - r of the piece, as dn_epi_seq): the state is loaded once, the tokens run
+// one after another, the state is stored once.  The columns of the state are independent in the recurrence, so a head is split
+// over 4 blocks of 32 columns; a column is held by 4 lanes of a warp, 32 rows each, in registers, and nothing but shuffles joins
+// them: no block barrier inside the token loop.  Bound by the latency of one token's chain (decay, S^T k, the ordered sum over
+// row groups, the update): 0.7 us per token, 44 us for 64 tokens of a layer (64 launches of gdn_fstep: 64 x 4 us).
+// Bit-identical to nb launches of gdn_fstep: the 16 partial sums of eight rows each are the same fma chains and are added in the same order
+// 0 .. 15 (four lanes pass the running sum on).  The sum of S^T q of a token is carried through beside the next token's S^T k:
+// it is off the recurrence.  The gated RMSNorm needs all 128 columns of a head: gdn_gate does it afterwards.
+// binds: 0 = cv fp16 [nb][C], 1 = la [nb][HV], 2 = beta [nb][HV], 3 = state pool, 4 = proj fp16 (row stride z_stride), 5 = conv state
+// pool (the last three inputs of the piece are written), 6 = o out fp16 [nb][HV*DV] (not normalised), 7 = slot ids (entry 0), 8 = gdn_args.
+// grid (4, HV) x 128
+template <bool TILED>
+__global__ void __launch_bounds__(128) gdn_seq_k(const __half *cv, const float *la, const float *beta, float *pool, const __half *proj, float *conv,
+                                                 __half *oo, const int32_t *sids, gdn_args a, uint32_t HK, uint32_t HV) {
+    constexpr int DK = 128, DV = 128, CW = 32;
+    extern __shared__ __align__(16) float seq_smem[];
+    float *kq = seq_smem;                              // [token][k 128 | q 128]
+    float2 *gb = (float2 *)(seq_smem + a.nb * 256);    // [token] decay, beta
+    pdl_sync();
+    const uint32_t cb = blockIdx.x, hv = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = a.nb;
+    const uint32_t hk = TILED ? hv % HK : hv / (HV / HK), q = lane >> 3, col = cb * CW + warp * 8 + (lane & 7);
+    const uint32_t C = 2 * HK * DK + HV * DV;
+    const uint32_t slot = (uint32_t)sids[0];
+    float *S = pool + (((size_t)slot * a.nlayers + a.layer) * HV + hv) * DK * DV + (size_t)(32 * q) * DV + col;
+    float s[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) s[i] = S[(size_t)i * DV];
+
+    // the piece's normalised q and k (expressions of gdn_fstep), decay and beta: tau = position in the piece, row nb - 1 - tau
+    for (uint32_t tau = warp; tau < nb; tau += 4) {
+        const __half *row = cv + (size_t)(nb - 1 - tau) * C;
+        const __half *qh = row + hk * DK, *kh = row + HK * DK + hk * DK;
+        const uint2 q4 = *(const uint2 *)(qh + 4 * lane), k4 = *(const uint2 *)(kh + 4 * lane);
+        const float2 qa = __half22float2(*(const __half2 *)&q4.x), qb = __half22float2(*(const __half2 *)&q4.y);
+        const float2 ka = __half22float2(*(const __half2 *)&k4.x), kb = __half22float2(*(const __half2 *)&k4.y);
+        const float qss = warp_sum(fmaf(qa.x, qa.x, fmaf(qa.y, qa.y, fmaf(qb.x, qb.x, qb.y * qb.y))));
+        const float kss = warp_sum(fmaf(ka.x, ka.x, fmaf(ka.y, ka.y, fmaf(kb.x, kb.x, kb.y * kb.y))));
+        const float rq_ = rsqrtf(qss / DK + GDN_EPS), rk_ = rsqrtf(kss / DK + GDN_EPS);
+        auto qnorm = [&](float v) { return __half2float(__float2half_rn(v * rq_ / DK)); };
+        auto knorm = [&](float v) { return __half2float(__float2half_rn(v * rk_ * rsqrtf((float)DK))); };
+        *(float4 *)(kq + tau * 256 + 4 * lane) = make_float4(knorm(ka.x), knorm(ka.y), knorm(kb.x), knorm(kb.y));
+        *(float4 *)(kq + tau * 256 + 128 + 4 * lane) = make_float4(qnorm(qa.x), qnorm(qa.y), qnorm(qb.x), qnorm(qb.y));
+        if (lane == 0) gb[tau] = make_float2(expf(la[(size_t)(nb - 1 - tau) * HV + hv]), beta[(size_t)(nb - 1 - tau) * HV + hv]);
+    }
+    // the conv state after the piece: its last three inputs (channels are spread over the launch's blocks; dn_epi_seq has read the old ones)
+    for (uint32_t ch = (hv * 4 + cb) * 128 + tid; ch < C; ch += 4 * HV * 128) {
+        float *st = conv + ((size_t)slot * a.nlayers + a.layer) * 3 * C + ch;
+        float nw[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int k = (int)nb - 3 + i;  // position in the piece; before it: the old state
+            nw[i] = k >= 0 ? __half2float(proj[(size_t)(2 - i) * a.z_stride + ch]) : st[(size_t)(3 + k) * C];
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) st[(size_t)i * C] = nw[i];
+    }
+    __syncthreads();
+
+    // running sum over the four lanes of a column: lane q adds its four group sums to what lane q - 1 hands over; the last one has the total
+    auto chain = [&](const float (&g)[4]) {
+        float m = ((g[0] + g[1]) + g[2]) + g[3];  // lanes q = 0: groups 0 .. 3
+#pragma unroll
+        for (uint32_t h = 1; h < 4; h++) {
+            const float v = __shfl_up_sync(0xffffffffu, m, 8);
+            if (q == h) m = (((v + g[0]) + g[1]) + g[2]) + g[3];
+        }
+        return m;
+    };
+    const __half *vrow = cv + 2 * HK * DK + hv * DV + col;
+    float og[4] = {0.f, 0.f, 0.f, 0.f};
+    __half vnext = vrow[(size_t)(nb - 1) * C];
+    for (uint32_t tau = 0; tau < nb; tau++) {
+        const float2 db = gb[tau];
+        const float v = __half2float(vnext);
+        if (tau + 1 < nb) vnext = vrow[(size_t)(nb - 2 - tau) * C];
+        const float4 *k4 = (const float4 *)(kq + tau * 256 + 32 * q), *q4 = (const float4 *)(kq + tau * 256 + 128 + 32 * q);
+        float kk[32], mg[4];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 x = k4[i];
+            kk[4 * i] = x.x; kk[4 * i + 1] = x.y; kk[4 * i + 2] = x.z; kk[4 * i + 3] = x.w;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            float m = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                s[8 * r + i] *= db.x;
+                m = fmaf(s[8 * r + i], kk[8 * r + i], m);
+            }
+            mg[r] = m;
+        }
+        const float mt = chain(mg), ot = chain(og);  // (the previous token's output rides along)
+        if (q == 3 && tau) oo[(size_t)(nb - tau) * HV * DV + hv * DV + col] = __float2half_rn(ot);
+        const float d = db.y * (v - __shfl_sync(0xffffffffu, mt, 24 + (lane & 7)));
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            float o = 0.f;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float4 x = q4[2 * r + i];
+                const float qq[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int e = 8 * r + 4 * i + j;
+                    s[e] = fmaf(kk[e], d, s[e]);
+                    o = fmaf(s[e], qq[j], o);
+                }
+            }
+            og[r] = o;
+        }
+    }
+    const float ot = chain(og);
+    if (q == 3) oo[(size_t)hv * DV + col] = __float2half_rn(ot);
+#pragma unroll
+    for (int i = 0; i < 32; i++) S[(size_t)i * DV] = s[i];
+}
+
+static cudaError_t launch_gdn_seq(const QwLaunch &L) {
+    const uint32_t HK = (uint32_t)L.def("HK", 16), HV = (uint32_t)L.def("HV", 32), DK = (uint32_t)L.def("DK", 128), DV = (uint32_t)L.def("DV", 128);
+    const bool tiled = L.def("GDN_TILED", 1) != 0;
+    const uint32_t C = 2 * HK * DK + HV * DV;
+    gdn_args a = L.bytes<gdn_args>(8);
+    QW_CHECK_ARG(DK == 128 && DV == 128 && HV % HK == 0 && L.has_bytes(8, 16) && a.nb >= 1 && a.nb <= GDN_SEQ_MAX && a.layer < a.nlayers && a.z_stride >= C);
+    for (int i = 0; i <= 7; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+    QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * C * 2 && L.avail(1) >= (size_t)a.nb * HV * 4 && L.avail(2) >= (size_t)a.nb * HV * 4 &&
+                 L.avail(4) >= ((size_t)(a.nb - 1) * a.z_stride + C) * 2 && L.avail(6) >= (size_t)a.nb * HV * DV * 2 && L.avail(7) >= 4);
+    const size_t smem = (size_t)a.nb * (256 * 4 + 8);
+    auto kern = tiled ? gdn_seq_k<true> : gdn_seq_k<false>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GDN_SEQ_MAX * (256 * 4 + 8));
+    if (e != cudaSuccess) return e;
+    qw_launch(kern, dim3(4, HV), 128, smem, L.stream, L.buf<__half>(0), L.buf<float>(1), L.buf<float>(2), L.buf<float>(3), L.buf<__half>(4), L.buf<float>(5),
+              L.buf<__half>(6), L.buf<int32_t>(7), a, HK, HV);
+    return cudaGetLastError();
+}
+QW_FAMILY(gdn_seq, launch_gdn_seq, 128)
+
+// Gated RMSNorm of gdn_seq's output, in the expressions of gdn_fstep: y = o * rsqrt(mean o^2 + eps) * w * sigmoid(z), in place.
+// binds: 0 = o fp16 [nb][HV*DV] (becomes y), 4 = z fp16 (row stride z_stride), 5 = norm weight fp32 [DV], 8 = gdn_args.  grid (HV, nb) x 128
+__global__ void __launch_bounds__(128) gdn_gate_k(__half *o, const __half *z, const float *nw, gdn_args a, uint32_t HV) {
+    constexpr int DV = 128;
+    __shared__ float red[4];
+    pdl_sync();
+    const uint32_t hv = blockIdx.x, t = blockIdx.y, c = threadIdx.x, lane = c & 31, warp = c >> 5;
+    __half *p = o + (size_t)t * HV * DV + hv * DV + c;
+    const float zz = __half2float(z[(size_t)t * a.z_stride + hv * DV + c]);
+    const float x = __half2float(*p);
+    const float ss = warp_sum(x * x);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    const float r = rsqrtf((((red[0] + red[1]) + red[2]) + red[3]) / DV + GDN_EPS);
+    *p = __float2half_rn(x * r * nw[c] * (1.0f / (1.0f + expf(-zz))));
+}
+static cudaError_t launch_gdn_gate(const QwLaunch &L) {
+    const uint32_t HV = (uint32_t)L.def("HV", 32), DV = (uint32_t)L.def("DV", 128);
+    gdn_args a = L.bytes<gdn_args>(8);
+    QW_CHECK_ARG(DV == 128 && L.has_bytes(8, 16) && a.nb >= 1 && a.nb <= GDN_SEQ_MAX && a.z_stride >= HV * DV);
+    QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(4) && L.buf<void>(5) && L.avail(0) >= (size_t)a.nb * HV * DV * 2 &&
+                 L.avail(4) >= ((size_t)(a.nb - 1) * a.z_stride + HV * DV) * 2 && L.avail(5) >= DV * 4);
+    qw_launch(gdn_gate_k, dim3(HV, a.nb), 128, 0, L.stream, L.buf<__half>(0), L.buf<__half>(4), L.buf<float>(5), a, HV);
+    return cudaGetLastError();
+}
+QW_FAMILY(gdn_gate, launch_gdn_gate, 128)

@@ -321,6 +321,28 @@ static cudaError_t launch_par_begin(const QwLaunch &L) {
 }
 QW_FAMILY(par_begin, launch_par_begin, 256)
 
+// Control block of a piece of a prompt: n consecutive tokens of one slot, newest first (row r = prompt position p0 + n - 1 - r), so
+// that the piece's last token is row 0.  The prompt was copied to the device once; nothing is read from the host per piece.
+// binds: 0 = prompt int32, 1 = control block [3][rows] (token, slot, position), 2 = {p0, n, slot, rows}
+struct par_chunk_args { uint32_t p0, n, slot, rows; };
+__global__ void par_chunk_k(const int32_t *prompt, int32_t *ctl, par_chunk_args a) {
+    pdl_sync();
+    for (uint32_t r = threadIdx.x; r < a.n; r += blockDim.x) {
+        const uint32_t pos = a.p0 + a.n - 1 - r;
+        ctl[r] = prompt[pos];
+        ctl[a.rows + r] = (int32_t)a.slot;
+        ctl[2 * a.rows + r] = (int32_t)pos;
+    }
+}
+static cudaError_t launch_par_chunk(const QwLaunch &L) {
+    const par_chunk_args a = L.bytes<par_chunk_args>(2);
+    QW_CHECK_ARG(L.has_bytes(2, 16) && L.buf<void>(0) && L.buf<void>(1) && a.n >= 1 && a.n <= a.rows && L.avail(0) >= ((size_t)a.p0 + a.n) * 4 &&
+                 L.avail(1) >= (size_t)a.rows * 12);
+    qw_launch(par_chunk_k, 1, 256, 0, L.stream, L.buf<int32_t>(0), L.buf<int32_t>(1), a);
+    return cudaGetLastError();
+}
+QW_FAMILY(par_chunk, launch_par_chunk, 256)
+
 // ------------------------------------------------------------------------------------------------ fill
 // Counter-based generator: byte i of a tensor with seed s is the low byte of mix64(s * 0x9E3779B97F4A7C15 + i)
 // (qwental_b200/synth.py holds the same functions in numpy).

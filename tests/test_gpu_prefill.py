@@ -1,0 +1,47 @@
+"""Prompt processing in pieces (qw_engine_par_prefill) against the decode step fed one token at a time: logits, recurrent and
+conv state and KV pages bit for bit, at prompt lengths around the edges of a piece, of the convolution's window and of a KV page."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    from qwental_b200.gpu import Gpu
+    g = Gpu()
+    yield g
+    g.close()
+
+
+def state_of(e, sid):
+    c = e.cfg
+    n_attn = c.layers // c.attn_every
+    pages = e.tap("pages", sid, np.int32)
+    kv = np.stack([e.tap("kvpage", int(p), np.float16).reshape(n_attn, 2, c.kvh, 256, c.hd) for p in pages])
+    kv = np.moveaxis(kv, 0, 3).reshape(n_attn, 2, c.kvh, -1, c.hd)[:, :, :, :e.pos(sid)]
+    return e.tap("sstate", sid, np.uint32), e.tap("cstate", sid, np.uint32), kv.view(np.uint16)
+
+
+@pytest.mark.parametrize("model", ["tiny", "wide", "wide_fma"])
+def test_prefill_equals_stepping_every_token(gpu, model):
+    from qwental_b200.engine import Engine, tiny_cfg, wide_cfg
+    e = Engine(gpu, tiny_cfg() if model == "tiny" else wide_cfg(fma=int(model == "wide_fma")))
+    try:
+        lengths = {1, 2, 3, 4, 5, 63, 64, 65, 67, 128, 257} if model != "wide_fma" else {3, 66}
+        text = np.random.default_rng(4).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(1, max(lengths) + 1):
+            if n > 1:
+                lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            e.seed_slot(5, 40, n)  # the slot was in use
+            got = e.prefill(5, text[:n])
+            assert e.pos(5) == n
+            if n > 1:
+                assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 5), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
