@@ -10,6 +10,7 @@
 // KD (K), NB (max tokens), YT_F32 (1: fp32 output, else fp16).
 #include "qmv_core.cuh"
 #include "qw_kern.h"
+#include "tmap.cuh"
 
 using namespace qw;
 
@@ -383,20 +384,13 @@ __global__ void __launch_bounds__(WARPS * TEAMS * 32, (WARPS * TEAMS == 8) ? 2 :
                     for (int i = 0; i < 4; i++) half_mma(A, i, zr, va[i], vb[i], (uint32_t)ps * 16 + 8 < p.nb, accp[ps]);
                 }
             };
-            if constexpr (GF == 21) {
-                const Iq3sHdr h0 = iq3s_hdr(rows, t), h1 = iq3s_hdr(rows + 8 * p.rs, t);
-                UnitHalf A;
-                iq3s_decode_half<0, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
-                run_half(A, 0);
-                iq3s_decode_half<1, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
-                run_half(A, 1);
-            } else {
-                UnitHalf A;
-                q8_decode_half<0>(rows, rows + 8 * p.rs, t, A);
-                run_half(A, 0);
-                q8_decode_half<1>(rows, rows + 8 * p.rs, t, A);
-                run_half(A, 1);
-            }
+            static_assert(GF == 21, "Q8_0 runs more than 16 tokens in the wide form");
+            const Iq3sHdr h0 = iq3s_hdr(rows, t), h1 = iq3s_hdr(rows + 8 * p.rs, t);
+            UnitHalf A;
+            iq3s_decode_half<0, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
+            run_half(A, 0);
+            iq3s_decode_half<1, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
+            run_half(A, 1);
 #pragma unroll
             for (int ps = 0; ps < 4; ps++) {
                 if ((uint32_t)ps >= passes) break;
@@ -455,7 +449,9 @@ template <int GF, int WARPS, int TEAMS, bool F32OUT, bool MP = false>
 static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) {
     // more than 16 tokens (at most 64): the form that decodes a unit once for all passes
     static const bool loop_passes = [] { const char *v = getenv("QW_QMV_PASSES"); return v && !strcmp(v, "loop"); }();  // for A/B timing
-    if (!MP && p.nb > 16 && p.nb <= 64 && !loop_passes) return qmv_mma2_go<GF, WARPS, TEAMS, F32OUT, true>(p, sm_count, st);
+    if constexpr (!MP && GF == 21) {
+        if (p.nb > 16 && p.nb <= 64 && !loop_passes) return qmv_mma2_go<GF, WARPS, TEAMS, F32OUT, true>(p, sm_count, st);
+    }
     const size_t smem = 128 + (GF == 21 ? 65536 : 0) + (size_t)TEAMS * 2 * WARPS * 2 * 32 * 16 +
                         (size_t)TEAMS * (GF == 8 ? 2 : QMV_STAGES) * ((16 * p.rs + 127) & ~127u);
     if (smem > 227 * 1024) return cudaErrorInvalidValue;
@@ -469,6 +465,241 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     const uint32_t want = (p.items + TEAMS - 1) / TEAMS, cap = (uint32_t)(sm_count * occ), grid = want < cap ? want : cap;
     qw_launch(k, grid, WARPS * TEAMS * 32, smem, st, p);
     return cudaGetLastError();
+}
+
+// ---- More than 16 tokens at K = 2048: a block owns a run of 16-row tiles and walks K in units of 256, so the activations reach a
+// block once per round of up to RG tiles instead of once per tile.  (The form above re-reads 256 KB of activations from L2 for each
+// 16 rows at 64 tokens: 2.5 GB for an output head of 330 MB -- L2 bandwidth was its bound.)  Two rings feed the block: weights (16-row boxes
+// of one Q8_0 unit, or of two IQ3_S units, whose 110 bytes do not start on 16-byte boundaries) and activations (one unit of all tokens,
+// 128-byte swizzled).  Warp = (row tile r, token part th): it decodes its tile's unit and runs it against every TS-th column tile.  A
+// unit's sum starts from zero and is added to the running total in unit order: the sums of qmv_mma2 in its slice order, bit for bit, without a
+// reduction across warps.  MMA column g of a tile holds token (g / 2) + 4 (g % 2), so that the eight lanes of a 16-byte shared load fall into
+// eight different chunks of the swizzle.
+// TS = warps that share a row tile.  2: the tiles of a block are few (a projection has 3 to 6 per SM) and the warps are what hides
+// latency.  1 (Q8_0, 16 tiles per SM and more): a unit is decoded once for all tokens, because the kernel is then bound by the
+// shared-memory pipe.
+// Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
+// IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
+// 40 of its cycles per unit of 16 rows x 32 weights.
+template <int GF, int TS>
+struct WideCfg {
+    static constexpr int RG = TS == 2 ? 7 : 11;              // row tiles per round: 14 + 1 warps of 128 registers, or 11 + 1 of 168
+    static constexpr int UPW = GF == 21 ? 2 : 1;             // units per weight stage
+    static constexpr int PITCH = GF == 21 ? 240 : 272;       // bytes between staged rows (eight rows: eight different groups of four banks)
+    static constexpr int WS = GF == 21 || TS == 1 ? 2 : 3, XS = 3;  // stages
+    static constexpr int TABB = GF == 21 ? 65536 : 0;
+    static constexpr int WBYTES = RG * 16 * PITCH;
+    static constexpr size_t smem(int CT) { return 1024 + 256 + (size_t)TABB + (size_t)WS * WBYTES + (size_t)XS * CT * TS * 8 * 512; }
+};
+static_assert(WideCfg<21, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 1>::smem(8) <= 227 * 1024, "shared memory of the wide matvec");
+
+// q8_sub_h for rows 272 bytes apart, in half the shared-memory cycles: 32-bit loads only, and lanes t >= 2 take their words in another
+// order, so that rows g and g + 1 do not meet in a bank (only the third load of an even block has two lanes per bank).
+template <int IB>
+__device__ __forceinline__ float q8_sub_272(uint32_t row, int t, uint32_t (&w)[4]) {
+    const bool sw = t >= 2;
+    const uint32_t a = row + 8 * t;
+    uint32_t lo, hi;
+    auto ld = [](uint32_t at) {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(at), "n"(34 * IB + (IB & 1 ? 2 : 0)));
+        return v;
+    };
+    if (IB & 1) {
+        const uint32_t x1 = ld(a + (sw ? 4 : 0)), x2 = ld(a + (sw ? 0 : 4));
+        lo = sw ? x2 : x1;
+        hi = sw ? x1 : x2;
+    } else {
+        const uint32_t x1 = ld(a + (sw ? 4 : 0)), x2 = ld(a + (sw ? 8 : 4)), x3 = ld(a + (sw ? 0 : 8));
+        const uint32_t w0 = sw ? x3 : x1, w1 = sw ? x1 : x2, w2 = sw ? x2 : x3;
+        lo = __byte_perm(w0, w1, 0x5432);
+        hi = __byte_perm(w1, w2, 0x5432);
+    }
+    q8_pairs(lo, hi, w);
+    return h2f((uint16_t)lds_u16<34 * IB>(row));
+}
+
+template <int GF, int IB>
+__device__ __forceinline__ void wide_decode(uint32_t u0, uint32_t u1, int t, const Iq3sHdr &h0, const Iq3sHdr &h1, uint32_t tabc, uint32_t (&a0)[4],
+                                            uint32_t (&a1)[4], float &da, float &db) {
+    uint32_t wa[4], wb[4];
+    if (GF == 21) {
+        da = iq3s_sub_h<IB, 128>(u0 + 2 * t, u0 + t, h0, tabc, wa);
+        db = iq3s_sub_h<IB, 128>(u1 + 2 * t, u1 + t, h1, tabc, wb);
+    } else {
+        da = q8_sub_272<IB>(u0, t, wa);
+        db = q8_sub_272<IB>(u1, t, wb);
+    }
+    a0[0] = wa[0]; a0[1] = wb[0]; a0[2] = wa[1]; a0[3] = wb[1];
+    a1[0] = wa[2]; a1[1] = wb[2]; a1[2] = wa[3]; a1[3] = wb[3];
+}
+
+// CT = column tiles of 8 tokens per warp: up to 8 CT TS tokens.  grid: at most one block per SM
+template <int GF, bool F32OUT, int TS, int CT>
+__global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wide_k(const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx,
+                                                                                    const QmvMmaP p, uint32_t rg) {
+    using C = WideCfg<GF, TS>;
+    constexpr int WS = C::WS, XS = C::XS, UPW = C::UPW, UNITS = 8, R = 8 * CT * TS, XBYTES = R * 512, CH = CT <= 4 ? CT : CT / 2;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;  // the swizzle pattern repeats every 1024 bytes
+    const uint32_t xs0 = base, ws0 = xs0 + XS * XBYTES, tab0 = ws0 + WS * C::WBYTES;
+    uint64_t *bars = (uint64_t *)(smem_raw + (tab0 + C::TABB - smem_u32(smem_raw)));
+    uint64_t *wfull = bars, *wempty = wfull + WS, *xfull = wempty + WS, *xempty = xfull + XS, *tbar = xempty + XS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t ncw = TS * rg;  // consumer warps; warp ncw is the producer
+    pdl_launch();
+    if (tid == 0) {
+        for (int s = 0; s < WS; s++) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], ncw); }
+        for (int s = 0; s < XS; s++) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], ncw); }
+        mbar_init(tbar, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    // this block's tiles, and the tiles of a round: both split evenly
+    const uint32_t t0 = (uint32_t)((uint64_t)blockIdx.x * p.items / gridDim.x), cnt = (uint32_t)((uint64_t)(blockIdx.x + 1) * p.items / gridDim.x) - t0;
+    const uint32_t rounds = (cnt + rg - 1) / rg;
+    if ((uint32_t)warp == ncw) {
+        if (lane == 0) {
+            bool ok = true;
+            if (GF == 21) {
+                mbar_expect_tx(tbar, C::TABB);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(tab0), "l"(p.tab->grid_h4), "r"(C::TABB),
+                             "r"(smem_u32(tbar))
+                             : "memory");
+            }
+            const uint32_t nw = rounds * (UNITS / UPW), nx = rounds * UNITS;
+            uint32_t jw = 0;
+            auto put_w = [&]() {  // weight stage number jw
+                const uint32_t s = jw % WS, r = jw / (UNITS / UPW), kp = jw % (UNITS / UPW);
+                if (jw >= WS && !mbar_wait(&wempty[s], (jw / WS - 1) & 1)) return false;
+                const uint32_t lo = cnt * r / rounds, n = cnt * (r + 1) / rounds - lo;
+                mbar_expect_tx(&wfull[s], n * 16 * C::PITCH);
+                const int xc = GF == 21 ? (int)((220 * kp) & ~15u) : (int)(136 * kp);  // bytes, or pairs of bytes
+                for (uint32_t i = 0; i < n; i++) tma_load_2d(ws0 + s * C::WBYTES + i * 16 * C::PITCH, &mw, xc, (int)((t0 + lo + i) * 16), &wfull[s]);
+                jw++;
+                return true;
+            };
+            while (jw < WS && jw < nw) put_w();  // the first weights do not depend on earlier kernels; the activations and the output do
+            pdl_wait();
+            for (uint32_t jx = 0; jx < nx && ok; jx++) {
+                const uint32_t s = jx % XS, u = jx % UNITS;
+                if (jx >= XS && !mbar_wait(&xempty[s], (jx / XS - 1) & 1)) { ok = false; break; }
+                mbar_expect_tx(&xfull[s], XBYTES);
+                for (uint32_t q = 0; q < 4; q++) tma_load_2d(xs0 + s * XBYTES + q * R * 128, &mx, (int)(u * 256 + q * 64), 0, &xfull[s]);
+                // weights as far ahead as their ring allows without holding up the activations of the stages already in it
+                if (jw < nw && jw * UPW <= jx + (WS - 1) * UPW) ok = put_w();
+            }
+            if (!ok) set_status(p.status, ST_MBAR_TIMEOUT | 12);
+        }
+        return;
+    }
+    pdl_wait();
+    const uint32_t r = (uint32_t)warp % rg, th = (uint32_t)warp / rg;
+    // (this warp's column tiles: th, th + TS, ...; rows past the last token read as zero)
+    const uint32_t tokr = (uint32_t)(g >> 1) | ((uint32_t)(g & 1) << 2);                      // token of MMA column g within a tile
+    const uint32_t xoff = th * 1024 + tokr * 128 + ((uint32_t)t ^ tokr) * 16, tabc = tab0 + (lane & 15) * 8;
+    const ZeroRegs zr = zero_regs();
+    bool ok = GF == 21 ? mbar_wait(tbar, 0) : true;
+    uint32_t jw = 0, jx = 0;
+    for (uint32_t rd = 0; rd < rounds && ok; rd++) {
+        const uint32_t lo = cnt * rd / rounds, n = cnt * (rd + 1) / rounds - lo;
+        float tot[CT][4];
+#pragma unroll
+        for (int i = 0; i < CT; i++) tot[i][0] = tot[i][1] = tot[i][2] = tot[i][3] = 0.f;
+#pragma unroll 1
+        for (uint32_t u = 0; u < UNITS; u++, jx++) {
+            if (u % UPW == 0 && !mbar_wait(&wfull[jw % WS], (jw / WS) & 1)) { ok = false; break; }
+            if (!mbar_wait(&xfull[jx % XS], (jx / XS) & 1)) { ok = false; break; }
+            if (r < n) {
+                const uint32_t u0 = ws0 + (jw % WS) * C::WBYTES + (r * 16 + g) * C::PITCH + (GF == 21 ? ((220 * (u / 2)) & 15) + (u & 1) * 110 : 0);
+                const uint32_t u1 = u0 + 8 * C::PITCH, xa = xs0 + (jx % XS) * XBYTES + xoff;
+                Iq3sHdr h0{}, h1{};
+                if (GF == 21) {
+                    h0 = iq3s_hdr(u0, t);
+                    h1 = iq3s_hdr(u1, t);
+                }
+                float acc[CT][4];
+#pragma unroll
+                for (int i = 0; i < CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+                // The MMAs of the column tiles are issued back to back, first halves then second halves, and the next sub-block is decoded before
+                // their results are used: in program order one tile after the other, every tile waited for its load and for two dependent MMAs.
+                uint32_t a0[4], a1[4];
+                float da, db;
+                wide_decode<GF, 0>(u0, u1, t, h0, h1, tabc, a0, a1, da, db);
+#define WIDE_SUB(IB)                                                                                                              \
+    {                                                                                                                             \
+        const uint32_t xb = (IB & 1 ? xa ^ 64u : xa) + (IB / 2) * R * 128;                                                        \
+        const float ea = da, eb = db;                                                                                             \
+        _Pragma("unroll") for (int c = 0; c < CT; c += CH) { /* CH column tiles at a time: registers */                           \
+            uint4 xv[CH];                                                                                                         \
+            float q[CH][4];                                                                                                       \
+            _Pragma("unroll") for (int i = 0; i < CH; i++) xv[i] = lds_v4(xb + (c + i) * TS * 1024);                              \
+            _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a0, xv[i].x, xv[i].y, zr.z);                             \
+            _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a1, xv[i].z, xv[i].w, q[i]);                             \
+            if (IB < 7 && c + CH == CT) wide_decode<GF, (IB < 7 ? IB + 1 : 7)>(u0, u1, t, h0, h1, tabc, a0, a1, da, db);          \
+            _Pragma("unroll") for (int i = 0; i < CH; i++) {                                                                      \
+                acc[c + i][0] = fmaf(ea, q[i][0], acc[c + i][0]);                                                                 \
+                acc[c + i][1] = fmaf(ea, q[i][1], acc[c + i][1]);                                                                 \
+                acc[c + i][2] = fmaf(eb, q[i][2], acc[c + i][2]);                                                                 \
+                acc[c + i][3] = fmaf(eb, q[i][3], acc[c + i][3]);                                                                 \
+            }                                                                                                                     \
+        }                                                                                                                         \
+    }
+                WIDE_SUB(0) WIDE_SUB(1) WIDE_SUB(2) WIDE_SUB(3) WIDE_SUB(4) WIDE_SUB(5) WIDE_SUB(6) WIDE_SUB(7)
+#undef WIDE_SUB
+#pragma unroll
+                for (int i = 0; i < CT; i++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) tot[i][k] += acc[i][k];
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&xempty[jx % XS]);
+                if (u % UPW == UPW - 1) mbar_arrive(&wempty[jw % WS]);
+            }
+            if (u % UPW == UPW - 1) jw++;
+        }
+        if (!ok || r >= n) continue;
+        const uint32_t row = (t0 + lo + r) * 16 + g;
+#pragma unroll
+        for (int i = 0; i < CT; i++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t col = (TS * i + th) * 8 + t + 4 * (k & 1), rw = row + 8 * (k >> 1);
+                if (col >= p.nb) continue;
+                if (F32OUT) ((float *)p.y)[(size_t)col * p.ystride + rw] = tot[i][k];
+                else ((__half *)p.y)[(size_t)col * p.ystride + rw] = __float2half_rn(tot[i][k]);
+            }
+    }
+    if (!ok && lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 13);
+}
+
+template <int GF, bool F32OUT, int TS>
+static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t grid, uint32_t per, cudaStream_t st) {
+    using C = WideCfg<GF, TS>;
+    CUtensorMap mw, mx;
+    constexpr int B = 2 / TS;  // column tiles per 16 tokens of a warp
+    const int n = p.nb <= 32 ? 2 : p.nb <= 48 ? 3 : 4, ct = n * B;
+    const bool mok = GF == 21 ? tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, p.rb, p.N, p.rb, 240, 16, CU_TENSOR_MAP_SWIZZLE_NONE)
+                              : tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.W, p.rb / 2, p.N, p.rb, 136, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (!mok || !tmap_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x, p.K, p.nb, (uint64_t)p.xstride * 2, 64, 16 * n, CU_TENSOR_MAP_SWIZZLE_128B))
+        return cudaErrorInvalidValue;
+    auto k = n == 2 ? qmv_wide_k<GF, F32OUT, TS, 2 * B> : n == 3 ? qmv_wide_k<GF, F32OUT, TS, 3 * B> : qmv_wide_k<GF, F32OUT, TS, 4 * B>;
+    const size_t smem = C::smem(ct);
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    // as many row tiles per round as split the block's tiles into equal rounds of at most RG
+    const uint32_t rounds = (per + C::RG - 1) / C::RG, rg = (per + rounds - 1) / rounds;
+    qw_launch(k, grid, (TS * rg + 1) * 32, smem, st, mw, mx, p, rg);
+    return cudaGetLastError();
+}
+template <int GF, bool F32OUT>
+static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) {
+    const uint32_t grid = p.items < (uint32_t)sm_count ? p.items : (uint32_t)sm_count, per = (p.items + grid - 1) / grid;  // one block per SM
+    if constexpr (GF == 8) {
+        if (per >= 16) return qmv_wide_ts<GF, F32OUT, 1>(p, grid, per, st);
+    }
+    return qmv_wide_ts<GF, F32OUT, 2>(p, grid, per, st);
 }
 
 // The grid and block given by the host are ignored (the kernels are persistent and size themselves).  Defines: GF (21 = IQ3_S,
@@ -520,6 +751,12 @@ static cudaError_t launch_qmv_mma(const QwLaunch &L) {
     }
 #define GO(G, M)                                                        \
     return f32 ? qmv_mma_nt<G, M, true>(p, L.sm_count, L.stream) : qmv_mma_nt<G, M, false>(p, L.sm_count, L.stream)
+    // More than 16 tokens: the activations no longer fit a warp's registers, and the wide form reads them from shared memory.  (The
+    // exchange between ranks is built into qmv_mma2 only.)
+    if (K == 2048 && a.nb > 16 && epx <= 1) {
+        if (gf == 21) return f32 ? qmv_wide_go<21, true>(p, L.sm_count, L.stream) : qmv_wide_go<21, false>(p, L.sm_count, L.stream);
+        return f32 ? qmv_wide_go<8, true>(p, L.sm_count, L.stream) : qmv_wide_go<8, false>(p, L.sm_count, L.stream);
+    }
     if (gf == 21 && K == 2048) return f32 ? qmv_mma2_go<21, 8, 2, true>(p, L.sm_count, L.stream) : qmv_mma2_go<21, 8, 2, false>(p, L.sm_count, L.stream);
     if (gf == 21 && K == 4096) return f32 ? qmv_mma2_go<21, 16, 1, true>(p, L.sm_count, L.stream) : qmv_mma2_go<21, 16, 1, false>(p, L.sm_count, L.stream);
     if (gf == 8 && K == 2048) return f32 ? qmv_mma2_go<8, 8, 1, true>(p, L.sm_count, L.stream) : qmv_mma2_go<8, 8, 1, false>(p, L.sm_count, L.stream);

@@ -350,19 +350,8 @@ __device__ __forceinline__ void half_mma(const UnitHalf &A, int i, const ZeroReg
     }
 }
 
-// Q8_0 through the same shared-space path: unit = eight 34-byte blocks of a row (src/ggml_dq.c:34-37).  The thread's
-// eight int8 values of block IB sit at byte 34*IB + 2 + 8t: 4-byte aligned for odd IB (two 32-bit loads), 2-byte aligned
-// for even IB (four 16-bit loads).  (q ^ 0x80) | 0x6400 is the half 1024 + (q + 128); subtracting 1152 is exact.
-template <int IB>
-__device__ __forceinline__ float q8_sub_h(uint32_t row_t, uint32_t row, uint32_t (&w)[4]) {
-    uint32_t lo, hi;
-    if (IB & 1) {
-        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(lo) : "r"(row_t), "n"(34 * IB + 2));
-        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(hi) : "r"(row_t), "n"(34 * IB + 6));
-    } else {
-        lo = lds_u16<34 * IB + 2>(row_t) | (lds_u16<34 * IB + 4>(row_t) << 16);
-        hi = lds_u16<34 * IB + 6>(row_t) | (lds_u16<34 * IB + 8>(row_t) << 16);
-    }
+// eight int8 (four in lo, four in hi) -> integer-valued fp16 pairs: (q ^ 0x80) | 0x6400 is the half 1024 + (q + 128); subtracting 1152 is exact
+__device__ __forceinline__ void q8_pairs(uint32_t lo, uint32_t hi, uint32_t (&w)[4]) {
     lo ^= 0x80808080u;
     hi ^= 0x80808080u;
     const uint32_t bias = 0x64806480u;
@@ -374,6 +363,22 @@ __device__ __forceinline__ float q8_sub_h(uint32_t row_t, uint32_t row, uint32_t
         const __half2 r = __hsub2(*(const __half2 *)&v[j], b2);
         w[j] = *(const uint32_t *)&r;
     }
+}
+
+// Q8_0 through the same shared-space path: unit = eight 34-byte blocks of a row (src/ggml_dq.c:34-37).  The thread's
+// eight int8 values of block IB sit at byte 34*IB + 2 + 8t: 4-byte aligned for odd IB (two 32-bit loads), 2-byte aligned
+// for even IB (four 16-bit loads).
+template <int IB>
+__device__ __forceinline__ float q8_sub_h(uint32_t row_t, uint32_t row, uint32_t (&w)[4]) {
+    uint32_t lo, hi;
+    if (IB & 1) {
+        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(lo) : "r"(row_t), "n"(34 * IB + 2));
+        asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(hi) : "r"(row_t), "n"(34 * IB + 6));
+    } else {
+        lo = lds_u16<34 * IB + 2>(row_t) | (lds_u16<34 * IB + 4>(row_t) << 16);
+        hi = lds_u16<34 * IB + 6>(row_t) | (lds_u16<34 * IB + 8>(row_t) << 16);
+    }
+    q8_pairs(lo, hi, w);
     return h2f((uint16_t)lds_u16<34 * IB>(row));
 }
 template <int IB>
@@ -411,22 +416,6 @@ __device__ __forceinline__ void unit_mma2_q8(uint32_t u0, uint32_t u1, int t, co
     sub_mma2_q8<5>(u0, u1, t, zr, xa[5], xb[5], second, acc);
     sub_mma2_q8<6>(u0, u1, t, zr, xa[6], xb[6], second, acc);
     sub_mma2_q8<7>(u0, u1, t, zr, xa[7], xb[7], second, acc);
-}
-
-// Q8_0 counterpart of iq3s_decode_half: blocks 4 HF .. 4 HF + 3 of the unit
-template <int HF>
-__device__ __forceinline__ void q8_decode_half(uint32_t u0, uint32_t u1, int t, UnitHalf &A) {
-    uint32_t wa[4], wb[4];
-#define QW_HALF_SUB(I)                                                            \
-    A.da[I] = q8_sub_h<4 * HF + I>(u0 + 8 * t, u0, wa);                           \
-    A.db[I] = q8_sub_h<4 * HF + I>(u1 + 8 * t, u1, wb);                           \
-    A.a0[I][0] = wa[0]; A.a0[I][1] = wb[0]; A.a0[I][2] = wa[1]; A.a0[I][3] = wb[1]; \
-    A.a1[I][0] = wa[2]; A.a1[I][1] = wb[2]; A.a1[I][2] = wa[3]; A.a1[I][3] = wb[3];
-    QW_HALF_SUB(0)
-    QW_HALF_SUB(1)
-    QW_HALF_SUB(2)
-    QW_HALF_SUB(3)
-#undef QW_HALF_SUB
 }
 
 __host__ __device__ constexpr int unit_bytes(int GF) { return GF == 21 ? 110 : 272; }

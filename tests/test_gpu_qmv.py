@@ -100,3 +100,22 @@ def test_bad_arguments_fail_the_batch_not_the_device(gpu):
     # the device is still usable
     W = synth.iq3s_rows(np.random.default_rng(3), 16, 2048)
     assert np.array_equal(bits(run_dq(gpu, 21, W, 2048)), bits(orc.dq_rows(21, W, 2048)))
+
+
+# More than 16 tokens at K = 2048 (the block-tiled form): rows equal to the same row alone, whose kernel is the one checked above.  Sizes:
+# fewer row tiles than SMs, an uneven split over the SMs, and a Q8_0 head large enough for one warp per row tile, 17 tiles on some SMs.
+@pytest.mark.parametrize("qtype,N", [(21, 16), (21, 16 * 149), (8, 48), (8, 16 * 300), (8, 16 * 2390)])
+@pytest.mark.parametrize("B", [17, 32, 33, 47, 64])
+def test_wide_matvec_rows_equal_the_row_alone(gpu, qtype, N, B):
+    rng = np.random.default_rng(N + B)
+    W = synth.quant_rows(rng, qtype, N, 2048)
+    x = synth.acts_fp16(rng, B, 2048)
+    y = run_qmv(gpu, "qmv_mma", qtype, W, 2048, x)
+    for b in range(B) if N < 5000 else (0, 7, 8, B // 2, B - 1):
+        assert np.array_equal(bits(run_qmv(gpu, "qmv_mma", qtype, W, 2048, x[b:b + 1])[0]), bits(y[b])), b
+    some = rng.integers(0, N, 64)
+    ref = orc.qmv_f64(qtype, W[some], 2048, x)
+    # fp16 products are exact, fp32 accumulation over K = 2048 terms: the bound of the test above
+    assert np.abs(y[:, some] - ref).max() <= 2e-5 * np.abs(ref).max()
+    y16 = run_qmv(gpu, "qmv_mma", qtype, W, 2048, x, f32=False)
+    assert np.array_equal(y16, y.astype(np.float16))
