@@ -280,20 +280,28 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // ------------------------------------------------------------------------------------------------ router + select in one launch
 // The role of moe_pre_gg's hand-over (kernels/moe_gg.metal:574-589): the block that finishes the router last (device
 // counter + fences) runs the selection.  Blocks of 512 threads: warp = (row blockIdx*4 + warp%4, token group warp/4); the
-// row sits in registers and the tokens in shared memory, both converted to fp32 once.
+// row sits in registers as fp32.  The tokens arrive as they are, fp16, by bulk copies of 16 tokens each -- up to three in flight -- and
+// are converted where they are used: a lane's 16-byte load feeds eight multiply-adds.  (Staged as fp32 by the block's own threads, every
+// token cost twice the shared-memory reads and a block barrier per 16 tokens with an L2 latency behind it; and 128 KB for even one
+// token kept the expert FFN's blocks from becoming resident early.)  64 tokens, 512 experts: 40.6 -> 26.7 us on a B200.
+// Up to four tokens -- one per warp at most -- are read straight from L2: staging them costs a copy's latency and saves nothing.
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
 // 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.
+constexpr uint32_t ROUTE_PASS = 16, ROUTE_STG = 3;  // tokens per copy, copies in flight
 template <int D>
 __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, unsigned *counter, moe_sel *ms,
-                                                   uint32_t E, uint32_t topk, sel_args a) {
+                                                   uint32_t E, uint32_t topk, sel_args a, unsigned *status) {
     constexpr int CH = D / 8 / 32;
-    // the tokens of one pass as fp32, converted once per block: [16 tokens][CH][2][32 lanes] float4, so that a lane's
-    // eight values of a chunk are two conflict-free 16-byte loads
-    extern __shared__ __align__(16) uint8_t route_smem[];
-    float4 *xs = (float4 *)route_smem;
+    extern __shared__ __align__(128) uint8_t route_smem[];  // [ROUTE_STG][16 tokens][D] fp16
+    __shared__ uint64_t full[ROUTE_STG];
     __shared__ bool last;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * 4 + (warp & 3), tg = warp >> 2;
+    const bool direct = a.nb <= 4;
     pdl_launch();
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < ROUTE_STG; s++) mbar_init(&full[s], 1);
+        mbar_init_fence();
+    }
     float wf[CH * 8];
     if (r <= E) {
         const uint4 *w = (const uint4 *)(r < E ? Wr + (size_t)r * D : Wsg);
@@ -309,45 +317,69 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
             }
         }
     }
+    if (!direct) __syncthreads();
     pdl_wait();  // the router row is static; the tokens are the previous kernel's output
-    // Passes of 16 tokens.  Each warp runs its tokens (tg, tg + 4, tg + 8, tg + 12) against its row; every dot product is
-    // the same single-lane chain as in moe_router (element k of lane l, chunk c is column (l + 32 c) * 8 + k), so logits
-    // are bit-identical.
-    for (uint32_t t0 = 0; t0 < a.nb; t0 += 16) {
-        const uint32_t nt = a.nb - t0 < 16 ? a.nb - t0 : 16;
-        if (t0) __syncthreads();
-        for (uint32_t e = threadIdx.x; e < nt * (D / 8); e += 512) {
-            const uint4 v = __ldcg((const uint4 *)(x + (size_t)t0 * D) + e);
-            const uint32_t tl = e / (D / 8), ce = e % (D / 8), c = ce >> 5, ln = ce & 31;
-            const float2 f0 = __half22float2(*(const __half2 *)&v.x), f1 = __half22float2(*(const __half2 *)&v.y);
-            const float2 f2 = __half22float2(*(const __half2 *)&v.z), f3 = __half22float2(*(const __half2 *)&v.w);
-            xs[((tl * CH + c) * 2 + 0) * 32 + ln] = make_float4(f0.x, f0.y, f1.x, f1.y);
-            xs[((tl * CH + c) * 2 + 1) * 32 + ln] = make_float4(f2.x, f2.y, f3.x, f3.y);
-        }
-        __syncthreads();
-        if (r <= E) {
-#pragma unroll 1
-            for (uint32_t tl = tg; tl < nt; tl += 4) {
-                const float4 *xt = xs + tl * CH * 64 + lane;
-                float acc = 0.f;
+    // Every dot product is the same single-lane chain as in moe_router (element k of lane l, chunk c is column (l + 32 c) * 8 + k), so
+    // logits are bit-identical.  v = this lane's chunks of the token.
+    auto dot = [&](const uint4 (&v)[CH]) {
+        float acc = 0.f;
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    const float4 u = xt[c * 64], v = xt[c * 64 + 32];
-                    acc = __fmaf_rn(wf[8 * c + 0], u.x, acc);
-                    acc = __fmaf_rn(wf[8 * c + 1], u.y, acc);
-                    acc = __fmaf_rn(wf[8 * c + 2], u.z, acc);
-                    acc = __fmaf_rn(wf[8 * c + 3], u.w, acc);
-                    acc = __fmaf_rn(wf[8 * c + 4], v.x, acc);
-                    acc = __fmaf_rn(wf[8 * c + 5], v.y, acc);
-                    acc = __fmaf_rn(wf[8 * c + 6], v.z, acc);
-                    acc = __fmaf_rn(wf[8 * c + 7], v.w, acc);
+        for (int c = 0; c < CH; c++) {
+            const uint32_t a4[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 f = __half22float2(*(const __half2 *)&a4[j]);
+                acc = __fmaf_rn(wf[8 * c + 2 * j], f.x, acc);
+                acc = __fmaf_rn(wf[8 * c + 2 * j + 1], f.y, acc);
+            }
+        }
+        return warp_sum_canon(acc);
+    };
+    if (direct) {
+        if (r <= E && tg < a.nb) {
+            const uint4 *xt = (const uint4 *)(x + (size_t)tg * D) + lane;
+            uint4 v[CH];
+#pragma unroll
+            for (int c = 0; c < CH; c++) v[c] = __ldcg(xt + 32 * c);
+            const float sum = dot(v);
+            if (lane == 0) logits[(size_t)tg * (E + 1) + r] = sum;
+        }
+    } else {
+        const uint32_t passes = (a.nb + ROUTE_PASS - 1) / ROUTE_PASS;
+        auto issue = [&](uint32_t ps) {
+            const uint32_t n = a.nb - ps * ROUTE_PASS < ROUTE_PASS ? a.nb - ps * ROUTE_PASS : ROUTE_PASS, s = ps % ROUTE_STG;
+            mbar_expect_tx(&full[s], n * D * 2);
+            bulk_g2s(route_smem + s * ROUTE_PASS * D * 2, x + (size_t)ps * ROUTE_PASS * D, n * D * 2, &full[s]);
+        };
+        if (threadIdx.x == 0)
+            for (uint32_t ps = 0; ps < passes && ps < ROUTE_STG; ps++) issue(ps);
+        bool ok = true;
+        for (uint32_t ps = 0; ps < passes; ps++) {  // a warp runs tokens tg, tg + 4, tg + 8, tg + 12 of a pass against its row
+            const uint32_t s = ps % ROUTE_STG, nt = a.nb - ps * ROUTE_PASS < ROUTE_PASS ? a.nb - ps * ROUTE_PASS : ROUTE_PASS;
+            if (ok && !mbar_wait(&full[s], (ps / ROUTE_STG) & 1)) {  // reported; the walk goes on without waiting again, so no barrier is left short
+                ok = false;
+                if (lane == 0) set_status(status, ST_MBAR_TIMEOUT | 14);
+            }
+            if (r <= E) {
+#pragma unroll 1
+                for (uint32_t tl = tg; tl < nt; tl += 4) {
+                    const uint4 *xt = (const uint4 *)(route_smem + (s * ROUTE_PASS + tl) * D * 2) + lane;
+                    uint4 v[CH];
+#pragma unroll
+                    for (int c = 0; c < CH; c++) v[c] = xt[32 * c];
+                    const float sum = dot(v);
+                    if (lane == 0) logits[(size_t)(ps * ROUTE_PASS + tl) * (E + 1) + r] = sum;
                 }
-                const float s = warp_sum_canon(acc);
-                if (lane == 0) logits[(size_t)(t0 + tl) * (E + 1) + r] = s;
+            }
+            if (ps + ROUTE_STG < passes) {
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    fence_proxy_async();
+                    issue(ps + ROUTE_STG);
+                }
             }
         }
     }
-    pdl_wait();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -362,10 +394,11 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
 
 template <int DD>
 static cudaError_t moe_route_go(const QwLaunch &L, unsigned grid, uint32_t E, uint32_t topk, const sel_args &a) {
-    cudaError_t e = cudaFuncSetAttribute(moe_route_k<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * DD * 4);
+    cudaError_t e = cudaFuncSetAttribute(moe_route_k<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_STG * ROUTE_PASS * DD * 2);
     if (e != cudaSuccess) return e;
-    qw_launch(moe_route_k<DD>, grid, 512, 16 * DD * 4, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), L.buf<unsigned>(4),
-              L.buf<moe_sel>(5), E, topk, a);
+    const uint32_t held = a.nb <= 4 ? 0 : a.nb < ROUTE_STG * ROUTE_PASS ? a.nb : ROUTE_STG * ROUTE_PASS;
+    qw_launch(moe_route_k<DD>, grid, 512, held * DD * 2, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), L.buf<unsigned>(4),
+              L.buf<moe_sel>(5), E, topk, a, (unsigned *)L.status);
     return cudaGetLastError();
 }
 
@@ -374,6 +407,7 @@ static cudaError_t launch_moe_route(const QwLaunch &L) {
     sel_args a = L.bytes<sel_args>(14);
     QW_CHECK_ARG(L.has_bytes(14, 12) && a.nb >= 1 && a.nb <= MOE_MAXB);
     for (int i = 0; i <= 5; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+    QW_CHECK_ARG(((uintptr_t)L.buf<void>(0) & 15) == 0 && ((uintptr_t)L.buf<void>(1) & 15) == 0 && ((uintptr_t)L.buf<void>(2) & 15) == 0);
     QW_CHECK_ARG(E % 32 == 0 && (E == 512 || E <= 256) && topk >= 1 && topk < MOE_MAXK && topk <= E);  // E <= the block's 512 threads
     QW_CHECK_ARG(L.avail(0) >= (size_t)E * D * 2 && L.avail(1) >= (size_t)D * 2 && L.avail(2) >= (size_t)a.nb * D * 2 &&
                  L.avail(3) >= (size_t)a.nb * (E + 1) * 4 && L.avail(4) >= 4 && L.avail(5) >= sizeof(moe_sel));
