@@ -203,3 +203,9 @@ def test_iq3x_recoding_is_lossless(gpu):
     got = y.download(np.float32, rows * K).reshape(rows, K)
     ref = orc.dq_rows(orc.IQ3_S, W, K)
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("B", [4, 5, 15, 17, 48, 49])
+def test_fused_router_at_the_edges_of_its_passes(gpu, B):
+    """moe_route reads up to four tokens directly and stages more by 16, three groups in flight: the comparison above at those edges."""
+    test_fused_router_select_equals_two_launches(gpu, B)
