@@ -25,11 +25,13 @@
 #include <vector>
 
 extern "C" size_t qw_moe_sel_bytes(void);
+extern "C" size_t qw_moe_sel_wide_bytes(void);
 
 namespace {
 
 constexpr int PAGE = 256;
-constexpr int ROWS = QW_PAR_MAX;  // rows of the control block: a step's slots, or the tokens of a piece of a prompt
+constexpr int ROWS = QW_PAR_MAX;      // rows of the control block of a step
+constexpr int PROWS = MOE_MAXB_WIDE;  // ... and of a piece of a prompt: its tokens
 std::string g_open_error;
 
 struct Slot {
@@ -90,6 +92,12 @@ struct qw_engine {
     // scratch
     qw_buf ctl_h{}, ctl_d{}, h{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
+    // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN.  Four times the tokens choose far fewer than four times the
+    // experts, so a wider piece reads and decodes fewer expert weights per token.
+    int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
+    qw_buf ctl_p{}, ffn_scr_w{};
+    qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_norm_cmb_rc_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
+              *k_group_w = nullptr, *k_ffn_w = nullptr;
     qw_buf mlog{}, msel{}, Hhi{}, Hlo{}, Pg{}, rcnt{};
     size_t sel_bytes = 0;
     // kernels
@@ -247,7 +255,7 @@ extern "C" qw_gpu *qw_engine_gpu(qw_engine *e) { return e ? e->g : nullptr; }
 extern "C" void qw_engine_close(qw_engine *e) {
     if (!e) return;
     qw_buf *all[] = {&e->emb, &e->lm_head, &e->dense, &e->small, &e->router, &e->exg, &e->exu, &e->exd, &e->shg, &e->shu, &e->shd, &e->kvpool,
-                     &e->ptab, &e->sstate, &e->cstate, &e->prompt_d, &e->ctl_h, &e->ctl_d, &e->h, &e->x, &e->proj, &e->cv, &e->la, &e->be, &e->gy, &e->qb,
+                     &e->ptab, &e->sstate, &e->cstate, &e->prompt_d, &e->ctl_p, &e->ffn_scr_w, &e->ctl_h, &e->ctl_d, &e->h, &e->x, &e->proj, &e->cv, &e->la, &e->be, &e->gy, &e->qb,
                      &e->part, &e->ya, &e->ob, &e->mo, &e->logits, &e->ids, &e->ids_h, &e->logits_h, &e->cand_h, &e->mlog, &e->msel, &e->Hhi, &e->Hlo, &e->Pg, &e->rcnt, &e->xq_gu, &e->xq_d, &e->xs_gu, &e->xs_d, &e->ffn_scr};
     // mappings of the other ranks' exchange buffers go first (their owners free the memory), then this rank's own
     for (int r = 0; r < 8; r++)
@@ -356,6 +364,23 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
                 ok = compile(e, "add_rmsnorm", "cmb_add_rmsnorm_rows", {{"CMB", 1}, {"TOPK", e->TOPK}, {"ROWCNT", 1}}, &e->k_norm_cmb_rc);
         }
     }
+    if (ok && c.ep_size == 1 && e->ffn_fused && c.max_ctx > ROWS) {
+        e->piece_rows = PROWS;
+        auto mw = md;
+        mw.push_back({"SELECT", 0});
+        mw.push_back({"WIDE", 1});
+        mw.push_back({"IQ3X", e->ffn_iq3x ? 1 : 0});
+        const std::vector<std::pair<const char *, long>> cw = {{"CMB", 1}, {"TOPK", e->TOPK}, {"ROWS", PROWS}, {"WIDE", 1}};
+        auto cr = cw;
+        cr.push_back({"ROWCNT", 1});
+        ok = compile(e, "kb_embed", "kb_embed_wide", {{"ROWS", PROWS}}, &e->k_embed_w) &&
+             compile(e, "add_rmsnorm", "rmsnorm_wide", {{"ADD", 0}, {"ROWS", PROWS}}, &e->k_norm0_w) &&
+             compile(e, "add_rmsnorm", "add_rmsnorm_wide", {{"ADD", 1}, {"ROWS", PROWS}}, &e->k_norm_w) &&
+             compile(e, "add_rmsnorm", "cmb_add_rmsnorm_wide", cw, &e->k_norm_cmb_w) &&
+             (!e->k_norm_cmb_rc || compile(e, "add_rmsnorm", "cmb_add_rmsnorm_rows_wide", cr, &e->k_norm_cmb_rc_w)) &&
+             compile(e, "moe_route", "moe_logits_wide", mw, &e->k_logits_w) && compile(e, "moe_topk_wide", "moe_topk_wide", mw, &e->k_topk_w) &&
+             compile(e, "moe_group_wide", "moe_group_wide", mw, &e->k_group_w) && compile(e, "moe_ffn", "moe_ffn_wide", mw, &e->k_ffn_w);
+    }
     ok = ok && compile(e, "k_topk", "k_topk", {}, &e->k_topk);
     e->k_ar = nullptr;
     if (ok && c.ep_size > 1) ok = compile(e, "ep_allreduce", "ep_allreduce", {}, &e->k_ar);
@@ -369,8 +394,8 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
     const size_t gu_bytes = (size_t)e->I * e->rbD;
     const int kvp = c.kv_pages > 0 ? c.kv_pages : c.max_slots * e->max_pages;
     const size_t page_bytes = (size_t)na * 2 * c.kvh * PAGE * c.hd * 2;
-    e->sel_bytes = align_up(qw_moe_sel_bytes(), 256);
-    const size_t B = QW_PAR_MAX;
+    e->sel_bytes = align_up(e->piece_rows > ROWS ? qw_moe_sel_wide_bytes() : qw_moe_sel_bytes(), 256);
+    const size_t B = QW_PAR_MAX, RB = (size_t)e->piece_rows;  // rows of a step / of any pass
     ok = new_buf(e, &e->emb, (size_t)e->V * e->D * 2) && new_buf(e, &e->lm_head, (size_t)e->V * e->rbV) && new_buf(e, &e->dense, dn) &&
          new_buf(e, &e->small, ((size_t)e->L * e->small_stride + e->D) * 4) && new_buf(e, &e->router, (size_t)e->L * (e->E + 1) * e->D * 2) &&
          new_buf(e, &e->exg, (size_t)e->L * e->EL * gu_bytes) && new_buf(e, &e->exu, (size_t)e->L * e->EL * gu_bytes) &&
@@ -378,19 +403,21 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->shu, (size_t)e->L * gu_bytes) && new_buf(e, &e->shd, (size_t)e->L * gu_bytes) &&
          new_buf(e, &e->kvpool, (size_t)kvp * page_bytes) && new_buf(e, &e->ptab, (size_t)c.max_slots * e->max_pages * 4) &&
          new_buf(e, &e->sstate, (size_t)c.max_slots * ng * c.hv * 128 * 128 * 4) && new_buf(e, &e->cstate, (size_t)c.max_slots * ng * 3 * e->C * 4) &&
-         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->ctl_d, 3 * ROWS * 4) && new_buf(e, &e->prompt_d, (size_t)c.max_ctx * 4) && new_buf(e, &e->h, B * e->D * 4) &&
-         new_buf(e, &e->x, B * e->D * 2) && new_buf(e, &e->proj, B * std::max(e->qkv_rows, e->gdn_rows) * 2) && new_buf(e, &e->cv, B * e->C * 2) &&
-         new_buf(e, &e->la, B * c.hv * 4) && new_buf(e, &e->be, B * c.hv * 4) && new_buf(e, &e->gy, B * e->KG * 2) &&
-         new_buf(e, &e->qb, B * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
-         new_buf(e, &e->ya, B * e->KA * 2) && new_buf(e, &e->ob, B * e->D * 2) && new_buf(e, &e->mo, B * e->D * 2) &&
+         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->ctl_d, 3 * ROWS * 4) && new_buf(e, &e->prompt_d, (size_t)c.max_ctx * 4) && new_buf(e, &e->h, RB * e->D * 4) &&
+         new_buf(e, &e->x, RB * e->D * 2) && new_buf(e, &e->proj, RB * std::max(e->qkv_rows, e->gdn_rows) * 2) && new_buf(e, &e->cv, RB * e->C * 2) &&
+         new_buf(e, &e->la, RB * c.hv * 4) && new_buf(e, &e->be, RB * c.hv * 4) && new_buf(e, &e->gy, RB * e->KG * 2) &&
+         new_buf(e, &e->qb, RB * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
+         new_buf(e, &e->ya, RB * e->KA * 2) && new_buf(e, &e->ob, RB * e->D * 2) && new_buf(e, &e->mo, B * e->D * 2) &&
          new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids, B * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
-         new_buf(e, &e->logits_h, B * (size_t)e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, B * (e->E + 1) * 4) &&
+         new_buf(e, &e->logits_h, B * (size_t)e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
          new_buf(e, &e->msel, (size_t)e->L * e->sel_bytes) && new_buf(e, &e->Hhi, B * (e->TOPK + 1) * e->I * 2) &&
-         new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, B * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
+         new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, RB * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
     if (ok) ok = qw_buf_zero(g, &e->msel, 0, e->msel.size) && qw_buf_zero(g, &e->Pg, 0, e->Pg.size) && qw_buf_zero(g, &e->Hhi, 0, e->Hhi.size) &&
                  qw_buf_zero(g, &e->Hlo, 0, e->Hlo.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) &&
                  qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size) && qw_buf_zero(g, &e->rcnt, 0, e->rcnt.size);  // rows past a slot's length are multiplied by probability 0: keep them finite
     if (ok && e->ffn_fused) ok = new_buf(e, &e->ffn_scr, MOE_FFN_SCRATCH_BYTES(e->I)) && qw_buf_zero(g, &e->ffn_scr, 0, e->ffn_scr.size);
+    if (ok && e->piece_rows > ROWS)
+        ok = new_buf(e, &e->ctl_p, 3 * PROWS * 4) && new_buf(e, &e->ffn_scr_w, MOE_FFN_SCRATCH_BYTES_WIDE(e->I)) && qw_buf_zero(g, &e->ffn_scr_w, 0, e->ffn_scr_w.size);
     if (ok && e->ffn_iq3x) {
         e->x_gus = (size_t)(e->I / 64) * (e->D / 512) * 128 * 272;
         e->x_dns = (size_t)(e->D / 128) * (e->I / 512) * 128 * 272;
@@ -526,12 +553,17 @@ struct gdn_args { uint32_t nb, layer, nlayers, z_stride; };
 struct sel_args { uint32_t nb, e_lo, e_hi; };
 
 void enc_qmv(qw_batch *b, qw_kernel *k, const qw_buf *W, size_t woff, uint32_t N, uint32_t K, const qw_buf *x, const qw_buf *y, uint32_t nb, uint32_t ystride,
-             size_t xoff = 0) {
+             size_t xoff = 0, size_t yoff = 0) {
+    if (nb > ROWS) {  // a wide piece (fp16 results): the matvec kernels take 64 rows at a time
+        for (uint32_t r = 0; r < nb; r += ROWS)
+            enc_qmv(b, k, W, woff, N, K, x, y, std::min<uint32_t>(ROWS, nb - r), ystride, xoff + (size_t)r * K * 2, yoff + (size_t)r * ystride * 2);
+        return;
+    }
     const qmv_args a = {N, K, ystride, nb};
     qw_batch_kernel(b, k);
     qw_batch_buf(b, 0, W, woff);
     qw_batch_buf(b, 3, x, xoff);
-    qw_batch_buf(b, 4, y, 0);
+    qw_batch_buf(b, 4, y, yoff);
     qw_batch_bytes(b, 5, &a, sizeof a);
     qw_batch_dispatch(b, (N + 7) / 8, 1, 1, 256, 1, 1);
 }
@@ -543,7 +575,9 @@ void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *delta, size_t w_off_float
     const bool cmb = delta == &e->Pg;
     const bool gathered = delta == &e->epx;  // slot sharding: the rows were stored by the ranks that own the slots
     const bool rows = cmb && e->k_norm_cmb_rc && e->ffn_fused && !e->ep_fused && !e->moe_probe;  // the FFN counts its output rows in
-    qw_batch_kernel(b, cmb ? (e->ep_fused ? e->k_norm_cmb_x : rows ? e->k_norm_cmb_rc : e->k_norm_cmb) : gathered ? e->k_norm_x : delta ? e->k_norm : e->k_norm0);
+    const bool wide = nb > ROWS;
+    if (wide) qw_batch_kernel(b, cmb ? (rows ? e->k_norm_cmb_rc_w : e->k_norm_cmb_w) : delta ? e->k_norm_w : e->k_norm0_w);
+    else qw_batch_kernel(b, cmb ? (e->ep_fused ? e->k_norm_cmb_x : rows ? e->k_norm_cmb_rc : e->k_norm_cmb) : gathered ? e->k_norm_x : delta ? e->k_norm : e->k_norm0);
     qw_batch_buf(b, 0, &e->h, 0);
     if (cmb) {
         qw_batch_buf(b, 5, &e->msel, (size_t)cmb_layer * e->sel_bytes);
@@ -552,7 +586,7 @@ void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *delta, size_t w_off_float
             qw_batch_buf(b, 7, &e->epx, 2 * e->pg_bytes);
             qw_batch_buf(b, 8, &e->rcnt, 64);
         } else qw_batch_buf(b, 6, &e->Pg, 0);
-        if (rows) qw_batch_buf(b, 9, &e->ffn_scr, 0);
+        if (rows) qw_batch_buf(b, 9, wide ? &e->ffn_scr_w : &e->ffn_scr, 0);
     } else if (delta) {
         qw_batch_buf(b, 1, delta, delta_off);
         if (gathered) {
@@ -579,11 +613,14 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                  const Piece *piece = nullptr) {
     const uint32_t D = e->D;
     const qw_buf *none = nullptr;
+    const bool wide = nb > ROWS;  // a piece of more than 64 tokens
+    const qw_buf *ctl = wide ? &e->ctl_p : &e->ctl_d;
+    const uint32_t CR = wide ? PROWS : ROWS;
     if (piece) {
-        const uint32_t a[4] = {piece->p0, nb, piece->slot, ROWS};
+        const uint32_t a[4] = {piece->p0, nb, piece->slot, CR};
         qw_batch_kernel(b, e->k_chunk);
         qw_batch_buf(b, 0, &e->prompt_d, 0);
-        qw_batch_buf(b, 1, &e->ctl_d, 0);
+        qw_batch_buf(b, 1, ctl, 0);
         qw_batch_bytes(b, 2, a, sizeof a);
         qw_batch_dispatch(b, 1, 1, 1, 256, 1, 1);
     } else if (from_host) {
@@ -596,9 +633,9 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     }
     {
         const uint32_t a[3] = {nb, D, (uint32_t)e->V};
-        qw_batch_kernel(b, e->k_embed);
+        qw_batch_kernel(b, wide ? e->k_embed_w : e->k_embed);
         qw_batch_buf(b, 0, &e->emb, 0);
-        qw_batch_buf(b, 1, &e->ctl_d, 0);
+        qw_batch_buf(b, 1, ctl, 0);
         qw_batch_buf(b, 2, &e->h, 0);
         qw_batch_bytes(b, 3, a, sizeof a);
         qw_batch_dispatch(b, (D + 255) / 256, nb, 1, 256, 1, 1);
@@ -639,34 +676,44 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_dispatch(b, 1, 1, 1, 32, 1, 1);
         } else if (w.attn) {
             enc_qmv(b, e->k_qmv_in_a, &e->dense, w.w_in, e->qkv_rows, D, &e->x, &e->proj, nbl, e->qkv_rows, xo);
-            const qsa_args qa = {nbl, (uint32_t)w.idx, (uint32_t)e->n_attn, e->qkv_rows, (uint32_t)e->max_pages, max_chunks, 0, 0};
-            qw_batch_kernel(b, e->k_prep);
-            qw_batch_buf(b, 0, &e->proj, 0);
-            qw_batch_buf(b, 1, &e->small, (w.small + 2 * D) * 4);
-            qw_batch_buf(b, 2, &e->small, (w.small + 2 * D + 256) * 4);
-            qw_batch_buf(b, 3, &e->qb, 0);
-            qw_batch_buf(b, 4, &e->kvpool, 0);
-            qw_batch_buf(b, 5, &e->ptab, 0);
-            qw_batch_buf(b, 6, &e->ctl_d, 2 * ROWS * 4 + co);
-            qw_batch_buf(b, 7, &e->ctl_d, ROWS * 4 + co);
-            qw_batch_bytes(b, 8, &qa, sizeof qa);
-            qw_batch_dispatch(b, e->QH + e->KVH, nbl, 1, 256, 1, 1);
-            qw_batch_kernel(b, e->k_attn);
-            qw_batch_buf(b, 0, &e->qb, 0);
-            qw_batch_buf(b, 1, &e->kvpool, 0);
-            qw_batch_buf(b, 2, &e->ptab, 0);
-            qw_batch_buf(b, 3, &e->ctl_d, 2 * ROWS * 4 + co);
-            qw_batch_buf(b, 4, &e->ctl_d, ROWS * 4 + co);
-            qw_batch_buf(b, 5, &e->part, 0);
-            qw_batch_bytes(b, 6, &qa, sizeof qa);
-            qw_batch_dispatch(b, max_chunks, e->KVH, nbl, 128, 1, 1);
-            qw_batch_kernel(b, e->k_merge);
-            qw_batch_buf(b, 0, &e->part, 0);
-            qw_batch_buf(b, 1, &e->proj, 0);
-            qw_batch_buf(b, 2, &e->ya, 0);
-            qw_batch_buf(b, 3, &e->ctl_d, 2 * ROWS * 4 + co);
-            qw_batch_bytes(b, 4, &qa, sizeof qa);
-            qw_batch_dispatch(b, e->QH, nbl, 1, 256, 1, 1);
+            // the attention kernels take up to 64 rows: one group of rows for a step, several for a wide piece -- all of its K and V first
+            auto group = [&](uint32_t r0) {
+                return qsa_args{std::min<uint32_t>(ROWS, nbl - r0), (uint32_t)w.idx, (uint32_t)e->n_attn, e->qkv_rows, (uint32_t)e->max_pages, max_chunks, 0, 0};
+            };
+            const size_t QR = (size_t)e->QH * e->HD * 2;  // bytes of a row of q
+            for (uint32_t r0 = 0; r0 < nbl; r0 += ROWS) {
+                const qsa_args qa = group(r0);
+                qw_batch_kernel(b, e->k_prep);
+                qw_batch_buf(b, 0, &e->proj, (size_t)r0 * e->qkv_rows * 2);
+                qw_batch_buf(b, 1, &e->small, (w.small + 2 * D) * 4);
+                qw_batch_buf(b, 2, &e->small, (w.small + 2 * D + 256) * 4);
+                qw_batch_buf(b, 3, &e->qb, r0 * QR);
+                qw_batch_buf(b, 4, &e->kvpool, 0);
+                qw_batch_buf(b, 5, &e->ptab, 0);
+                qw_batch_buf(b, 6, ctl, (2 * CR + r0) * 4 + co);
+                qw_batch_buf(b, 7, ctl, (CR + r0) * 4 + co);
+                qw_batch_bytes(b, 8, &qa, sizeof qa);
+                qw_batch_dispatch(b, e->QH + e->KVH, qa.nb, 1, 256, 1, 1);
+            }
+            for (uint32_t r0 = 0; r0 < nbl; r0 += ROWS) {
+                const qsa_args qa = group(r0);
+                qw_batch_kernel(b, e->k_attn);
+                qw_batch_buf(b, 0, &e->qb, r0 * QR);
+                qw_batch_buf(b, 1, &e->kvpool, 0);
+                qw_batch_buf(b, 2, &e->ptab, 0);
+                qw_batch_buf(b, 3, ctl, (2 * CR + r0) * 4 + co);
+                qw_batch_buf(b, 4, ctl, (CR + r0) * 4 + co);
+                qw_batch_buf(b, 5, &e->part, 0);
+                qw_batch_bytes(b, 6, &qa, sizeof qa);
+                qw_batch_dispatch(b, max_chunks, e->KVH, qa.nb, 128, 1, 1);
+                qw_batch_kernel(b, e->k_merge);
+                qw_batch_buf(b, 0, &e->part, 0);
+                qw_batch_buf(b, 1, &e->proj, (size_t)r0 * e->qkv_rows * 2);
+                qw_batch_buf(b, 2, &e->ya, (size_t)r0 * e->KA * 2);
+                qw_batch_buf(b, 3, ctl, (2 * CR + r0) * 4 + co);
+                qw_batch_bytes(b, 4, &qa, sizeof qa);
+                qw_batch_dispatch(b, e->QH, qa.nb, 1, 256, 1, 1);
+            }
             enc_out_proj(e->k_qmv_o_a, e->k_qmv_o_a_x, w.w_out, e->KA, &e->ya);
         } else {
             enc_qmv(b, e->k_qmv_in_g, &e->dense, w.w_in, e->gdn_rows, D, &e->x, &e->proj, nbl, e->gdn_rows, xo);
@@ -681,7 +728,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_buf(b, 5, &e->cv, 0);
             qw_batch_buf(b, 6, &e->la, 0);
             qw_batch_buf(b, 7, &e->be, 0);
-            qw_batch_buf(b, 8, &e->ctl_d, ROWS * 4 + co);
+            qw_batch_buf(b, 8, ctl, CR * 4 + co);
             qw_batch_bytes(b, 9, &ea, sizeof ea);
             qw_batch_dispatch(b, (e->C + 2 * e->HV + 255) / 256, nbl, 1, 256, 1, 1);
             const gdn_args ga = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
@@ -694,7 +741,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             if (piece) qw_batch_buf(b, 5, &e->cstate, 0);
             else qw_batch_buf(b, 5, &e->small, sa + 2 * e->HV * 4);
             qw_batch_buf(b, 6, &e->gy, 0);
-            qw_batch_buf(b, 7, &e->ctl_d, ROWS * 4 + co);
+            qw_batch_buf(b, 7, ctl, CR * 4 + co);
             qw_batch_bytes(b, 8, &ga, sizeof ga);
             qw_batch_dispatch(b, e->HV, nbl, 1, 512, 1, 1);
             if (piece) {
@@ -711,7 +758,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
         // ---- MoE (gg_moe, src/engine.c:568-646)
         const size_t gu_bytes = (size_t)e->I * e->rbD, ex_bytes = (size_t)e->EL * gu_bytes, selo = (size_t)l * e->sel_bytes;
         const sel_args sa = {nb, (uint32_t)e->e_lo, (uint32_t)(e->e_lo + e->EL)};
-        qw_batch_kernel(b, e->k_route);  // router logits + top-k + grouping in one launch
+        qw_batch_kernel(b, wide ? e->k_logits_w : e->k_route);  // router logits + top-k + grouping in one launch; of a wide piece the logits
         qw_batch_buf(b, 0, &e->router, (size_t)l * (e->E + 1) * D * 2);
         qw_batch_buf(b, 1, &e->router, ((size_t)l * (e->E + 1) + e->E) * D * 2);
         qw_batch_buf(b, 2, &e->x, 0);
@@ -720,6 +767,17 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
         qw_batch_buf(b, 5, &e->msel, selo);
         qw_batch_bytes(b, 14, &sa, sizeof sa);
         qw_batch_dispatch(b, (e->E + 1 + 7) / 8, 1, 1, 1024, 1, 1);
+        if (wide) {
+            qw_batch_kernel(b, e->k_topk_w);
+            qw_batch_buf(b, 0, &e->mlog, 0);
+            qw_batch_buf(b, 1, &e->msel, selo);
+            qw_batch_bytes(b, 2, &sa, sizeof sa);
+            qw_batch_dispatch(b, (nb + 3) / 4, 1, 1, 128, 1, 1);
+            qw_batch_kernel(b, e->k_group_w);
+            qw_batch_buf(b, 1, &e->msel, selo);
+            qw_batch_bytes(b, 2, &sa, sizeof sa);
+            qw_batch_dispatch(b, 1, 1, 1, 512, 1, 1);
+        }
         const uint32_t ebase = (uint32_t)e->e_lo;
         const bool zero_first = e->c.ep_size > 1 && !e->ep_fused;  // rows of experts held elsewhere must read as zero before the NCCL exchange
         // the down projection's output: Pg, or (fused exchange) Pg[layer parity] of every rank -- two buffers suffice because a rank
@@ -737,7 +795,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 const fill_args z = {0, (uint64_t)nb * (e->TOPK + 1) * D * 4, 0, 0, 0.f, 0.f};
                 enc_fill(e, b, &e->Pg, 0, z);
             }
-            qw_batch_kernel(b, e->ep_fused ? e->k_ffn_x : e->moe_probe ? e->k_ffn_probe : e->k_ffn);  // gate/up, SiLU * up and down of every chosen expert in one launch
+            qw_batch_kernel(b, wide ? e->k_ffn_w : e->ep_fused ? e->k_ffn_x : e->moe_probe ? e->k_ffn_probe : e->k_ffn);  // gate/up, SiLU * up and down of every chosen expert in one launch
             if (e->ffn_iq3x) {
                 qw_batch_buf(b, 0, &e->xq_gu, (size_t)l * e->EL * e->x_gus);
                 qw_batch_buf(b, 2, &e->xs_gu, (size_t)l * e->x_gus);
@@ -753,7 +811,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             }
             qw_batch_buf(b, 4, &e->x, 0);
             qw_batch_buf(b, 5, &e->msel, selo);
-            qw_batch_buf(b, 8, &e->ffn_scr, 0);
+            qw_batch_buf(b, 8, wide ? &e->ffn_scr_w : &e->ffn_scr, 0);
             bind_pg();
             qw_batch_dispatch(b, e->I / 16, nb * e->TOPK + 1, 1, 256, 1, 1);
         } else {
@@ -885,6 +943,7 @@ void end_step(qw_engine *e, const int *sids, int B, int nsteps, double wall_ms) 
 // non-zero; the next step must not find them: they would let down pieces start before their H is complete.
 void after_failed_step(qw_engine *e) {
     if (e->ffn_scr.size) qw_buf_zero(e->g, &e->ffn_scr, 0, MOE_FFN_SYNC_BYTES);
+    if (e->ffn_scr_w.size) qw_buf_zero(e->g, &e->ffn_scr_w, 0, MOE_FFN_SYNC_BYTES_WIDE);
 }
 
 }  // namespace
@@ -1043,10 +1102,10 @@ extern "C" int qw_engine_par_step_sample(qw_engine *e, const int *sids, const in
 }
 
 // Prompt processing for one slot (src/engine.h:81), from an empty slot -- recurrent and conv state zero, no KV.  The prompt runs in
-// pieces of up to ROWS tokens, each one pass over the weights, submitted back to back; a token's arithmetic is that of the decode
+// pieces of up to piece_rows tokens, each one pass over the weights, submitted back to back; a token's arithmetic is that of the decode
 // step, so "prefill then step" equals stepping every token, bit for bit.  (There is no prefix cache: *cached = 0.)
-// Measured on a B200, 48 layers: 419 tokens 91 ms (one token at a time: 1200 ms), 45 tokens 11 ms (124 ms).  A piece's cost is that of a
-// step of as many slots; smaller pieces would read the weights more often, larger ones need wider kernels.
+// Measured on a B200: 48 layers, 419 tokens 1206 ms one token at a time, 81.2 ms in pieces of 64, 50.6 ms in pieces of 256; 12 layers, 1700 tokens
+// 80.0 -> 46.8 ms.  64 tokens choose about 370 of 512 experts, 256 nearly all: per token a quarter of the weights is left to decode.
 extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32_t *prompt, int np, int *cached) {
     if (cached) *cached = 0;
     if (!e || sid < 0 || sid >= (int)e->slots.size() || !prompt || np < 1 || np >= e->c.max_ctx) return e ? (e->fail("par_prefill: bad arguments"), nullptr) : nullptr;
@@ -1078,8 +1137,8 @@ extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32
     }
     int n = 0;
     for (int p0 = 0; p0 < np && ok; p0 += n) {
-        n = std::min(ROWS, np - p0);
-        int perm[ROWS], sids[ROWS], lo, hi;
+        n = std::min(e->moe_probe ? ROWS : e->piece_rows, np - p0);
+        int perm[PROWS], sids[PROWS], lo, hi;
         std::fill(sids, sids + n, sid);
         qw_ep_row_order(sids, n, e->slot_shard ? e->c.ep_size : 1, e->slot_shard ? e->c.ep_rank : 0, perm, &lo, &hi);  // one slot: all rows are this rank's, or none
         e->row_lo = (uint32_t)lo;

@@ -42,8 +42,12 @@ namespace {
 
 constexpr int FFN_CW = 16;                       // consumer warps
 constexpr int FFN_THREADS = (FFN_CW + 1) * 32;   // + the producer warp
-constexpr int FFN_MAXITEMS = MOE_FFN_MAXITEMS;   // see moe_sel.h: the scratch buffer
-constexpr int FFN_SYNC_BYTES = MOE_FFN_SYNC_BYTES;
+// see moe_sel.h: the selection record and the scratch buffer of a step (WIDE 0) and of a piece of a prompt (WIDE 1)
+template <int WIDE>
+struct FfnRec {
+    typedef moe_sel_t<WIDE ? MOE_MAXB_WIDE : MOE_MAXB> sel;
+    static constexpr uint32_t MAXITEMS = WIDE ? MOE_FFN_MAXITEMS_WIDE : MOE_FFN_MAXITEMS, ROWCNT = WIDE ? MOE_FFN_ROWCNT_WIDE : MOE_FFN_ROWCNT;
+};
 constexpr int FFN_PITCH = 240;                   // IQ3_S: bytes between staged gate/up rows
 constexpr int FFN_D = 2048, FFN_I = 512;         // the shapes this kernel is built for (the launcher refuses others)
 constexpr int FFN_MAXG = 520;                    // groups kept in shared memory: E <= 512 experts (+ end markers)
@@ -69,12 +73,12 @@ struct FfnP {
     const uint8_t *Wg, *Sg;   // IQ3X: routed / shared gate + up stages (IQ3_S copies go through the tensor maps)
     const __half *x;          // tokens fp16 [nb][D]
     float *Pg;                // [nb][topk+1][D]
-    const moe_sel *ms;
+    const void *ms;           // moe_sel, or moe_sel_wide
     const QwTables *tab;
     unsigned *status;
     uint32_t ebase;
-    unsigned *sync;           // [0 .. FFN_MAXITEMS) per-item counters of finished gate/up warps, [FFN_MAXITEMS] finished blocks; all zero between launches
-    __half *H;                // [FFN_MAXITEMS][2][8][I]
+    unsigned *sync;           // [0 .. MAXITEMS) per-item counters of finished gate/up warps, [MAXITEMS] finished blocks; all zero between launches
+    __half *H;                // [item][2][8][I]
     float *PgR[8];            // expert-parallel exchange: Pg of every rank (see moe_dn in k_moe.cu)
     EpPeers ep;
 };
@@ -96,7 +100,8 @@ struct __align__(16) FfnItem {
 };
 // item number w -> (group, pass): routed groups first (pre[] = passes before each group, in shared memory), then the shared
 // expert's passes.  The group's entries and expert come from the selection record in global memory.
-__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const moe_sel *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
+template <class SEL>
+__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const SEL *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
     FfnItem it{};
     const uint32_t routed = pre[U];
     uint32_t cnt;
@@ -123,7 +128,8 @@ __device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const moe_sel *
     return it;
 }
 // column col of the item -> (token, rank)
-__device__ __forceinline__ void ffn_entry(const moe_sel *ms, const FfnItem &it, uint32_t topk, uint32_t col, uint32_t &tok, uint32_t &rank) {
+template <class SEL>
+__device__ __forceinline__ void ffn_entry(const SEL *ms, const FfnItem &it, uint32_t topk, uint32_t col, uint32_t &tok, uint32_t &rank) {
     if (it.shared) {
         tok = it.c0 + col;
         rank = topk;
@@ -326,10 +332,11 @@ __device__ __forceinline__ void x_unit(uint32_t rec0, uint32_t rec1, int kh, int
 // TMA boxes and bulk copies through the same ring, but the consumers only read every staged byte once (16-byte loads) and
 // compute nothing -- the role of the reference's pure-read probes (bench/moe_bw.c:1-3, bench/qmv.c:357-382).
 // (17 warps put five on one scheduler, whose 16 K registers then allow 96 per thread)
-template <bool PROBE, int FMT>
+template <bool PROBE, int FMT, int WIDE>
 __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(const __grid_constant__ CUtensorMap mG, const __grid_constant__ CUtensorMap mU,
                                                            const __grid_constant__ CUtensorMap mSG, const __grid_constant__ CUtensorMap mSU, const FfnP p) {
     using C = FfnCfg<FMT>;
+    using Rec = FfnRec<WIDE>;
     constexpr int FFN_STG = C::STG, FFN_SLOT = C::SLOT;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *bars = (uint64_t *)smem;
@@ -367,13 +374,13 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
         *(uint4 *)(smem + C::OFF_TAB + 16 * tid) = make_uint4(*(const uint32_t *)&m0, *(const uint32_t *)&a0, *(const uint32_t *)&m1, *(const uint32_t *)&a1);
     }
     pdl_wait();  // the selection record, the tokens and Pg belong to earlier kernels
-    const moe_sel *ms = p.ms;
+    const typename Rec::sel *ms = (const typename Rec::sel *)p.ms;
     // passes before every group: independent loads, so the table is in shared memory after one latency
     for (uint32_t i = tid; i < FFN_MAXG; i += FFN_THREADS) pre[i] = ms->pre[i];
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
     uint32_t items = pre[U] + (p.Sd ? (nb + 7) / 8 : 0);
-    if (items > FFN_MAXITEMS) {  // cannot happen with E <= 512 and 64 tokens; never index past the flags
+    if (items > Rec::MAXITEMS) {  // cannot happen with E <= 512 and 64 (256) tokens; never index past the flags
         if (tid == 0) set_status(p.status, ST_BAD_ARG | 5);
         items = 0;
     }
@@ -694,8 +701,8 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                     __syncwarp();
                     if (g == 0) {
                         __threadfence();  // the warp's stores (cumulative over the warp barrier) before the counts
-                        if (oo[0] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[0] / D, 1u);
-                        if (oo[1] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[1] / D, 1u);
+                        if (oo[0] != 0xffffffffu) atomicAdd(p.sync + Rec::ROWCNT + oo[0] / D, 1u);
+                        if (oo[1] != 0xffffffffu) atomicAdd(p.sync + Rec::ROWCNT + oo[1] / D, 1u);
                     }
                 }
             }
@@ -707,9 +714,9 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     __syncthreads();
     if (tid == 0 && !PROBE) {
         __threadfence();
-        if (atomicAdd(p.sync + FFN_MAXITEMS, 1u) == gridDim.x - 1) {
+        if (atomicAdd(p.sync + Rec::MAXITEMS, 1u) == gridDim.x - 1) {
             for (uint32_t i = 0; i < items; i++) p.sync[i] = 0;
-            p.sync[FFN_MAXITEMS] = 0;
+            p.sync[Rec::MAXITEMS] = 0;
         }
     }
     if (p.ep.nranks > 1) ep_publish(p.ep);
@@ -776,16 +783,19 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     p.Wd = L.buf<uint8_t>(6);
     p.Wg = Wg;
     p.Sg = Sg;
+    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 256 rows of tokens (one GPU only)
+    const bool wide = L.def("WIDE", 0) != 0;
     p.sync = L.buf<unsigned>(8);
-    QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= MOE_FFN_SCRATCH_BYTES(I));
-    p.H = (__half *)((uint8_t *)p.sync + FFN_SYNC_BYTES);
+    QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I) : MOE_FFN_SCRATCH_BYTES(I)));
+    QW_CHECK_ARG(!wide || (L.def("EPX", 0) <= 1 && L.def("PROBE", 0) == 0));
+    p.H = (__half *)((uint8_t *)p.sync + (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
     p.Sd = shared ? L.buf<uint8_t>(7) : nullptr;
     p.x = L.buf<__half>(4);
-    p.ms = L.buf<moe_sel>(5);
+    p.ms = L.buf<void>(5);
     p.Pg = L.buf<float>(9);
     p.tab = (const QwTables *)L.tables;
     p.status = L.status;
-    QW_CHECK_ARG(Wg && Wu && p.Wd && p.x && p.ms && p.Pg && L.avail(5) >= sizeof(moe_sel));
+    QW_CHECK_ARG(Wg && Wu && p.Wd && p.x && p.ms && p.Pg && L.avail(5) >= (wide ? sizeof(moe_sel_wide) : sizeof(moe_sel)));
     QW_CHECK_ARG(!shared || (Sg && Su && p.Sd));
     if (x4) {
         const size_t gus = (size_t)(I / 64) * (D / 512) * IQ3X_STAGE, dns = (size_t)(D / 128) * (I / 512) * IQ3X_STAGE;
@@ -795,7 +805,7 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
         QW_CHECK_ARG(L.avail(0) >= wsz && L.avail(1) >= wsz && L.avail(6) >= wsz && (!shared || (L.avail(2) >= ssz && L.avail(3) >= ssz && L.avail(7) >= ssz)));
     }
     QW_CHECK_ARG((((uintptr_t)Wg | (uintptr_t)Wu | (uintptr_t)p.Wd | (uintptr_t)Sg | (uintptr_t)Su | (uintptr_t)p.Sd | (uintptr_t)p.x) & 15) == 0);
-    QW_CHECK_ARG(L.avail(9) >= (size_t)MOE_MAXB * (topk + 1) * D * 4 && L.avail(4) >= (size_t)D * 2);
+    QW_CHECK_ARG(L.avail(9) >= (size_t)(wide ? MOE_MAXB_WIDE : MOE_MAXB) * (topk + 1) * D * 4 && L.avail(4) >= (size_t)D * 2);
     p.ep = EpPeers{};
     p.ep.nranks = 1;
     if (L.def("EPX", 0) > 1) {
@@ -821,7 +831,8 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
         QW_CHECK_ARG(mG && mU && mSG && mSU);
     }
     const bool probe = L.def("PROBE", 0) != 0;  // PROBE defined 1: the copy-only twin (outputs are not written)
-    auto kern = x4 ? (probe ? moe_ffn_k<true, 1> : moe_ffn_k<false, 1>) : (probe ? moe_ffn_k<true, 0> : moe_ffn_k<false, 0>);
+    auto kern = wide ? (x4 ? moe_ffn_k<false, 1, 1> : moe_ffn_k<false, 0, 1>)
+                : x4 ? (probe ? moe_ffn_k<true, 1, 0> : moe_ffn_k<false, 1, 0>) : (probe ? moe_ffn_k<true, 0, 0> : moe_ffn_k<false, 0, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;  // the blocks wait for one another's H: all of them must be resident together

@@ -27,7 +27,7 @@ __global__ void kb_embed_k(const __half *emb, const int32_t *tok, float *h, uint
 }
 static cudaError_t launch_kb_embed(const QwLaunch &L) {
     struct { uint32_t nb, D, V; } a = L.bytes<decltype(a)>(3);
-    QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(1) && L.buf<void>(2) && L.has_bytes(3, 12) && a.nb >= 1 && a.nb <= 64);
+    QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(1) && L.buf<void>(2) && L.has_bytes(3, 12) && a.nb >= 1 && a.nb <= (uint32_t)L.def("ROWS", 64));
     QW_CHECK_ARG(L.avail(0) >= (size_t)a.V * a.D * 2 && L.avail(1) >= a.nb * 4 && L.avail(2) >= (size_t)a.nb * a.D * 4);
     qw_launch(kb_embed_k, dim3((a.D + 255) / 256, a.nb), 256, 0, L.stream, L.buf<__half>(0), L.buf<int32_t>(1), L.buf<float>(2), a.D, a.V);
     return cudaGetLastError();
@@ -37,7 +37,8 @@ QW_FAMILY(kb_embed, launch_kb_embed, 256)
 // binds: 0 = h fp32 [nb][D], 1 = delta fp16 [nb][D] (only with ADD defined 1: h is then updated in place),
 // 2 = w fp32 [D], 3 = x out fp16 [nb][D], 4 = {nb, D}.  With CMB defined 1 the delta is not read from memory but is
 // the MoE combine of moe_cmb (rank-ordered weighted sum of Pg plus the shared expert, rounded to fp16) computed on
-// the fly: 5 = moe_sel, 6 = Pg fp32 [nb][TOPK+1][D], define TOPK.  grid nb x 256
+// the fly: 5 = moe_sel, 6 = Pg fp32 [nb][TOPK+1][D], define TOPK.  ROWS = the most rows (default 64); WIDE defined 1: bind 5 is a
+// moe_sel_wide.  grid nb x 256
 template <int MODE>  // 0: norm only, 1: h += delta, 2: h += fp16(combine)
 __global__ void __launch_bounds__(1024) add_rmsnorm_k(float *h, const __half *delta, const float *w, __half *x, uint32_t D, const moe_sel *ms,
                                                      const float *Pg, uint32_t topk, const unsigned *flags, const unsigned *seq, uint32_t nranks,
@@ -54,8 +55,9 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_k(float *h, const __half *de
     float *hr = h + (size_t)t * D;
     float wk[MOE_MAXK];
     if (MODE == 2) {
+        const float *wr = &ms->w[0][0] + t * (MOE_MAXK + 1);  // (moe_sel and moe_sel_wide keep w in the same place)
 #pragma unroll
-        for (uint32_t s = 0; s < MOE_MAXK; s++) wk[s] = s <= topk ? ms->w[t][s] : 0.f;
+        for (uint32_t s = 0; s < MOE_MAXK; s++) wk[s] = s <= topk ? wr[s] : 0.f;
     }
     // a thread's values stay in registers between the two passes (D <= 4 * blockDim; beyond that they are read back)
     float vv[4] = {0.f, 0.f, 0.f, 0.f};
@@ -148,8 +150,9 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256) cmb_rmsnorm_cl_
     }
     if (nranks > 1) ep_wait(flags, seq, nranks, status);
     float wk[MOE_MAXK], pv[MOE_MAXK];
+    const float *wr = &ms->w[0][0] + t * (MOE_MAXK + 1);  // (moe_sel and moe_sel_wide keep w in the same place)
 #pragma unroll
-    for (uint32_t s = 0; s < MOE_MAXK; s++) wk[s] = s <= topk ? ms->w[t][s] : 0.f;
+    for (uint32_t s = 0; s < MOE_MAXK; s++) wk[s] = s <= topk ? wr[s] : 0.f;
 #pragma unroll
     for (uint32_t s = 0; s < MOE_MAXK; s++) pv[s] = s <= topk ? __ldcg(Pg + ((size_t)t * (topk + 1) + s) * D + d) : 0.f;
     float v = h[(size_t)t * D + d];
@@ -181,11 +184,13 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256) cmb_rmsnorm_cl_
 }
 static cudaError_t launch_add_rmsnorm(const QwLaunch &L) {
     struct { uint32_t nb, D; } a = L.bytes<decltype(a)>(4);
-    QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(2) && L.buf<void>(3) && L.has_bytes(4, 8) && a.nb >= 1 && a.nb <= 64);
+    QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(2) && L.buf<void>(3) && L.has_bytes(4, 8) && a.nb >= 1 && a.nb <= (uint32_t)L.def("ROWS", 64));
     QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * a.D * 4 && L.avail(2) >= (size_t)a.D * 4 && L.avail(3) >= (size_t)a.nb * a.D * 2);
     if (L.def("CMB", 0)) {
         const uint32_t topk = (uint32_t)L.def("TOPK", 10);
-        QW_CHECK_ARG(L.buf<void>(5) && L.buf<void>(6) && L.avail(5) >= sizeof(moe_sel) && L.avail(6) >= (size_t)a.nb * (topk + 1) * a.D * 4 && topk < MOE_MAXK);
+        const bool wide = L.def("WIDE", 0) != 0;
+        QW_CHECK_ARG(a.nb <= (wide ? MOE_MAXB_WIDE : MOE_MAXB));
+        QW_CHECK_ARG(L.buf<void>(5) && L.buf<void>(6) && L.avail(5) >= (wide ? sizeof(moe_sel_wide) : sizeof(moe_sel)) && L.avail(6) >= (size_t)a.nb * (topk + 1) * a.D * 4 && topk < MOE_MAXK);
         // EPX = number of expert-parallel ranks whose down projections store into Pg: 7 = this rank's flag array
         // (one sequence number per rank), 8 = this rank's sequence counter
         const uint32_t nranks = (uint32_t)L.def("EPX", 1);
@@ -194,8 +199,8 @@ static cudaError_t launch_add_rmsnorm(const QwLaunch &L) {
             // ROWCNT defined 1 (one GPU, after moe_ffn): 9 = the FFN's scratch buffer, whose per-row counters replace the wait for the launch
             unsigned *rowcnt = nullptr;
             if (L.def("ROWCNT", 0)) {
-                QW_CHECK_ARG(nranks == 1 && L.buf<unsigned>(9) && L.avail(9) >= MOE_FFN_SYNC_BYTES && (a.nb * (topk + 1)) <= MOE_MAXB * MOE_MAXK);
-                rowcnt = L.buf<unsigned>(9) + MOE_FFN_ROWCNT;
+                QW_CHECK_ARG(nranks == 1 && L.buf<unsigned>(9) && L.avail(9) >= (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
+                rowcnt = L.buf<unsigned>(9) + (wide ? MOE_FFN_ROWCNT_WIDE : MOE_FFN_ROWCNT);
             }
             qw_launch(cmb_rmsnorm_cl_k, a.nb * 8, 256, 0, L.stream, L.buf<float>(0), L.buf<float>(2), L.buf<__half>(3), L.buf<moe_sel>(5), L.buf<float>(6), topk,
                       nranks > 1 ? L.buf<unsigned>(7) : nullptr, nranks > 1 ? L.buf<unsigned>(8) : nullptr, nranks, rowcnt, (unsigned *)L.status);

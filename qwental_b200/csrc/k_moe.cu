@@ -73,147 +73,146 @@ struct sel_args {
     uint32_t nb, e_lo, e_hi;
 };
 
-// Body of the selection for one block of NTH threads (NTH >= E: thread e owns expert e in the scans).  Logits are read with .cg loads: in the fused router + select
-// kernel they were written by other blocks of the same launch.
-template <int NTH>
-__device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms, uint32_t E, uint32_t topk, sel_args a) {
-    __shared__ uint32_t mlo[MOE_MAXE], mhi[MOE_MAXE], pos[MOE_MAXE], grp[MOE_MAXE];  // token bit masks per expert
-    __shared__ uint16_t sid[MOE_MAXB * MOE_MAXK];
-    __shared__ uint32_t wsum[2][32];
-    __shared__ uint64_t cand_s[NTH / 32][32 + MOE_MAXK];  // per warp: candidates of the fast top-k path, then the winners' keys
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+// Top-k of one token by one warp: lane owns experts lane, lane + 32, ... (coalesced reads).  Equal logits -> lowest expert id: within a
+// lane the strict '>' keeps the lowest id, across lanes the smallest id among the lanes holding the maximum wins.  Logits are read with
+// .cg loads: in the fused router + select kernel they were written by other blocks of the same launch.  cs = the warp's [32 + MOE_MAXK]
+// words: candidates of the fast path, then the winners' keys.  ids may be nullptr.
+__device__ __forceinline__ void moe_topk_row(const float *lg, uint32_t E, uint32_t topk, uint32_t lane, uint64_t *cs, int32_t *ids, uint16_t *sid, float *w) {
     const uint32_t PER = E / 32;
-    constexpr uint32_t NW = NTH / 32;
-    for (uint32_t e = tid; e < MOE_MAXE; e += NTH) mlo[e] = mhi[e] = 0;
-    // 1. top-k per token: one warp per token, lane owns experts lane, lane + 32, ... (coalesced reads).  Equal
-    //    logits -> lowest expert id: within a lane the strict '>' keeps the lowest id, across lanes the smallest id
-    //    among the lanes holding the maximum wins.
-    for (uint32_t t = warp; t < a.nb; t += NW) {
-        const float *lg = logits + (size_t)t * (E + 1);
-        // Logits as order-preserving unsigned keys (a float's bits with the sign folded), so a maximum is one hardware
-        // warp reduction.  Equal floats give equal keys (a logit is never -0: every dot product starts from +0).
-        auto key_of = [&](uint32_t j) {
-            const uint32_t u = __float_as_uint(__ldcg(lg + lane + 32 * j));
-            return u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
-        };
-        uint32_t pkey = 0;
-        if (PER == 16) {
-            uint32_t kv[16];
+    // Logits as order-preserving unsigned keys (a float's bits with the sign folded), so a maximum is one hardware
+    // warp reduction.  Equal floats give equal keys (a logit is never -0: every dot product starts from +0).
+    auto key_of = [&](uint32_t j) {
+        const uint32_t u = __float_as_uint(__ldcg(lg + lane + 32 * j));
+        return u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+    };
+    uint32_t pkey = 0;
+    if (PER == 16) {
+        uint32_t kv[16];
 #pragma unroll
-            for (uint32_t j = 0; j < 16; j++) kv[j] = key_of(j);
-            // Fast path.  T = the topk-th largest of the 32 lane maxima: at least topk values are >= T, so the winners are
-            // among the values >= T -- usually little more than topk of them.  If they fit one per lane, each lane takes
-            // one candidate and finds its rank by counting the candidates that beat it (larger key, or equal key and
-            // lower id); ranks are distinct because ids are.  Otherwise (many equal logits) the general path below runs.
-            uint32_t lm = kv[0];
+        for (uint32_t j = 0; j < 16; j++) kv[j] = key_of(j);
+        // Fast path.  T = the topk-th largest of the 32 lane maxima: at least topk values are >= T, so the winners are
+        // among the values >= T -- usually little more than topk of them.  If they fit one per lane, each lane takes
+        // one candidate and finds its rank by counting the candidates that beat it (larger key, or equal key and
+        // lower id); ranks are distinct because ids are.  Otherwise (many equal logits) the general path below runs.
+        uint32_t lm = kv[0];
 #pragma unroll
-            for (uint32_t j = 1; j < 16; j++) lm = max(lm, kv[j]);
-            uint32_t cur = lm, T = 0;
-            for (uint32_t k = 0; k < topk; k++) {
-                T = __reduce_max_sync(0xffffffffu, cur);
-                const uint32_t who = __ffs(__ballot_sync(0xffffffffu, cur == T)) - 1;
-                if (lane == who) cur = 0;  // (a real key is never 0: that would be the bit pattern of -NaN)
+        for (uint32_t j = 1; j < 16; j++) lm = max(lm, kv[j]);
+        uint32_t cur = lm, T = 0;
+        for (uint32_t k = 0; k < topk; k++) {
+            T = __reduce_max_sync(0xffffffffu, cur);
+            const uint32_t who = __ffs(__ballot_sync(0xffffffffu, cur == T)) - 1;
+            if (lane == who) cur = 0;  // (a real key is never 0: that would be the bit pattern of -NaN)
+        }
+        uint32_t cnt = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 16; j++) cnt += kv[j] >= T;
+        uint32_t pre = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= (uint32_t)o) pre += n;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
+        if (total <= 32) {
+            uint32_t at = pre - cnt;
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j++)
+                if (kv[j] >= T) cs[at++] = ((uint64_t)kv[j] << 32) | (0xffffffffu - (lane + 32 * j));
+            __syncwarp();
+            const uint64_t mine = lane < total ? cs[lane] : 0;
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < total; j++) rank += __shfl_sync(0xffffffffu, mine, j) > mine;
+            if (lane < total && rank < topk) {
+                const uint32_t id = 0xffffffffu - (uint32_t)mine;
+                if (ids) ids[rank] = (int32_t)id;
+                sid[rank] = (uint16_t)id;
+                cs[32 + rank] = mine >> 32;  // key of rank r, for the softmax below
             }
-            uint32_t cnt = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < 16; j++) cnt += kv[j] >= T;
-            uint32_t pre = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t n = __shfl_up_sync(0xffffffffu, pre, o);
-                if (lane >= (uint32_t)o) pre += n;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, pre, 31);
-            if (total <= 32) {
-                uint64_t *cs = cand_s[warp];
-                uint32_t at = pre - cnt;
-#pragma unroll
-                for (uint32_t j = 0; j < 16; j++)
-                    if (kv[j] >= T) cs[at++] = ((uint64_t)kv[j] << 32) | (0xffffffffu - (lane + 32 * j));
-                __syncwarp();
-                const uint64_t mine = lane < total ? cs[lane] : 0;
-                uint32_t rank = 0;
-                for (uint32_t j = 0; j < total; j++) rank += __shfl_sync(0xffffffffu, mine, j) > mine;
-                if (lane < total && rank < topk) {
-                    const uint32_t id = 0xffffffffu - (uint32_t)mine;
-                    ms->ids[t][rank] = (int32_t)id;
-                    sid[t * MOE_MAXK + rank] = (uint16_t)id;
-                    cs[32 + rank] = mine >> 32;  // key of rank r, for the softmax below
-                }
-                __syncwarp();
-                if (lane < topk) pkey = (uint32_t)cs[32 + lane];
-                __syncwarp();
-            } else {
-            // General path: the lane sorts its 16 (key, ~id) pairs once
-            uint64_t s[16];
-#pragma unroll
-            for (uint32_t j = 0; j < 16; j++) s[j] = ((uint64_t)kv[j] << 32) | (0xffffffffu - (lane + 32 * j));
-#define CE(A, B)                          \
-    {                                     \
-        const uint64_t x_ = s[A], y_ = s[B]; \
-        const bool sw_ = y_ > x_;         \
-        s[A] = sw_ ? y_ : x_;             \
-        s[B] = sw_ ? x_ : y_;             \
-    }
-            CE(0, 1) CE(2, 3) CE(4, 5) CE(6, 7) CE(8, 9) CE(10, 11) CE(12, 13) CE(14, 15) CE(0, 2) CE(1, 3) CE(4, 6) CE(5, 7) CE(8, 10) CE(9, 11) CE(12, 14) CE(13, 15) CE(1, 2) CE(5, 6) CE(9, 10) CE(13, 14) CE(0, 4) CE(1, 5) CE(2, 6) CE(3, 7) CE(8, 12) CE(9, 13) CE(10, 14) CE(11, 15) CE(2, 4) CE(3, 5) CE(10, 12) CE(11, 13) CE(1, 2) CE(3, 4) CE(5, 6) CE(9, 10) CE(11, 12) CE(13, 14) CE(0, 8) CE(1, 9) CE(2, 10) CE(3, 11) CE(4, 12) CE(5, 13) CE(6, 14) CE(7, 15) CE(4, 8) CE(5, 9) CE(6, 10) CE(7, 11) CE(2, 4) CE(3, 5) CE(6, 8) CE(7, 9) CE(10, 12) CE(11, 13) CE(1, 2) CE(3, 4) CE(5, 6) CE(7, 8) CE(9, 10) CE(11, 12) CE(13, 14)
-#undef CE
-            for (uint32_t k = 0; k < topk; k++) {
-                const uint32_t hk = (uint32_t)(s[0] >> 32), hi_ = (uint32_t)s[0];
-                const uint32_t m = __reduce_max_sync(0xffffffffu, hk);
-                const uint32_t nid = __reduce_max_sync(0xffffffffu, hk == m ? hi_ : 0u);  // largest ~id = lowest id
-                const uint32_t id = 0xffffffffu - nid;
-                if (lane == 0) {
-                    ms->ids[t][k] = (int32_t)id;
-                    sid[t * MOE_MAXK + k] = (uint16_t)id;
-                }
-                if (lane == k) pkey = m;
-                if (lane == (id & 31)) {  // pop the head
-#pragma unroll
-                    for (uint32_t j = 0; j < 15; j++) s[j] = s[j + 1];
-                    s[15] = 0;
-                }
-            }
-            }  // general path
+            __syncwarp();
+            if (lane < topk) pkey = (uint32_t)cs[32 + lane];
+            __syncwarp();
         } else {
-            uint32_t v[8];  // small expert counts (E <= 256): rescan the lane's few values every round
+        // General path: the lane sorts its 16 (key, ~id) pairs once
+        uint64_t s[16];
 #pragma unroll
-            for (uint32_t j = 0; j < 8; j++) v[j] = j < PER ? key_of(j) : 0u;
-            for (uint32_t k = 0; k < topk; k++) {
-                uint32_t b0 = v[0], j0 = 0;
+        for (uint32_t j = 0; j < 16; j++) s[j] = ((uint64_t)kv[j] << 32) | (0xffffffffu - (lane + 32 * j));
+#define CE(A, B)                          \
+{                                     \
+    const uint64_t x_ = s[A], y_ = s[B]; \
+    const bool sw_ = y_ > x_;         \
+    s[A] = sw_ ? y_ : x_;             \
+    s[B] = sw_ ? x_ : y_;             \
+}
+        CE(0, 1) CE(2, 3) CE(4, 5) CE(6, 7) CE(8, 9) CE(10, 11) CE(12, 13) CE(14, 15) CE(0, 2) CE(1, 3) CE(4, 6) CE(5, 7) CE(8, 10) CE(9, 11) CE(12, 14) CE(13, 15) CE(1, 2) CE(5, 6) CE(9, 10) CE(13, 14) CE(0, 4) CE(1, 5) CE(2, 6) CE(3, 7) CE(8, 12) CE(9, 13) CE(10, 14) CE(11, 15) CE(2, 4) CE(3, 5) CE(10, 12) CE(11, 13) CE(1, 2) CE(3, 4) CE(5, 6) CE(9, 10) CE(11, 12) CE(13, 14) CE(0, 8) CE(1, 9) CE(2, 10) CE(3, 11) CE(4, 12) CE(5, 13) CE(6, 14) CE(7, 15) CE(4, 8) CE(5, 9) CE(6, 10) CE(7, 11) CE(2, 4) CE(3, 5) CE(6, 8) CE(7, 9) CE(10, 12) CE(11, 13) CE(1, 2) CE(3, 4) CE(5, 6) CE(7, 8) CE(9, 10) CE(11, 12) CE(13, 14)
+#undef CE
+        for (uint32_t k = 0; k < topk; k++) {
+            const uint32_t hk = (uint32_t)(s[0] >> 32), hi_ = (uint32_t)s[0];
+            const uint32_t m = __reduce_max_sync(0xffffffffu, hk);
+            const uint32_t nid = __reduce_max_sync(0xffffffffu, hk == m ? hi_ : 0u);  // largest ~id = lowest id
+            const uint32_t id = 0xffffffffu - nid;
+            if (lane == 0) {
+                if (ids) ids[k] = (int32_t)id;
+                sid[k] = (uint16_t)id;
+            }
+            if (lane == k) pkey = m;
+            if (lane == (id & 31)) {  // pop the head
 #pragma unroll
-                for (uint32_t j = 1; j < 8; j++)
-                    if (j < PER && v[j] > b0) { b0 = v[j]; j0 = j; }
-                const uint32_t m = __reduce_max_sync(0xffffffffu, b0);
-                const uint32_t id = __reduce_min_sync(0xffffffffu, b0 == m ? lane + 32 * j0 : 0xffffffffu);
-                if (lane == 0) {
-                    ms->ids[t][k] = (int32_t)id;
-                    sid[t * MOE_MAXK + k] = (uint16_t)id;
-                }
-                if (lane == k) pkey = m;
-                const uint32_t bl = id & 31, bj = id >> 5;
-#pragma unroll
-                for (uint32_t j = 0; j < 8; j++) v[j] = (lane == bl && j == bj) ? 0u : v[j];  // below every real key
+                for (uint32_t j = 0; j < 15; j++) s[j] = s[j + 1];
+                s[15] = 0;
             }
         }
-        const float pk = __uint_as_float(pkey ^ ((pkey >> 31) ? 0x80000000u : 0xffffffffu));
-        const float mx = __shfl_sync(0xffffffffu, pk, 0), ex = expf(pk - mx);
-        float sm = 0.f;
-        for (uint32_t k = 0; k < topk; k++) sm = __fadd_rn(sm, __shfl_sync(0xffffffffu, ex, k));  // rank order
-        if (lane < topk) ms->w[t][lane] = ex / sm;
-        if (lane == topk) ms->w[t][topk] = 1.0f / (1.0f + expf(-__ldcg(lg + E)));
+        }  // general path
+    } else {
+        uint32_t v[8];  // small expert counts (E <= 256): rescan the lane's few values every round
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++) v[j] = j < PER ? key_of(j) : 0u;
+        for (uint32_t k = 0; k < topk; k++) {
+            uint32_t b0 = v[0], j0 = 0;
+#pragma unroll
+            for (uint32_t j = 1; j < 8; j++)
+                if (j < PER && v[j] > b0) { b0 = v[j]; j0 = j; }
+            const uint32_t m = __reduce_max_sync(0xffffffffu, b0);
+            const uint32_t id = __reduce_min_sync(0xffffffffu, b0 == m ? lane + 32 * j0 : 0xffffffffu);
+            if (lane == 0) {
+                if (ids) ids[k] = (int32_t)id;
+                sid[k] = (uint16_t)id;
+            }
+            if (lane == k) pkey = m;
+            const uint32_t bl = id & 31, bj = id >> 5;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++) v[j] = (lane == bl && j == bj) ? 0u : v[j];  // below every real key
+        }
     }
-    __syncthreads();
-    // 2. group by expert.  mask[e] = tokens that chose e; an entry's place inside its group is the number of
+    const float pk = __uint_as_float(pkey ^ ((pkey >> 31) ? 0x80000000u : 0xffffffffu));
+    const float mx = __shfl_sync(0xffffffffu, pk, 0), ex = expf(pk - mx);
+    float sm = 0.f;
+    for (uint32_t k = 0; k < topk; k++) sm = __fadd_rn(sm, __shfl_sync(0xffffffffu, ex, k));  // rank order
+    if (lane < topk) w[lane] = ex / sm;
+    if (lane == topk) w[topk] = 1.0f / (1.0f + expf(-__ldcg(lg + E)));
+}
+
+// Grouping of nb tokens' chosen experts (sid [token][MOE_MAXK]) by one block of NTH >= E threads: thread e owns expert e in the scans.
+template <int NTH, class SEL, int W>
+__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][MOE_MAXE]) {
+    __shared__ uint32_t pos[MOE_MAXE];
+    __shared__ uint32_t wsum[2][32];
+    constexpr uint32_t NW = NTH / 32;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // group by expert.  mask[e] = tokens that chose e; an entry's place inside its group is the number of
     //    earlier tokens in the mask, so groups are filled in token order without any serial scan.
     const uint32_t nent = a.nb * topk;
     for (uint32_t i = tid; i < nent; i += NTH) {
         const uint32_t t = i / topk, e = sid[t * MOE_MAXK + (i - t * topk)];
-        if (e >= a.e_lo && e < a.e_hi) atomicOr(t < 32 ? &mlo[e] : &mhi[e], 1u << (t & 31));
+        if (e >= a.e_lo && e < a.e_hi) atomicOr(&mask[t >> 5][e], 1u << (t & 31));
     }
     __syncthreads();
     {   // exclusive scans over experts (thread e = expert e): entries (low 16 bits of one word) and passes of 8 entries
         // (high 16 bits: what the gate/up and down kernels enumerate their work units by), and non-empty flags
-        const uint32_t c0 = tid < E ? __popc(mlo[tid]) + __popc(mhi[tid]) : 0, f = c0 ? 1u : 0u, c = c0 | (((c0 + 7) / 8) << 16);
+        uint32_t c0 = 0;
+        if (tid < E)
+#pragma unroll
+            for (int q = 0; q < W; q++) c0 += __popc(mask[q][tid]);
+        const uint32_t f = c0 ? 1u : 0u, c = c0 | (((c0 + 7) / 8) << 16);
         uint32_t sc = c, sf = f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -236,7 +235,6 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
         const uint32_t bc = warp ? wsum[0][warp - 1] : 0, bf = warp ? wsum[1][warp - 1] : 0;
         const uint32_t ex = bc + sc - c;  // exclusive prefix: entries | passes << 16
         pos[tid] = ex & 0xffffu;          // first entry of expert tid
-        grp[tid] = bf + sf - f;           // group number of expert tid (if non-empty)
         if (c0) {
             ms->ue[bf + sf - f] = tid;
             ms->off[bf + sf - f] = ex & 0xffffu;
@@ -254,11 +252,68 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
     for (uint32_t i = tid; i < nent; i += NTH) {
         const uint32_t t = i / topk, k = i - t * topk, e = sid[t * MOE_MAXK + k];
         if (e >= a.e_lo && e < a.e_hi) {
-            const uint32_t before = t < 32 ? __popc(mlo[e] & ((1u << t) - 1)) : __popc(mlo[e]) + __popc(mhi[e] & ((1u << (t - 32)) - 1));
+            uint32_t before = __popc(mask[t >> 5][e] & ((1u << (t & 31)) - 1));
+            for (uint32_t q = 0; q < t >> 5; q++) before += __popc(mask[q][e]);
             ms->ent[pos[e] + before] = (uint16_t)((t << 8) | k);
         }
     }
 }
+
+// Body of the selection of up to 64 tokens for one block of NTH threads.
+template <int NTH>
+__device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms, uint32_t E, uint32_t topk, sel_args a) {
+    __shared__ uint32_t mask[2][MOE_MAXE];  // token bit masks per expert
+    __shared__ uint16_t sid[MOE_MAXB * MOE_MAXK];
+    __shared__ uint64_t cand_s[NTH / 32][32 + MOE_MAXK];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    for (uint32_t e = tid; e < MOE_MAXE; e += NTH) mask[0][e] = mask[1][e] = 0;
+    for (uint32_t t = warp; t < a.nb; t += NTH / 32)
+        moe_topk_row(logits + (size_t)t * (E + 1), E, topk, tid & 31, cand_s[warp], ms->ids[t], sid + t * MOE_MAXK, ms->w[t]);
+    __syncthreads();
+    moe_group_body<NTH>(sid, ms, E, topk, a, mask);
+}
+
+// ---- a piece of a prompt (up to 256 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
+// part is moe_route with SELECT defined 0.  (In moe_route's one last block 256 tokens would be 16 rounds of top-k.)
+// moe_topk_wide binds: 0 = logits [nb][E+1], 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid ceil(nb/4) x 128
+__global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_sel_wide *ms, uint32_t E, uint32_t topk, uint32_t nb) {
+    __shared__ uint64_t cand_s[4][32 + MOE_MAXK];
+    pdl_sync();
+    const uint32_t warp = threadIdx.x >> 5, t = blockIdx.x * 4 + warp;
+    if (t < nb) moe_topk_row(logits + (size_t)t * (E + 1), E, topk, threadIdx.x & 31, cand_s[warp], t < MOE_MAXB ? ms->ids[t] : nullptr, ms->sid[t], ms->w[t]);
+}
+// moe_group_wide binds: 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid 1 x 512
+__global__ void __launch_bounds__(512) moe_group_wide_k(moe_sel_wide *ms, uint32_t E, uint32_t topk, sel_args a) {
+    __shared__ uint32_t mask[MOE_MAXB_WIDE / 32][MOE_MAXE];
+    pdl_launch();
+    for (uint32_t e = threadIdx.x; e < MOE_MAXE; e += 512)
+#pragma unroll
+        for (int q = 0; q < MOE_MAXB_WIDE / 32; q++) mask[q][e] = 0;
+    __syncthreads();
+    pdl_wait();
+    moe_group_body<512>(&ms->sid[0][0], (moe_sel_t<MOE_MAXB_WIDE> *)ms, E, topk, a, mask);
+}
+static bool moe_wide_check(const QwLaunch &L, const sel_args &a, uint32_t E, uint32_t topk) {
+    return L.buf<void>(1) && L.has_bytes(2, 12) && E % 32 == 0 && (E == 512 || E <= 256) && topk >= 1 && topk < MOE_MAXK && topk <= E && a.nb >= 1 &&
+           a.nb <= MOE_MAXB_WIDE && L.avail(1) >= sizeof(moe_sel_wide);
+}
+static cudaError_t launch_moe_topk_wide(const QwLaunch &L) {
+    const uint32_t E = (uint32_t)L.def("E", 512), topk = (uint32_t)L.def("TOPK", 10);
+    const sel_args a = L.bytes<sel_args>(2);
+    QW_CHECK_ARG(moe_wide_check(L, a, E, topk) && L.buf<void>(0) && L.avail(0) >= (size_t)a.nb * (E + 1) * 4);
+    qw_launch(moe_topk_wide_k, (a.nb + 3) / 4, 128, 0, L.stream, L.buf<float>(0), L.buf<moe_sel_wide>(1), E, topk, a.nb);
+    return cudaGetLastError();
+}
+QW_FAMILY(moe_topk_wide, launch_moe_topk_wide, 128)
+static cudaError_t launch_moe_group_wide(const QwLaunch &L) {
+    const uint32_t E = (uint32_t)L.def("E", 512), topk = (uint32_t)L.def("TOPK", 10);
+    sel_args a = L.bytes<sel_args>(2);
+    QW_CHECK_ARG(moe_wide_check(L, a, E, topk));
+    if (a.e_hi > E) a.e_hi = E;
+    qw_launch(moe_group_wide_k, 1, 512, 0, L.stream, L.buf<moe_sel_wide>(1), E, topk, a);
+    return cudaGetLastError();
+}
+QW_FAMILY(moe_group_wide, launch_moe_group_wide, 512)
 
 __global__ void __launch_bounds__(1024) moe_select_k(const float *logits, moe_sel *ms, uint32_t E, uint32_t topk, sel_args a) {
     pdl_sync();
@@ -286,11 +341,12 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // token kept the expert FFN's blocks from becoming resident early.)  64 tokens, 512 experts: 40.6 -> 26.7 us on a B200.
 // Up to four tokens -- one per warp at most -- are read straight from L2: staging them costs a copy's latency and saves nothing.
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
-// 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.
+// 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.  With SELECT defined 0 only the
+// logits are computed, of up to 256 tokens (binds 4 and 5 are not used).
 constexpr uint32_t ROUTE_PASS = 16, ROUTE_STG = 3;  // tokens per copy, copies in flight
 template <int D>
 __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, unsigned *counter, moe_sel *ms,
-                                                   uint32_t E, uint32_t topk, sel_args a, unsigned *status) {
+                                                   uint32_t E, uint32_t topk, sel_args a, bool select, unsigned *status) {
     constexpr int CH = D / 8 / 32;
     extern __shared__ __align__(128) uint8_t route_smem[];  // [ROUTE_STG][16 tokens][D] fp16
     __shared__ uint64_t full[ROUTE_STG];
@@ -380,6 +436,7 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
             }
         }
     }
+    if (!select) return;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -398,19 +455,20 @@ static cudaError_t moe_route_go(const QwLaunch &L, unsigned grid, uint32_t E, ui
     if (e != cudaSuccess) return e;
     const uint32_t held = a.nb <= 4 ? 0 : a.nb < ROUTE_STG * ROUTE_PASS ? a.nb : ROUTE_STG * ROUTE_PASS;
     qw_launch(moe_route_k<DD>, grid, 512, held * DD * 2, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), L.buf<unsigned>(4),
-              L.buf<moe_sel>(5), E, topk, a, (unsigned *)L.status);
+              L.buf<moe_sel>(5), E, topk, a, L.def("SELECT", 1) != 0, (unsigned *)L.status);
     return cudaGetLastError();
 }
 
 static cudaError_t launch_moe_route(const QwLaunch &L) {
     const uint32_t E = (uint32_t)L.def("E", 512), D = (uint32_t)L.def("D", 2048), topk = (uint32_t)L.def("TOPK", 10);
     sel_args a = L.bytes<sel_args>(14);
-    QW_CHECK_ARG(L.has_bytes(14, 12) && a.nb >= 1 && a.nb <= MOE_MAXB);
-    for (int i = 0; i <= 5; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+    const bool select = L.def("SELECT", 1) != 0;
+    QW_CHECK_ARG(L.has_bytes(14, 12) && a.nb >= 1 && a.nb <= (select ? MOE_MAXB : MOE_MAXB_WIDE));
+    for (int i = 0; i <= (select ? 5 : 3); i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
     QW_CHECK_ARG(((uintptr_t)L.buf<void>(0) & 15) == 0 && ((uintptr_t)L.buf<void>(1) & 15) == 0 && ((uintptr_t)L.buf<void>(2) & 15) == 0);
     QW_CHECK_ARG(E % 32 == 0 && (E == 512 || E <= 256) && topk >= 1 && topk < MOE_MAXK && topk <= E);  // E <= the block's 512 threads
     QW_CHECK_ARG(L.avail(0) >= (size_t)E * D * 2 && L.avail(1) >= (size_t)D * 2 && L.avail(2) >= (size_t)a.nb * D * 2 &&
-                 L.avail(3) >= (size_t)a.nb * (E + 1) * 4 && L.avail(4) >= 4 && L.avail(5) >= sizeof(moe_sel));
+                 L.avail(3) >= (size_t)a.nb * (E + 1) * 4 && (!select || (L.avail(4) >= 4 && L.avail(5) >= sizeof(moe_sel))));
     if (a.e_hi > E) a.e_hi = E;
     const unsigned grid = (E + 1 + 3) / 4;  // (the grid given by the host is ignored)
     if (D == 2048) return moe_route_go<2048>(L, grid, E, topk, a);
@@ -914,3 +972,4 @@ QW_FAMILY(moe_cmb, launch_moe_cmb, 256)
 
 // size of struct moe_sel for hosts that allocate it (bind 1 of moe_select)
 extern "C" size_t qw_moe_sel_bytes(void) { return sizeof(moe_sel); }
+extern "C" size_t qw_moe_sel_wide_bytes(void) { return sizeof(moe_sel_wide); }

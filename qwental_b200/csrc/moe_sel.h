@@ -8,17 +8,23 @@
 
 // Result of the selection, read by the gate/up, down and combine kernels (role of struct gg_sel,
 // kernels/moe_gg.metal:110-116).  Groups are in expert-id order; a group's entries are in token order.
-struct moe_sel {
+// MAXB = 64: a step.  MAXB = 256: a piece of a prompt; the fields up to w sit at the same offsets in both.
+template <int MAXB>
+struct moe_sel_t {
     uint32_t U;                               // groups (distinct experts in [e_lo, e_hi) that were chosen)
     uint32_t nb, topk, pad;
-    int32_t ids[MOE_MAXB][MOE_MAXK];          // chosen experts per token, rank order
-    float w[MOE_MAXB][MOE_MAXK + 1];          // routed weights, then the shared gate at [topk]
+    int32_t ids[MOE_MAXB][MOE_MAXK];          // chosen experts of the first 64 tokens, rank order
+    float w[MAXB][MOE_MAXK + 1];              // routed weights, then the shared gate at [topk]
     uint32_t ue[MOE_MAXE];                    // expert of group u
     uint32_t off[MOE_MAXE + 1];               // entries of group u: ent[off[u] .. off[u+1])
-    uint16_t ent[MOE_MAXB * MOE_MAXK];        // token << 8 | rank
+    uint16_t ent[MAXB * MOE_MAXK];            // token << 8 | rank
     uint32_t pre[MOE_MAXE + 2];               // passes of 8 entries in the groups before u (pre[U] = all routed passes)
 };
-
+typedef moe_sel_t<MOE_MAXB> moe_sel;
+#define MOE_MAXB_WIDE 256  // an entry keeps its token in 8 bits
+struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
+    uint16_t sid[MOE_MAXB_WIDE][MOE_MAXK];    // chosen experts of every token: from the top-k to the grouping
+};
 
 // Scratch buffer of the fused expert-FFN kernel (k_ffn.cu): the items' counters and the finished-block counter in the first
 // MOE_FFN_SYNC_BYTES (all zero between launches: the owner zeroes the buffer once), then H [item][2 planes][8 columns][I] fp16.
@@ -32,3 +38,8 @@ struct moe_sel {
 #define MOE_FFN_ROWCNT 1024
 #define MOE_FFN_ROW_DONE(D) ((D) / 128 * 8)
 #define MOE_FFN_SCRATCH_BYTES(I) ((size_t)MOE_FFN_SYNC_BYTES + (size_t)MOE_FFN_MAXITEMS * 16 * (I) * 2)
+// The same for a piece of a prompt of up to 256 tokens, in a buffer of its own: at most 512 + 256 x 15 / 8 + 32 items, 256 x 16 output rows.
+#define MOE_FFN_MAXITEMS_WIDE 1024
+#define MOE_FFN_ROWCNT_WIDE 2048
+#define MOE_FFN_SYNC_BYTES_WIDE 32768
+#define MOE_FFN_SCRATCH_BYTES_WIDE(I) ((size_t)MOE_FFN_SYNC_BYTES_WIDE + (size_t)MOE_FFN_MAXITEMS_WIDE * 16 * (I) * 2)

@@ -45,3 +45,24 @@ def test_prefill_equals_stepping_every_token(gpu, model):
                 assert np.array_equal(a, b), n
     finally:
         e.close()
+
+
+def test_wide_pieces_equal_stepping_every_token(gpu):
+    """Pieces of 65 to 256 tokens (512 experts, ten per token: several passes per expert and most experts chosen), at the edges of a piece,
+    of the groups of 64 rows inside it and of what is left for a second and third piece."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(experts=512, topk=10, max_slots=2))
+    try:
+        lengths = {65, 127, 192, 193, 255, 256, 257, 321, 512, 577}
+        text = np.random.default_rng(5).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
