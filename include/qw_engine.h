@@ -60,6 +60,9 @@ const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32_t *prompt,
 /* src/engine.h:91.  One decode step for B slots (sids distinct, 1 <= B <= QW_PAR_MAX): returns [B][vocab] fp32
  * logits in host-visible memory, valid until the next step; NULL on failure.  *gpu_ms = device time. */
 const float *qw_engine_par_step(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms);
+/* The same step with the logits copied to the caller's buffer [B][vocab] (any host memory; the copy is fastest into pinned memory,
+ * QW_BUF_HOSTIO).  0 or -1. */
+int qw_engine_par_step_into(qw_engine *e, const int *sids, const int32_t *toks, int B, float *logits, double *gpu_ms);
 /* The same step with the arg-max fused on the device (ties -> lowest id, as src/engine.c:6144-6148):
  * returns B token ids in host-visible memory; logits are not copied to the host. */
 const int32_t *qw_engine_par_step_greedy(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms);

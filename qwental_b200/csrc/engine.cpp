@@ -409,7 +409,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->qb, RB * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
          new_buf(e, &e->ya, RB * e->KA * 2) && new_buf(e, &e->ob, RB * e->D * 2) && new_buf(e, &e->mo, B * e->D * 2) &&
          new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids, B * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
-         new_buf(e, &e->logits_h, B * (size_t)e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
+         new_buf(e, &e->logits_h, (size_t)c.max_slots * e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
          new_buf(e, &e->msel, (size_t)e->L * e->sel_bytes) && new_buf(e, &e->Hhi, B * (e->TOPK + 1) * e->I * 2) &&
          new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, RB * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
     if (ok) ok = qw_buf_zero(g, &e->msel, 0, e->msel.size) && qw_buf_zero(g, &e->Pg, 0, e->Pg.size) && qw_buf_zero(g, &e->Hhi, 0, e->Hhi.size) &&
@@ -948,19 +948,27 @@ void after_failed_step(qw_engine *e) {
 
 }  // namespace
 
-extern "C" const float *qw_engine_par_step(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms) {
+extern "C" int qw_engine_par_step_into(qw_engine *e, const int *sids, const int32_t *toks, int B, float *logits, double *gpu_ms) {
     const double t0 = qw_now();
+    if (e && !logits) return e->fail("par_step: no buffer for the logits"), -1;
     const uint32_t mc = begin_step(e, sids, toks, B, 1);
-    if (!mc) return nullptr;
+    if (!mc) return -1;
     qw_batch *b = qw_batch_begin(e->g, false);
     encode_step(e, b, (uint32_t)B, mc, true, 0);
     const double secs = qw_batch_end(b);
-    if (secs < 0) return after_failed_step(e), e->fail("par_step: device batch failed"), nullptr;
-    for (int j = 0; j < B; j++)  // device row j is the caller's row perm[j]
-        if (!qw_buf_download(e->g, &e->logits, (size_t)j * e->V * 4, (float *)e->logits_h.ptr + (size_t)e->perm[j] * e->V, (size_t)e->V * 4))
-            return e->fail("par_step: logits copy failed"), nullptr;
+    if (secs < 0) return after_failed_step(e), e->fail("par_step: device batch failed"), -1;
+    for (int j = 0, n; j < B; j += n) {  // device row j is the caller's row perm[j]: runs of consecutive rows travel together
+        for (n = 1; j + n < B && e->perm[j + n] == e->perm[j] + n; n++) {}
+        if (!qw_buf_download(e->g, &e->logits, (size_t)j * e->V * 4, logits + (size_t)e->perm[j] * e->V, (size_t)n * e->V * 4))
+            return e->fail("par_step: logits copy failed"), -1;
+    }
     if (gpu_ms) *gpu_ms = secs * 1e3;
     end_step(e, sids, B, 1, (qw_now() - t0) * 1e3);
+    return 0;
+}
+
+extern "C" const float *qw_engine_par_step(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms) {
+    if (!e || qw_engine_par_step_into(e, sids, toks, B, (float *)e->logits_h.ptr, gpu_ms) != 0) return nullptr;
     return (const float *)e->logits_h.ptr;
 }
 

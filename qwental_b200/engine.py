@@ -8,7 +8,7 @@ from dataclasses import dataclass
 import numpy as np
 
 from . import lib as _lib
-from .gpu import Gpu, GpuError
+from .gpu import HOSTIO, Gpu, GpuError
 
 
 class ModelCfg(C.Structure):
@@ -30,6 +30,7 @@ def _bind(L):
         "qw_engine_par_slots": (C.c_int, [vp]), "qw_engine_par_pick": (C.c_int, [vp, i32p, C.c_int, C.c_ulonglong]),
         "qw_engine_par_seed": (C.c_int, [vp, C.c_int, C.c_int, C.c_ulonglong]),
         "qw_engine_par_step": (C.POINTER(C.c_float), [vp, ip, i32p, C.c_int, C.POINTER(C.c_double)]),
+        "qw_engine_par_step_into": (C.c_int, [vp, vp, vp, C.c_int, vp, vp]),
         "qw_engine_par_step_greedy": (i32p, [vp, ip, i32p, C.c_int, C.POINTER(C.c_double)]),
         "qw_engine_par_decode_greedy": (C.c_int, [vp, ip, i32p, C.c_int, C.c_int, i32p, C.POINTER(C.c_double)]),
         "qw_engine_par_finish": (None, [vp, C.c_int, i32p, C.c_int]), "qw_engine_par_cost": (C.c_double, [vp, C.c_int]),
@@ -88,6 +89,53 @@ def wide_cfg(**over) -> ModelCfg:
     return default_cfg(**base)
 
 
+class _HostRows:
+    """Pinned host buffers for a step's logits [rows][cols].  The device copies into one and `Engine.step` hands it out as an array; it
+    comes back when the array and every view of it are gone.  Copying the rows out of one fixed buffer into fresh pages instead cost as
+    much as half of the device's step for a full server: 64 x 151936 logits are 39 MB.  At most KEEP buffers exist; a caller who holds
+    more results than that gets copies."""
+
+    KEEP = 3
+    SMALL = 1 << 17  # below this many bytes a copy is cheaper than the bookkeeping
+
+    def __init__(self, gpu: Gpu, rows: int, cols: int):
+        self.gpu, self.cols, self.size, self.made, self.free = gpu, cols, rows * cols * 4, 0, []
+        if self.size >= self.SMALL:  # two to begin with: a loop's next step runs while the last one's logits are still held
+            self.free = [b for b in (self._make(), self._make()) if b]
+
+    def _make(self):
+        try:
+            b = self.gpu.buf(self.size, HOSTIO)
+        except GpuError:
+            return None
+        self.made += 1
+        return b
+
+    def lease(self, rows: int):
+        if rows * self.cols * 4 < self.SMALL or self.free is None:
+            return None
+        try:
+            b = self.free.pop()
+        except IndexError:
+            b = self._make() if self.made < self.KEEP else None
+        return _Lease(self, b, (rows, self.cols)) if b else None
+
+    def close(self):  # what is handed out is freed with its array
+        self.made, self.free = self.KEEP, None
+
+
+class _Lease:
+    """The owner of an array over a buffer of _HostRows."""
+
+    def __init__(self, pool: _HostRows, buf, shape):
+        self.pool, self.buf = pool, buf
+        self.__array_interface__ = dict(shape=shape, typestr="<f4", data=(buf.b.ptr, False), version=3)
+
+    def __del__(self):
+        if self.pool.free is not None:
+            self.pool.free.append(self.buf)
+
+
 class Engine:
     def __init__(self, gpu: Gpu, cfg: ModelCfg):
         self.L = gpu.L
@@ -96,6 +144,7 @@ class Engine:
         self.e = self.L.qw_engine_open_synth(gpu.g, C.byref(cfg))
         if not self.e:
             raise GpuError("qw_engine_open_synth: " + self.L.qw_engine_error(None).decode())
+        self._host = _HostRows(gpu, cfg.max_slots, cfg.vocab)
 
     def error(self) -> str:
         return self.L.qw_engine_error(self.e).decode()
@@ -121,9 +170,14 @@ class Engine:
         return s, t
 
     def step(self, sids, toks):
-        """One decode step: fp32 logits [B][vocab] (copied out of the engine's host buffer) and device ms."""
+        """One decode step: fp32 logits [B][vocab] (an array of the caller's own) and device ms."""
         s, t = self._rows(sids, toks)
         ms = C.c_double()
+        own = self._host.lease(len(s)) if len(s) <= self.cfg.max_slots else None
+        if own:
+            if self.L.qw_engine_par_step_into(self.e, s.ctypes.data, t.ctypes.data, len(s), own.buf.b.ptr, C.addressof(ms)) != 0:
+                raise GpuError("par_step: " + self.error())
+            return np.asarray(own), ms.value
         p = self.L.qw_engine_par_step(self.e, s.ctypes.data_as(C.POINTER(C.c_int)), t.ctypes.data_as(C.POINTER(C.c_int32)), len(s), C.byref(ms))
         if not p:
             raise GpuError("par_step: " + self.error())
@@ -215,6 +269,7 @@ class Engine:
 
     def close(self):
         if self.e:
+            self._host.close()
             self.L.qw_engine_close(self.e)
             self.e = None
 

@@ -260,3 +260,27 @@ def test_benchmark_engine_full_depth_batched_equals_alone_and_graph_replay(gpu):
         assert np.array_equal(lg.view(np.uint32), lb.view(np.uint32))
     finally:
         e.close()
+
+
+def test_step_logits_belong_to_the_caller(gpu):
+    """Logits of earlier steps keep their values while they (or views of them) are held, however many; they outlive the engine."""
+    from qwental_b200.engine import Engine, _HostRows, tiny_cfg
+    cfg = tiny_cfg(vocab=8192)
+    assert 8 * cfg.vocab * 4 >= _HostRows.SMALL > cfg.vocab * 4
+    a, b = Engine(gpu, cfg), Engine(gpu, cfg)
+    for e in (a, b):
+        for s in range(8):
+            e.seed_slot(s, 20 + s, 100 + s)
+    rng = np.random.default_rng(6)
+    held, want = [], []
+    for k in range(8):
+        rows = list(range(8)) if k % 3 else [5]
+        toks = rng.integers(0, cfg.vocab, len(rows)).astype(np.int32)
+        lg, _ = a.step(rows, toks)
+        assert lg.flags.writeable and lg.flags.c_contiguous and lg.dtype == np.float32 and lg.shape == (len(rows), cfg.vocab)
+        held.append(lg[1:] if len(rows) > 1 else lg)
+        want.append(b.step(rows, toks)[0][-len(held[-1]):].copy())  # given back at once: the next step reuses its buffer
+    a.close()
+    for x, y in zip(held, want):
+        assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
+    b.close()
