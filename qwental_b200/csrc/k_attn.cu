@@ -224,23 +224,30 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
-constexpr int AT_WARP_BYTES = 16384;  // per warp: K tile 8 KB + V tile 8 KB (4 swizzled boxes of 16 rows x 128 B each)
+// STG = 1: one tile of K and one of V per warp and three blocks per SM -- many warps hide one another's copies.  STG = 3, for launches with
+// no more tasks than one block per SM has warps: nobody else hides a warp's copies then, and with one tile in flight each of a page's 16
+// steps waited a whole memory latency (1.3 us); three tiles of both in a ring.  One slot of 25000 tokens, 48 layers on a B200: 3.07 -> 2.97 ms per
+// step; five slots of up to 12000 tokens (at most 470 tasks) and one of 1000 tokens within 1 %.
+constexpr int AT_TILE_BYTES = 16384;  // K tile 8 KB + V tile 8 KB (4 swizzled boxes of 16 rows x 128 B each)
 constexpr int AT_TAB_BYTES = 1024;    // per block: first task of every slot [65], tokens [64], slot id [64]
-constexpr int AT_SMEM = 4 * AT_WARP_BYTES + 64 + AT_TAB_BYTES + 1024;
-constexpr int AT_BLOCKS_PER_SM = 3;   // what the shared memory and the registers of the kernel allow
+constexpr int AT_FEW_STG = 3;
+constexpr int at_smem(int stg) { return 4 * stg * AT_TILE_BYTES + 128 + AT_TAB_BYTES + 1024; }
+constexpr int at_blocks_per_sm(int stg) { return stg == 1 ? 3 : 1; }  // what the shared memory and the registers of the kernel allow
 
+template <int STG>
 __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CUtensorMap tm, const __half *q, const int32_t *pt, const int32_t *posv,
                                                       const int32_t *sids, float *part, qsa_args a, uint32_t QH, uint32_t KVH, unsigned *status) {
     constexpr uint32_t HD = 256;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // swizzled boxes need 1024-byte alignment
-    uint8_t *Kb = smem + warp * AT_WARP_BYTES, *Vb = Kb + 8192;
-    uint64_t *bars = (uint64_t *)(smem + 4 * AT_WARP_BYTES) + warp * 2;
-    uint32_t *first = (uint32_t *)(smem + 4 * AT_WARP_BYTES + 64), *ntokv = first + 65, *sidv = ntokv + 64;
+    uint8_t *Kb = smem + warp * STG * AT_TILE_BYTES, *Vb = Kb + 8192;
+    constexpr int NBAR = STG == 1 ? 2 : STG;  // STG = 1: K and V on their own; else one per tile pair
+    uint64_t *bars = (uint64_t *)(smem + 4 * STG * AT_TILE_BYTES) + warp * NBAR;
+    uint32_t *first = (uint32_t *)(smem + 4 * STG * AT_TILE_BYTES + 128), *ntokv = first + 65, *sidv = ntokv + 64;
     if (lane == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+#pragma unroll
+        for (int k = 0; k < NBAR; k++) mbar_init(&bars[k], 1);
         mbar_init_fence();
     }
     pdl_sync();
@@ -306,12 +313,38 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
     const int vrows = (int)(KVH * QSA_PAGE);  // rows from a page's K tile to its V tile
     uint32_t kph = 0, vph = 0;  // copies waited for so far on the K / V barrier (their parity selects the phase)
     bool ok = true;
-    uint32_t i = blockIdx.x * 4 + warp;
+    uint32_t i = STG == 1 ? blockIdx.x * 4 + warp : warp * gridDim.x + blockIdx.x;  // (few tasks go to different SMs first)
     Task cur{};
+    // STG > 1: the ring is fed tile by tile over the warp's tasks, STG tiles ahead of the one in work (tile number n of the warp)
+    uint32_t n = 0, fi = i, fs = 0;
+    Task ft{};
+    auto feed = [&](uint32_t at) {
+        if (fi >= tasks) return;
+        const uint32_t st = at % STG;
+        if (lane == 0) {
+            fence_proxy_async();  // the warp's reads of the stage (ordered by __syncwarp) before the async-proxy writes
+            mbar_expect_tx(&bars[st], AT_TILE_BYTES);
+#pragma unroll
+            for (int db = 0; db < 4; db++) {
+                tma_load_2d(Kb + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + (int)fs * 16, &bars[st]);
+                tma_load_2d(Vb + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + vrows + (int)fs * 16, &bars[st]);
+            }
+        }
+        if (++fs == (ft.n + 15) / 16) {
+            fs = 0;
+            fi += W;
+            if (fi < tasks) ft = task_of(fi);
+        }
+    };
     if (i < tasks) {
         cur = task_of(i);
-        load(Kb, &bars[0], cur.rowK);
-        load(Vb, &bars[1], cur.rowK + vrows);
+        if (STG == 1) {
+            load(Kb, &bars[0], cur.rowK);
+            load(Vb, &bars[1], cur.rowK + vrows);
+        } else {
+            ft = cur;
+            for (uint32_t k = 0; k < STG; k++) feed(k);
+        }
     }
     while (i < tasks && ok) {
         const uint32_t steps = (cur.n + 15) / 16;
@@ -335,18 +368,21 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
         for (int dt = 0; dt < 16; dt++) o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f;
         float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
         for (uint32_t step = 0; step < steps; step++) {
-            if (!mbar_wait(&bars[0], kph & 1)) { ok = false; break; }
+            const uint32_t so = STG == 1 ? 0 : n % STG * AT_TILE_BYTES;
+            if (!(STG == 1 ? mbar_wait(&bars[0], kph & 1) : mbar_wait(&bars[n % STG], n / STG & 1))) { ok = false; break; }
             kph++;
             float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int ks = 0; ks < 16; ks++) {
                 uint32_t af[4];
-                ldsm_x4(af, kbase + (ks >> 2) * 2048 + ((((ks & 3) * 2 + (mi >> 1)) ^ r8) << 4));
+                ldsm_x4(af, kbase + so + (ks >> 2) * 2048 + ((((ks & 3) * 2 + (mi >> 1)) ^ r8) << 4));
                 mma_f16(s, af, qf[ks][0], qf[ks][1], s);
             }
-            __syncwarp();
-            if (step + 1 < steps) load(Kb, &bars[0], cur.rowK + (int)(step + 1) * 16);
-            else if (more) load(Kb, &bars[0], nxt.rowK);
+            if (STG == 1) {
+                __syncwarp();
+                if (step + 1 < steps) load(Kb, &bars[0], cur.rowK + (int)(step + 1) * 16);
+                else if (more) load(Kb, &bars[0], nxt.rowK);
+            }
             const uint32_t ta = step * 16 + g;
             if (ta >= cur.n) s[0] = s[1] = -INFINITY;
             if (ta + 8 >= cur.n) s[2] = s[3] = -INFINITY;
@@ -383,17 +419,24 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
                 return __byte_perm(__shfl_sync(0xffffffffu, u, srcA), __shfl_sync(0xffffffffu, u, srcB), sel);
             };
             const uint32_t b0 = to_b(h01), b1 = to_b(h23), c0 = to_b(r01), c1 = to_b(r23);
-            if (!mbar_wait(&bars[1], vph & 1)) { ok = false; break; }
+            if (STG == 1 && !mbar_wait(&bars[1], vph & 1)) { ok = false; break; }
             vph++;
+            // four dim tiles at a time: the two MMAs of a tile depend on one another, back to back the second would wait for the first
 #pragma unroll
-            for (int dt = 0; dt < 16; dt++) {
-                uint32_t af[4];
-                ldsm_x4_t(af, vbase + (dt >> 2) * 2048 + ((((dt & 3) * 2 + (mi & 1)) ^ r8) << 4));
-                mma_f16(o[dt], af, b0, b1, o[dt]);
-                mma_f16(o[dt], af, c0, c1, o[dt]);
+            for (int dq = 0; dq < 4; dq++) {
+                uint32_t af[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) ldsm_x4_t(af[j], vbase + so + dq * 2048 + (((j * 2 + (mi & 1)) ^ r8) << 4));
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f16(o[4 * dq + j], af[j], b0, b1, o[4 * dq + j]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f16(o[4 * dq + j], af[j], c0, c1, o[4 * dq + j]);
             }
             __syncwarp();
-            if (step + 1 < steps) load(Vb, &bars[1], cur.rowK + vrows + (int)(step + 1) * 16);
+            if (STG > 1) {
+                feed(n + STG);
+                n++;
+            } else if (step + 1 < steps) load(Vb, &bars[1], cur.rowK + vrows + (int)(step + 1) * 16);
             else if (more) load(Vb, &bars[1], nxt.rowK + vrows);
         }
         if (!ok) break;
@@ -456,6 +499,19 @@ static const CUtensorMap *attn_tensor_map(void *pool, size_t bytes) {
     return &(cache[key] = tm);
 }
 
+// Persistent: as many blocks as fit on the device at once, or fewer when the step cannot have that many tasks.  most = the most tasks the
+// launch can have (slots x chunks x kv heads); with up to one per warp of a block on every SM the deep ring is the faster form.
+struct AttnLaunch {
+    decltype(&qsa_attn_mma_k<1>) k;
+    uint32_t grid;
+    int smem;
+};
+static AttnLaunch attn_launch(uint32_t most, uint32_t sms) {
+    if (most <= 4 * sms) return {qsa_attn_mma_k<AT_FEW_STG>, most < sms ? most : sms, at_smem(AT_FEW_STG)};
+    const uint32_t blocks = (most + 3) / 4, cap = sms * at_blocks_per_sm(1);
+    return {qsa_attn_mma_k<1>, blocks < cap ? blocks : cap, at_smem(1)};
+}
+
 static cudaError_t launch_qsa_attn_mma(const QwLaunch &L) {
     uint32_t QH, KVH, HD;
     QW_CHECK_ARG(qsa_dims(L, QH, KVH, HD));
@@ -466,13 +522,10 @@ static cudaError_t launch_qsa_attn_mma(const QwLaunch &L) {
     QW_CHECK_ARG(((uintptr_t)L.buf<void>(1) & 15) == 0 && L.avail(1) >= 512 && L.avail(1) / 512 < 0x7fffffffull);
     const CUtensorMap *tm = attn_tensor_map(L.buf<void>(1), L.avail(1) / 512 * 512);
     QW_CHECK_ARG(tm != nullptr);
-    const size_t smem = AT_SMEM;
-    cudaError_t e = cudaFuncSetAttribute(qsa_attn_mma_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const AttnLaunch at = attn_launch(a.nb * a.max_chunks * KVH, (uint32_t)L.sm_count);
+    const cudaError_t e = cudaFuncSetAttribute(at.k, cudaFuncAttributeMaxDynamicSharedMemorySize, at.smem);
     if (e != cudaSuccess) return e;
-    // persistent: as many blocks as fit on the device at once, or fewer when the step cannot have that many tasks
-    const uint32_t most = (a.nb * a.max_chunks * KVH + 3) / 4, cap = (uint32_t)L.sm_count * AT_BLOCKS_PER_SM;
-    qw_launch(qsa_attn_mma_k, most < cap ? most : cap, 128, smem, L.stream, *tm, L.buf<__half>(0), L.buf<int32_t>(2), L.buf<int32_t>(3),
-                                                                          L.buf<int32_t>(4), L.buf<float>(5), a, QH, KVH, L.status);
+    qw_launch(at.k, at.grid, 128, at.smem, L.stream, *tm, L.buf<__half>(0), L.buf<int32_t>(2), L.buf<int32_t>(3), L.buf<int32_t>(4), L.buf<float>(5), a, QH, KVH, L.status);
     return cudaGetLastError();
 }
 QW_FAMILY(qsa_attn, launch_qsa_attn_mma, 128)
@@ -602,14 +655,13 @@ extern "C" int qw_attn_decode_static(const void *q, const void *kv_pool, size_t 
     CUtensorMap tm;  // encoded on the stack: no allocation
     if (!attn_encode_map(&tm, kv_pool, kv_pool_bytes / 512 * 512)) return fail(-3, "tensor map encoding failed");
     qsa_args a = {nb, layer, nlayers, qkv_stride, max_pages, max_chunks, 0, 0};
-    const size_t smem = AT_SMEM;
-    cudaError_t e = cudaFuncSetAttribute(qsa_attn_mma_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fail(-3, cudaGetErrorString(e));
     cudaStream_t st = (cudaStream_t)stream;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return fail(-3, "cannot read the SM count");
-    const uint32_t most = (nb * max_chunks * KVH + 3) / 4, cap = (uint32_t)sms * AT_BLOCKS_PER_SM;
-    qsa_attn_mma_k<<<most < cap ? most : cap, 128, smem, st>>>(tm, (const __half *)q, page_table, pos, slot_ids, part, a, QH, KVH, nullptr);
+    const AttnLaunch at = attn_launch(nb * max_chunks * KVH, (uint32_t)sms);
+    cudaError_t e = cudaFuncSetAttribute(at.k, cudaFuncAttributeMaxDynamicSharedMemorySize, at.smem);
+    if (e != cudaSuccess) return fail(-3, cudaGetErrorString(e));
+    at.k<<<at.grid, 128, at.smem, st>>>(tm, (const __half *)q, page_table, pos, slot_ids, part, a, QH, KVH, nullptr);
     qsa_merge_k<<<dim3(QH, nb), 512, 0, st>>>(part, (const __half *)qkv, (__half *)y, pos, a, QH);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(-3, cudaGetErrorString(e));

@@ -193,3 +193,14 @@ def test_gdn_batched_equals_alone(gpu):
         sid = d["sids"][r]
         assert np.array_equal(gya[0].view(np.uint16), gy[r].view(np.uint16))
         assert np.array_equal(Sa[sid, 1].view(np.uint32), S[sid, 1].view(np.uint32))
+
+
+def test_attention_core_forms_agree(gpu):
+    """40 slots x 9 chunks are more tasks than the deep-ring form of the core takes, a slot alone is few: the same bits from both, at context
+    lengths around its 16-token tiles, its ring of three of them and a page."""
+    lens = [0, 1, 14, 15, 16, 31, 32, 33, 47, 48, 49, 63, 64, 65, 79, 80, 81, 239, 240, 241, 254, 255, 256, 257, 271, 272, 273, 303, 304, 305,
+            511, 512, 513, 700, 1023, 1024, 1025, 1500, 2047, 2049]
+    core, d = attn_setup(gpu, lens, seed=40)
+    y = attn_run(gpu, core, d, range(len(lens)))
+    for r in range(len(lens)):
+        assert np.array_equal(attn_run(gpu, core, d, [r])[0].view(np.uint16), y[r].view(np.uint16)), lens[r]
