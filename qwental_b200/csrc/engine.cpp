@@ -92,7 +92,7 @@ struct qw_engine {
     // scratch
     qw_buf ctl_h{}, ctl_d{}, h{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
-    // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN.  Four times the tokens choose far fewer than four times the
+    // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN.  Eight times the tokens choose far fewer than eight times the
     // experts, so a wider piece reads and decodes fewer expert weights per token.
     int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
     qw_buf ctl_p{}, ffn_scr_w{};
@@ -1112,8 +1112,9 @@ extern "C" int qw_engine_par_step_sample(qw_engine *e, const int *sids, const in
 // Prompt processing for one slot (src/engine.h:81), from an empty slot -- recurrent and conv state zero, no KV.  The prompt runs in
 // pieces of up to piece_rows tokens, each one pass over the weights, submitted back to back; a token's arithmetic is that of the decode
 // step, so "prefill then step" equals stepping every token, bit for bit.  (There is no prefix cache: *cached = 0.)
-// Measured on a B200: 48 layers, 419 tokens 1206 ms one token at a time, 81.2 ms in pieces of 64, 50.6 ms in pieces of 256; 12 layers, 1700 tokens
-// 80.0 -> 46.8 ms.  64 tokens choose about 370 of 512 experts, 256 nearly all: per token a quarter of the weights is left to decode.
+// Measured on a B200 for pieces of up to 1, 64, 256 and 512 tokens: 48 layers, 419 tokens 1206, 81.2, 50.0 and 43.3 ms; 12 layers, 1700 tokens
+// 1362, 80.0, 46.7 and 41.9 ms.  64 tokens choose about 370 of 512 experts, 256 nearly all; from there on fuller passes of eight
+// tokens per expert are what a wider piece still gains.
 extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32_t *prompt, int np, int *cached) {
     if (cached) *cached = 0;
     if (!e || sid < 0 || sid >= (int)e->slots.size() || !prompt || np < 1 || np >= e->c.max_ctx) return e ? (e->fail("par_prefill: bad arguments"), nullptr) : nullptr;

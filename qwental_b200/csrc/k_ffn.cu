@@ -135,8 +135,8 @@ __device__ __forceinline__ void ffn_entry(const SEL *ms, const FfnItem &it, uint
         rank = topk;
     } else {
         const uint32_t en = ms->ent[it.e0 + it.c0 + col];
-        tok = en >> 8;
-        rank = en & 255;
+        tok = en >> SEL::TOK;
+        rank = en & ((1u << SEL::TOK) - 1);
     }
 }
 
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
     uint32_t items = pre[U] + (p.Sd ? (nb + 7) / 8 : 0);
-    if (items > Rec::MAXITEMS) {  // cannot happen with E <= 512 and 64 (256) tokens; never index past the flags
+    if (items > Rec::MAXITEMS) {  // cannot happen with E <= 512 and 64 (512) tokens; never index past the flags
         if (tid == 0) set_status(p.status, ST_BAD_ARG | 5);
         items = 0;
     }
@@ -783,7 +783,7 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     p.Wd = L.buf<uint8_t>(6);
     p.Wg = Wg;
     p.Sg = Sg;
-    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 256 rows of tokens (one GPU only)
+    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 512 rows of tokens (one GPU only)
     const bool wide = L.def("WIDE", 0) != 0;
     p.sync = L.buf<unsigned>(8);
     QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I) : MOE_FFN_SCRATCH_BYTES(I)));

@@ -192,8 +192,8 @@ __device__ __forceinline__ void moe_topk_row(const float *lg, uint32_t E, uint32
 }
 
 // Grouping of nb tokens' chosen experts (sid [token][MOE_MAXK]) by one block of NTH >= E threads: thread e owns expert e in the scans.
-template <int NTH, class SEL, int W>
-__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][MOE_MAXE]) {
+template <int NTH, class SEL, int W, int ME>
+__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][ME]) {
     __shared__ uint32_t pos[MOE_MAXE];
     __shared__ uint32_t wsum[2][32];
     constexpr uint32_t NW = NTH / 32;
@@ -254,7 +254,7 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
         if (e >= a.e_lo && e < a.e_hi) {
             uint32_t before = __popc(mask[t >> 5][e] & ((1u << (t & 31)) - 1));
             for (uint32_t q = 0; q < t >> 5; q++) before += __popc(mask[q][e]);
-            ms->ent[pos[e] + before] = (uint16_t)((t << 8) | k);
+            ms->ent[pos[e] + before] = (uint16_t)((t << SEL::TOK) | k);
         }
     }
 }
@@ -273,8 +273,8 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
     moe_group_body<NTH>(sid, ms, E, topk, a, mask);
 }
 
-// ---- a piece of a prompt (up to 256 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
-// part is moe_route with SELECT defined 0.  (In moe_route's one last block 256 tokens would be 16 rounds of top-k.)
+// ---- a piece of a prompt (up to 512 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
+// part is moe_route with SELECT defined 0.  (In moe_route's one last block 512 tokens would be 32 rounds of top-k.)
 // moe_topk_wide binds: 0 = logits [nb][E+1], 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid ceil(nb/4) x 128
 __global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_sel_wide *ms, uint32_t E, uint32_t topk, uint32_t nb) {
     __shared__ uint64_t cand_s[4][32 + MOE_MAXK];
@@ -284,11 +284,10 @@ __global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_
 }
 // moe_group_wide binds: 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid 1 x 512
 __global__ void __launch_bounds__(512) moe_group_wide_k(moe_sel_wide *ms, uint32_t E, uint32_t topk, sel_args a) {
-    __shared__ uint32_t mask[MOE_MAXB_WIDE / 32][MOE_MAXE];
+    __shared__ uint32_t mask[MOE_MAXB_WIDE / 32][512];  // (E <= 512)
     pdl_launch();
-    for (uint32_t e = threadIdx.x; e < MOE_MAXE; e += 512)
 #pragma unroll
-        for (int q = 0; q < MOE_MAXB_WIDE / 32; q++) mask[q][e] = 0;
+    for (int q = 0; q < MOE_MAXB_WIDE / 32; q++) mask[q][threadIdx.x] = 0;
     __syncthreads();
     pdl_wait();
     moe_group_body<512>(&ms->sid[0][0], (moe_sel_t<MOE_MAXB_WIDE> *)ms, E, topk, a, mask);
@@ -342,7 +341,7 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // Up to four tokens -- one per warp at most -- are read straight from L2: staging them costs a copy's latency and saves nothing.
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
 // 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.  With SELECT defined 0 only the
-// logits are computed, of up to 256 tokens (binds 4 and 5 are not used).
+// logits are computed, of up to 512 tokens (binds 4 and 5 are not used).
 constexpr uint32_t ROUTE_PASS = 16, ROUTE_STG = 3;  // tokens per copy, copies in flight
 template <int D>
 __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, unsigned *counter, moe_sel *ms,

@@ -8,7 +8,7 @@
 
 // Result of the selection, read by the gate/up, down and combine kernels (role of struct gg_sel,
 // kernels/moe_gg.metal:110-116).  Groups are in expert-id order; a group's entries are in token order.
-// MAXB = 64: a step.  MAXB = 256: a piece of a prompt; the fields up to w sit at the same offsets in both.
+// MAXB = 64: a step.  MAXB = 512: a piece of a prompt; the fields up to w sit at the same offsets in both.
 template <int MAXB>
 struct moe_sel_t {
     uint32_t U;                               // groups (distinct experts in [e_lo, e_hi) that were chosen)
@@ -17,11 +17,12 @@ struct moe_sel_t {
     float w[MAXB][MOE_MAXK + 1];              // routed weights, then the shared gate at [topk]
     uint32_t ue[MOE_MAXE];                    // expert of group u
     uint32_t off[MOE_MAXE + 1];               // entries of group u: ent[off[u] .. off[u+1])
-    uint16_t ent[MAXB * MOE_MAXK];            // token << 8 | rank
+    static constexpr int TOK = MAXB > 256 ? 4 : 8;  // bits of an entry below its token
+    uint16_t ent[MAXB * MOE_MAXK];            // token << TOK | rank
     uint32_t pre[MOE_MAXE + 2];               // passes of 8 entries in the groups before u (pre[U] = all routed passes)
 };
 typedef moe_sel_t<MOE_MAXB> moe_sel;
-#define MOE_MAXB_WIDE 256  // an entry keeps its token in 8 bits
+#define MOE_MAXB_WIDE 512
 struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
     uint16_t sid[MOE_MAXB_WIDE][MOE_MAXK];    // chosen experts of every token: from the top-k to the grouping
 };
@@ -38,8 +39,8 @@ struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
 #define MOE_FFN_ROWCNT 1024
 #define MOE_FFN_ROW_DONE(D) ((D) / 128 * 8)
 #define MOE_FFN_SCRATCH_BYTES(I) ((size_t)MOE_FFN_SYNC_BYTES + (size_t)MOE_FFN_MAXITEMS * 16 * (I) * 2)
-// The same for a piece of a prompt of up to 256 tokens, in a buffer of its own: at most 512 + 256 x 15 / 8 + 32 items, 256 x 16 output rows.
-#define MOE_FFN_MAXITEMS_WIDE 1024
-#define MOE_FFN_ROWCNT_WIDE 2048
-#define MOE_FFN_SYNC_BYTES_WIDE 32768
+// The same for a piece of a prompt of up to 512 tokens, in a buffer of its own: at most 512 + 512 x 15 / 8 + 64 items, 512 x 16 output rows.
+#define MOE_FFN_MAXITEMS_WIDE 1600
+#define MOE_FFN_ROWCNT_WIDE 4096
+#define MOE_FFN_SYNC_BYTES_WIDE 65536
 #define MOE_FFN_SCRATCH_BYTES_WIDE(I) ((size_t)MOE_FFN_SYNC_BYTES_WIDE + (size_t)MOE_FFN_MAXITEMS_WIDE * 16 * (I) * 2)

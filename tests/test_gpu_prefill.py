@@ -48,12 +48,12 @@ def test_prefill_equals_stepping_every_token(gpu, model):
 
 
 def test_wide_pieces_equal_stepping_every_token(gpu):
-    """Pieces of 65 to 256 tokens (512 experts, ten per token: several passes per expert and most experts chosen), at the edges of a piece,
+    """Pieces of 65 to 512 tokens (512 experts, ten per token: several passes per expert and most experts chosen), at the edges of a piece,
     of the groups of 64 rows inside it and of what is left for a second and third piece."""
     from qwental_b200.engine import Engine, wide_cfg
     e = Engine(gpu, wide_cfg(experts=512, topk=10, max_slots=2))
     try:
-        lengths = {65, 127, 192, 193, 255, 256, 257, 321, 512, 577}
+        lengths = {65, 127, 192, 193, 255, 256, 257, 321, 511, 512, 513, 577}
         text = np.random.default_rng(5).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
         e.prefill(0, text[:1])  # slot 0 steps every token
         for n in range(2, max(lengths) + 1):
