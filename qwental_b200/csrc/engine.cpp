@@ -90,7 +90,7 @@ struct qw_engine {
     std::vector<int> free_pages;
     unsigned long long clock = 0;
     // scratch
-    qw_buf ctl_h{}, ctl_d{}, h{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
+    qw_buf ctl_h{}, ctl_d{}, h{}, h2{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
     // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN.  Eight times the tokens choose far fewer than eight times the
     // experts, so a wider piece reads and decodes fewer expert weights per token.
@@ -103,6 +103,10 @@ struct qw_engine {
     // kernels
     qw_kernel *k_begin, *k_embed, *k_norm, *k_norm0, *k_norm_cmb, *k_route, *k_adv_feed, *k_qmv_in_a, *k_qmv_in_g, *k_qmv_o_a, *k_qmv_o_g, *k_lm, *k_prep, *k_attn, *k_merge, *k_epi, *k_gdn, *k_router, *k_select,
         *k_chunk, *k_epi_seq, *k_gdn_seq, *k_gdn_gate, *k_gu, *k_dn, *k_cmb, *k_argmax, *k_adv, *k_fill, *k_ar;
+    // Up to four rows on one GPU: the residual add + norm before the router runs inside the router's launch, which writes the residual
+    // stream to the other one of h and h2 (h_last: where the last pass left it).
+    qw_kernel *k_route_n = nullptr;
+    const qw_buf *h_last = nullptr;
     bool ep_ready = false;
     // fused exchange: each rank's down projection stores its rows straight into every rank's Pg (peer memory)
     bool ep_fused = false;
@@ -255,7 +259,7 @@ extern "C" qw_gpu *qw_engine_gpu(qw_engine *e) { return e ? e->g : nullptr; }
 extern "C" void qw_engine_close(qw_engine *e) {
     if (!e) return;
     qw_buf *all[] = {&e->emb, &e->lm_head, &e->dense, &e->small, &e->router, &e->exg, &e->exu, &e->exd, &e->shg, &e->shu, &e->shd, &e->kvpool,
-                     &e->ptab, &e->sstate, &e->cstate, &e->prompt_d, &e->ctl_p, &e->ffn_scr_w, &e->ctl_h, &e->ctl_d, &e->h, &e->x, &e->proj, &e->cv, &e->la, &e->be, &e->gy, &e->qb,
+                     &e->ptab, &e->sstate, &e->cstate, &e->prompt_d, &e->ctl_p, &e->ffn_scr_w, &e->ctl_h, &e->ctl_d, &e->h, &e->h2, &e->x, &e->proj, &e->cv, &e->la, &e->be, &e->gy, &e->qb,
                      &e->part, &e->ya, &e->ob, &e->mo, &e->logits, &e->ids, &e->ids_h, &e->logits_h, &e->cand_h, &e->mlog, &e->msel, &e->Hhi, &e->Hlo, &e->Pg, &e->rcnt, &e->xq_gu, &e->xq_d, &e->xs_gu, &e->xs_d, &e->ffn_scr};
     // mappings of the other ranks' exchange buffers go first (their owners free the memory), then this rank's own
     for (int r = 0; r < 8; r++)
@@ -364,6 +368,11 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
                 ok = compile(e, "add_rmsnorm", "cmb_add_rmsnorm_rows", {{"CMB", 1}, {"TOPK", e->TOPK}, {"ROWCNT", 1}}, &e->k_norm_cmb_rc);
         }
     }
+    if (ok && c.ep_size == 1 && e->D == 2048) {
+        auto mn = md;
+        mn.push_back({"NORM", 1});
+        ok = compile(e, "moe_route", "norm_moe_route", mn, &e->k_route_n);
+    }
     if (ok && c.ep_size == 1 && e->ffn_fused && c.max_ctx > ROWS) {
         e->piece_rows = PROWS;
         auto mw = md;
@@ -403,7 +412,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->shu, (size_t)e->L * gu_bytes) && new_buf(e, &e->shd, (size_t)e->L * gu_bytes) &&
          new_buf(e, &e->kvpool, (size_t)kvp * page_bytes) && new_buf(e, &e->ptab, (size_t)c.max_slots * e->max_pages * 4) &&
          new_buf(e, &e->sstate, (size_t)c.max_slots * ng * c.hv * 128 * 128 * 4) && new_buf(e, &e->cstate, (size_t)c.max_slots * ng * 3 * e->C * 4) &&
-         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->ctl_d, 3 * ROWS * 4) && new_buf(e, &e->prompt_d, (size_t)c.max_ctx * 4) && new_buf(e, &e->h, RB * e->D * 4) &&
+         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->ctl_d, 3 * ROWS * 4) && new_buf(e, &e->prompt_d, (size_t)c.max_ctx * 4) && new_buf(e, &e->h, RB * e->D * 4) && new_buf(e, &e->h2, 4 * e->D * 4) &&
          new_buf(e, &e->x, RB * e->D * 2) && new_buf(e, &e->proj, RB * std::max(e->qkv_rows, e->gdn_rows) * 2) && new_buf(e, &e->cv, RB * e->C * 2) &&
          new_buf(e, &e->la, RB * c.hv * 4) && new_buf(e, &e->be, RB * c.hv * 4) && new_buf(e, &e->gy, RB * e->KG * 2) &&
          new_buf(e, &e->qb, RB * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
@@ -570,7 +579,7 @@ void enc_qmv(qw_batch *b, qw_kernel *k, const qw_buf *W, size_t woff, uint32_t N
 
 // h (+)= the previous block's output, x = rmsnorm(h) * w.  delta == &e->Pg means "the MoE combine of layer cmb_layer",
 // computed inside the norm kernel from Pg and that layer's selection record.
-void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *delta, size_t w_off_floats, uint32_t nb, int cmb_layer = -1, size_t delta_off = 0) {
+void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *h, const qw_buf *delta, size_t w_off_floats, uint32_t nb, int cmb_layer = -1, size_t delta_off = 0) {
     const uint32_t a[2] = {nb, (uint32_t)e->D};
     const bool cmb = delta == &e->Pg;
     const bool gathered = delta == &e->epx;  // slot sharding: the rows were stored by the ranks that own the slots
@@ -578,7 +587,7 @@ void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *delta, size_t w_off_float
     const bool wide = nb > ROWS;
     if (wide) qw_batch_kernel(b, cmb ? (rows ? e->k_norm_cmb_rc_w : e->k_norm_cmb_w) : delta ? e->k_norm_w : e->k_norm0_w);
     else qw_batch_kernel(b, cmb ? (e->ep_fused ? e->k_norm_cmb_x : rows ? e->k_norm_cmb_rc : e->k_norm_cmb) : gathered ? e->k_norm_x : delta ? e->k_norm : e->k_norm0);
-    qw_batch_buf(b, 0, &e->h, 0);
+    qw_batch_buf(b, 0, h, 0);
     if (cmb) {
         qw_batch_buf(b, 5, &e->msel, (size_t)cmb_layer * e->sel_bytes);
         if (e->ep_fused) {
@@ -640,6 +649,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
         qw_batch_bytes(b, 3, a, sizeof a);
         qw_batch_dispatch(b, (D + 255) / 256, nb, 1, 256, 1, 1);
     }
+    const qw_buf *hb = &e->h;      // the residual stream
     const qw_buf *pending = none;  // block output not yet added to the residual stream
     // rows of the token mixers: all of them, or (slot sharding) the rows [lo, lo + nbl) whose slots this rank owns
     const uint32_t lo = e->slot_shard ? e->row_lo : 0, nbl = e->slot_shard ? e->row_hi - e->row_lo : nb;
@@ -669,7 +679,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     };
     for (int l = 0; l < e->L; l++) {
         const LayerW &w = e->layers[l];
-        enc_norm(e, b, pending, w.small, nb, l - 1);  // h += previous block (the MoE combine of layer l-1); x = rmsnorm(h) * w1
+        enc_norm(e, b, hb, pending, w.small, nb, l - 1);  // h += previous block (the MoE combine of layer l-1); x = rmsnorm(h) * w1
         if (nbl == 0) {  // no row of this rank in the step: only tell the others so
             qw_batch_kernel(b, e->k_pub);
             bind_peers(0, false);
@@ -754,17 +764,26 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             }
             enc_out_proj(e->k_qmv_o_g, e->k_qmv_o_g_x, w.w_out, e->KG, &e->gy);
         }
-        enc_norm(e, b, obuf, w.small + D, nb, -1, obo);  // h += mixer output (all rows); x = rmsnorm(h) * w2
+        const bool norm_in_route = nb <= 4 && e->k_route_n;
+        if (!norm_in_route) enc_norm(e, b, hb, obuf, w.small + D, nb, -1, obo);  // h += mixer output (all rows); x = rmsnorm(h) * w2
         // ---- MoE (gg_moe, src/engine.c:568-646)
         const size_t gu_bytes = (size_t)e->I * e->rbD, ex_bytes = (size_t)e->EL * gu_bytes, selo = (size_t)l * e->sel_bytes;
         const sel_args sa = {nb, (uint32_t)e->e_lo, (uint32_t)(e->e_lo + e->EL)};
-        qw_batch_kernel(b, wide ? e->k_logits_w : e->k_route);  // router logits + top-k + grouping in one launch; of a wide piece the logits
+        qw_batch_kernel(b, wide ? e->k_logits_w : norm_in_route ? e->k_route_n : e->k_route);  // router logits + top-k + grouping in one launch; of a wide piece the logits
         qw_batch_buf(b, 0, &e->router, (size_t)l * (e->E + 1) * D * 2);
         qw_batch_buf(b, 1, &e->router, ((size_t)l * (e->E + 1) + e->E) * D * 2);
         qw_batch_buf(b, 2, &e->x, 0);
         qw_batch_buf(b, 3, &e->mlog, 0);
         qw_batch_buf(b, 4, &e->rcnt, 0);
         qw_batch_buf(b, 5, &e->msel, selo);
+        if (norm_in_route) {
+            const qw_buf *hn = hb == &e->h ? &e->h2 : &e->h;
+            qw_batch_buf(b, 6, hb, 0);
+            qw_batch_buf(b, 7, obuf, obo);
+            qw_batch_buf(b, 8, &e->small, (w.small + D) * 4);
+            qw_batch_buf(b, 9, hn, 0);
+            hb = hn;
+        }
         qw_batch_bytes(b, 14, &sa, sizeof sa);
         qw_batch_dispatch(b, (e->E + 1 + 7) / 8, 1, 1, 1024, 1, 1);
         if (wide) {
@@ -852,7 +871,8 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     }
     // (a piece: h and x of row 0 -- the newest token -- and its logits if the prompt ends there; a piece in the middle still needs the
     // combine of its last layer for nothing, but the kernel also returns the FFN's row counters to zero)
-    enc_norm(e, b, pending, e->final_norm, nb, e->L - 1);
+    enc_norm(e, b, hb, pending, e->final_norm, nb, e->L - 1);
+    e->h_last = hb;
     if (piece) {
         if (piece->last) enc_qmv(b, e->k_lm, &e->lm_head, 0, (uint32_t)e->V, D, &e->x, &e->logits, 1, (uint32_t)e->V);
         return;
@@ -1211,7 +1231,7 @@ extern "C" size_t qw_engine_tap(qw_engine *e, const char *name, int index, void 
     const size_t gu = (size_t)e->I * e->rbD, B = (size_t)e->lastB;
     const int ng = std::max(1, e->n_gdn), na = std::max(1, e->n_attn);
     const bool lay = index >= 0 && index < e->L;
-    if (!strcmp(name, "h")) { b = &e->h; n = B * e->D * 4; }
+    if (!strcmp(name, "h")) { b = e->h_last ? e->h_last : &e->h; n = B * e->D * 4; }
     else if (!strcmp(name, "logits")) { b = &e->logits; n = B * e->V * 4; }
     else if (!strcmp(name, "x")) { b = &e->x; n = B * e->D * 2; }
     else if (!strcmp(name, "emb")) { b = &e->emb; n = (size_t)e->V * e->D * 2; }

@@ -342,16 +342,27 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
 // 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.  With SELECT defined 0 only the
 // logits are computed, of up to 512 tokens (binds 4 and 5 are not used).
+// With NORM defined 1 (D = 2048, up to four tokens) the launch begins with the residual add + RMSNorm before the router, in the order of
+// add_rmsnorm: 6 = h fp32 [nb][D], 7 = delta fp16 [nb][D], 8 = w fp32 [D], 9 = h out (another buffer: every block reads h), 2 = x out.
+// Every block normalises all tokens for itself -- 12 KB of L2 reads per token and block -- and the first one stores h and x; that is
+// cheaper than a launch that does it once as long as the tokens are few: a step of one slot, 48 layers, 2.96 -> 2.84 ms on a B200.
 constexpr uint32_t ROUTE_PASS = 16, ROUTE_STG = 3;  // tokens per copy, copies in flight
+constexpr uint32_t ROUTE_DIRECT = 4;                // up to this many tokens nothing is staged, and NORM is possible
+struct RouteNorm {
+    const float *h, *w;
+    const __half *delta;
+    float *hout;
+    __half *xout;
+};
 template <int D>
 __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, unsigned *counter, moe_sel *ms,
-                                                   uint32_t E, uint32_t topk, sel_args a, bool select, unsigned *status) {
+                                                   uint32_t E, uint32_t topk, sel_args a, bool select, RouteNorm nm, unsigned *status) {
     constexpr int CH = D / 8 / 32;
     extern __shared__ __align__(128) uint8_t route_smem[];  // [ROUTE_STG][16 tokens][D] fp16
     __shared__ uint64_t full[ROUTE_STG];
     __shared__ bool last;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * 4 + (warp & 3), tg = warp >> 2;
-    const bool direct = a.nb <= 4;
+    const bool direct = a.nb <= ROUTE_DIRECT;
     pdl_launch();
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < ROUTE_STG; s++) mbar_init(&full[s], 1);
@@ -372,8 +383,57 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
             }
         }
     }
+    constexpr int NV = D / 512 > 0 ? D / 512 : 1;  // values of a row per thread, as add_rmsnorm's blocks of 512 threads hold them
+    float nw[NV];
+    if (nm.h)
+#pragma unroll
+        for (int i = 0; i < NV; i++) nw[i] = nm.w[threadIdx.x + 512 * i];
     if (!direct) __syncthreads();
-    pdl_wait();  // the router row is static; the tokens are the previous kernel's output
+    pdl_wait();  // the router row and the norm weights are static; the tokens are the previous kernel's output
+    if (D == 2048 && nm.h) {
+        __shared__ float part[ROUTE_DIRECT][16];
+        float v[ROUTE_DIRECT][NV], ss[ROUTE_DIRECT];
+#pragma unroll
+        for (uint32_t t = 0; t < ROUTE_DIRECT; t++) {
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+                const size_t at = (size_t)t * D + threadIdx.x + 512 * i;
+                v[t][i] = 0.f;
+                if (t < a.nb) v[t][i] = __ldcg(nm.h + at) + __half2float(__ldcg(nm.delta + at));
+            }
+        }
+#pragma unroll
+        for (uint32_t t = 0; t < ROUTE_DIRECT; t++) {
+            ss[t] = 0.f;
+#pragma unroll
+            for (int i = 0; i < NV; i++) ss[t] = fmaf(v[t][i], v[t][i], ss[t]);
+        }
+#pragma unroll
+        for (int off = 16; off; off >>= 1)
+#pragma unroll
+            for (uint32_t t = 0; t < ROUTE_DIRECT; t++) ss[t] += __shfl_xor_sync(0xffffffffu, ss[t], off);
+        if (lane == 0)
+#pragma unroll
+            for (uint32_t t = 0; t < ROUTE_DIRECT; t++) part[t][warp] = ss[t];
+        __syncthreads();
+        __half *xs = (__half *)route_smem;
+#pragma unroll
+        for (uint32_t t = 0; t < ROUTE_DIRECT; t++) {
+            if (t >= a.nb) break;
+            const float r = rsqrtf(warp_sum(lane < 16 ? part[t][lane] : 0.f) / D + 1e-6f);
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+                const uint32_t d = threadIdx.x + 512 * i;
+                const __half xv = __float2half_rn(v[t][i] * r * nw[i]);
+                xs[t * D + d] = xv;
+                if (blockIdx.x == 0) {
+                    nm.hout[(size_t)t * D + d] = v[t][i];
+                    nm.xout[(size_t)t * D + d] = xv;
+                }
+            }
+        }
+        __syncthreads();
+    }
     // Every dot product is the same single-lane chain as in moe_router (element k of lane l, chunk c is column (l + 32 c) * 8 + k), so
     // logits are bit-identical.  v = this lane's chunks of the token.
     auto dot = [&](const uint4 (&v)[CH]) {
@@ -392,10 +452,10 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
     };
     if (direct) {
         if (r <= E && tg < a.nb) {
-            const uint4 *xt = (const uint4 *)(x + (size_t)tg * D) + lane;
+            const uint4 *xt = (const uint4 *)(x + (size_t)tg * D) + lane, *xn = (const uint4 *)(route_smem + tg * D * 2) + lane;
             uint4 v[CH];
 #pragma unroll
-            for (int c = 0; c < CH; c++) v[c] = __ldcg(xt + 32 * c);
+            for (int c = 0; c < CH; c++) v[c] = nm.h ? xn[32 * c] : __ldcg(xt + 32 * c);
             const float sum = dot(v);
             if (lane == 0) logits[(size_t)tg * (E + 1) + r] = sum;
         }
@@ -452,9 +512,17 @@ template <int DD>
 static cudaError_t moe_route_go(const QwLaunch &L, unsigned grid, uint32_t E, uint32_t topk, const sel_args &a) {
     cudaError_t e = cudaFuncSetAttribute(moe_route_k<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_STG * ROUTE_PASS * DD * 2);
     if (e != cudaSuccess) return e;
-    const uint32_t held = a.nb <= 4 ? 0 : a.nb < ROUTE_STG * ROUTE_PASS ? a.nb : ROUTE_STG * ROUTE_PASS;
+    RouteNorm nm{};
+    if (L.def("NORM", 0)) {
+        QW_CHECK_ARG(DD == 2048 && a.nb <= ROUTE_DIRECT);
+        for (int i = 6; i <= 9; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+        QW_CHECK_ARG(L.avail(6) >= (size_t)a.nb * DD * 4 && L.avail(7) >= (size_t)a.nb * DD * 2 && L.avail(8) >= DD * 4 && L.avail(9) >= (size_t)a.nb * DD * 4);
+        nm = {L.buf<float>(6), L.buf<float>(8), L.buf<__half>(7), L.buf<float>(9), L.buf<__half>(2)};
+        QW_CHECK_ARG(nm.h != nm.hout);
+    }
+    const uint32_t held = a.nb <= ROUTE_DIRECT ? (nm.h ? a.nb : 0) : a.nb < ROUTE_STG * ROUTE_PASS ? a.nb : ROUTE_STG * ROUTE_PASS;
     qw_launch(moe_route_k<DD>, grid, 512, held * DD * 2, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), L.buf<unsigned>(4),
-              L.buf<moe_sel>(5), E, topk, a, L.def("SELECT", 1) != 0, (unsigned *)L.status);
+              L.buf<moe_sel>(5), E, topk, a, L.def("SELECT", 1) != 0, nm, (unsigned *)L.status);
     return cudaGetLastError();
 }
 
