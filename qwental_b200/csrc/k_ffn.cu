@@ -332,7 +332,7 @@ __device__ __forceinline__ void x_unit(uint32_t rec0, uint32_t rec1, int kh, int
 // TMA boxes and bulk copies through the same ring, but the consumers only read every staged byte once (16-byte loads) and
 // compute nothing -- the role of the reference's pure-read probes (bench/moe_bw.c:1-3, bench/qmv.c:357-382).
 // (17 warps put five on one scheduler, whose 16 K registers then allow 96 per thread)
-template <bool PROBE, int FMT, int WIDE>
+template <bool PROBE, int FMT, int WIDE, bool HALF = false>
 __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(const __grid_constant__ CUtensorMap mG, const __grid_constant__ CUtensorMap mU,
                                                            const __grid_constant__ CUtensorMap mSG, const __grid_constant__ CUtensorMap mSU, const FfnP p) {
     using C = FfnCfg<FMT>;
@@ -387,18 +387,23 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     const uint32_t slot0 = smem_u32(stage0);
     // this block's pieces: gate/up tiles [a_lo, a_hi) of the items x GT list, then down tiles [b_lo, b_hi) of the items x DT list
     const uint32_t G = gridDim.x, bx_ = blockIdx.x;
-    uint32_t a_lo = (uint32_t)((uint64_t)bx_ * items * GT / G), a_hi = (uint32_t)((uint64_t)(bx_ + 1) * items * GT / G);
+    // HALF: few items (one or two slots).  Gate/up pieces are halved -- half of the row groups, 32 indices -- as long as every block gets at
+    // most one.  A piece is then a chain of four stages with half the warps decoding, and H is complete sooner.  (A variant of its own:
+    // in the others the registers would not suffice.)  A step of one slot, 48 layers: 2.83 -> 2.69 ms on a B200.
+    static_assert(!HALF || FMT == 1, "half pieces are cut from IQ3X stages");
+    const uint32_t spl = HALF && 2 * items * GT <= G ? 1 : 0, GTS = GT << spl;
+    uint32_t a_lo = (uint32_t)((uint64_t)bx_ * items * GTS / G), a_hi = (uint32_t)((uint64_t)(bx_ + 1) * items * GTS / G);
     uint32_t b_lo = (uint32_t)((uint64_t)bx_ * items * DT / G), b_hi = (uint32_t)((uint64_t)(bx_ + 1) * items * DT / G);
     // the few items those shares touch, looked up once (thread k: item k of the gate/up share, thread FFN_RECS + k: of the down share)
-    const uint32_t wa0 = a_lo / GT, wb0 = b_lo / DT;
-    if ((a_hi > a_lo && (a_hi - 1) / GT - wa0 >= FFN_RECS) || (b_hi > b_lo && (b_hi - 1) / DT - wb0 >= FFN_RECS)) {  // a grid far smaller than the device's
+    const uint32_t wa0 = a_lo / GTS, wb0 = b_lo / DT;
+    if ((a_hi > a_lo && (a_hi - 1) / GTS - wa0 >= FFN_RECS) || (b_hi > b_lo && (b_hi - 1) / DT - wb0 >= FFN_RECS)) {  // a grid far smaller than the device's
         if (tid == 0) set_status(p.status, ST_BAD_ARG | 6);
         a_hi = a_lo;
         b_hi = b_lo;
     }
     if (tid < 2 * FFN_RECS) {
         const uint32_t k = tid % FFN_RECS, w = (tid < FFN_RECS ? wa0 : wb0) + k;
-        const bool need = tid < FFN_RECS ? (a_hi > a_lo && w <= (a_hi - 1) / GT) : (b_hi > b_lo && w <= (b_hi - 1) / DT);
+        const bool need = tid < FFN_RECS ? (a_hi > a_lo && w <= (a_hi - 1) / GTS) : (b_hi > b_lo && w <= (b_hi - 1) / DT);
         if (need) recs[tid] = ffn_item(pre, ms, U, nb, p.ebase, w);
     }
     __syncthreads();
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
             Src sc{};
             uint32_t cur = 0xffffffffu;
             for (uint32_t a = a_lo; a < a_hi; a++) {
-                const uint32_t w = a / GT, gt = a - w * GT;
+                const uint32_t w = a / GTS, gh = a - w * GTS, gt = gh >> spl;
                 const bool sw = w != cur;
                 FfnItem it{};
                 if (sw) {
@@ -473,8 +478,13 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                     sc = src_of(it);
                 }
                 for (uint32_t kp = 0; kp < KP; kp++, j++) {
-                    const uint32_t dst = slot_for(FMT ? IQ3X_STAGE : 2 * 64 * FFN_PITCH);
-                    if (FMT == 1) {  // one contiguous stage
+                    const uint32_t dst = slot_for(FMT ? IQ3X_STAGE >> spl : 2 * 64 * FFN_PITCH);
+                    if (HALF && spl) {  // half of the gate rows and of the up rows, in their places
+                        const uint32_t o = (gh & 1) * 32 * IQ3X_REC;
+                        const uint8_t *src = sc.wg + ((size_t)gt * KP + kp) * IQ3X_STAGE + o;
+                        bulk_s(dst + o, src, 32 * IQ3X_REC, &full[j % FFN_STG]);
+                        bulk_s(dst + o + 64 * IQ3X_REC, src + 64 * IQ3X_REC, 32 * IQ3X_REC, &full[j % FFN_STG]);
+                    } else if (FMT == 1) {  // one contiguous stage
                         bulk_s(dst, sc.wg + ((size_t)gt * KP + kp) * IQ3X_STAGE, IQ3X_STAGE, &full[j % FFN_STG]);
                     } else {
                         const int xc = (int)((220 * kp) & ~15u), yr = (int)(sc.erow * I + gt * 64);
@@ -592,7 +602,8 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
         // ---- gate/up pieces: tiles of 64 intermediate indices
         uint32_t cur = 0xffffffffu, have = 0, ncols = 0, xb0 = 0;
         for (uint32_t a = a_lo; a < a_hi; a++) {
-            const uint32_t w = a / GT, gt = a - w * GT;
+            const uint32_t w = a / GTS, gh = a - w * GTS, gt = gh >> spl;
+            const bool mine = !spl || (uint32_t)r >> 2 == (gh & 1);  // a half piece has rows for half of the row groups
             if (w != cur) {
                 if (cur != 0xffffffffu) act_release();
                 cur = w;
@@ -607,14 +618,14 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                 if (PROBE) probe_read(st, FMT ? IQ3X_STAGE : 128 * FFN_PITCH, sink);
                 else if (FMT == 1) {
                     const uint32_t rec0 = st + (8 * r + g) * IQ3X_REC;
-                    x_unit<1>(rec0, rec0 + 64 * IQ3X_REC, kh, t, stab, zr, bx, bx, have, acc);
+                    if (mine) x_unit<1>(rec0, rec0 + 64 * IQ3X_REC, kh, t, stab, zr, bx, bx, have, acc);
                 } else {
                     const uint32_t u0 = st + (8 * r + g) * FFN_PITCH + ((220 * kp) & 15) + kh * 110, u1 = u0 + 64 * FFN_PITCH;
                     ffn_unit<1>(u0, u1, t, tabl, zr, bx, bx, have, acc);
                 }
                 release();
             }
-            if (PROBE) continue;
+            if (PROBE || !mine) continue;
             pair_sum(acc);
             if (!kh) {
                 // acc[0], acc[1] = gate of index 64 gt + 8 r + g for columns 2t, 2t + 1; acc[2], acc[3] = up.  H travels to the
@@ -831,7 +842,10 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
         QW_CHECK_ARG(mG && mU && mSG && mSU);
     }
     const bool probe = L.def("PROBE", 0) != 0;  // PROBE defined 1: the copy-only twin (outputs are not written)
-    auto kern = wide ? (x4 ? moe_ffn_k<false, 1, 1> : moe_ffn_k<false, 0, 1>)
+    // HALF defined 1: the variant for few items (IQ3X; the other kinds ignore it)
+    const bool half = L.def("HALF", 0) != 0;
+    auto kern = x4 && half && !probe && !wide ? moe_ffn_k<false, 1, 0, true>
+                : wide ? (x4 ? moe_ffn_k<false, 1, 1> : moe_ffn_k<false, 0, 1>)
                 : x4 ? (probe ? moe_ffn_k<true, 1, 0> : moe_ffn_k<false, 1, 0>) : (probe ? moe_ffn_k<true, 0, 0> : moe_ffn_k<false, 0, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
