@@ -97,7 +97,7 @@ struct qw_engine {
     int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
     qw_buf ctl_p{}, ffn_scr_w{};
     qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_norm_cmb_rc_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
-              *k_group_w = nullptr, *k_ffn_w = nullptr;
+              *k_group_w = nullptr, *k_ffn_w = nullptr, *k_qmv_in_w = nullptr, *k_qmv_oa_w = nullptr, *k_qmv_og_w = nullptr;
     qw_buf mlog{}, msel{}, Hhi{}, Hlo{}, Pg{}, rcnt{};
     size_t sel_bytes = 0;
     // kernels
@@ -391,6 +391,10 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
              compile(e, "add_rmsnorm", "cmb_add_rmsnorm_wide", cw, &e->k_norm_cmb_w) &&
              (!e->k_norm_cmb_rc || compile(e, "add_rmsnorm", "cmb_add_rmsnorm_rows_wide", cr, &e->k_norm_cmb_rc_w)) &&
              compile(e, "moe_route", "moe_logits_wide", mw, &e->k_logits_w) && compile(e, "moe_topk_wide", "moe_topk_wide", mw, &e->k_topk_w) &&
+             (c.fma || (e->KA != 2048 && e->KA != 4096) || (e->KG != 2048 && e->KG != 4096) ||  // (else the matvecs go by 64 rows)
+              (compile(e, "qmv_mma", "qmv_in_wide", {{"GF", 21}, {"KD", (long)e->D}, {"ROWS", PROWS}, {"YT_F32", 0}}, &e->k_qmv_in_w) &&
+               compile(e, "qmv_mma", "qmv_out_attn_wide", {{"GF", 21}, {"KD", (long)e->KA}, {"ROWS", PROWS}, {"YT_F32", 0}}, &e->k_qmv_oa_w) &&
+               compile(e, "qmv_mma", "qmv_out_gdn_wide", {{"GF", 21}, {"KD", (long)e->KG}, {"ROWS", PROWS}, {"YT_F32", 0}}, &e->k_qmv_og_w))) &&
              compile(e, "moe_group_wide", "moe_group_wide", mw, &e->k_group_w) && compile(e, "moe_ffn", "moe_ffn_wide", mw, &e->k_ffn_w);
     }
     ok = ok && compile(e, "k_topk", "k_topk", {}, &e->k_topk);
@@ -564,11 +568,13 @@ struct dn_epi_args { uint32_t nb, layer, nlayers, proj_stride; };
 struct gdn_args { uint32_t nb, layer, nlayers, z_stride; };
 struct sel_args { uint32_t nb, e_lo, e_hi; };
 
-void enc_qmv(qw_batch *b, qw_kernel *k, const qw_buf *W, size_t woff, uint32_t N, uint32_t K, const qw_buf *x, const qw_buf *y, uint32_t nb, uint32_t ystride,
+// kw: the kernel that takes a wide piece as a whole, nullptr where there is none
+void enc_qmv(qw_batch *b, qw_kernel *k, qw_kernel *kw, const qw_buf *W, size_t woff, uint32_t N, uint32_t K, const qw_buf *x, const qw_buf *y, uint32_t nb, uint32_t ystride,
              size_t xoff = 0, size_t yoff = 0) {
-    if (nb > ROWS) {  // a wide piece (fp16 results): the matvec kernels take 64 rows at a time
+    if (nb > ROWS && kw) k = kw;
+    else if (nb > ROWS) {  // a wide piece (fp16 results), 64 rows at a time
         for (uint32_t r = 0; r < nb; r += ROWS)
-            enc_qmv(b, k, W, woff, N, K, x, y, std::min<uint32_t>(ROWS, nb - r), ystride, xoff + (size_t)r * K * 2, yoff + (size_t)r * ystride * 2);
+            enc_qmv(b, k, nullptr, W, woff, N, K, x, y, std::min<uint32_t>(ROWS, nb - r), ystride, xoff + (size_t)r * K * 2, yoff + (size_t)r * ystride * 2);
         return;
     }
     const qmv_args a = {N, K, ystride, nb};
@@ -669,8 +675,8 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_buf(b, 24 + r, &e->ep_peer[r], 2 * e->pg_bytes);
         }
     };
-    auto enc_out_proj = [&](qw_kernel *plain, qw_kernel *shared, size_t woff, uint32_t K, const qw_buf *in) {
-        if (!e->slot_shard) return enc_qmv(b, plain, &e->dense, woff, D, K, in, &e->ob, nb, D);
+    auto enc_out_proj = [&](qw_kernel *plain, qw_kernel *piecew, qw_kernel *shared, size_t woff, uint32_t K, const qw_buf *in) {
+        if (!e->slot_shard) return enc_qmv(b, plain, piecew, &e->dense, woff, D, K, in, &e->ob, nb, D);
         const qmv_args a = {D, K, D, nbl};
         qw_batch_kernel(b, shared);
         qw_batch_buf(b, 0, &e->dense, woff);
@@ -688,7 +694,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             bind_peers(0, false);
             qw_batch_dispatch(b, 1, 1, 1, 32, 1, 1);
         } else if (w.attn) {
-            enc_qmv(b, e->k_qmv_in_a, &e->dense, w.w_in, e->qkv_rows, D, &e->x, &e->proj, nbl, e->qkv_rows, xo);
+            enc_qmv(b, e->k_qmv_in_a, e->k_qmv_in_w, &e->dense, w.w_in, e->qkv_rows, D, &e->x, &e->proj, nbl, e->qkv_rows, xo);
             // the attention kernels take up to 64 rows: one group of rows for a step, several for a wide piece -- all of its K and V first
             auto group = [&](uint32_t r0) {
                 return qsa_args{std::min<uint32_t>(ROWS, nbl - r0), (uint32_t)w.idx, (uint32_t)e->n_attn, e->qkv_rows, (uint32_t)e->max_pages, max_chunks, 0, 0};
@@ -727,9 +733,9 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 qw_batch_bytes(b, 4, &qa, sizeof qa);
                 qw_batch_dispatch(b, e->QH, qa.nb, 1, 256, 1, 1);
             }
-            enc_out_proj(e->k_qmv_o_a, e->k_qmv_o_a_x, w.w_out, e->KA, &e->ya);
+            enc_out_proj(e->k_qmv_o_a, e->k_qmv_oa_w, e->k_qmv_o_a_x, w.w_out, e->KA, &e->ya);
         } else {
-            enc_qmv(b, e->k_qmv_in_g, &e->dense, w.w_in, e->gdn_rows, D, &e->x, &e->proj, nbl, e->gdn_rows, xo);
+            enc_qmv(b, e->k_qmv_in_g, e->k_qmv_in_w, &e->dense, w.w_in, e->gdn_rows, D, &e->x, &e->proj, nbl, e->gdn_rows, xo);
             const size_t so = (w.small + 2 * D) * 4, sa = so + (size_t)e->C * 16;
             const dn_epi_args ea = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
             qw_batch_kernel(b, piece ? e->k_epi_seq : e->k_epi);
@@ -765,7 +771,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 qw_batch_bytes(b, 8, &ga, sizeof ga);
                 qw_batch_dispatch(b, e->HV, nbl, 1, 128, 1, 1);
             }
-            enc_out_proj(e->k_qmv_o_g, e->k_qmv_o_g_x, w.w_out, e->KG, &e->gy);
+            enc_out_proj(e->k_qmv_o_g, e->k_qmv_og_w, e->k_qmv_o_g_x, w.w_out, e->KG, &e->gy);
         }
         const bool norm_in_route = nb <= 4 && e->k_route_n;
         if (!norm_in_route) enc_norm(e, b, hb, obuf, w.small + D, nb, -1, obo);  // h += mixer output (all rows); x = rmsnorm(h) * w2
@@ -878,10 +884,10 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     enc_norm(e, b, hb, pending, e->final_norm, nb, e->L - 1);
     e->h_last = hb;
     if (piece) {
-        if (piece->last) enc_qmv(b, e->k_lm, &e->lm_head, 0, (uint32_t)e->V, D, &e->x, &e->logits, 1, (uint32_t)e->V);
+        if (piece->last) enc_qmv(b, e->k_lm, nullptr, &e->lm_head, 0, (uint32_t)e->V, D, &e->x, &e->logits, 1, (uint32_t)e->V);
         return;
     }
-    enc_qmv(b, e->k_lm, &e->lm_head, 0, (uint32_t)e->V, D, &e->x, &e->logits, nb, (uint32_t)e->V);
+    enc_qmv(b, e->k_lm, nullptr, &e->lm_head, 0, (uint32_t)e->V, D, &e->x, &e->logits, nb, (uint32_t)e->V);
     if (sample == 3) {  // the 256 best (id, logit) pairs of every row, written straight into host-visible memory
         const uint32_t a[3] = {nb, (uint32_t)e->V, 256};
         qw_batch_kernel(b, e->k_topk);

@@ -130,7 +130,7 @@ static bool qmv_common_check(const QwLaunch &L, qmv_args &a, int &gf, uint32_t &
     if (!(gf == 21 || gf == 8) || K == 0 || K % 256 != 0) return false;
     rb = gf == 21 ? K / 256 * 110 : K / 32 * 34;
     if (!L.buf<uint8_t>(0) || !L.buf<__half>(3) || !L.buf<void>(4) || !L.has_bytes(5, 12)) return false;
-    if (a.nb == 0 || a.nb > 64 || a.N == 0 || a.xstride < K || a.xstride % 8 != 0 || a.ystride < a.N) return false;
+    if (a.nb == 0 || a.nb > (uint32_t)L.def("ROWS", 64) || a.N == 0 || a.xstride < K || a.xstride % 8 != 0 || a.ystride < a.N) return false;
     if (((uintptr_t)L.buf<__half>(3) & 15) != 0) return false;
     if (L.avail(0) < (size_t)a.N * rb) return false;
     if (L.avail(3) < ((size_t)(a.nb - 1) * a.xstride + K) * 2) return false;
@@ -534,12 +534,15 @@ __device__ __forceinline__ void wide_decode(uint32_t u0, uint32_t u1, int t, con
     a1[0] = wa[2]; a1[1] = wb[2]; a1[2] = wa[3]; a1[3] = wb[3];
 }
 
-// CT = column tiles of 8 tokens per warp: up to 8 CT TS tokens.  grid: at most one block per SM
-template <int GF, bool F32OUT, int TS, int CT>
+// CT = column tiles of 8 tokens per warp: up to 8 CT TS tokens per block; more tokens (a piece of a prompt) are groups of 64 that share
+// the grid: blocks_per_group blocks each, so that a group's blocks have many row tiles and run them side by side.  One launch for all groups
+// instead of one per 64 tokens, and K = 4096 here instead of in qmv_mma2: a prompt of 419 tokens, 48 layers, 42.5 -> 39.6 ms, 1700 tokens, 12
+// layers, 41.2 -> 38.9 ms on a B200.  UNITS = K / 256.  grid: at most one block per SM
+template <int GF, bool F32OUT, int TS, int CT, int UNITS>
 __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wide_k(const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx,
-                                                                                    const QmvMmaP p, uint32_t rg) {
+                                                                                    const QmvMmaP p, uint32_t rg, uint32_t blocks_per_group) {
     using C = WideCfg<GF, TS>;
-    constexpr int WS = C::WS, XS = C::XS, UPW = C::UPW, UNITS = 8, R = 8 * CT * TS, XBYTES = R * 512, CH = CT <= 4 ? CT : CT / 2;
+    constexpr int WS = C::WS, XS = C::XS, UPW = C::UPW, R = 8 * CT * TS, XBYTES = R * 512, CH = CT <= 4 ? CT : CT / 2;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;  // the swizzle pattern repeats every 1024 bytes
     const uint32_t xs0 = base, ws0 = xs0 + XS * XBYTES, tab0 = ws0 + WS * C::WBYTES;
@@ -556,7 +559,8 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
     }
     __syncthreads();
     // this block's tiles, and the tiles of a round: both split evenly
-    const uint32_t t0 = (uint32_t)((uint64_t)blockIdx.x * p.items / gridDim.x), cnt = (uint32_t)((uint64_t)(blockIdx.x + 1) * p.items / gridDim.x) - t0;
+    const uint32_t c0 = blockIdx.x / blocks_per_group * 64, bi = blockIdx.x % blocks_per_group;  // first token of the group, block within it
+    const uint32_t t0 = (uint32_t)((uint64_t)bi * p.items / blocks_per_group), cnt = (uint32_t)((uint64_t)(bi + 1) * p.items / blocks_per_group) - t0;
     const uint32_t rounds = (cnt + rg - 1) / rg;
     if ((uint32_t)warp == ncw) {
         if (lane == 0) {
@@ -585,7 +589,7 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
                 const uint32_t s = jx % XS, u = jx % UNITS;
                 if (jx >= XS && !mbar_wait(&xempty[s], (jx / XS - 1) & 1)) { ok = false; break; }
                 mbar_expect_tx(&xfull[s], XBYTES);
-                for (uint32_t q = 0; q < 4; q++) tma_load_2d(xs0 + s * XBYTES + q * R * 128, &mx, (int)(u * 256 + q * 64), 0, &xfull[s]);
+                for (uint32_t q = 0; q < 4; q++) tma_load_2d(xs0 + s * XBYTES + q * R * 128, &mx, (int)(u * 256 + q * 64), (int)c0, &xfull[s]);
                 // weights as far ahead as their ring allows without holding up the activations of the stages already in it
                 if (jw < nw && jw * UPW <= jx + (WS - 1) * UPW) ok = put_w();
             }
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
         for (int i = 0; i < CT; i++)
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const uint32_t col = (TS * i + th) * 8 + t + 4 * (k & 1), rw = row + 8 * (k >> 1);
+                const uint32_t col = c0 + (TS * i + th) * 8 + t + 4 * (k & 1), rw = row + 8 * (k >> 1);
                 if (col >= p.nb) continue;
                 if (F32OUT) ((float *)p.y)[(size_t)col * p.ystride + rw] = tot[i][k];
                 else ((__half *)p.y)[(size_t)col * p.ystride + rw] = __float2half_rn(tot[i][k]);
@@ -674,8 +678,8 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
     if (!ok && lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 13);
 }
 
-template <int GF, bool F32OUT, int TS>
-static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t grid, uint32_t per, cudaStream_t st) {
+template <int GF, bool F32OUT, int TS, int UNITS>
+static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t groups, uint32_t bpg, uint32_t per, cudaStream_t st) {
     using C = WideCfg<GF, TS>;
     CUtensorMap mw, mx;
     constexpr int B = 2 / TS;  // column tiles per 16 tokens of a warp
@@ -684,22 +688,24 @@ static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t grid, uint32_t per, cu
                               : tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.W, p.rb / 2, p.N, p.rb, 136, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (!mok || !tmap_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x, p.K, p.nb, (uint64_t)p.xstride * 2, 64, 16 * n, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
-    auto k = n == 2 ? qmv_wide_k<GF, F32OUT, TS, 2 * B> : n == 3 ? qmv_wide_k<GF, F32OUT, TS, 3 * B> : qmv_wide_k<GF, F32OUT, TS, 4 * B>;
+    auto k = n == 2 ? qmv_wide_k<GF, F32OUT, TS, 2 * B, UNITS> : n == 3 ? qmv_wide_k<GF, F32OUT, TS, 3 * B, UNITS> : qmv_wide_k<GF, F32OUT, TS, 4 * B, UNITS>;
     const size_t smem = C::smem(ct);
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     // as many row tiles per round as split the block's tiles into equal rounds of at most RG
     const uint32_t rounds = (per + C::RG - 1) / C::RG, rg = (per + rounds - 1) / rounds;
-    qw_launch(k, grid, (TS * rg + 1) * 32, smem, st, mw, mx, p, rg);
+    qw_launch(k, groups * bpg, (TS * rg + 1) * 32, smem, st, mw, mx, p, rg, bpg);
     return cudaGetLastError();
 }
-template <int GF, bool F32OUT>
+template <int GF, bool F32OUT, int UNITS = 8>
 static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) {
-    const uint32_t grid = p.items < (uint32_t)sm_count ? p.items : (uint32_t)sm_count, per = (p.items + grid - 1) / grid;  // one block per SM
+    // one block per SM, shared evenly by the groups of 64 tokens
+    const uint32_t groups = (p.nb + 63) / 64, most = (uint32_t)sm_count / groups > 0 ? (uint32_t)sm_count / groups : 1, bpg = p.items < most ? p.items : most;
+    const uint32_t per = (p.items + bpg - 1) / bpg;
     if constexpr (GF == 8) {
-        if (per >= 16) return qmv_wide_ts<GF, F32OUT, 1>(p, grid, per, st);
+        if (per >= 16) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
     }
-    return qmv_wide_ts<GF, F32OUT, 2>(p, grid, per, st);
+    return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }
 
 // The grid and block given by the host are ignored (the kernels are persistent and size themselves).  Defines: GF (21 = IQ3_S,
@@ -756,6 +762,12 @@ static cudaError_t launch_qmv_mma(const QwLaunch &L) {
     if (K == 2048 && a.nb > 16 && epx <= 1) {
         if (gf == 21) return f32 ? qmv_wide_go<21, true>(p, L.sm_count, L.stream) : qmv_wide_go<21, false>(p, L.sm_count, L.stream);
         return f32 ? qmv_wide_go<8, true>(p, L.sm_count, L.stream) : qmv_wide_go<8, false>(p, L.sm_count, L.stream);
+    }
+    // More than 64 tokens (ROWS defined: a piece of a prompt) at K = 4096 too: with 64 a block would have one row tile, with several groups of
+    // tokens it has enough to keep its warps busy.
+    if (a.nb > 64) {
+        QW_CHECK_ARG(gf == 21 && K == 4096 && epx <= 1);
+        return f32 ? qmv_wide_go<21, true, 16>(p, L.sm_count, L.stream) : qmv_wide_go<21, false, 16>(p, L.sm_count, L.stream);
     }
     if (gf == 21 && K == 2048) return f32 ? qmv_mma2_go<21, 8, 2, true>(p, L.sm_count, L.stream) : qmv_mma2_go<21, 8, 2, false>(p, L.sm_count, L.stream);
     if (gf == 21 && K == 4096) return f32 ? qmv_mma2_go<21, 16, 1, true>(p, L.sm_count, L.stream) : qmv_mma2_go<21, 16, 1, false>(p, L.sm_count, L.stream);

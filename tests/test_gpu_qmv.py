@@ -119,3 +119,28 @@ def test_wide_matvec_rows_equal_the_row_alone(gpu, qtype, N, B):
     assert np.abs(y[:, some] - ref).max() <= 2e-5 * np.abs(ref).max()
     y16 = run_qmv(gpu, "qmv_mma", qtype, W, 2048, x, f32=False)
     assert np.array_equal(y16, y.astype(np.float16))
+
+
+@pytest.mark.parametrize("N,K", [(2048, 4096), (16 * 149, 2048), (48, 4096)])
+@pytest.mark.parametrize("B", [65, 128, 130, 419, 512])
+def test_matvec_of_a_prompt_piece_equals_groups_of_64(gpu, N, K, B):
+    """ROWS defined: up to 512 rows in one launch, groups of 64 sharing the grid; each group the bits of a launch of its own, which the tests
+    above tie to single rows.  More rows than ROWS, and more than 64 without it, are refused."""
+    from qwental_b200.gpu import GpuError
+    rng = np.random.default_rng(N + B)
+    W = synth.iq3s_rows(rng, N, K)
+    x = synth.acts_fp16(rng, B, K)
+    k = gpu.compile("qmv_mma", "qmv_piece_%d" % K, GF=21, KD=K, ROWS=512, YT_F32=0)
+    wb, xb, yb = gpu.buf_from(W), gpu.buf_from(x), gpu.buf(B * N * 2).zero()
+
+    def run(kern, rows):
+        gpu.batch().kernel(kern).buf(0, wb).buf(3, xb).buf(4, yb).bytes(5, np.array([N, K, N, rows], np.uint32)).dispatch(((N + 7) // 8,), (256,)).end()
+
+    run(k, B)
+    y = yb.download(np.float16, B * N).reshape(B, N)
+    for r in range(0, B, 64):
+        assert np.array_equal(y[r:r + 64].view(np.uint16), run_qmv(gpu, "qmv_mma", 21, W, K, x[r:r + 64], f32=False).view(np.uint16)), r
+    plain = gpu.compile("qmv_mma", "qmv_no_piece_%d" % K, GF=21, KD=K, YT_F32=0)
+    for kern, rows in ((plain, 65), (k, 513)):
+        with pytest.raises(GpuError):
+            run(kern, rows)
