@@ -92,7 +92,7 @@ struct qw_engine {
     // scratch
     qw_buf ctl_h{}, ctl_d{}, h{}, h2{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
-    // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN.  Eight times the tokens choose far fewer than eight times the
+    // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN on IQ3X.  Eight times the tokens choose far fewer than eight times the
     // experts, so a wider piece reads and decodes fewer expert weights per token.
     int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
     qw_buf ctl_p{}, ffn_scr_w{};
@@ -376,7 +376,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
         mn.push_back({"NORM", 1});
         ok = compile(e, "moe_route", "norm_moe_route", mn, &e->k_route_n);
     }
-    if (ok && c.ep_size == 1 && e->ffn_fused && c.max_ctx > ROWS) {
+    if (ok && c.ep_size == 1 && e->ffn_iq3x && c.max_ctx > ROWS) {
         e->piece_rows = PROWS;
         auto mw = md;
         mw.push_back({"SELECT", 0});

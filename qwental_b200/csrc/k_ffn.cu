@@ -794,11 +794,12 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     p.Wd = L.buf<uint8_t>(6);
     p.Wg = Wg;
     p.Sg = Sg;
-    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 512 rows of tokens (one GPU only)
+    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 512 rows of tokens; one GPU only
     const bool wide = L.def("WIDE", 0) != 0;
     p.sync = L.buf<unsigned>(8);
     QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I) : MOE_FFN_SCRATCH_BYTES(I)));
-    QW_CHECK_ARG(!wide || (L.def("EPX", 0) <= 1 && L.def("PROBE", 0) == 0));
+    // and only IQ3X: with one block per SM a share of its items would not fit FFN_RECS.
+    QW_CHECK_ARG(!wide || (x4 && L.def("EPX", 0) <= 1 && L.def("PROBE", 0) == 0));
     p.H = (__half *)((uint8_t *)p.sync + (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
     p.Sd = shared ? L.buf<uint8_t>(7) : nullptr;
     p.x = L.buf<__half>(4);
@@ -844,8 +845,7 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     const bool probe = L.def("PROBE", 0) != 0;  // PROBE defined 1: the copy-only twin (outputs are not written)
     // HALF defined 1: the variant for few items (IQ3X; the other kinds ignore it)
     const bool half = L.def("HALF", 0) != 0;
-    auto kern = x4 && half && !probe && !wide ? moe_ffn_k<false, 1, 0, true>
-                : wide ? (x4 ? moe_ffn_k<false, 1, 1> : moe_ffn_k<false, 0, 1>)
+    auto kern = wide ? moe_ffn_k<false, 1, 1> : x4 && half && !probe ? moe_ffn_k<false, 1, 0, true>
                 : x4 ? (probe ? moe_ffn_k<true, 1, 0> : moe_ffn_k<false, 1, 0>) : (probe ? moe_ffn_k<true, 0, 0> : moe_ffn_k<false, 0, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -66,3 +66,22 @@ def test_wide_pieces_equal_stepping_every_token(gpu):
                 assert np.array_equal(a, b), n
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("ffn", ["fused", "split"])
+def test_prompts_with_the_other_expert_kernels(gpu, ffn, monkeypatch):
+    """Engines whose experts are not re-coded run prompts in pieces of 64: nearly all of 512 experts chosen, several pieces."""
+    from qwental_b200.engine import Engine, wide_cfg
+    monkeypatch.setenv("QW_MOE_FFN", ffn)
+    e = Engine(gpu, wide_cfg(experts=512, topk=10, max_slots=2))
+    try:
+        text = np.random.default_rng(7).integers(0, e.cfg.vocab, 200).astype(np.int32)
+        e.prefill(0, text[:1])
+        for n in range(2, len(text) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+        got = e.prefill(1, text)
+        assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32))
+        for a, b in zip(state_of(e, 1), state_of(e, 0)):
+            assert np.array_equal(a, b)
+    finally:
+        e.close()
