@@ -425,7 +425,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->qb, RB * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
          new_buf(e, &e->ya, RB * e->KA * 2) && new_buf(e, &e->ob, RB * e->D * 2) && new_buf(e, &e->mo, B * e->D * 2) &&
          new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids, B * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
-         new_buf(e, &e->logits_h, (size_t)c.max_slots * e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
+         new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
          new_buf(e, &e->msel, (size_t)e->L * e->sel_bytes) && new_buf(e, &e->Hhi, B * (e->TOPK + 1) * e->I * 2) &&
          new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, RB * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
     if (ok) ok = qw_buf_zero(g, &e->msel, 0, e->msel.size) && qw_buf_zero(g, &e->Pg, 0, e->Pg.size) && qw_buf_zero(g, &e->Hhi, 0, e->Hhi.size) &&
@@ -998,7 +998,14 @@ extern "C" int qw_engine_par_step_into(qw_engine *e, const int *sids, const int3
 }
 
 extern "C" const float *qw_engine_par_step(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms) {
-    if (!e || qw_engine_par_step_into(e, sids, toks, B, (float *)e->logits_h.ptr, gpu_ms) != 0) return nullptr;
+    if (!e) return nullptr;
+    if (B > 1 && B <= (int)e->slots.size() && e->logits_h.size < (size_t)B * e->V * 4) {  // one row at first (prompts need no more): pinned memory is slow to get
+        qw_buf all{};
+        if (!new_buf(e, &all, e->slots.size() * e->V * 4, QW_BUF_HOSTIO)) return nullptr;
+        qw_buf_free(&e->logits_h);
+        e->logits_h = all;
+    }
+    if (qw_engine_par_step_into(e, sids, toks, B, (float *)e->logits_h.ptr, gpu_ms) != 0) return nullptr;
     return (const float *)e->logits_h.ptr;
 }
 

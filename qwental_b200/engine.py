@@ -100,8 +100,8 @@ class _HostRows:
 
     def __init__(self, gpu: Gpu, rows: int, cols: int):
         self.gpu, self.cols, self.size, self.made, self.free = gpu, cols, rows * cols * 4, 0, []
-        if self.size >= self.SMALL:  # two to begin with: a loop's next step runs while the last one's logits are still held
-            self.free = [b for b in (self._make(), self._make()) if b]
+        if self.size >= self.SMALL:  # one to begin with; a loop that holds the last step's logits during the next one gets its second there
+            self.free = [b for b in [self._make()] if b]
 
     def _make(self):
         try:
