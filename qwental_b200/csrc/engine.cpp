@@ -106,6 +106,7 @@ struct qw_engine {
     // Up to four rows on one GPU: the residual add + norm before the router runs inside the router's launch, which writes the residual
     // stream to the other one of h and h2 (h_last: where the last pass left it).
     qw_kernel *k_route_n = nullptr;
+    qw_kernel *k_epi_e = nullptr, *k_gdn_e = nullptr;  // Gated DeltaNet with EARLY, where a step may use it
     const qw_buf *h_last = nullptr;
     bool ep_ready = false;
     // fused exchange: each rank's down projection stores its rows straight into every rank's Pg (peer memory)
@@ -341,13 +342,16 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
     // QW_MOE_FFN=split keeps the two-launch family, QW_MOE_FFN=fused runs moe_ffn on the raw IQ3_S blocks
     e->ffn_fused = e->D == 2048 && e->I == 512 && !(fm && !strcmp(fm, "split"));
     e->ffn_iq3x = e->ffn_fused && !(fm && !strcmp(fm, "fused"));
-    // EARLY: the GDN kernels read their per-slot state before they wait for the previous kernel.  Allowed when every layer ends in a
-    // launch that fills all SMs (moe_ffn) and there are at least two layers: see gdn_fstep_k.
-    std::vector<std::pair<const char *, long>> gd = {{"HK", c.hk}, {"HV", c.hv}, {"DK", 128}, {"DV", 128}, {"GDN_TILED", 1},
-                                                      {"EARLY", e->ffn_fused && e->L >= 2 ? 1 : 0}};
+    std::vector<std::pair<const char *, long>> gd = {{"HK", c.hk}, {"HV", c.hv}, {"DK", 128}, {"DV", 128}, {"GDN_TILED", 1}};
     ok = ok && compile(e, "dn_epi", "dn_epi", gd, &e->k_epi) && compile(e, "gdn_fstep", "gdn_fstep", gd, &e->k_gdn) &&
          compile(e, "dn_epi_seq", "dn_epi_seq", gd, &e->k_epi_seq) && compile(e, "gdn_seq", "gdn_seq", gd, &e->k_gdn_seq) &&
          compile(e, "gdn_gate", "gdn_gate", gd, &e->k_gdn_gate) && compile(e, "par_chunk", "par_chunk", {}, &e->k_chunk);
+    // EARLY: the GDN kernels read the slot table and their per-slot state before they wait for the previous kernel.  Where every layer ends in
+    // a launch that fills all SMs (moe_ffn), the layers of a step from the third on may: see gdn_fstep_k and encode_step.
+    if (ok && e->ffn_fused && e->L > 2) {
+        gd.push_back({"EARLY", 1});
+        ok = compile(e, "dn_epi", "dn_epi_early", gd, &e->k_epi_e) && compile(e, "gdn_fstep", "gdn_fstep_early", gd, &e->k_gdn_e);
+    }
     // expert-parallel: the shared expert is computed by rank 0 only, so the exchange can sum whole buffers
     std::vector<std::pair<const char *, long>> md = {{"E", e->E}, {"EL", e->EL}, {"D", D}, {"I", e->I}, {"TOPK", e->TOPK},
                                                       {"SHARED", c.ep_rank == 0 ? 1 : 0}, {"RESID", 0}};
@@ -735,10 +739,13 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             }
             enc_out_proj(e->k_qmv_o_a, e->k_qmv_oa_w, e->k_qmv_o_a_x, w.w_out, e->KA, &e->ya);
         } else {
+            // Reading ahead of the wait needs two FFN launches between par_begin, which writes the slot table, and the reader; a step whose
+            // control block is already on the device (fed by the step before, which the host has waited for) has no such writer.
+            const bool early = !piece && e->k_gdn_e && (l >= 2 || !from_host);
             enc_qmv(b, e->k_qmv_in_g, e->k_qmv_in_w, &e->dense, w.w_in, e->gdn_rows, D, &e->x, &e->proj, nbl, e->gdn_rows, xo);
             const size_t so = (w.small + 2 * D) * 4, sa = so + (size_t)e->C * 16;
             const dn_epi_args ea = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
-            qw_batch_kernel(b, piece ? e->k_epi_seq : e->k_epi);
+            qw_batch_kernel(b, piece ? e->k_epi_seq : early ? e->k_epi_e : e->k_epi);
             qw_batch_buf(b, 0, &e->proj, 0);
             qw_batch_buf(b, 1, &e->small, so);
             qw_batch_buf(b, 2, &e->cstate, 0);
@@ -751,7 +758,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_bytes(b, 9, &ea, sizeof ea);
             qw_batch_dispatch(b, (e->C + 2 * e->HV + 255) / 256, nbl, 1, 256, 1, 1);
             const gdn_args ga = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
-            qw_batch_kernel(b, piece ? e->k_gdn_seq : e->k_gdn);
+            qw_batch_kernel(b, piece ? e->k_gdn_seq : early ? e->k_gdn_e : e->k_gdn);
             qw_batch_buf(b, 0, &e->cv, 0);
             qw_batch_buf(b, 1, &e->la, 0);
             qw_batch_buf(b, 2, &e->be, 0);

@@ -36,8 +36,8 @@ __global__ void __launch_bounds__(256) dn_epi_k(const __half *proj, const float 
     const uint32_t g = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
     const __half *pr = proj + (size_t)t * a.proj_stride;
     if (g < C) {
-        // early: the conv state (last written by this kernel one step ago), the static weights and the slot table are read before
-        // the wait for the projection (see gdn_fstep_k for when that is allowed)
+        // early: the slot table, the conv state and the static weights are read before the wait for the projection (see gdn_fstep_k for
+        // when that is allowed)
         float *st = pool + ((size_t)sids[t] * a.nlayers + a.layer) * 3 * C;
         const float s0 = st[g], s1 = st[C + g], s2 = st[2 * C + g];
         const float4 w = *(const float4 *)(cw + 4 * (size_t)g);
@@ -149,11 +149,12 @@ __global__ void __launch_bounds__(512, 2) gdn_fstep_k(const __half *cv, const fl
     const __half *row = cv + (size_t)t * C;
     float4 *S = (float4 *)(pool + (((size_t)sids[t] * a.nlayers + a.layer) * HV + hv) * DK * DV) + c4;
 
-    // State rows into registers: the long-latency part.  With EARLY defined 1 they are requested before the wait for the previous
-    // kernel.  The state of this (slot, layer, head) was last written by this kernel one step ago and the slot table at the step's
-    // start.  A launch cannot begin before every block of its predecessor has started; the host defines EARLY only when at least two
-    // launches that fill every SM (moe_ffn: as many blocks as fit the device) lie between those writers and this launch -- the later
-    // one cannot have started all its blocks before the earlier one has left, and that one has waited for everything before it.
+    // State rows into registers: the long-latency part.  With EARLY defined 1 they, and the slot id they are found by, are requested before the
+    // wait for the previous kernel.  The state was last written in an earlier batch, which the host has waited for; the slot table by
+    // par_begin at the start of this step, possibly.  A launch cannot begin before every block of its predecessor has started, but that alone says
+    // little: the small launches of a layer can all be resident while par_begin still reads the host's memory.  So the host runs this form
+    // only behind two launches that fill every SM (moe_ffn: as many blocks as fit the device) after par_begin: the later one cannot have
+    // started all its blocks before the earlier one has left, and that one has waited for everything before it.
     float4 s[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) s[i] = S[(size_t)(8 * rq + i) * (DV / 4)];

@@ -284,3 +284,48 @@ def test_step_logits_belong_to_the_caller(gpu):
     for x, y in zip(held, want):
         assert np.array_equal(x.view(np.uint32), y.view(np.uint32))
     b.close()
+
+
+def test_slot_table_is_read_ahead_only_behind_two_full_launches(gpu):
+    """A step that begins with the control block's copy (par_begin) writes the slot table its GDN kernels find their state by: up to the second
+    FFN launch after it they wait for the previous kernel first (the plain forms); from the third layer on, and in steps fed on the device, they
+    may read ahead.  And rows that change their slots from step to step get the states of their own slots."""
+    import ctypes as C
+    from qwental_b200.engine import Engine, wide_cfg
+    a, b = Engine(gpu, wide_cfg(layers=6)), Engine(gpu, wide_cfg(layers=6))
+    try:
+        def kernels(run):
+            gpu.L.qw_profile_enable(gpu.g, True)
+            run()
+            names = [gpu.L.qw_profile_get(gpu.g, i, C.byref(C.c_double())).decode() for i in range(gpu.L.qw_profile_count(gpu.g))]
+            gpu.L.qw_profile_enable(gpu.g, False)
+            return names
+        gdn = lambda names: [n for n in names if n.startswith(("dn_epi", "gdn_fstep"))]
+        for e in (a, b):
+            for s in range(8):
+                e.seed_slot(s, 100 + 30 * s, 50 + s)
+        plain, ahead = ["dn_epi", "gdn_fstep"], ["dn_epi_early", "gdn_fstep_early"]
+        k1 = kernels(lambda: a.step([0, 1], [1, 2]))
+        assert "par_begin" in k1 and gdn(k1) == 2 * plain + 3 * ahead  # layers 0, 1 | 2, 4, 5 (3 is attention)
+        k2 = kernels(lambda: a.decode_greedy([2, 3], [5, 6], 2))  # what is profiled is the last batch: the step fed on the device
+        assert "par_begin" not in k2 and gdn(k2) == 5 * ahead
+        b.step([0, 1], [1, 2])
+        b.decode_greedy([2, 3], [5, 6], 2)
+        gpu.L.qw_gpu_set_graphs(gpu.g, True)
+        rng = np.random.default_rng(8)
+        try:
+            for _ in range(40):
+                rows = rng.permutation(8)[:rng.integers(1, 5)]
+                toks = rng.integers(0, a.cfg.vocab, len(rows))
+                la, _ = a.step(rows, toks)
+                for i, s in enumerate(rows):
+                    lb, _ = b.step([s], toks[i:i + 1])
+                    assert np.array_equal(la[i].view(np.uint32), lb[0].view(np.uint32))
+        finally:
+            gpu.L.qw_gpu_set_graphs(gpu.g, False)
+        for s in range(8):
+            assert np.array_equal(a.tap("sstate", s, np.uint32), b.tap("sstate", s, np.uint32))
+            assert np.array_equal(a.tap("cstate", s, np.uint32), b.tap("cstate", s, np.uint32))
+    finally:
+        a.close()
+        b.close()
