@@ -540,6 +540,7 @@ extern "C" int qw_engine_par_seed(qw_engine *e, int sid, int ctx_len, unsigned l
     enc_fill(e, b, &e->cstate, (size_t)sid * cst * 4, {mix64(seed ^ 0x434Full), cst, 0, 4, 1.0f, 0.f});
     if (qw_batch_end(b) < 0) {
         e->fail("slot seeding failed");
+        release_slot(e, sid);
         return -1;
     }
     return 0;
@@ -1166,11 +1167,17 @@ extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32
         if (prompt[i] < 0 || prompt[i] >= e->V) return e->fail("par_prefill: token %d out of range", prompt[i]), nullptr;
     if (e->slots[sid].used) release_slot(e, sid);
     Slot &s = e->slots[sid];
-    if (!reserve_pages(e, sid, np + 1)) return nullptr;
+    // a prompt that fails leaves its slot free: pieces of it may be in the state already, and no step must run on that
+    auto failed = [&](const char *what) {
+        e->fail("par_prefill: %s", what);
+        release_slot(e, sid);
+        return (const float *)nullptr;
+    };
+    if (!reserve_pages(e, sid, np + 1)) return release_slot(e, sid), nullptr;
     s.used = true;
     s.pos = 0;
     s.last_use = ++e->clock;
-    if (!qw_buf_upload(e->g, &e->prompt_d, 0, prompt, (size_t)np * 4)) return e->fail("par_prefill: prompt upload failed"), nullptr;
+    if (!qw_buf_upload(e->g, &e->prompt_d, 0, prompt, (size_t)np * 4)) return failed("prompt upload failed");
     std::vector<qw_batch *> flight;  // submitted, oldest first: a few pieces ahead keep the device busy, more would only hold host memory
     bool ok = true;
     auto submit = [&](qw_batch *b) {
@@ -1203,8 +1210,8 @@ extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32
         submit(b);
     }
     for (qw_batch *b : flight) ok = qw_batch_wait(b) >= 0 && ok;
-    if (!ok) return after_failed_step(e), e->fail("par_prefill: device batch failed"), nullptr;
-    if (!qw_buf_download(e->g, &e->logits, 0, e->logits_h.ptr, (size_t)e->V * 4)) return e->fail("par_prefill: logits copy failed"), nullptr;
+    if (!ok) return after_failed_step(e), failed("device batch failed");
+    if (!qw_buf_download(e->g, &e->logits, 0, e->logits_h.ptr, (size_t)e->V * 4)) return failed("logits copy failed");
     s.pos = np;
     s.last_use = ++e->clock;
     e->last_sids.assign(1, sid);

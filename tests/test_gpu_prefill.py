@@ -85,3 +85,28 @@ def test_prompts_with_the_other_expert_kernels(gpu, ffn, monkeypatch):
             assert np.array_equal(a, b)
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("n,kernel,family,broken,whole", [(40, "gdn_gate", "gdn_gate", dict(DV=64), dict()), (540, "kb_embed", "kb_embed", dict(ROWS=8), dict())])
+def test_a_failed_prompt_frees_its_slot(gpu, n, kernel, family, broken, whole):
+    """A launch that the host refuses (a kernel specialised so that its argument check fails) in the first piece, or in the last one after a piece
+    of 512 tokens has gone through: the prompt fails, its slot is free -- no step runs on what the pieces left -- and the same prompt works afterwards."""
+    from qwental_b200.engine import Engine, wide_cfg
+    from qwental_b200.gpu import GpuError
+    e = Engine(gpu, wide_cfg(max_slots=2, kv_pages=4))
+    try:
+        text = np.random.default_rng(n).integers(0, e.cfg.vocab, n).astype(np.int32)
+        want = e.prefill(1, text)
+        e.finish(1)
+        gpu.compile(family, kernel, HK=16, HV=32, **broken)
+        with pytest.raises(GpuError):
+            e.prefill(0, text)
+        gpu.compile(family, kernel, HK=16, HV=32, **whole)
+        assert e.pos(0) == -1 and e.mem() == 0
+        with pytest.raises(GpuError, match="not in use"):
+            e.step([0], [1])
+        got = e.prefill(1, text)  # all pages are there again, and nothing of the failed launches is left
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        assert e.pos(1) == n
+    finally:
+        e.close()
