@@ -986,35 +986,47 @@ void after_failed_step(qw_engine *e) {
 
 }  // namespace
 
-extern "C" int qw_engine_par_step_into(qw_engine *e, const int *sids, const int32_t *toks, int B, float *logits, double *gpu_ms) {
+namespace {
+// A step whose logits go to `logits`, or to logits_h where that is nullptr: returns where they are, nullptr on failure.  logits_h holds one row at
+// first (prompts need no more, and pinned memory is slow to get); the first step of several rows gets one for all slots.  The old one, which
+// the caller may still be reading, goes only when that step has succeeded.
+const float *step_logits(qw_engine *e, const int *sids, const int32_t *toks, int B, float *logits, double *gpu_ms) {
     const double t0 = qw_now();
-    if (e && !logits) return e->fail("par_step: no buffer for the logits"), -1;
     const uint32_t mc = begin_step(e, sids, toks, B, 1);
-    if (!mc) return -1;
+    if (!mc) return nullptr;
+    qw_buf grown{};
+    if (!logits && e->logits_h.size < (size_t)B * e->V * 4 && !new_buf(e, &grown, e->slots.size() * e->V * 4, QW_BUF_HOSTIO)) return nullptr;
+    float *dst = logits ? logits : (float *)(grown.handle ? grown.ptr : e->logits_h.ptr);
+    auto failed = [&](const char *what) {
+        e->fail("par_step: %s", what);
+        qw_buf_free(&grown);
+        return (const float *)nullptr;
+    };
     qw_batch *b = qw_batch_begin(e->g, false);
     encode_step(e, b, (uint32_t)B, mc, true, 0);
     const double secs = qw_batch_end(b);
-    if (secs < 0) return after_failed_step(e), e->fail("par_step: device batch failed"), -1;
+    if (secs < 0) return after_failed_step(e), failed("device batch failed");
     for (int j = 0, n; j < B; j += n) {  // device row j is the caller's row perm[j]: runs of consecutive rows travel together
         for (n = 1; j + n < B && e->perm[j + n] == e->perm[j] + n; n++) {}
-        if (!qw_buf_download(e->g, &e->logits, (size_t)j * e->V * 4, logits + (size_t)e->perm[j] * e->V, (size_t)n * e->V * 4))
-            return e->fail("par_step: logits copy failed"), -1;
+        if (!qw_buf_download(e->g, &e->logits, (size_t)j * e->V * 4, dst + (size_t)e->perm[j] * e->V, (size_t)n * e->V * 4)) return failed("logits copy failed");
+    }
+    if (grown.handle) {
+        qw_buf_free(&e->logits_h);
+        e->logits_h = grown;
     }
     if (gpu_ms) *gpu_ms = secs * 1e3;
     end_step(e, sids, B, 1, (qw_now() - t0) * 1e3);
-    return 0;
+    return dst;
+}
+}  // namespace
+
+extern "C" int qw_engine_par_step_into(qw_engine *e, const int *sids, const int32_t *toks, int B, float *logits, double *gpu_ms) {
+    if (e && !logits) return e->fail("par_step: no buffer for the logits"), -1;
+    return step_logits(e, sids, toks, B, logits, gpu_ms) ? 0 : -1;
 }
 
 extern "C" const float *qw_engine_par_step(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms) {
-    if (!e) return nullptr;
-    if (B > 1 && B <= (int)e->slots.size() && e->logits_h.size < (size_t)B * e->V * 4) {  // one row at first (prompts need no more): pinned memory is slow to get
-        qw_buf all{};
-        if (!new_buf(e, &all, e->slots.size() * e->V * 4, QW_BUF_HOSTIO)) return nullptr;
-        qw_buf_free(&e->logits_h);
-        e->logits_h = all;
-    }
-    if (qw_engine_par_step_into(e, sids, toks, B, (float *)e->logits_h.ptr, gpu_ms) != 0) return nullptr;
-    return (const float *)e->logits_h.ptr;
+    return step_logits(e, sids, toks, B, nullptr, gpu_ms);
 }
 
 extern "C" const int32_t *qw_engine_par_step_greedy(qw_engine *e, const int *sids, const int32_t *toks, int B, double *gpu_ms) {

@@ -329,3 +329,37 @@ def test_slot_table_is_read_ahead_only_behind_two_full_launches(gpu):
     finally:
         a.close()
         b.close()
+
+
+def test_a_rejected_step_leaves_the_last_logits_readable(gpu):
+    """qw_engine_par_step gets memory for all rows with the first step of several rows.  The logits of a prompt stay where they are while such
+    calls are rejected (a slot that is not in use, a slot twice, a token out of range) or fail on the device; the next good step replaces them."""
+    import ctypes as C
+    from qwental_b200.engine import Engine, tiny_cfg
+    e = Engine(gpu, tiny_cfg())
+    try:
+        e.seed_slot(3, 50, 1)
+        e.seed_slot(4, 60, 2)
+        prompt = np.array([5, 17, 300], np.int32)
+        L, V = e.L, e.cfg.vocab
+        ip, i32p = C.POINTER(C.c_int), C.POINTER(C.c_int32)
+        p = C.cast(L.qw_engine_par_prefill(e.e, 0, prompt.ctypes.data, 3, None), C.POINTER(C.c_float))
+        want = np.ctypeslib.as_array(p, shape=(V,)).copy()
+
+        def step(sids, toks):
+            s, t = np.array(sids, np.int32), np.array(toks, np.int32)
+            return L.qw_engine_par_step(e.e, s.ctypes.data_as(ip), t.ctypes.data_as(i32p), len(s), None)
+        for sids, toks in (([0, 5], [1, 1]), ([3, 3], [1, 1]), ([3, 4], [1, V])):
+            assert not step(sids, toks)
+            assert np.array_equal(np.ctypeslib.as_array(p, shape=(V,)).view(np.uint32), want.view(np.uint32)), sids
+        gpu.compile("kb_embed", "kb_embed", ROWS=1)  # two rows are refused at launch
+        assert not step([3, 4], [1, 2])
+        gpu.compile("kb_embed", "kb_embed")
+        assert np.array_equal(np.ctypeslib.as_array(p, shape=(V,)).view(np.uint32), want.view(np.uint32))
+        q = step([3, 4], [1, 2])
+        both = np.ctypeslib.as_array(q, shape=(2, V)).copy()
+        e.seed_slot(4, 60, 2)
+        alone = step([4], [2])
+        assert np.array_equal(np.ctypeslib.as_array(alone, shape=(V,)).view(np.uint32), both[1].view(np.uint32))
+    finally:
+        e.close()
