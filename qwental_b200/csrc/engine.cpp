@@ -434,7 +434,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, RB * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
     if (ok) ok = qw_buf_zero(g, &e->msel, 0, e->msel.size) && qw_buf_zero(g, &e->Pg, 0, e->Pg.size) && qw_buf_zero(g, &e->Hhi, 0, e->Hhi.size) &&
                  qw_buf_zero(g, &e->Hlo, 0, e->Hlo.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) &&
-                 qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size) && qw_buf_zero(g, &e->rcnt, 0, e->rcnt.size);  // rows past a slot's length are multiplied by probability 0: keep them finite
+                 qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size) && qw_buf_zero(g, &e->rcnt, 0, e->rcnt.size);
     if (ok && e->ffn_fused) ok = new_buf(e, &e->ffn_scr, MOE_FFN_SCRATCH_BYTES(e->I)) && qw_buf_zero(g, &e->ffn_scr, 0, e->ffn_scr.size);
     if (ok && e->piece_rows > ROWS)
         ok = new_buf(e, &e->ctl_p, 3 * PROWS * 4) && new_buf(e, &e->ffn_scr_w, MOE_FFN_SCRATCH_BYTES_WIDE(e->I)) && qw_buf_zero(g, &e->ffn_scr_w, 0, e->ffn_scr_w.size);

@@ -421,6 +421,13 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
             const uint32_t b0 = to_b(h01), b1 = to_b(h23), c0 = to_b(r01), c1 = to_b(r23);
             if (STG == 1 && !mbar_wait(&bars[1], vph & 1)) { ok = false; break; }
             vph++;
+            if (const uint32_t left = cur.n - step * 16; left < 16) {
+                // Rows of the tile past the slot's length: their probabilities are 0, but the page may hold anything there -- a later token of the same
+                // prompt, or what an earlier conversation left -- and 0 times an infinity or a NaN would reach every head.  Zeros instead.
+                for (uint32_t r = left; r < 16; r++) *(uint4 *)(Vb + so + (lane >> 3) * 2048 + r * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async();  // before the next copy into this tile
+                __syncwarp();
+            }
             // four dim tiles at a time: the two MMAs of a tile depend on one another, back to back the second would wait for the first
 #pragma unroll
             for (int dq = 0; dq < 4; dq++) {

@@ -204,3 +204,20 @@ def test_attention_core_forms_agree(gpu):
     y = attn_run(gpu, core, d, range(len(lens)))
     for r in range(len(lens)):
         assert np.array_equal(attn_run(gpu, core, d, [r])[0].view(np.uint16), y[r].view(np.uint16)), lens[r]
+
+
+@pytest.mark.parametrize("family", ["qsa_attn", "qsa_attn_simt"])
+@pytest.mark.parametrize("lens", [[0, 13, 14, 15, 16, 30, 31, 253, 254, 255, 256, 300], [0, 5, 15, 100, 254, 700] * 10 + [1023, 1024, 1039, 1500]])
+def test_what_lies_behind_a_slots_length_does_not_matter(gpu, family, lens):
+    """Rows of a slot's last page past its length: infinities and NaN there (a later token of a prompt whose values overflowed, or an earlier
+    conversation's) change no bit.  Few tasks and many: both forms of the core; 16 tokens per tile."""
+    core, d = attn_setup(gpu, lens, seed=3 + len(lens), family=family)
+    clean = attn_run(gpu, core, d, range(len(lens)))
+    assert np.isfinite(clean.astype(np.float32)).all()
+    pool = core.pool.download(np.float16, core.pool.size // 2).reshape(-1, 2, 2, KVH, 256, HD)
+    ptab = core.ptab.download(np.int32, core.ptab.size // 4).reshape(-1, d["max_pages"])
+    for r, L in enumerate(lens):
+        rest = pool[ptab[d["sids"][r], L // 256], 1, :, :, L % 256 + 1:]
+        rest[:] = [np.inf, -np.inf, np.nan][r % 3]
+    core.pool.upload(pool)
+    assert np.array_equal(attn_run(gpu, core, d, range(len(lens))).view(np.uint16), clean.view(np.uint16))
