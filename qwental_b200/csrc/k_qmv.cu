@@ -384,13 +384,19 @@ __global__ void __launch_bounds__(WARPS * TEAMS * 32, (WARPS * TEAMS == 8) ? 2 :
                     for (int i = 0; i < 4; i++) half_mma(A, i, zr, va[i], vb[i], (uint32_t)ps * 16 + 8 < p.nb, accp[ps]);
                 }
             };
-            static_assert(GF == 21, "Q8_0 runs more than 16 tokens in the wide form");
-            const Iq3sHdr h0 = iq3s_hdr(rows, t), h1 = iq3s_hdr(rows + 8 * p.rs, t);
             UnitHalf A;
-            iq3s_decode_half<0, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
-            run_half(A, 0);
-            iq3s_decode_half<1, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
-            run_half(A, 1);
+            if constexpr (GF == 21) {
+                const Iq3sHdr h0 = iq3s_hdr(rows, t), h1 = iq3s_hdr(rows + 8 * p.rs, t);
+                iq3s_decode_half<0, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
+                run_half(A, 0);
+                iq3s_decode_half<1, TS>(rows, rows + 8 * p.rs, t, h0, h1, tabc, A);
+                run_half(A, 1);
+            } else {
+                q8_decode_half<0>(rows, rows + 8 * p.rs, t, A);
+                run_half(A, 0);
+                q8_decode_half<1>(rows, rows + 8 * p.rs, t, A);
+                run_half(A, 1);
+            }
 #pragma unroll
             for (int ps = 0; ps < 4; ps++) {
                 if ((uint32_t)ps >= passes) break;
@@ -449,7 +455,7 @@ template <int GF, int WARPS, int TEAMS, bool F32OUT, bool MP = false>
 static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) {
     // more than 16 tokens (at most 64): the form that decodes a unit once for all passes
     static const bool loop_passes = [] { const char *v = getenv("QW_QMV_PASSES"); return v && !strcmp(v, "loop"); }();  // for A/B timing
-    if constexpr (!MP && GF == 21) {
+    if constexpr (!MP) {
         if (p.nb > 16 && p.nb <= 64 && !loop_passes) return qmv_mma2_go<GF, WARPS, TEAMS, F32OUT, true>(p, sm_count, st);
     }
     const size_t smem = 128 + (GF == 21 ? 65536 : 0) + (size_t)TEAMS * 2 * WARPS * 2 * 32 * 16 +
@@ -467,7 +473,7 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     return cudaGetLastError();
 }
 
-// ---- More than 16 tokens at K = 2048: a block owns a run of 16-row tiles and walks K in units of 256, so the activations reach a
+// ---- More than 16 tokens and many rows at K = 2048: a block owns a run of 16-row tiles and walks K in units of 256, so the activations reach a
 // block once per round of up to RG tiles instead of once per tile.  (The form above re-reads 256 KB of activations from L2 for each
 // 16 rows at 64 tokens: 2.5 GB for an output head of 330 MB -- L2 bandwidth was its bound.)  Two rings feed the block: weights (16-row boxes
 // of one Q8_0 unit, or of two IQ3_S units, whose 110 bytes do not start on 16-byte boundaries) and activations (one unit of all tokens,
@@ -708,6 +714,25 @@ static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }
 
+// More than 16 tokens at K = 2048: the wide form, or the one that decodes a unit once for all passes of 16 tokens (qmv_mma2 with MP)?  A
+// block of the wide form walks K alone and costs the same for one row tile as for a few, and its copies and barriers come first; MP splits
+// K over 8 warps, but reads the activations once per tile: the more tokens, the fewer tiles make up for it.  Time of MP over time of wide on a
+// B200, 148 SMs, IQ3_S / Q8_0:
+//   row tiles        17 tokens     24 tokens     32 tokens     41 tokens     48 tokens     64 tokens
+//    16             0.85 / 0.69   0.85 / 0.69   0.88 / 0.72   0.84 / 0.77   0.87 / 0.77   0.86 / 0.69
+//   128             0.83 / 0.83   0.85 / 0.86   0.89 / 0.89   0.88 / 0.97   0.93 / 1.00   0.92 / 0.89
+//   185             0.79 / 0.75   0.85 / 0.76   0.92 / 0.85   0.96 / 1.00   1.05 / 1.12   1.10 / 1.09
+//   296             0.81 / 0.78   0.85 / 0.83   0.92 / 0.88   0.99 / 1.05   1.09 / 1.16   1.13 / 1.15
+//   370             1.02 / 0.93   1.05 / 1.05   1.11 / 1.15   1.19 / 1.25   1.27 / 1.34   1.31 / 1.34
+//   592             0.96 / 0.97   1.02 / 1.05   1.10 / 1.13   1.24 / 1.33   1.36 / 1.47   1.44 / 1.49
+//   772             1.02 / 1.02   1.05 / 1.10   1.14 / 1.21   1.31 / 1.39   1.41 / 1.50   1.52 / 1.57
+// So: wide beyond 4, 2 or 1 row tiles per SM (up to 21, up to 42, more tokens).  One more tile than that costs MP little, a last round for few
+// teams, and wide a whole round (297 tiles: 0.85 to 1.05): an eighth is added.
+static bool qmv_wide_pays(uint32_t items, uint32_t nb, uint32_t sms) {
+    const uint32_t per_sm = nb <= 21 ? 4 : nb <= 42 ? 2 : 1;
+    return 8 * items > (8 * per_sm + 1) * sms;
+}
+
 // The grid and block given by the host are ignored (the kernels are persistent and size themselves).  Defines: GF (21 = IQ3_S,
 // 8 = Q8_0), KD, YT_F32; EPX = ranks of a slot-sharded projection whose rows go to every rank (see below).
 static cudaError_t launch_qmv_mma(const QwLaunch &L) {
@@ -758,8 +783,8 @@ static cudaError_t launch_qmv_mma(const QwLaunch &L) {
 #define GO(G, M)                                                        \
     return f32 ? qmv_mma_nt<G, M, true>(p, L.sm_count, L.stream) : qmv_mma_nt<G, M, false>(p, L.sm_count, L.stream)
     // More than 16 tokens: the activations no longer fit a warp's registers, and the wide form reads them from shared memory.  (The
-    // exchange between ranks is built into qmv_mma2 only.)
-    if (K == 2048 && a.nb > 16 && epx <= 1) {
+    // exchange between ranks is built into qmv_mma2 only, more than 64 tokens into the wide form.)
+    if (K == 2048 && a.nb > 16 && epx <= 1 && (a.nb > 64 || qmv_wide_pays(p.items, a.nb, (uint32_t)L.sm_count))) {
         if (gf == 21) return f32 ? qmv_wide_go<21, true>(p, L.sm_count, L.stream) : qmv_wide_go<21, false>(p, L.sm_count, L.stream);
         return f32 ? qmv_wide_go<8, true>(p, L.sm_count, L.stream) : qmv_wide_go<8, false>(p, L.sm_count, L.stream);
     }

@@ -418,6 +418,22 @@ __device__ __forceinline__ void unit_mma2_q8(uint32_t u0, uint32_t u1, int t, co
     sub_mma2_q8<7>(u0, u1, t, zr, xa[7], xb[7], second, acc);
 }
 
+// Q8_0 counterpart of iq3s_decode_half: blocks 4 HF .. 4 HF + 3 of the unit
+template <int HF>
+__device__ __forceinline__ void q8_decode_half(uint32_t u0, uint32_t u1, int t, UnitHalf &A) {
+    uint32_t wa[4], wb[4];
+#define QW_HALF_SUB(I)                                                            \
+    A.da[I] = q8_sub_h<4 * HF + I>(u0 + 8 * t, u0, wa);                           \
+    A.db[I] = q8_sub_h<4 * HF + I>(u1 + 8 * t, u1, wb);                           \
+    A.a0[I][0] = wa[0]; A.a0[I][1] = wb[0]; A.a0[I][2] = wa[1]; A.a0[I][3] = wb[1]; \
+    A.a1[I][0] = wa[2]; A.a1[I][1] = wb[2]; A.a1[I][2] = wa[3]; A.a1[I][3] = wb[3];
+    QW_HALF_SUB(0)
+    QW_HALF_SUB(1)
+    QW_HALF_SUB(2)
+    QW_HALF_SUB(3)
+#undef QW_HALF_SUB
+}
+
 __host__ __device__ constexpr int unit_bytes(int GF) { return GF == 21 ? 110 : 272; }
 
 }  // namespace qw

@@ -144,3 +144,17 @@ def test_matvec_of_a_prompt_piece_equals_groups_of_64(gpu, N, K, B):
     for kern, rows in ((plain, 65), (k, 513)):
         with pytest.raises(GpuError):
             run(kern, rows)
+
+
+# Around the row-tile counts (on 148 SMs) where 17 to 21, 22 to 42 and more tokens change from one form to the other.
+@pytest.mark.parametrize("qtype", [21, 8])
+@pytest.mark.parametrize("tiles", [166, 167, 314, 315, 610, 611])
+def test_both_forms_of_more_than_16_tokens_agree_with_the_row_alone(gpu, qtype, tiles):
+    rng = np.random.default_rng(tiles)
+    W = synth.quant_rows(rng, qtype, 16 * tiles, 2048)
+    x = synth.acts_fp16(rng, 64, 2048)
+    alone = {b: run_qmv(gpu, "qmv_mma", qtype, W, 2048, x[b:b + 1])[0] for b in (0, 15, 16, 20, 21, 41, 42, 63)}
+    for B in (17, 21, 22, 42, 43, 64):
+        y = run_qmv(gpu, "qmv_mma", qtype, W, 2048, x[:B])
+        for b, want in alone.items():
+            assert b >= B or np.array_equal(bits(y[b]), bits(want)), (B, b)
