@@ -123,7 +123,7 @@ struct qw_engine {
     qw_buf xq_gu{}, xq_d{}, xs_gu{}, xs_d{};  // routed gate+up / down and the shared expert's, per layer
     qw_buf ffn_scr{};  // moe_ffn's scratch (moe_sel.h): per-item counters, zero between launches, and H
     size_t x_gus = 0, x_dns = 0;              // IQ3X bytes of one expert's gate+up / down
-    qw_kernel *k_ffn = nullptr, *k_ffn_h = nullptr, *k_ffn_x = nullptr, *k_ffn_probe = nullptr, *k_pack = nullptr;
+    qw_kernel *k_ffn = nullptr, *k_ffn_x = nullptr, *k_ffn_probe = nullptr, *k_pack = nullptr;
     bool moe_probe = false;  // measurement only: the copy-only twin of moe_ffn runs in its place (outputs are not produced)
     // slot sharding on top of the fused exchange: attention / GDN (their projections included) run only for the rows whose
     // slot this rank owns (slot % ep_size == ep_rank); the out-projection stores its rows into every rank's `ob` and publishes
@@ -365,10 +365,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
             mf.push_back({"IQ3X", e->ffn_iq3x ? 1 : 0});
             auto mp = mf;
             mp.push_back({"PROBE", 1});
-            auto mh = mf;
-            mh.push_back({"HALF", 1});
-            if (e->ffn_iq3x && c.ep_size == 1) ok = compile(e, "moe_ffn", "moe_ffn_few", mh, &e->k_ffn_h);
-            ok = ok && compile(e, "moe_ffn", "moe_ffn", mf, &e->k_ffn) && compile(e, "moe_ffn", "moe_ffn_copy_probe", mp, &e->k_ffn_probe) &&
+            ok = compile(e, "moe_ffn", "moe_ffn", mf, &e->k_ffn) && compile(e, "moe_ffn", "moe_ffn_copy_probe", mp, &e->k_ffn_probe) &&
                  (!e->ffn_iq3x || compile(e, "iq3x_pack", "iq3x_pack", {}, &e->k_pack));
             const char *cw = getenv("QW_CMB_WAIT");  // QW_CMB_WAIT=launch: the combine + norm waits for the FFN's whole launch, as with any other kernel
             if (ok && c.ep_size == 1 && e->D == 2048 && !(cw && !strcmp(cw, "launch")))
@@ -831,8 +828,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 const fill_args z = {0, (uint64_t)nb * (e->TOPK + 1) * D * 4, 0, 0, 0.f, 0.f};
                 enc_fill(e, b, &e->Pg, 0, z);
             }
-            qw_batch_kernel(b, wide ? e->k_ffn_w : e->ep_fused ? e->k_ffn_x : e->moe_probe ? e->k_ffn_probe
-                               : e->k_ffn_h && nb * e->TOPK + 1 <= 24 ? e->k_ffn_h : e->k_ffn);  // gate/up, SiLU * up and down of every chosen expert in one launch
+            qw_batch_kernel(b, wide ? e->k_ffn_w : e->ep_fused ? e->k_ffn_x : e->moe_probe ? e->k_ffn_probe : e->k_ffn);  // gate/up, SiLU * up and down of every chosen expert in one launch
             if (e->ffn_iq3x) {
                 qw_batch_buf(b, 0, &e->xq_gu, (size_t)l * e->EL * e->x_gus);
                 qw_batch_buf(b, 2, &e->xs_gu, (size_t)l * e->x_gus);
@@ -849,6 +845,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_buf(b, 4, &e->x, 0);
             qw_batch_buf(b, 5, &e->msel, selo);
             qw_batch_buf(b, 8, wide ? &e->ffn_scr_w : &e->ffn_scr, 0);
+            qw_batch_bytes(b, 13, &nb, 4);
             bind_pg();
             qw_batch_dispatch(b, e->I / 16, nb * e->TOPK + 1, 1, 256, 1, 1);
         } else {

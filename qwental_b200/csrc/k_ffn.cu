@@ -32,6 +32,7 @@
 #include "qmv_core.cuh"
 #include "qw_kern.h"
 #include <cuda.h>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -387,11 +388,10 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     const uint32_t slot0 = smem_u32(stage0);
     // this block's pieces: gate/up tiles [a_lo, a_hi) of the items x GT list, then down tiles [b_lo, b_hi) of the items x DT list
     const uint32_t G = gridDim.x, bx_ = blockIdx.x;
-    // HALF: few items (one or two slots).  Gate/up pieces are halved -- half of the row groups, 32 indices -- as long as every block gets at
-    // most one.  A piece is then a chain of four stages with half the warps decoding, and H is complete sooner.  (A variant of its own:
-    // in the others the registers would not suffice.)  A step of one slot, 48 layers: 2.83 -> 2.69 ms on a B200.
+    // HALF: few items.  Gate/up pieces are halved -- half of the row groups, 32 indices -- so that a piece is a chain of four stages with half
+    // the warps decoding, and H is complete sooner.  (A variant of its own: in the others the registers would not suffice.)
     static_assert(!HALF || FMT == 1, "half pieces are cut from IQ3X stages");
-    const uint32_t spl = HALF && 2 * items * GT <= G ? 1 : 0, GTS = GT << spl;
+    constexpr uint32_t spl = HALF ? 1 : 0, GTS = GT << spl;
     uint32_t a_lo = (uint32_t)((uint64_t)bx_ * items * GTS / G), a_hi = (uint32_t)((uint64_t)(bx_ + 1) * items * GTS / G);
     uint32_t b_lo = (uint32_t)((uint64_t)bx_ * items * DT / G), b_hi = (uint32_t)((uint64_t)(bx_ + 1) * items * DT / G);
     // the few items those shares touch, looked up once (thread k: item k of the gate/up share, thread FFN_RECS + k: of the down share)
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                 }
                 for (uint32_t kp = 0; kp < KP; kp++, j++) {
                     const uint32_t dst = slot_for(FMT ? IQ3X_STAGE >> spl : 2 * 64 * FFN_PITCH);
-                    if (HALF && spl) {  // half of the gate rows and of the up rows, in their places
+                    if (HALF) {  // half of the gate rows and of the up rows, in their places
                         const uint32_t o = (gh & 1) * 32 * IQ3X_REC;
                         const uint8_t *src = sc.wg + ((size_t)gt * KP + kp) * IQ3X_STAGE + o;
                         bulk_s(dst + o, src, 32 * IQ3X_REC, &full[j % FFN_STG]);
@@ -769,7 +769,8 @@ const CUtensorMap *ffn_tensor_map(const void *base, uint64_t pitch, uint64_t row
 // binds: 0 = routed gate, 1 = routed up [EL][I][rbD], 2 = shared gate, 3 = shared up (used unless SHARED is defined 0),
 // 4 = x fp16 [nb][D], 5 = moe_sel, 6 = routed down [EL][D][rbI], 7 = shared down, 8 = scratch (MOE_FFN_SCRATCH_BYTES(I) of
 // moe_sel.h, zeroed once by the owner, private to one stream), 9 = Pg fp32 [64][TOPK+1][D],
-// 10 = id of the first expert held in the weight buffers (optional, default 0); with EPX = ranks also 11, 12, 16 + r,
+// 10 = id of the first expert held in the weight buffers (optional, default 0), 13 = {nb} (optional: lets the launcher split the work of few
+// tokens further); with EPX = ranks also 11, 12, 16 + r,
 // 24 + r as for moe_dn.  defines: E, D, I, TOPK, EL, SHARED, EPX.  The host's grid and block are ignored.
 // With IQ3X defined 1 the weights are the re-coded form of iq3x.cuh (made by iq3x_pack): 0 = routed gate + up
 // [EL][I/64][D/512] stages, 2 = the shared expert's, 6 = routed down [EL][D/128][I/512] stages, 7 = the shared expert's;
@@ -843,9 +844,14 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
         QW_CHECK_ARG(mG && mU && mSG && mSU);
     }
     const bool probe = L.def("PROBE", 0) != 0;  // PROBE defined 1: the copy-only twin (outputs are not written)
-    // HALF defined 1: the variant for few items (IQ3X; the other kinds ignore it)
-    const bool half = L.def("HALF", 0) != 0;
-    auto kern = wide ? moe_ffn_k<false, 1, 1> : x4 && half && !probe ? moe_ffn_k<false, 1, 0, true>
+    // Half pieces while nearly every block gets at most one of them, by the items that nb tokens (bind 13; without it never) choose on average: up to
+    // 19 on 148 SMs.  Beyond that some blocks run two, and the variant itself costs 1 to 2 %.  Step time with whole pieces over step time with half
+    // pieces on a B200 (items): 512 experts, top-10, 1 to 4 slots 1.057 (11), 0.994 (20.8), 0.986 (30), 0.997 (39); 32 experts, top-4, 5 to 8 slots
+    // 1.038 (17), 1.015 (18.8), 0.999 (20.2), 0.990 (21.5); 256 experts, top-2, 8 and 10 slots 1.044 (16.5), 0.986 (21).
+    const uint32_t nb = L.has_bytes(13, 4) ? L.bytes<uint32_t>(13) : 0, grid = (uint32_t)(L.sm_count * per_sm);
+    const double items = E * (1 - pow(1 - (double)topk / E, (double)nb)) + (nb + 7) / 8;
+    const bool half = x4 && !wide && !probe && p.ep.nranks == 1 && nb >= 1 && 2 * items * (I / 64) <= grid * (33.0 / 32);
+    auto kern = wide ? moe_ffn_k<false, 1, 1> : half ? moe_ffn_k<false, 1, 0, true>
                 : x4 ? (probe ? moe_ffn_k<true, 1, 0> : moe_ffn_k<false, 1, 0>) : (probe ? moe_ffn_k<true, 0, 0> : moe_ffn_k<false, 0, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -853,7 +859,7 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, FFN_THREADS, smem);
     if (e != cudaSuccess) return e;
     QW_CHECK_ARG(occ >= per_sm);
-    qw_launch(kern, L.sm_count * per_sm, FFN_THREADS, smem, L.stream, *mG, *mU, *mSG, *mSU, p);
+    qw_launch(kern, grid, FFN_THREADS, smem, L.stream, *mG, *mU, *mSG, *mSU, p);
     return cudaGetLastError();
 }
 QW_FAMILY(moe_ffn, launch_moe_ffn, 512)

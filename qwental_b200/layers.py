@@ -109,7 +109,8 @@ class MoeLayer:
             b.kernel(self.k_ffn).buf(0, self.Xgu)
             if self.Sg is not None:
                 b.buf(2, self.XSgu).buf(7, self.XSd)
-            b.buf(4, x).buf(5, self.sel).buf(6, self.Xd).buf(8, self.ffn_scr).buf(9, self.Pg).dispatch((I // 16, nb * self.topk + 1), (256,))
+            b.buf(4, x).buf(5, self.sel).buf(6, self.Xd).buf(8, self.ffn_scr).buf(9, self.Pg).bytes(13, u32(nb)) \
+                .dispatch((I // 16, nb * self.topk + 1), (256,))
         elif self.fused_ffn:
             b.kernel(self.k_ffn).buf(0, self.Wg).buf(1, self.Wu)
             if self.Sg is not None:

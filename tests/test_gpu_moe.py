@@ -209,3 +209,18 @@ def test_iq3x_recoding_is_lossless(gpu):
 def test_fused_router_at_the_edges_of_its_passes(gpu, B):
     """moe_route reads up to four tokens directly and stages more by 16, three groups in flight: the comparison above at those edges."""
     test_fused_router_select_equals_two_launches(gpu, B)
+
+
+@pytest.mark.parametrize("topk,edge", [(10, 1), (4, 5), (1, 18)])
+def test_half_pieces_of_few_items_give_the_same_rows(gpu, topk, edge):
+    """moe_ffn halves its gate/up pieces while the tokens choose few enough experts (64 of them here) that a block gets one half piece: up to `edge`
+    tokens on 148 SMs.  A row is the same from both forms."""
+    D, I, E = 2048, 512, 64
+    layer, h, _ = make_layer(gpu, E, D, I, topk, seed=20 + topk, ffn="iq3x")
+    x = synth.acts_fp16(np.random.default_rng(topk), edge + 1, D)
+    whole = run_layer(gpu, layer, x)
+    ids = layer.read_sel(edge + 1)[1]
+    few = run_layer(gpu, layer, x[:edge])
+    assert np.array_equal(few.view(np.uint16), whole[:edge].view(np.uint16))
+    ref, _, _ = orc.moe_ref(x, h["Wr"], h["wsg"], h["gate"], h["up"], h["down"], h["sg"], h["su"], h["sd"], D, I, topk, ids=ids)
+    assert np.abs(few.astype(np.float64) - ref[:edge]).max() < 2e-3 * np.abs(ref).max()  # the bound of the layer test above
