@@ -16,6 +16,10 @@ extern "C" {
  * that the host touches every step. */
 enum { QW_BUF_SHARED = 0, QW_BUF_DEVICE = 1, QW_BUF_HOSTIO = 2 };
 bool qw_buf_new_kind(qw_gpu *g, size_t size, int kind, qw_buf *out);
+/* Bytes [offset, offset + size) of a buffer as a buffer of their own, with range checks of their own: one device allocation above 2 MB
+ * costs 0.3 ms and more whatever its size, so many buffers are better cut out of one.  Freeing a slice frees no memory; free the
+ * slices before the whole. */
+bool qw_buf_slice(const qw_buf *whole, size_t offset, size_t size, qw_buf *out);
 
 /* Copies between host memory and any buffer, ordered after everything already submitted on the current
  * stream; they return when the copy is complete.  false on a range or CUDA error. */

@@ -89,7 +89,8 @@ struct qw_engine {
     std::vector<Slot> slots;
     std::vector<int> free_pages;
     unsigned long long clock = 0;
-    // scratch
+    // scratch: slices of `scratch`, but for the pinned ones, part and logits
+    qw_buf scratch{};
     qw_buf ctl_h{}, ctl_d{}, h{}, h2{}, x{}, proj{}, cv{}, la{}, be{}, gy{}, qb{}, part{}, ya{}, ob{}, mo{}, logits{}, ids{}, ids_h{}, logits_h{}, cand_h{};
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
     // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN on IQ3X.  Eight times the tokens choose far fewer than eight times the
@@ -267,6 +268,7 @@ extern "C" void qw_engine_close(qw_engine *e) {
         if (r != e->c.ep_rank && e->ep_peer[r].handle) qw_buf_free(&e->ep_peer[r]);
     qw_buf_free(&e->epx);
     for (qw_buf *b : all) qw_buf_free(b);
+    qw_buf_free(&e->scratch);
     delete e;
 }
 
@@ -411,8 +413,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
     const size_t gu_bytes = (size_t)e->I * e->rbD;
     const int kvp = c.kv_pages > 0 ? c.kv_pages : c.max_slots * e->max_pages;
     const size_t page_bytes = (size_t)na * 2 * c.kvh * PAGE * c.hd * 2;
-    e->sel_bytes = align_up(e->piece_rows > ROWS ? qw_moe_sel_wide_bytes() : qw_moe_sel_bytes(), 256);
-    const size_t B = QW_PAR_MAX, RB = (size_t)e->piece_rows;  // rows of a step / of any pass
+    const size_t B = QW_PAR_MAX;
     ok = new_buf(e, &e->emb, (size_t)e->V * e->D * 2) && new_buf(e, &e->lm_head, (size_t)e->V * e->rbV) && new_buf(e, &e->dense, dn) &&
          new_buf(e, &e->small, ((size_t)e->L * e->small_stride + e->D) * 4) && new_buf(e, &e->router, (size_t)e->L * (e->E + 1) * e->D * 2) &&
          new_buf(e, &e->exg, (size_t)e->L * e->EL * gu_bytes) && new_buf(e, &e->exu, (size_t)e->L * e->EL * gu_bytes) &&
@@ -420,21 +421,39 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->shu, (size_t)e->L * gu_bytes) && new_buf(e, &e->shd, (size_t)e->L * gu_bytes) &&
          new_buf(e, &e->kvpool, (size_t)kvp * page_bytes) && new_buf(e, &e->ptab, (size_t)c.max_slots * e->max_pages * 4) &&
          new_buf(e, &e->sstate, (size_t)c.max_slots * ng * c.hv * 128 * 128 * 4) && new_buf(e, &e->cstate, (size_t)c.max_slots * ng * 3 * e->C * 4) &&
-         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->ctl_d, 3 * ROWS * 4) && new_buf(e, &e->prompt_d, (size_t)c.max_ctx * 4) && new_buf(e, &e->h, RB * e->D * 4) && new_buf(e, &e->h2, 4 * e->D * 4) &&
-         new_buf(e, &e->x, RB * e->D * 2) && new_buf(e, &e->proj, RB * std::max(e->qkv_rows, e->gdn_rows) * 2) && new_buf(e, &e->cv, RB * e->C * 2) &&
-         new_buf(e, &e->la, RB * c.hv * 4) && new_buf(e, &e->be, RB * c.hv * 4) && new_buf(e, &e->gy, RB * e->KG * 2) &&
-         new_buf(e, &e->qb, RB * c.qh * c.hd * 2) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
-         new_buf(e, &e->ya, RB * e->KA * 2) && new_buf(e, &e->ob, RB * e->D * 2) && new_buf(e, &e->mo, B * e->D * 2) &&
-         new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids, B * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
-         new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO) && new_buf(e, &e->mlog, RB * (e->E + 1) * 4) &&
-         new_buf(e, &e->msel, (size_t)e->L * e->sel_bytes) && new_buf(e, &e->Hhi, B * (e->TOPK + 1) * e->I * 2) &&
-         new_buf(e, &e->Hlo, B * (e->TOPK + 1) * e->I * 2) && new_buf(e, &e->Pg, RB * (e->TOPK + 1) * e->D * 4) && new_buf(e, &e->rcnt, 256);
-    if (ok) ok = qw_buf_zero(g, &e->msel, 0, e->msel.size) && qw_buf_zero(g, &e->Pg, 0, e->Pg.size) && qw_buf_zero(g, &e->Hhi, 0, e->Hhi.size) &&
-                 qw_buf_zero(g, &e->Hlo, 0, e->Hlo.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) &&
-                 qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size) && qw_buf_zero(g, &e->rcnt, 0, e->rcnt.size);
-    if (ok && e->ffn_fused) ok = new_buf(e, &e->ffn_scr, MOE_FFN_SCRATCH_BYTES(e->I)) && qw_buf_zero(g, &e->ffn_scr, 0, e->ffn_scr.size);
-    if (ok && e->piece_rows > ROWS)
-        ok = new_buf(e, &e->ctl_p, 3 * PROWS * 4) && new_buf(e, &e->ffn_scr_w, MOE_FFN_SCRATCH_BYTES_WIDE(e->I)) && qw_buf_zero(g, &e->ffn_scr_w, 0, e->ffn_scr_w.size);
+         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
+         new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
+         new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO);
+    // The rest of the scratch memory in one allocation.  With wide pieces it is some 120 MB more; where they are not there, prompts run in
+    // pieces of 64 tokens instead.
+    while (ok) {
+        const size_t RB = (size_t)e->piece_rows;  // the most rows of a pass
+        const bool wide = RB > ROWS;
+        e->sel_bytes = align_up(wide ? qw_moe_sel_wide_bytes() : qw_moe_sel_bytes(), 256);
+        const std::pair<qw_buf *, size_t> cut[] = {
+            {&e->ctl_d, 3 * ROWS * 4}, {&e->prompt_d, (size_t)c.max_ctx * 4}, {&e->h, RB * e->D * 4}, {&e->h2, 4 * (size_t)e->D * 4}, {&e->x, RB * e->D * 2},
+            {&e->proj, RB * std::max(e->qkv_rows, e->gdn_rows) * 2}, {&e->cv, RB * e->C * 2}, {&e->la, RB * c.hv * 4}, {&e->be, RB * c.hv * 4},
+            {&e->gy, RB * e->KG * 2}, {&e->qb, RB * c.qh * c.hd * 2}, {&e->ya, RB * e->KA * 2}, {&e->ob, RB * e->D * 2}, {&e->mo, B * e->D * 2}, {&e->ids, B * 4},
+            {&e->mlog, RB * (e->E + 1) * 4}, {&e->msel, (size_t)e->L * e->sel_bytes}, {&e->Hhi, B * (e->TOPK + 1) * e->I * 2},
+            {&e->Hlo, B * (e->TOPK + 1) * e->I * 2}, {&e->Pg, RB * (e->TOPK + 1) * e->D * 4}, {&e->rcnt, 256},
+            {&e->ffn_scr, e->ffn_fused ? MOE_FFN_SCRATCH_BYTES(e->I) : 0}, {&e->ctl_p, wide ? 3 * PROWS * 4 : 0}, {&e->ffn_scr_w, wide ? MOE_FFN_SCRATCH_BYTES_WIDE(e->I) : 0}};
+        auto room = [](size_t n) { return align_up(n, 256) + 256; };  // (the spare bytes that an allocation has, see qw_buf_new_kind)
+        size_t total = 0, at = 0;
+        for (auto &k : cut) total += k.second ? room(k.second) : 0;
+        if (!new_buf(e, &e->scratch, total)) {
+            ok = wide;
+            e->piece_rows = ROWS;
+            if (ok) e->err.clear();
+            continue;
+        }
+        for (auto &k : cut)
+            if (k.second) {
+                ok = ok && qw_buf_slice(&e->scratch, at, k.second, k.first);
+                at += room(k.second);
+            }
+        break;
+    }
+    if (ok) ok = qw_buf_zero(g, &e->scratch, 0, e->scratch.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) && qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size);
     if (ok && e->ffn_iq3x) {
         e->x_gus = (size_t)(e->I / 64) * (e->D / 512) * 128 * 272;
         e->x_dns = (size_t)(e->D / 128) * (e->I / 512) * 128 * 272;

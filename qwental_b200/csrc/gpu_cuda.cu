@@ -65,7 +65,7 @@ struct BufRec {
     void *dev;
     void *host;
     size_t size;
-    int kind;      // QW_BUF_*; 3 = wrap (device copy, host pointer is the caller's)
+    int kind;      // QW_BUF_*; 3 = wrap (device copy, host pointer is the caller's), 4 = imported, 5 = slice (the memory is another buffer's)
     int device;
 };
 
@@ -362,10 +362,23 @@ extern "C" void qw_buf_free(qw_buf *b) {
     BufRec *r = (BufRec *)b->handle;
     cudaSetDevice(r->device);
     if (r->kind == QW_BUF_HOSTIO) cudaFreeHost(r->host);
+    else if (r->kind == 5) {}
     else if (r->kind == 4) cudaIpcCloseMemHandle(r->dev);
     else cudaFree(r->dev);
     delete r;
     memset(b, 0, sizeof *b);
+}
+
+extern "C" bool qw_buf_slice(const qw_buf *whole, size_t offset, size_t size, qw_buf *out) {
+    if (!out) return false;
+    memset(out, 0, sizeof *out);
+    if (!whole || !whole->handle || size == 0 || offset > whole->size || size > whole->size - offset) return false;
+    const BufRec *w = (const BufRec *)whole->handle;
+    BufRec *r = new BufRec{(char *)w->dev + offset, w->host ? (char *)w->host + offset : nullptr, size, 5, w->device};
+    out->handle = r;
+    out->ptr = r->host;
+    out->size = size;
+    return true;
 }
 
 extern "C" void *qw_pool_push(void) { return nullptr; }

@@ -47,6 +47,7 @@ def load() -> C.CDLL:
         "qw_on_battery": (b, []), "qw_now": (d, []),
         # qw_gpu_ext.h
         "qw_buf_new_kind": (b, [vp, sz, C.c_int, P(QwBuf)]),
+        "qw_buf_slice": (b, [P(QwBuf), sz, sz, P(QwBuf)]),
         "qw_buf_upload": (b, [vp, P(QwBuf), sz, vp, sz]), "qw_buf_download": (b, [vp, P(QwBuf), sz, vp, sz]),
         "qw_buf_zero": (b, [vp, P(QwBuf), sz, sz]), "qw_buf_device_ptr": (vp, [P(QwBuf)]),
         "qw_gpu_stream_handle": (vp, [vp, C.c_int]), "qw_gpu_last_error": (cp, [vp]),

@@ -363,3 +363,22 @@ def test_a_rejected_step_leaves_the_last_logits_readable(gpu):
         assert np.array_equal(np.ctypeslib.as_array(alone, shape=(V,)).view(np.uint32), both[1].view(np.uint32))
     finally:
         e.close()
+
+
+def test_slices_of_a_buffer(gpu):
+    """qw_buf_slice: the bytes of the whole, ranges of its own, freed without the whole's memory; out of range is refused."""
+    import ctypes as C
+    from qwental_b200.lib import QwBuf
+    L, whole = gpu.L, gpu.buf_from(np.arange(4096, dtype=np.uint32))
+    part = QwBuf()
+    assert L.qw_buf_slice(C.byref(whole.b), 1024, 512, C.byref(part)) and part.size == 512
+    got = np.empty(128, np.uint32)
+    assert L.qw_buf_download(gpu.g, C.byref(part), 0, got.ctypes.data, 512) and np.array_equal(got, np.arange(256, 384))
+    assert not L.qw_buf_download(gpu.g, C.byref(part), 4, got.ctypes.data, 512)
+    assert L.qw_buf_zero(gpu.g, C.byref(part), 0, 512)
+    L.qw_buf_free(C.byref(part))
+    want = np.arange(4096, dtype=np.uint32)
+    want[256:384] = 0
+    assert np.array_equal(whole.download(np.uint32, 4096), want)
+    for off, n in ((16384, 1), (16000, 385), (0, 16385), (0, 0), (2 ** 64 - 8, 16)):
+        assert not L.qw_buf_slice(C.byref(whole.b), off, n, C.byref(part)), (off, n)
