@@ -131,7 +131,8 @@ int qw_engine_set_moe_probe(qw_engine *e, int on);
 
 /* Debug taps for the parity tests (role of the reference's QW_MOE_TEST / QW_DN_TAP dumps, src/engine.c:7942-7999):
  * copy a named internal buffer to the host; dst == NULL returns the size.  Last step: "h" fp32 [B][D],
- * "x" fp16 [B][D], "logits" fp32 [B][V], "sel" (layer index: the MoE selection record).  Weights by layer index:
+ * "x" fp16 [B][D], "logits" fp32 [B][V], "sel" (layer index: the MoE selection record); after a prompt they, and
+ * qw_engine_last_step_bytes, describe a step of its last token.  Weights by layer index:
  * "w_in", "w_out", "small", "router", "exg", "exu", "exd", "shg", "shu", "shd"; "emb", "lm_head", "final_norm".
  * State: "sstate" / "cstate" / "pages" by slot, "kvpage" by page id.  Returns bytes copied, 0 on error. */
 size_t qw_engine_tap(qw_engine *e, const char *name, int index, void *dst, size_t cap);

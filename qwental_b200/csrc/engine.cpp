@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -141,6 +142,7 @@ struct qw_engine {
     std::vector<int> last_sids;
     long long last_ctx = 0;
     int last_own = 0;  // rows of the last step whose token mixers ran on this rank
+    bool last_piece = false;  // the last pass was a piece of a prompt: its records describe all of its rows, lastB = 1 is its row 0
 
     bool fail(const char *fmt, ...) {
         char buf[512];
@@ -977,6 +979,7 @@ uint32_t begin_step(qw_engine *e, const int *sids, const int32_t *toks, int B, i
 void end_step(qw_engine *e, const int *sids, int B, int nsteps, double wall_ms) {
     e->last_sids.assign(sids, sids + B);
     e->lastB = B;
+    e->last_piece = false;
     e->last_ctx = 0;
     e->last_own = 0;
     for (int i = 0; i < B; i++) {
@@ -1244,6 +1247,7 @@ extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32
     s.last_use = ++e->clock;
     e->last_sids.assign(1, sid);
     e->lastB = 1;  // row 0 of the last piece is the prompt's last token
+    e->last_piece = true;
     const bool own = !e->slot_shard || sid % e->c.ep_size == e->c.ep_rank;
     e->last_ctx = own ? np : 0;
     e->last_own = own;
@@ -1258,6 +1262,31 @@ extern "C" int qw_engine_set_moe_probe(qw_engine *e, int on) {
 
 extern "C" double qw_engine_par_cost(qw_engine *e, int B) { return e && B >= 1 && B <= QW_PAR_MAX ? e->cost[B] : 0; }
 
+// The selection record of layer l as the last step left it.  After a prompt: the one a step of its last token would have left (that token is row 0
+// of the piece; both kinds of record keep the first rows' ids and w in the same places).
+static bool read_sel(qw_engine *e, int l, moe_sel *m) {
+    const size_t at = (size_t)l * e->sel_bytes;
+    if (!e->last_piece) return qw_buf_download(e->g, &e->msel, at, m, sizeof *m);
+    memset(m, 0, sizeof *m);
+    if (!qw_buf_download(e->g, &e->msel, at, m, offsetof(moe_sel, w) + sizeof m->w[0])) return false;
+    memset(m->ids[1], 0, sizeof m->ids - sizeof m->ids[0]);
+    m->U = 0;
+    m->nb = 1;
+    std::vector<std::pair<int, int>> chosen;  // (expert, rank)
+    for (int k = 0; k < e->TOPK; k++)
+        if (m->ids[0][k] >= e->e_lo && m->ids[0][k] < e->e_lo + e->EL) chosen.push_back({m->ids[0][k], k});
+    std::sort(chosen.begin(), chosen.end());
+    for (auto &c : chosen) {
+        m->ue[m->U] = (uint32_t)c.first;
+        m->off[m->U] = m->pre[m->U] = m->U;
+        m->ent[m->U] = (uint16_t)c.second;
+        m->U++;
+    }
+    m->off[m->U] = m->U;
+    for (uint32_t u = m->U; u < MOE_MAXE + 2; u++) m->pre[u] = m->U;
+    return true;
+}
+
 extern "C" void qw_engine_last_step_bytes(qw_engine *e, qw_step_bytes *o) {
     if (!o) return;
     memset(o, 0, sizeof *o);
@@ -1266,7 +1295,8 @@ extern "C" void qw_engine_last_step_bytes(qw_engine *e, qw_step_bytes *o) {
     int usum = 0;
     for (int l = 0; l < e->L; l++) {
         uint32_t U = 0;
-        qw_buf_download(e->g, &e->msel, (size_t)l * e->sel_bytes, &U, 4);
+        if (moe_sel m; !e->last_piece) qw_buf_download(e->g, &e->msel, (size_t)l * e->sel_bytes, &U, 4);
+        else if (read_sel(e, l, &m)) U = m.U;
         usum += (int)U;
         const double nexp = (double)U + (e->c.ep_rank == 0 ? 1 : 0);  // the shared expert runs on rank 0
         o->moe += nexp * (e->ffn_iq3x ? (double)(e->x_gus + e->x_dns) : 3 * gu) + (double)(e->E + 1) * e->D * 2;
@@ -1306,7 +1336,13 @@ extern "C" size_t qw_engine_tap(qw_engine *e, const char *name, int index, void 
     else if (!strcmp(name, "shg") && lay) { b = &e->shg; off = (size_t)index * gu; n = gu; }
     else if (!strcmp(name, "shu") && lay) { b = &e->shu; off = (size_t)index * gu; n = gu; }
     else if (!strcmp(name, "shd") && lay) { b = &e->shd; off = (size_t)index * gu; n = gu; }
-    else if (!strcmp(name, "sel") && lay) { b = &e->msel; off = (size_t)index * e->sel_bytes; n = qw_moe_sel_bytes(); }
+    else if (!strcmp(name, "sel") && lay) {
+        moe_sel m;
+        if (!dst) return sizeof m;
+        if (sizeof m > cap || !read_sel(e, index, &m)) return 0;
+        memcpy(dst, &m, sizeof m);
+        return sizeof m;
+    }
     else if (!strcmp(name, "sstate") && index >= 0 && index < (int)e->slots.size()) { n = (size_t)ng * e->HV * 128 * 128 * 4; b = &e->sstate; off = (size_t)index * n; }
     else if (!strcmp(name, "cstate") && index >= 0 && index < (int)e->slots.size()) { n = (size_t)ng * 3 * e->C * 4; b = &e->cstate; off = (size_t)index * n; }
     else if (!strcmp(name, "kvpage") && index >= 0) { n = (size_t)na * 2 * e->KVH * PAGE * e->HD * 2; b = &e->kvpool; off = (size_t)index * n; }

@@ -110,3 +110,34 @@ def test_a_failed_prompt_frees_its_slot(gpu, n, kernel, family, broken, whole):
         assert e.pos(1) == n
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("n", [2, 40, 130, 600])
+def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
+    """The selection record and the step's byte counts after a prompt (pieces of up to 64 tokens and of up to 512 keep different records on the
+    device) equal those after stepping its last token; h, x and logits are that token's."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(experts=256, topk=6, max_slots=2))
+    try:
+        text = np.random.default_rng(n).integers(0, e.cfg.vocab, n).astype(np.int32)
+
+        def records():
+            out = []
+            for l in range(e.cfg.layers):
+                r = e.tap("sel", l, np.uint8)
+                U, nb, topk = (int(v) for v in r[:12].view(np.uint32))
+                at = np.cumsum([16, 64 * 16 * 4, 64 * 17 * 4, 1024 * 4, 1025 * 4, 1024 * 2])
+                f = lambda i, t, k: r[at[i]:].view(np.uint8)[:k * np.dtype(t).itemsize].view(t).tolist()
+                out.append((U, nb, topk, f(0, np.int32, topk), f(1, np.uint32, topk + 1), f(2, np.uint32, U), f(3, np.uint32, U + 1), f(4, np.uint16, U),
+                            f(5, np.uint32, U + 1)))
+            b = e.step_bytes()
+            return out, [getattr(b, k) for k, _ in b._fields_], [e.tap(t, 0, np.uint16).tolist() for t in ("h", "x", "logits")]
+        e.prefill(0, text)
+        got = records()
+        e.prefill(1, text[:-1])
+        e.step([1], text[-1:])
+        want = records()
+        assert all(r[0] == 6 and r[1] == 1 for r in want[0])
+        assert got == want
+    finally:
+        e.close()
