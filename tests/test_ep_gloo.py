@@ -115,6 +115,20 @@ def test_row_order_edge_cases():
         ep.row_order([1], 2, 2)
 
 
+@pytest.mark.parametrize("nranks", [1, 2, 3, 8])
+@pytest.mark.parametrize("sid", [0, 1, 6, 63])
+@pytest.mark.parametrize("n", [1, 2, 63, 64])
+def test_a_piece_of_a_prompt_is_one_ranks(nranks, sid, n):
+    """The rows of a piece all carry the same slot id: its owner gets all of them in their order, the other ranks none."""
+    for rank in range(nranks):
+        perm, lo, hi = ep.row_order([sid] * n, nranks, rank)
+        assert perm.tolist() == list(range(n))
+        if rank == sid % nranks:
+            assert (lo, hi) == (0, n)
+        else:
+            assert lo == hi
+
+
 def free_port():
     s = socket.socket()
     s.bind(("127.0.0.1", 0))

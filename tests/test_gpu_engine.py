@@ -195,7 +195,7 @@ def test_benchmark_layer_shapes_match_fp64_reference(gpu):
 
 
 def test_prefill_is_the_decode_path_token_by_token(gpu):
-    """qw_engine_par_prefill feeds a prompt through the decode step: prefill(p) equals prefill(p[:-1]) followed by one
+    """qw_engine_par_prefill, in pieces, computes what the decode step computes token by token: prefill(p) equals prefill(p[:-1]) followed by one
     step of p[-1], bit for bit; the result does not depend on the slot; a slot that was in use is emptied first; a
     prefilled slot steps together with a seeded one exactly as it steps alone."""
     from qwental_b200.engine import Engine, tiny_cfg

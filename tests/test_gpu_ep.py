@@ -2,8 +2,8 @@
 replicated.  Two exchanges are covered: one NCCL all-reduce per MoE layer, and the fused one (the down projection
 stores its rows into every rank's buffer over NVLink and the next norm waits on sequence flags).  With the fused exchange
 on full-size layer shapes the slots are sharded too: attention and Gated DeltaNet run only on the rank that owns a slot and
-the out-projection's rows are gathered the same way -- covered with rows on both ranks and with a step in which one rank
-owns no row at all.  The logits of every rank must be bit-identical to the single-GPU step (each exchanged row has exactly
+the out-projection's rows are gathered the same way -- covered with rows on both ranks, with a step in which one rank
+owns no row at all and with prompts, whose pieces are one rank's.  The logits of every rank must be bit-identical to the single-GPU step (each exchanged row has exactly
 one contributor)."""
 import os
 
@@ -33,7 +33,11 @@ def _steps(eng):
         ids_g, _ = eng.decode_greedy(SIDS, [1, 2, 3], 4)
     finally:
         eng.gpu.L.qw_gpu_set_graphs(eng.gpu.g, False)
-    return l1, l2, l3, ids, ids_g
+    # prompts of three pieces into a slot of each rank (with slot sharding the other rank only publishes), then a step of both with a third
+    text = np.random.default_rng(3).integers(0, eng.cfg.vocab, 150).astype(np.int32)
+    p = [eng.prefill(4, text), eng.prefill(1, text[:131])]
+    l4, _ = eng.step([1, 2, 4], [3, 4, 5])
+    return l1, l2, l3, ids, ids_g, np.concatenate([np.stack(p), l4])
 
 
 def _worker(rank, world, uid, q, up, down):
@@ -88,6 +92,7 @@ def test_expert_parallel_step_bit_identical_to_single_gpu(fused):
         for got, want in zip(r[1:4], ref[:3]):
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), r[0]
         assert np.array_equal(r[4], ref[3]) and np.array_equal(r[5], ref[4]), r[0]
+        assert np.array_equal(r[6].view(np.uint32), ref[5].view(np.uint32)), r[0]
 
 
 def test_missing_peer_is_reported_not_waited_for_forever():

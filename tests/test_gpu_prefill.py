@@ -53,7 +53,7 @@ def test_wide_pieces_equal_stepping_every_token(gpu):
     from qwental_b200.engine import Engine, wide_cfg
     e = Engine(gpu, wide_cfg(experts=512, topk=10, max_slots=2))
     try:
-        lengths = {65, 127, 192, 193, 255, 256, 257, 321, 511, 512, 513, 577}
+        lengths = {65, 127, 192, 193, 255, 256, 257, 321, 511, 512, 513, 515, 550, 576, 577}
         text = np.random.default_rng(5).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
         e.prefill(0, text[:1])  # slot 0 steps every token
         for n in range(2, max(lengths) + 1):
