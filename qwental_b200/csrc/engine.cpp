@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <string>
 #include <vector>
 
@@ -439,20 +440,23 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
             {&e->mlog, RB * (e->E + 1) * 4}, {&e->msel, (size_t)e->L * e->sel_bytes}, {&e->Hhi, B * (e->TOPK + 1) * e->I * 2},
             {&e->Hlo, B * (e->TOPK + 1) * e->I * 2}, {&e->Pg, RB * (e->TOPK + 1) * e->D * 4}, {&e->rcnt, 256},
             {&e->ffn_scr, e->ffn_fused ? MOE_FFN_SCRATCH_BYTES(e->I) : 0}, {&e->ctl_p, wide ? 3 * PROWS * 4 : 0}, {&e->ffn_scr_w, wide ? MOE_FFN_SCRATCH_BYTES_WIDE(e->I) : 0}};
-        auto room = [](size_t n) { return align_up(n, 256) + 256; };  // (the spare bytes that an allocation has, see qw_buf_new_kind)
-        size_t total = 0, at = 0;
-        for (auto &k : cut) total += k.second ? room(k.second) : 0;
+        // Buffers of a megabyte and more begin at 2 MB boundaries, as if allocated one by one; the others follow, packed.  (All packed, a step of 16
+        // slots takes 0.6 % longer.)  256 spare bytes behind each, see qw_buf_new_kind.
+        size_t at[std::size(cut)], total = 0;
+        for (int big = 1; big >= 0; big--)
+            for (size_t i = 0; i < std::size(cut); i++) {
+                if ((cut[i].second >= (1u << 20)) != (big == 1)) continue;
+                at[i] = total = align_up(total, big ? 2u << 20 : 256);
+                total += cut[i].second + 256;
+            }
         if (!new_buf(e, &e->scratch, total)) {
             ok = wide;
             e->piece_rows = ROWS;
             if (ok) e->err.clear();
             continue;
         }
-        for (auto &k : cut)
-            if (k.second) {
-                ok = ok && qw_buf_slice(&e->scratch, at, k.second, k.first);
-                at += room(k.second);
-            }
+        for (size_t i = 0; i < std::size(cut); i++)
+            if (cut[i].second) ok = ok && qw_buf_slice(&e->scratch, at[i], cut[i].second, cut[i].first);
         break;
     }
     if (ok) ok = qw_buf_zero(g, &e->scratch, 0, e->scratch.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) && qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size);
