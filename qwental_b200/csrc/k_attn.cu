@@ -19,7 +19,7 @@
 // length, so a slot's result is bit-identical alone or in any batch.
 #include "common.cuh"
 #include "qw_kern.h"
-#include <cuda.h>
+#include "tmap.cuh"
 #include <cstdio>
 #include <map>
 #include <mutex>
@@ -212,11 +212,6 @@ QW_FAMILY(qsa_attn_simt, launch_qsa_attn, 256)
 //            B = the probabilities moved from accumulator layout to operand layout with four shuffles
 // The 8 query heads of the kv head fill the MMA's N dimension exactly: nothing is padded.  What a task computes depends
 // only on its slot's own length, never on which warp runs it or on the other slots of the batch.
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tm, int x, int y, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-                 "l"(tm), "r"(x), "r"(y), "r"(smem_u32(bar))
-                 : "memory");
-}
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
@@ -304,7 +299,7 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
             fence_proxy_async();  // the warp's reads of this buffer (ordered by __syncwarp) before the async-proxy writes
             mbar_expect_tx(bar, 8192);
 #pragma unroll
-            for (int db = 0; db < 4; db++) tma_load_2d(dst + db * 2048, &tm, db * 64, row, bar);
+            for (int db = 0; db < 4; db++) tma_load_2d(smem_u32(dst) + db * 2048, &tm, db * 64, row, bar);
         }
     };
     // ldmatrix lane roles: matrix mi = lane / 8, row r8 = lane % 8 (the swizzle key of that row)
@@ -326,8 +321,8 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
             mbar_expect_tx(&bars[st], AT_TILE_BYTES);
 #pragma unroll
             for (int db = 0; db < 4; db++) {
-                tma_load_2d(Kb + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + (int)fs * 16, &bars[st]);
-                tma_load_2d(Vb + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + vrows + (int)fs * 16, &bars[st]);
+                tma_load_2d(smem_u32(Kb) + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + (int)fs * 16, &bars[st]);
+                tma_load_2d(smem_u32(Vb) + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, ft.rowK + vrows + (int)fs * 16, &bars[st]);
             }
         }
         if (++fs == (ft.n + 15) / 16) {
@@ -473,27 +468,12 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
     if (!ok && lane == 0) set_status(status, ST_MBAR_TIMEOUT | 4);
 }
 
-// cuTensorMapEncodeTiled is a driver entry point; it is looked up through the runtime so that the library has no link
-// dependency on libcuda (it must load, without running anything, on machines that have no driver).
-typedef CUresult (*qw_encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                       const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                       CUtensorMapFloatOOBfill);
+// The pool seen as [rows of one token of one kv head][256 halves]
 static bool attn_encode_map(CUtensorMap *tm, const void *pool, size_t bytes) {
-    static qw_encode_tiled_fn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess || !p) return false;
-        fn = (qw_encode_tiled_fn)p;
-    }
-    const cuuint64_t gdim[2] = {256, (cuuint64_t)(bytes / 512)};
-    const cuuint64_t gstride[1] = {512};
-    const cuuint32_t box[2] = {64, 16}, estr[2] = {1, 1};
-    return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)pool, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return tmap_2d(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, pool, 256, bytes / 512, 512, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
-// One tensor map per KV pool: the pool seen as [rows of one token of one kv head][256 halves]
+// One tensor map per KV pool
 static const CUtensorMap *attn_tensor_map(void *pool, size_t bytes) {
     static std::mutex mu;
     static std::map<std::pair<void *, size_t>, CUtensorMap> cache;

@@ -31,7 +31,7 @@
 #include "moe_sel.h"
 #include "qmv_core.cuh"
 #include "qw_kern.h"
-#include <cuda.h>
+#include "tmap.cuh"
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -84,11 +84,6 @@ struct FfnP {
     EpPeers ep;
 };
 
-__device__ __forceinline__ void tma_box_2d(uint32_t dst, const CUtensorMap *tm, int x, int y, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(tm),
-                 "r"(x), "r"(y), "r"(smem_u32(bar))
-                 : "memory");
-}
 __device__ __forceinline__ void bulk_s(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {  // 1-D bulk copy to a shared-space address
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
@@ -488,8 +483,8 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                         bulk_s(dst, sc.wg + ((size_t)gt * KP + kp) * IQ3X_STAGE, IQ3X_STAGE, &full[j % FFN_STG]);
                     } else {
                         const int xc = (int)((220 * kp) & ~15u), yr = (int)(sc.erow * I + gt * 64);
-                        tma_box_2d(dst, sc.tg, xc, yr, &full[j % FFN_STG]);
-                        tma_box_2d(dst + 64 * FFN_PITCH, sc.tu, xc, yr, &full[j % FFN_STG]);
+                        tma_load_2d(dst, sc.tg, xc, yr, &full[j % FFN_STG]);
+                        tma_load_2d(dst + 64 * FFN_PITCH, sc.tu, xc, yr, &full[j % FFN_STG]);
                     }
                     if (sw && kp == 0) {  // the tokens of a new item's columns, requested after its first weights (the longer wait)
                         const uint32_t r0 = act_for(it.ncols, it.ncols * D * 2, false);
@@ -733,25 +728,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     if (p.ep.nranks > 1) ep_publish(p.ep);
 }
 
-// ---- tensor maps: an expert tensor [rows][pitch bytes] seen as a 2-D byte array, box = 240 bytes x 64 rows, no swizzle.
-// cuTensorMapEncodeTiled is a driver entry point; it is looked up through the runtime so that the library has no link
-// dependency on libcuda.
-typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                    const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-bool ffn_encode_map(CUtensorMap *tm, const void *base, uint64_t pitch, uint64_t rows) {
-    static encode_tiled_fn fn = nullptr;
-    if (!fn) {
-        void *q = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &qr) != cudaSuccess || !q) return false;
-        fn = (encode_tiled_fn)q;
-    }
-    const cuuint64_t gdim[2] = {pitch, rows};
-    const cuuint64_t gstride[1] = {pitch};
-    const cuuint32_t box[2] = {FFN_PITCH, 64}, estr[2] = {1, 1};
-    return fn(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void *)base, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
+// ---- tensor maps: an expert tensor [rows][pitch bytes] seen as a 2-D byte array, box = 240 bytes x 64 rows, no swizzle
 const CUtensorMap *ffn_tensor_map(const void *base, uint64_t pitch, uint64_t rows) {
     static std::mutex mu;
     static std::map<std::tuple<const void *, uint64_t, uint64_t>, CUtensorMap> cache;
@@ -760,7 +737,7 @@ const CUtensorMap *ffn_tensor_map(const void *base, uint64_t pitch, uint64_t row
     auto itc = cache.find(key);
     if (itc != cache.end()) return &itc->second;
     CUtensorMap tm;
-    if (!ffn_encode_map(&tm, base, pitch, rows)) return nullptr;
+    if (!tmap_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, pitch, rows, pitch, FFN_PITCH, 64, CU_TENSOR_MAP_SWIZZLE_NONE)) return nullptr;
     return &(cache[key] = tm);
 }
 
