@@ -221,8 +221,10 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
 
 // STG = 1: one tile of K and one of V per warp and three blocks per SM -- many warps hide one another's copies.  STG = 3, for launches with
 // no more tasks than one block per SM has warps: nobody else hides a warp's copies then, and with one tile in flight each of a page's 16
-// steps waited a whole memory latency (1.3 us); three tiles of both in a ring.  One slot of 25000 tokens, 48 layers on a B200: 3.07 -> 2.97 ms per
-// step; five slots of up to 12000 tokens (at most 470 tasks) and one of 1000 tokens within 1 %.
+// steps waited a whole memory latency (1.3 us); three tiles of both in a ring.  Measured on a B200, step time with STG = 1 over step time
+// with STG = 3, 12 layers: 1 slot of 6000 to 48000 tokens 1.04 to 1.03, 2 slots of 6000 to 36000 1.035 to 1.02, 3 of 3000 to 24000 1.03 to 1.02, 5 of 3000
+// to 12000 and 8 of 1000 to 9000 1.00 to 1.01; a prompt's group of 64 rows in its first 1024 tokens (prep, core and merge alone) 1.20 to 1.29, of
+// 8 rows in its first 4096 1.07 to 1.36.  (Prep, core and merge alone, back to back, one slot of 25000 or 48000 tokens: 0.94 and 0.97.)
 constexpr int AT_TILE_BYTES = 16384;  // K tile 8 KB + V tile 8 KB (4 swizzled boxes of 16 rows x 128 B each)
 constexpr int AT_TAB_BYTES = 1024;    // per block: first task of every slot [65], tokens [64], slot id [64]
 constexpr int AT_FEW_STG = 3;
