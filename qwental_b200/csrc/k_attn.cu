@@ -224,11 +224,12 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
 // steps waited a whole memory latency (1.3 us); three tiles of both in a ring.  Measured on a B200, step time with STG = 1 over step time
 // with STG = 3, 12 layers: 1 slot of 6000 to 48000 tokens 1.04 to 1.03, 2 slots of 6000 to 36000 1.035 to 1.02, 3 of 3000 to 24000 1.03 to 1.02, 5 of 3000
 // to 12000 and 8 of 1000 to 9000 1.00 to 1.01; a prompt's group of 64 rows in its first 1024 tokens (prep, core and merge alone) 1.20 to 1.29, of
-// 8 rows in its first 4096 1.07 to 1.36.  (Prep, core and merge alone, back to back, one slot of 25000 or 48000 tokens: 0.94 and 0.97.)
+// 8 rows in its first 4096 1.07 to 1.36.
 constexpr int AT_TILE_BYTES = 16384;  // K tile 8 KB + V tile 8 KB (4 swizzled boxes of 16 rows x 128 B each)
-constexpr int AT_TAB_BYTES = 1024;    // per block: first task of every slot [65], tokens [64], slot id [64]
+constexpr int AT_TAB_BYTES = 896;     // per block: first task of every slot [65], tokens [64], slot id [64]
+constexpr int AT_ZERO_BYTES = 3 * 2048 + 128;  // a row of zeros for each of a V tile's boxes, as far apart as the boxes
 constexpr int AT_FEW_STG = 3;
-constexpr int at_smem(int stg) { return 4 * stg * AT_TILE_BYTES + 128 + AT_TAB_BYTES + 1024; }
+constexpr int at_smem(int stg) { return 4 * stg * AT_TILE_BYTES + 128 + AT_TAB_BYTES + AT_ZERO_BYTES + 1024; }
 constexpr int at_blocks_per_sm(int stg) { return stg == 1 ? 3 : 1; }  // what the shared memory and the registers of the kernel allow
 
 template <int STG>
@@ -242,6 +243,8 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
     constexpr int NBAR = STG == 1 ? 2 : STG;  // STG = 1: K and V on their own; else one per tile pair
     uint64_t *bars = (uint64_t *)(smem + 4 * STG * AT_TILE_BYTES) + warp * NBAR;
     uint32_t *first = (uint32_t *)(smem + 4 * STG * AT_TILE_BYTES + 128), *ntokv = first + 65, *sidv = ntokv + 64;
+    const uint32_t zeros = smem_u32(first) + AT_TAB_BYTES;
+    first[(AT_TAB_BYTES + warp * 2048) / 4 + lane] = 0;
     if (lane == 0) {
 #pragma unroll
         for (int k = 0; k < NBAR; k++) mbar_init(&bars[k], 1);
@@ -306,7 +309,8 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
     };
     // ldmatrix lane roles: matrix mi = lane / 8, row r8 = lane % 8 (the swizzle key of that row)
     const uint32_t mi = lane >> 3, r8 = lane & 7;
-    const uint32_t kbase = smem_u32(Kb) + ((mi & 1) * 8 + r8) * 128, vbase = smem_u32(Vb) + ((mi >> 1) * 8 + r8) * 128;
+    const uint32_t vrow = (mi >> 1) * 8 + r8;  // token of the V tile whose row this lane addresses
+    const uint32_t kbase = smem_u32(Kb) + ((mi & 1) * 8 + r8) * 128, vbase = smem_u32(Vb) + vrow * 128;
     const int vrows = (int)(KVH * QSA_PAGE);  // rows from a page's K tile to its V tile
     uint32_t kph = 0, vph = 0;  // copies waited for so far on the K / V barrier (their parity selects the phase)
     bool ok = true;
@@ -418,19 +422,17 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
             const uint32_t b0 = to_b(h01), b1 = to_b(h23), c0 = to_b(r01), c1 = to_b(r23);
             if (STG == 1 && !mbar_wait(&bars[1], vph & 1)) { ok = false; break; }
             vph++;
-            if (const uint32_t left = cur.n - step * 16; left < 16) {
-                // Rows of the tile past the slot's length: their probabilities are 0, but the page may hold anything there -- a later token of the same
-                // prompt, or what an earlier conversation left -- and 0 times an infinity or a NaN would reach every head.  Zeros instead.
-                for (uint32_t r = left; r < 16; r++) *(uint4 *)(Vb + so + (lane >> 3) * 2048 + r * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
-                fence_proxy_async();  // before the next copy into this tile
-                __syncwarp();
-            }
+            // Rows of the tile past the slot's length: their probabilities are 0, but the page may hold anything there -- a later token of the same
+            // prompt, or what an earlier conversation left -- and 0 times an infinity or a NaN would reach every head.  Lanes that address such a row
+            // read zeros instead: one select per step, prep, core and merge of one slot of 6000 tokens 26.0 -> 26.3 us.  (Zeroing the tile's rows in
+            // place: 26.8; a branch in the step keeps V's loads behind the softmax.)
+            const uint32_t va = step * 16 + vrow < cur.n ? vbase + so : zeros;
             // four dim tiles at a time: the two MMAs of a tile depend on one another, back to back the second would wait for the first
 #pragma unroll
             for (int dq = 0; dq < 4; dq++) {
                 uint32_t af[4][4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) ldsm_x4_t(af[j], vbase + so + dq * 2048 + (((j * 2 + (mi & 1)) ^ r8) << 4));
+                for (int j = 0; j < 4; j++) ldsm_x4_t(af[j], va + dq * 2048 + (((j * 2 + (mi & 1)) ^ r8) << 4));
 #pragma unroll
                 for (int j = 0; j < 4; j++) mma_f16(o[4 * dq + j], af[j], b0, b1, o[4 * dq + j]);
 #pragma unroll
