@@ -3,8 +3,8 @@
  *
  * The reference's qw_engine_par_step (src/engine.c:8795) splits more than 8 slots into groups that each re-read
  * all weights; here one step advances up to QW_PAR_MAX slots with a single pass over the weights.
- * Out of scope here (see the reference for them): prefill, speculative decoding, prefix cache, snapshots, the
- * tokenizer and server.  Because prefill is out of scope a slot's context is created by qw_engine_par_seed.
+ * Out of scope here (see the reference for them): speculative decoding, prefix cache, snapshots, the tokenizer and server.
+ * A slot's context is a prompt's (qw_engine_par_prefill) or synthetic (qw_engine_par_seed).
  */
 #ifndef QW_ENGINE_H
 #define QW_ENGINE_H
@@ -50,8 +50,8 @@ int qw_engine_par_slots(qw_engine *e);               /* src/engine.h:78 */
 /* src/engine.h:80: a slot whose bit in `busy` is clear, preferring never-used ones, else the least recently
  * used; -1 if none.  (The prompt is not used for prefix matching: the prefix cache is out of scope.) */
 int qw_engine_par_pick(qw_engine *e, const int32_t *prompt, int np, unsigned long long busy);
-/* Stands in for qw_engine_par_prefill (src/engine.h:81): gives slot sid a context of ctx_len tokens whose KV
- * pages, GDN state and conv state are seeded synthetic values (K, V ~ N(0,1); S ~ N(0, 0.01)).  0 or -1. */
+/* For measurements: gives slot sid a context of ctx_len tokens whose KV
+ * pages, GDN state and conv state are seeded synthetic values (K, V ~ N(0,1); S ~ N(0, 0.01)).  0, or -1 (the slot is then free). */
 int qw_engine_par_seed(qw_engine *e, int sid, int ctx_len, unsigned long long seed);
 /* src/engine.h:81.  Processes a prompt into slot sid (released first if it was in use) and returns the logits of its last
  * position ([vocab], valid until the next step that succeeds), NULL on failure (the slot is then free).  The prompt runs in pieces of up to 512 tokens, each one

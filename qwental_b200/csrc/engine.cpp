@@ -6,7 +6,7 @@
 // Differences by design:
 //   - one weight pass for up to 64 slots (the reference splits into groups of <= 8, src/engine.c:8783-8814);
 //   - per-slot kernels (attention core, GDN recurrence, conv state) take the slot as a grid dimension and find
-//     the slot's state through tables in device memory, so a step is ~12 dispatches per layer for any batch
+//     the slot's state through tables in device memory, so a step is 7 to 9 dispatches per layer for any batch
 //     (the reference issues 3 more per slot, src/engine.c:8948-8959, 8992-9007);
 //   - KV lives in 256-token pages drawn from one pool; a slot owns a page list;
 //   - the step's control data (token, slot id, position per row) is read once from pinned host memory and kept
