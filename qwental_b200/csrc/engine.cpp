@@ -427,7 +427,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
          new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids_h, B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
          new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO);
-    // The rest of the scratch memory in one allocation.  With wide pieces it is some 120 MB more; where they are not there, prompts run in
+    // The rest of the scratch memory in one allocation.  With wide pieces it is some 100 MB more; where they are not to be had, prompts run in
     // pieces of 64 tokens instead.
     while (ok) {
         const size_t RB = (size_t)e->piece_rows;  // the most rows of a pass
