@@ -18,7 +18,7 @@ using namespace qw;
 
 #define GDN_EPS 1e-6f
 #define GDN_SEQ_MAX 512   // tokens of one launch of the sequence kernels
-#define GDN_SEQ_CHUNK 32  // tokens of one of gdn_seq's two staging buffers
+#define GDN_SEQ_CHUNK 16  // tokens of one of gdn_seq's two staging buffers
 
 // proj row layout (fp16, stride PS): [q: HK*DK | k: HK*DK | v: HV*DV | z: HV*DV | a: HV | b: HV]
 struct dn_epi_args {
@@ -263,38 +263,69 @@ QW_FAMILY(gdn_fstep, launch_gdn_fstep, 512)
 // ------------------------------------------------------------------------------------------------ recurrence over a piece of a prompt
 // nb consecutive tokens of ONE slot (row r = token nb - 1 - r of the piece, as dn_epi_seq): the state is loaded once, the tokens run
 // one after another, the state is stored once.  The columns of the state are independent in the recurrence, so a head is split
-// over 4 blocks of 32 columns; a column is held by 4 lanes of a warp, 32 rows each, in registers, and nothing but shuffles joins
-// them: no block barrier inside the token loop.  Four more warps prepare the next 32 tokens in shared memory meanwhile: normalised k and q
-// (the four row groups of a token 36 floats apart, so that the four lanes of a column read different banks), v, decay and beta.
-// Bound by the latency of one token's chain (decay, S^T k, the ordered sum over row groups, the update).  Before the staging warps, the spread
-// row groups and v in shared memory a token took 0.9 us; a 419-token prompt of 48 layers went from 86.6 to 81.3 ms on a B200.
-// Bit-identical to nb launches of gdn_fstep: the 16 partial sums of eight rows each are the same fma chains and are added in the same order
-// 0 .. 15 (four lanes pass the running sum on).  The sum of S^T q of a token is carried through beside the next token's S^T k:
-// it is off the recurrence.  The gated RMSNorm needs all 128 columns of a head: gdn_gate does it afterwards.
+// over 4 blocks of 32 columns and a block over 4 warps of 8; no block barrier inside the token loop.  A lane holds row groups j and j + 8
+// (eight rows each) of two columns as fp32 pairs (row of group j, row of group j + 8): the packed fp32 instructions run both groups' chains at
+// once, and an operand read from shared memory serves two columns.  Four more warps work beside them, a buffer ahead and a buffer behind: they
+// prepare the next 16 tokens in shared memory (normalised k and q as such pairs, v, decay and beta) and add up the outputs of the last 16.
+// Bound by the latency of one token's chain: decay, the fma chain of S^T k, the 16 group sums through shared memory, their ordered sum, the
+// update.  Everything else is off it: S^T q of a token runs beside the next token's sums, and its 16 group sums are left to the other warps.
+// 419 tokens on a B200: 146 -> 95 us (before, a lane held 32 rows of one column: every fma its own instruction and its own operand from shared
+// memory, the running sum handed on by four shuffles); prompts of 419 tokens, 48 layers, 40.3 -> 38.4 ms.
+// Bit-identical to nb launches of gdn_fstep: the 16 partial sums of eight rows each are the same fma chains and are added in the same order.
+// The gated RMSNorm needs all 128 columns of a head: gdn_gate does it afterwards.
 // binds: 0 = cv fp16 [nb][C], 1 = la [nb][HV], 2 = beta [nb][HV], 3 = state pool, 4 = proj fp16 (row stride z_stride), 5 = conv state
 // pool (the last three inputs of the piece are written), 6 = o out fp16 [nb][HV*DV] (not normalised), 7 = slot ids (entry 0), 8 = gdn_args.
 // grid (4, HV) x 256
-constexpr uint32_t SEQ_TOK = 324, SEQ_Q = 144, SEQ_V = 288, SEQ_GB = 320;  // floats of a staged token; q, v, {decay, beta} within it
+// Floats of a staged token: k and q as 8 lane groups of 8 pairs (16 floats, 20 apart: the eight lanes of a 16-byte load read different banks),
+// v, then {decay, decay, beta}.  Sums of 16 row groups: a column's 16 floats, 20 apart.
+constexpr uint32_t SEQ_Q = 160, SEQ_V = 320, SEQ_GB = 352, SEQ_TOK = 356, SEQ_COL = 20, SEQ_OUT = 32 * SEQ_COL;
+constexpr size_t SEQ_SMEM = (2 * GDN_SEQ_CHUNK * (SEQ_TOK + SEQ_OUT) + 2 * SEQ_OUT) * 4;  // tokens, sums of S^T q, sums of S^T k of two tokens
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 halves_of(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 template <bool TILED>
-__global__ void __launch_bounds__(256) gdn_seq_k(const __half *cv, const float *la, const float *beta, float *pool, const __half *proj, float *conv,
+__global__ void __launch_bounds__(256, 1) gdn_seq_k(const __half *cv, const float *la, const float *beta, float *pool, const __half *proj, float *conv,
                                                  __half *oo, const int32_t *sids, gdn_args a, uint32_t HK, uint32_t HV) {
-    constexpr int DK = 128, DV = 128, CW = 32;
-    extern __shared__ __align__(16) float seq_smem[];  // [2][GDN_SEQ_CHUNK][SEQ_TOK]
+    constexpr int DK = 128, DV = 128, CW = 32, CH = GDN_SEQ_CHUNK;
+    extern __shared__ __align__(16) float seq_smem[];
+    float *osum = seq_smem + 2 * CH * SEQ_TOK, *msum = osum + 2 * CH * SEQ_OUT;
     pdl_sync();
     const uint32_t cb = blockIdx.x, hv = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = a.nb;
-    const uint32_t hk = TILED ? hv % HK : hv / (HV / HK), q = lane >> 3, col = cb * CW + (warp & 3) * 8 + (lane & 7);
+    const uint32_t hk = TILED ? hv % HK : hv / (HV / HK), j = lane & 7, cp = lane >> 3, col = cb * CW + (warp & 3) * 8 + 2 * cp;
     const uint32_t C = 2 * HK * DK + HV * DV;
     const uint32_t slot = (uint32_t)sids[0];
-    const bool runs = warp < 4;  // warps 0 .. 3 hold the state
-    float *S = pool + (((size_t)slot * a.nlayers + a.layer) * HV + hv) * DK * DV + (size_t)(32 * q) * DV + col;
-    float s[32];
+    const bool runs = warp < 4;  // warps 0 .. 3 hold the state: rows 8 j + i and 8 (j + 8) + i of columns col and col + 1
+    float *S = pool + (((size_t)slot * a.nlayers + a.layer) * HV + hv) * DK * DV + (size_t)(8 * j) * DV + col;
+    f32x2 s0[8], s1[8];
 #pragma unroll
-    for (int i = 0; i < 32; i++) s[i] = runs ? S[(size_t)i * DV] : 0.f;
+    for (int i = 0; i < 8; i++) {
+        const float2 x = runs ? *(const float2 *)(S + (size_t)i * DV) : make_float2(0.f, 0.f), y = runs ? *(const float2 *)(S + (size_t)(64 + i) * DV) : x;
+        s0[i] = pair_of(x.x, y.x);
+        s1[i] = pair_of(x.y, y.y);
+    }
 
     // tokens c0 .. of the piece (position tau: row nb - 1 - tau) into their buffer, this warp being number w of `warps`: expressions of gdn_fstep
     auto stage = [&](uint32_t c0, uint32_t w, uint32_t warps) {
-        const uint32_t c1 = c0 + GDN_SEQ_CHUNK < nb ? c0 + GDN_SEQ_CHUNK : nb;
-        float *buf = seq_smem + (c0 / GDN_SEQ_CHUNK & 1) * GDN_SEQ_CHUNK * SEQ_TOK;
+        const uint32_t c1 = c0 + CH < nb ? c0 + CH : nb;
+        float *buf = seq_smem + (c0 / CH & 1) * CH * SEQ_TOK;
 #pragma unroll 4
         for (uint32_t tau = c0 + w; tau < c1; tau += warps) {
             const __half *row = cv + (size_t)(nb - 1 - tau) * C;
@@ -309,11 +340,37 @@ __global__ void __launch_bounds__(256) gdn_seq_k(const __half *cv, const float *
             const float rq_ = rsqrtf(qss / DK + GDN_EPS), rk_ = rsqrtf(kss / DK + GDN_EPS);
             auto qnorm = [&](float x) { return __half2float(__float2half_rn(x * rq_ / DK)); };
             auto knorm = [&](float x) { return __half2float(__float2half_rn(x * rk_ * rsqrtf((float)DK))); };
-            float *tk = buf + (tau - c0) * SEQ_TOK, *at = tk + 36 * (lane >> 3) + 4 * (lane & 7);
-            *(float4 *)at = make_float4(knorm(ka.x), knorm(ka.y), knorm(kb.x), knorm(kb.y));
-            *(float4 *)(at + SEQ_Q) = make_float4(qnorm(qa.x), qnorm(qa.y), qnorm(qb.x), qnorm(qb.y));
+            // this lane's four rows are rows 4 (lane % 2) .. of row group lane / 2
+            float *tk = buf + (tau - c0) * SEQ_TOK, *at = tk + (lane >> 1 & 7) * 20 + 8 * (lane & 1) + (lane >> 4);
+            at[0] = knorm(ka.x); at[2] = knorm(ka.y); at[4] = knorm(kb.x); at[6] = knorm(kb.y);
+            at += SEQ_Q;
+            at[0] = qnorm(qa.x); at[2] = qnorm(qa.y); at[4] = qnorm(qb.x); at[6] = qnorm(qb.y);
             tk[SEQ_V + lane] = __half2float(v);
-            if (lane == 0) *(float2 *)(tk + SEQ_GB) = make_float2(expf(lg), bt);
+            if (lane == 0) {
+                const float gd = expf(lg);
+                *(float4 *)(tk + SEQ_GB) = make_float4(gd, gd, bt, 0.f);
+            }
+        }
+    };
+    // 16 group sums in order
+    auto sum16 = [](const float *p) {
+        float m = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float4 y = ((const float4 *)p)[i];
+            m = i ? m + y.x : y.x;
+            m += y.y;
+            m += y.z;
+            m += y.w;
+        }
+        return m;
+    };
+    // outputs whose group sums rounds i0 .. i1 - 1 of the token loop have left, lane = column
+    auto outputs = [&](uint32_t i0, uint32_t i1, uint32_t w, uint32_t warps) {
+#pragma unroll 4
+        for (uint32_t i = i0 + w; i < i1; i += warps) {
+            const float o = sum16(osum + (i & (2 * CH - 1)) * SEQ_OUT + lane * SEQ_COL);
+            if (i) oo[(size_t)(nb - i) * HV * DV + hv * DV + cb * CW + lane] = __float2half_rn(o);  // (round i: token i - 1)
         }
     };
     stage(0, warp, 8);
@@ -331,77 +388,91 @@ __global__ void __launch_bounds__(256) gdn_seq_k(const __half *cv, const float *
     }
     __syncthreads();
 
-    // running sum over the four lanes of a column: lane q adds its four group sums to what lane q - 1 hands over; the last one has the total
-    auto chain = [&](const float (&g)[4]) {
-        float m = ((g[0] + g[1]) + g[2]) + g[3];  // lanes q = 0: groups 0 .. 3
+    auto load8 = [](f32x2 (&x)[8], const float *p) {
 #pragma unroll
-        for (uint32_t h = 1; h < 4; h++) {
-            const float v = __shfl_up_sync(0xffffffffu, m, 8);
-            if (q == h) m = (((v + g[0]) + g[1]) + g[2]) + g[3];
+        for (int i = 0; i < 4; i++) {
+            const ulonglong2 y = ((const ulonglong2 *)p)[i];
+            x[2 * i] = y.x;
+            x[2 * i + 1] = y.y;
         }
-        return m;
     };
-    auto load32 = [](float (&x)[32], const float *p) {
+    // the group sums j and j + 8 of this lane's two columns, in the order of the columns of the block
+    auto put = [&](float *p, f32x2 m0, f32x2 m1) {
+        const float2 x = halves_of(m0), y = halves_of(m1);
+        p[j] = x.x;
+        p[j + 8] = x.y;
+        p[SEQ_COL + j] = y.x;
+        p[SEQ_COL + j + 8] = y.y;
+    };
+    const uint32_t wc = (warp & 3) * 8;  // first column of the warp within the block
+    f32x2 qq[8];                         // q of the token before: its S^T q is added up a round later
+#pragma unroll
+    for (int i = 0; i < 8; i++) qq[i] = 0;
+    auto out_sums = [&](uint32_t round) {
+        f32x2 o0 = 0, o1 = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const float4 y = ((const float4 *)p)[i];
-            x[4 * i] = y.x; x[4 * i + 1] = y.y; x[4 * i + 2] = y.z; x[4 * i + 3] = y.w;
+            o0 = fma2(s0[i], qq[i], o0);
+            o1 = fma2(s1[i], qq[i], o1);
         }
+        put(osum + (round & (2 * CH - 1)) * SEQ_OUT + (wc + 2 * cp) * SEQ_COL, o0, o1);
     };
-    float og[4] = {0.f, 0.f, 0.f, 0.f};
-    for (uint32_t c0 = 0; c0 < nb; c0 += GDN_SEQ_CHUNK) {
-        const uint32_t c1 = c0 + GDN_SEQ_CHUNK < nb ? c0 + GDN_SEQ_CHUNK : nb;
+    for (uint32_t c0 = 0; c0 < nb; c0 += CH) {
+        const uint32_t c1 = c0 + CH < nb ? c0 + CH : nb;
         if (!runs) {
             if (c1 < nb) stage(c1, warp - 4, 4);
+            if (c0) outputs(c0 - CH, c0, warp - 4, 4);
         } else {
-            const float *tk = seq_smem + (c0 / GDN_SEQ_CHUNK & 1) * GDN_SEQ_CHUNK * SEQ_TOK;
-            float kk[32];
-            load32(kk, tk + 36 * q);
-            float2 db = *(const float2 *)(tk + SEQ_GB);
-            float v = tk[SEQ_V + warp * 8 + (lane & 7)];
+            const float *tk = seq_smem + (c0 / CH & 1) * CH * SEQ_TOK;
+            f32x2 kk[8];
+            load8(kk, tk + 20 * j);
+            float4 gb = *(const float4 *)(tk + SEQ_GB);
+            float v = tk[SEQ_V + wc + j];
 #pragma unroll 2
             for (uint32_t tau = c0; tau < c1; tau++) {
-                float mg[4], qq[32], kn[32];
-                load32(qq, tk + SEQ_Q + 36 * q);
+                f32x2 d0[8], d1[8], m0 = 0, m1 = 0;
+                const f32x2 gg = pair_of(gb.x, gb.y);
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    float m = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        s[8 * r + i] *= db.x;
-                        m = fmaf(s[8 * r + i], kk[8 * r + i], m);
-                    }
-                    mg[r] = m;
+                for (int i = 0; i < 8; i++) {
+                    d0[i] = mul2(s0[i], gg);
+                    d1[i] = mul2(s1[i], gg);
+                    m0 = fma2(d0[i], kk[i], m0);
+                    m1 = fma2(d1[i], kk[i], m1);
                 }
-                const float mt = chain(mg), ot = chain(og);  // (the previous token's output rides along)
-                if (q == 3 && tau) oo[(size_t)(nb - tau) * HV * DV + hv * DV + col] = __float2half_rn(ot);
-                if (tau + 1 < c1) tk += SEQ_TOK;  // the next token's operands (the last one reads its own again)
-                load32(kn, tk + 36 * q);
-                const float d = db.y * (v - __shfl_sync(0xffffffffu, mt, 24 + (lane & 7)));
-                db = *(const float2 *)(tk + SEQ_GB);
-                v = tk[SEQ_V + warp * 8 + (lane & 7)];
+                float *ms = msum + (tau & 1) * SEQ_OUT + wc * SEQ_COL;  // two of them: a warp barrier lies between a read and the next write
+                put(ms + 2 * cp * SEQ_COL, m0, m1);
+                __syncwarp();
+                const float mt = sum16(ms + j * SEQ_COL);  // lanes j, j + 8, ..: column j of the warp
+                out_sums(tau);                             // (of the token before)
+                const float *tn = tau + 1 < c1 ? tk + SEQ_TOK : tk;
+                load8(qq, tk + SEQ_Q + 20 * j);
+                const float d = gb.z * (v - mt);
+                const float da = __shfl_sync(0xffffffffu, d, 2 * cp), db = __shfl_sync(0xffffffffu, d, 2 * cp + 1);
+                const f32x2 dd0 = pair_of(da, da), dd1 = pair_of(db, db);
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    float o = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int e = 8 * r + i;
-                        s[e] = fmaf(kk[e], d, s[e]);
-                        o = fmaf(s[e], qq[e], o);
-                    }
-                    og[r] = o;
+                for (int i = 0; i < 8; i++) {
+                    s0[i] = fma2(kk[i], dd0, d0[i]);
+                    s1[i] = fma2(kk[i], dd1, d1[i]);
                 }
-#pragma unroll
-                for (int i = 0; i < 32; i++) kk[i] = kn[i];
+                tk = tn;  // the next token's operands (the last one reads its own again)
+                load8(kk, tk + 20 * j);
+                gb = *(const float4 *)(tk + SEQ_GB);
+                v = tk[SEQ_V + wc + j];
             }
         }
         __syncthreads();
     }
-    if (!runs) return;
-    const float ot = chain(og);
-    if (q == 3) oo[(size_t)hv * DV + col] = __float2half_rn(ot);
+    if (runs) {
+        out_sums(nb);
 #pragma unroll
-    for (int i = 0; i < 32; i++) S[(size_t)i * DV] = s[i];
+        for (int i = 0; i < 8; i++) {
+            const float2 x = halves_of(s0[i]), y = halves_of(s1[i]);
+            *(float2 *)(S + (size_t)i * DV) = make_float2(x.x, y.x);
+            *(float2 *)(S + (size_t)(64 + i) * DV) = make_float2(x.y, y.y);
+        }
+    }
+    __syncthreads();
+    outputs((nb - 1) / CH * CH, nb + 1, warp, 8);
 }
 
 static cudaError_t launch_gdn_seq(const QwLaunch &L) {
@@ -413,11 +484,10 @@ static cudaError_t launch_gdn_seq(const QwLaunch &L) {
     for (int i = 0; i <= 7; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
     QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * C * 2 && L.avail(1) >= (size_t)a.nb * HV * 4 && L.avail(2) >= (size_t)a.nb * HV * 4 &&
                  L.avail(4) >= ((size_t)(a.nb - 1) * a.z_stride + C) * 2 && L.avail(6) >= (size_t)a.nb * HV * DV * 2 && L.avail(7) >= 4);
-    const size_t smem = (size_t)(a.nb > GDN_SEQ_CHUNK ? 2 * GDN_SEQ_CHUNK : a.nb) * SEQ_TOK * 4;
     auto kern = tiled ? gdn_seq_k<true> : gdn_seq_k<false>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * GDN_SEQ_CHUNK * SEQ_TOK * 4);
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SEQ_SMEM);
     if (e != cudaSuccess) return e;
-    qw_launch(kern, dim3(4, HV), 256, smem, L.stream, L.buf<__half>(0), L.buf<float>(1), L.buf<float>(2), L.buf<float>(3), L.buf<__half>(4), L.buf<float>(5),
+    qw_launch(kern, dim3(4, HV), 256, SEQ_SMEM, L.stream, L.buf<__half>(0), L.buf<float>(1), L.buf<float>(2), L.buf<float>(3), L.buf<__half>(4), L.buf<float>(5),
               L.buf<__half>(6), L.buf<int32_t>(7), a, HK, HV);
     return cudaGetLastError();
 }

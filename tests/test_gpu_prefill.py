@@ -47,6 +47,26 @@ def test_prefill_equals_stepping_every_token(gpu, model):
         e.close()
 
 
+def test_recurrence_around_the_edges_of_its_buffers(gpu):
+    """The recurrence stages 16 tokens at a time and adds up outputs a buffer later: one less, as many and one more than one to four buffers."""
+    from qwental_b200.engine import Engine, tiny_cfg
+    e = Engine(gpu, tiny_cfg())
+    try:
+        lengths = {15, 16, 17, 18, 31, 32, 33, 34, 47, 48, 49}
+        text = np.random.default_rng(9).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(5, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 5), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
+
+
 def test_wide_pieces_equal_stepping_every_token(gpu):
     """Pieces of 65 to 512 tokens (512 experts, ten per token: several passes per expert and most experts chosen), at the edges of a piece,
     of the groups of 64 rows inside it and of what is left for a second and third piece."""
