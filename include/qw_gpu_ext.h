@@ -48,6 +48,13 @@ void qw_gpu_set_graphs(qw_gpu *g, bool on);
  * instantiating a graph costs more than launching it once). */
 void qw_batch_plain(qw_batch *b);
 
+/* Replaying without recording again.  A submitted batch that ran as a CUDA graph has a ticket (0: it did not, or failed);
+ * qw_batch_replay submits the same work once more -- same kernels, buffers, offsets and inline bytes, on the same stream -- and
+ * returns a batch to wait for.  NULL: the ticket is void (the graph was dropped, graphs are off, profiling is on, another
+ * stream is current, the launch mode changed) and the batch has to be recorded.  The buffers must still exist. */
+unsigned long long qw_batch_ticket(const qw_batch *b);
+qw_batch *qw_batch_replay(qw_gpu *g, unsigned long long ticket);
+
 /* Programmatic dependent launch for the kernels of later batches (default on; QW_PDL=0 in the environment turns it
  * off): each kernel may start while its predecessor drains and waits on the device for the predecessor's results. */
 void qw_gpu_set_pdl(qw_gpu *g, bool on);

@@ -100,14 +100,19 @@ struct qw_gpu {
     std::string err;
     unsigned long long launches;
     bool graphs;
-    // CUDA graphs of recorded batches, keyed by a hash of everything a replay depends on (kernel, its specialisation, grid,
-    // threadgroup memory, bound addresses, inline bytes, stream, dependent-launch mode); the key bytes are kept and compared
-    // on a hit.  Cleared whenever a kernel is re-specialised or the launch mode changes; capped in size.
+    // CUDA graphs of recorded batches, keyed by a hash of everything a replay depends on (kernel, grid, threadgroup memory, bound
+    // addresses, inline bytes, stream, dependent-launch mode); the key is kept and compared on a hit.  Cleared whenever a kernel is
+    // re-specialised or the launch mode changes; capped in size.  A ticket names an entry for qw_batch_replay; it is never given out twice.
     struct GraphEnt {
         cudaGraphExec_t exec;
-        std::vector<uint8_t> key;
+        std::vector<uint64_t> key;
+        unsigned long long ticket, launches;
+        cudaStream_t stream;
+        std::string pdl_off;
     };
     std::unordered_map<uint64_t, GraphEnt> graph_cache;
+    std::unordered_map<unsigned long long, GraphEnt *> tickets;
+    unsigned long long last_ticket;
     void *tables;
     unsigned *status_host, *status_dev;
 };
@@ -124,11 +129,13 @@ struct qw_batch {
     std::vector<cudaEvent_t> pev;  // profiling: 2 per dispatch
     bool submitted, failed;
     bool plain;  // launched directly even when graphs are on: it is not going to be replayed
+    unsigned long long ticket;
 };
 
 static void graph_cache_clear(qw_gpu *g) {
     for (auto &kv : g->graph_cache) cudaGraphExecDestroy(kv.second.exec);
     g->graph_cache.clear();
+    g->tickets.clear();
 }
 
 static void set_err(qw_gpu *g, const char *what, cudaError_t e) {
@@ -486,6 +493,7 @@ extern "C" qw_batch *qw_batch_begin(qw_gpu *g, bool /*concurrent*/) {
     b->cur_tg = 0;
     b->e0 = b->e1 = nullptr;
     b->submitted = b->failed = b->plain = false;
+    b->ticket = 0;
     b->recs.reserve(1024);
     return b;
 }
@@ -547,10 +555,26 @@ extern "C" void qw_batch_plain(qw_batch *b) {
 extern "C" void qw_batch_barrier(qw_batch *) {}
 extern "C" void qw_batch_flush(qw_batch *) {}
 
-static uint64_t hash_bytes(uint64_t h, const void *p, size_t n) {
-    const uint8_t *c = (const uint8_t *)p;
-    for (size_t i = 0; i < n; i++) h = (h ^ c[i]) * 0x100000001B3ull;
-    return h;
+static uint64_t hash_words(const uint64_t *w, size_t n) {  // four chains, so that the multiplies overlap
+    uint64_t h[4] = {0xcbf29ce484222325ull, 0x9e3779b97f4a7c15ull, 0xbf58476d1ce4e5b9ull, 0x94d049bb133111ebull};
+    for (size_t i = 0; i < n; i++) {
+        uint64_t &c = h[i & 3];
+        c = (c ^ w[i]) * 0x100000001B3ull;
+        c ^= c >> 29;
+    }
+    uint64_t r = n;
+    for (uint64_t c : h) r = (r ^ c) * 0x100000001B3ull;
+    return r ^ (r >> 32);
+}
+static const char *pdl_off_env() {
+    const char *p = getenv("QW_PDL_OFF");
+    return p ? p : "";
+}
+static cudaError_t replay(qw_gpu *g, const qw_gpu::GraphEnt &e) {
+    g->launches += e.launches;
+    const cudaError_t r = cudaGraphLaunch(e.exec, e.stream);
+    if (r != cudaSuccess) set_err(g, "graph launch", r);
+    return r;
 }
 
 static cudaError_t launch_one(qw_batch *b, const Rec &r) {
@@ -603,32 +627,36 @@ extern "C" void qw_batch_submit(qw_batch *b) {
     }
     cudaEventRecord(b->e0, b->stream);
     if (g->graphs && !b->plain && !g->profile && b->recs.size() > 1) {
-        std::vector<uint8_t> key;
-        key.reserve(b->recs.size() * 320);
-        auto put = [&](const void *p, size_t n) { key.insert(key.end(), (const uint8_t *)p, (const uint8_t *)p + n); };
-        for (const Rec &r : b->recs) {
-            put(&r.k, sizeof r.k);
-            put(&r.k->fam, sizeof r.k->fam);
-            for (auto &kv : r.k->defs.v) {
-                put(kv.first.data(), kv.first.size());
-                put(&kv.second, sizeof kv.second);
-            }
-            put(&r.gx, 6 * sizeof(unsigned));
-            put(&r.tgmem, sizeof r.tgmem);
-            for (int i = 0; i < 32; i++) {
-                put(&r.b[i].ptr, sizeof(void *));
-                put(&r.b[i].blen, 4);
-                if (r.b[i].blen) put(b->arena.data() + r.b[i].boff, r.b[i].blen);
-            }
+        std::vector<uint64_t> key;
+        key.reserve(b->recs.size() * 32);
+        for (const Rec &r : b->recs) {  // (a kernel that is specialised anew keeps its address, but clears the cache)
             qw_pdl_current_family(r.k->fam->name);
-            const uint8_t pdl = qw_pdl_enabled() ? 1 : 0;
-            put(&pdl, 1);
+            key.push_back((uint64_t)(uintptr_t)r.k);
+            key.push_back((uint64_t)r.gx << 32 | r.gy);
+            key.push_back((uint64_t)r.gz << 32 | r.tx);
+            key.push_back((uint64_t)r.ty << 32 | r.tz);
+            key.push_back((uint64_t)r.tgmem << 1 | (qw_pdl_enabled() ? 1 : 0));
+            for (int i = 0; i < 32; i++) {
+                const QwBind &d = r.b[i];
+                if (!d.ptr && !d.blen) continue;
+                key.push_back((uint64_t)i << 32 | d.blen);
+                if (!d.blen) {
+                    key.push_back((uint64_t)(uintptr_t)d.ptr);
+                    key.push_back(d.avail);
+                } else {
+                    const size_t at = key.size();
+                    key.resize(at + (d.blen + 7) / 8, 0);
+                    memcpy(key.data() + at, b->arena.data() + d.boff, d.blen);
+                }
+            }
+            key.push_back(~0ull);
         }
-        put(&b->stream, sizeof b->stream);
-        const uint64_t h = hash_bytes(0xcbf29ce484222325ull, key.data(), key.size());
+        key.push_back((uint64_t)(uintptr_t)b->stream);
+        const uint64_t h = hash_words(key.data(), key.size());
         auto it = g->graph_cache.find(h);
         if (it != g->graph_cache.end() && it->second.key != key) {  // a hash collision: the stored graph is another batch's
             cudaGraphExecDestroy(it->second.exec);
+            g->tickets.erase(it->second.ticket);
             g->graph_cache.erase(it);
             it = g->graph_cache.end();
         }
@@ -655,16 +683,34 @@ extern "C" void qw_batch_submit(qw_batch *b) {
                 b->failed = true;
                 return;
             }
-            it = g->graph_cache.emplace(h, qw_gpu::GraphEnt{exec, std::move(key)}).first;
+            it = g->graph_cache.emplace(h, qw_gpu::GraphEnt{exec, std::move(key), ++g->last_ticket, b->recs.size(), b->stream, pdl_off_env()}).first;
+            g->tickets[it->second.ticket] = &it->second;  // (entries do not move)
         }
-        cudaError_t e = cudaGraphLaunch(it->second.exec, b->stream);
-        if (e != cudaSuccess) {
-            set_err(g, "graph launch", e);
-            b->failed = true;
-        }
-        g->launches += b->recs.size();
+        b->ticket = it->second.ticket;
+        if (replay(g, it->second) != cudaSuccess) b->failed = true;
     } else run_records(b);
     cudaEventRecord(b->e1, b->stream);
+}
+
+extern "C" unsigned long long qw_batch_ticket(const qw_batch *b) { return b && b->submitted && !b->failed ? b->ticket : 0; }
+
+extern "C" qw_batch *qw_batch_replay(qw_gpu *g, unsigned long long ticket) {
+    if (!g || !g->graphs || g->profile) return nullptr;
+    const auto it = g->tickets.find(ticket);
+    if (it == g->tickets.end() || it->second->stream != g->stream[g->cur] || it->second->pdl_off != pdl_off_env()) return nullptr;
+    cudaSetDevice(g->dev);
+    qw_batch *b = new qw_batch();
+    b->g = g;
+    b->stream = g->stream[g->cur];
+    b->ticket = ticket;
+    b->submitted = true;
+    b->failed = b->plain = false;
+    cudaEventCreate(&b->e0);
+    cudaEventCreate(&b->e1);
+    cudaEventRecord(b->e0, b->stream);
+    b->failed = replay(g, *it->second) != cudaSuccess;
+    cudaEventRecord(b->e1, b->stream);
+    return b;
 }
 
 extern "C" bool qw_batch_poll(qw_batch *b) {

@@ -245,8 +245,9 @@ static cudaError_t launch_ep_publish(const QwLaunch &L) {
 QW_FAMILY(ep_publish, launch_ep_publish, 32)
 
 // binds: 0 = logits fp32 [nb][V], 1 = ids out int32 [nb], 2 = {nb, V}, 3 = second ids out (with IDS2 defined 1,
-// e.g. a host-visible copy).  grid nb x 1024
-__global__ void __launch_bounds__(1024) k_argmax_k(const float *lg, int32_t *ids, int32_t *ids2, uint32_t V) {
+// e.g. a host-visible copy).  With ALT defined 1 also 4 = a position: with an odd one the second ids go 64 places further, so that the
+// host can read a step's while the next step runs.  grid nb x 1024
+__global__ void __launch_bounds__(1024) k_argmax_k(const float *lg, int32_t *ids, int32_t *ids2, uint32_t V, const int32_t *pos) {
     __shared__ float bv[32];
     __shared__ uint32_t bi[32];
     pdl_sync();
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(1024) k_argmax_k(const float *lg, int32_t *ids
         }
         if (lane == 0) {
             ids[t] = (int32_t)idx;
-            if (ids2) ids2[t] = (int32_t)idx;
+            if (ids2) ids2[t + (pos ? (*pos & 1) * 64 : 0)] = (int32_t)idx;
         }
     }
 }
@@ -287,8 +288,10 @@ static cudaError_t launch_k_argmax(const QwLaunch &L) {
     QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(1) && L.has_bytes(2, 8) && a.nb >= 1 && a.nb <= 64 && a.V >= 1);
     QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * a.V * 4 && L.avail(1) >= a.nb * 4);
     int32_t *ids2 = L.def("IDS2", 0) ? L.buf<int32_t>(3) : nullptr;
-    if (L.def("IDS2", 0)) QW_CHECK_ARG(ids2 && L.avail(3) >= a.nb * 4);
-    qw_launch(k_argmax_k, a.nb, 1024, 0, L.stream, L.buf<float>(0), L.buf<int32_t>(1), ids2, a.V);
+    const bool alt = ids2 && L.def("ALT", 0);
+    const int32_t *pos = alt ? L.buf<int32_t>(4) : nullptr;
+    if (L.def("IDS2", 0)) QW_CHECK_ARG(ids2 && L.avail(3) >= (alt ? 64 + a.nb : a.nb) * 4 && (!alt || (pos && L.avail(4) >= 4)));
+    qw_launch(k_argmax_k, a.nb, 1024, 0, L.stream, L.buf<float>(0), L.buf<int32_t>(1), ids2, a.V, pos);
     return cudaGetLastError();
 }
 QW_FAMILY(k_argmax, launch_k_argmax, 1024)

@@ -382,3 +382,39 @@ def test_slices_of_a_buffer(gpu):
     assert np.array_equal(whole.download(np.uint32, 4096), want)
     for off, n in ((16384, 1), (16000, 385), (0, 16385), (0, 0), (2 ** 64 - 8, 16)):
         assert not L.qw_buf_slice(C.byref(whole.b), off, n, C.byref(part)), (off, n)
+
+
+@pytest.mark.parametrize("start", [64, 65])
+def test_replayed_steps_and_their_ids(gpu, start):
+    """Greedy chains whose steps are submitted ahead leave their ids in alternating halves by the first row's position: chains of 1, 2 and 5
+    steps from even and odd positions, recorded and replayed, against one step at a time; and again after another engine has registered the same
+    kernels anew, which drops the recorded graphs."""
+    from qwental_b200.engine import Engine, tiny_cfg
+    a, b = Engine(gpu, tiny_cfg()), Engine(gpu, tiny_cfg())
+    rows, toks = [2, 0, 1], np.array([3, 1, 2], np.int32)
+
+    def run(e, n, ahead):
+        for i, s in enumerate(rows):
+            e.seed_slot(s, start + 7 * i, 90 + i)
+        if ahead:
+            return e.decode_greedy(rows, toks, n)[0], e.step(rows, toks)[0]
+        ids, cur = [], toks
+        for _ in range(n):
+            cur = np.array(e.step_greedy(rows, cur)[0], np.int32)
+            ids.append(cur)
+        return np.array(ids), e.step(rows, toks)[0]
+
+    try:
+        want = {n: run(b, n, False) for n in (1, 2, 5)}
+        gpu.L.qw_gpu_set_graphs(gpu.g, True)
+        for rnd in range(3):
+            for n in (1, 2, 5):
+                for ahead in (True, False):
+                    ids, lg = run(a, n, ahead)
+                    assert np.array_equal(ids, want[n][0]) and np.array_equal(lg.view(np.uint32), want[n][1].view(np.uint32)), (rnd, n, ahead)
+            if rnd == 1:
+                Engine(gpu, tiny_cfg()).close()
+    finally:
+        gpu.L.qw_gpu_set_graphs(gpu.g, False)
+        a.close()
+        b.close()
