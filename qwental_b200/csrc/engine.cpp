@@ -668,7 +668,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                  const Piece *piece = nullptr) {
     const uint32_t D = e->D;
     const qw_buf *none = nullptr;
-    const bool wide = nb > ROWS;  // a piece of more than 64 tokens
+    bool wide = nb > ROWS;  // a piece of more than 64 tokens
     const qw_buf *ctl = wide ? &e->ctl_p : &e->ctl_d;
     const uint32_t CR = wide ? PROWS : ROWS;
     if (piece) {
@@ -698,7 +698,8 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     const qw_buf *hb = &e->h;      // the residual stream
     const qw_buf *pending = none;  // block output not yet added to the residual stream
     // rows of the token mixers: all of them, or (slot sharding) the rows [lo, lo + nbl) whose slots this rank owns
-    const uint32_t lo = e->slot_shard ? e->row_lo : 0, nbl = e->slot_shard ? e->row_hi - e->row_lo : nb;
+    const uint32_t lo = e->slot_shard ? e->row_lo : 0;
+    uint32_t nbl = e->slot_shard ? e->row_hi - e->row_lo : nb;
     const size_t xo = (size_t)lo * D * 2, co = (size_t)lo * 4;  // byte offsets of row lo in x / ob and in the control arrays
     const qw_buf *obuf = e->slot_shard ? &e->epx : &e->ob;
     const size_t obo = e->slot_shard ? e->ob_off : 0;
@@ -725,6 +726,16 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
     };
     for (int l = 0; l < e->L; l++) {
         const LayerW &w = e->layers[l];
+        // Of a piece, the last layer only has to bring the KV cache and the recurrent state forward; what follows it is wanted for the prompt's
+        // last token alone -- row 0 of the last piece, which goes on as a step of one row.  (Ranks that share the experts keep all rows: their
+        // exchange is built for one row count per pass.)  Prompts of 45 and 419 tokens, 48 layers: 1.013x, 1.017x; of 1700 tokens, 12 layers: 36.3 ->
+        // 33.7 ms on a B200.
+        const bool state_only = piece && l == e->L - 1 && e->c.ep_size == 1;
+        auto row0_goes_on = [&] {
+            nb = nbl = 1;
+            wide = false;
+            return piece->last;
+        };
         enc_norm(e, b, hb, pending, w.small, nb, l - 1);  // h += previous block (the MoE combine of layer l-1); x = rmsnorm(h) * w1
         if (nbl == 0) {  // no row of this rank in the step: only tell the others so
             qw_batch_kernel(b, e->k_pub);
@@ -751,6 +762,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 qw_batch_bytes(b, 8, &qa, sizeof qa);
                 qw_batch_dispatch(b, e->QH + e->KVH, qa.nb, 1, 256, 1, 1);
             }
+            if (state_only && !row0_goes_on()) return;
             for (uint32_t r0 = 0; r0 < nbl; r0 += ROWS) {
                 const qsa_args qa = group(r0);
                 qw_batch_kernel(b, e->k_attn);
@@ -790,7 +802,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_buf(b, 8, ctl, CR * 4 + co);
             qw_batch_bytes(b, 9, &ea, sizeof ea);
             qw_batch_dispatch(b, (e->C + 2 * e->HV + 255) / 256, nbl, 1, 256, 1, 1);
-            const gdn_args ga = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
+            gdn_args ga = {nbl, (uint32_t)w.idx, (uint32_t)e->n_gdn, e->gdn_rows};
             qw_batch_kernel(b, piece ? e->k_gdn_seq : early ? e->k_gdn_e : e->k_gdn);
             qw_batch_buf(b, 0, &e->cv, 0);
             qw_batch_buf(b, 1, &e->la, 0);
@@ -803,7 +815,9 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_buf(b, 7, ctl, CR * 4 + co);
             qw_batch_bytes(b, 8, &ga, sizeof ga);
             qw_batch_dispatch(b, e->HV, nbl, 1, 512, 1, 1);
+            if (state_only && !row0_goes_on()) return;
             if (piece) {
+                ga.nb = nbl;
                 qw_batch_kernel(b, e->k_gdn_gate);
                 qw_batch_buf(b, 0, &e->gy, 0);
                 qw_batch_buf(b, 4, &e->proj, (size_t)e->C * 2);
@@ -919,8 +933,8 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
         }
         pending = &e->Pg;  // combined, rounded to fp16 and added to the residual stream inside the next norm kernel
     }
-    // (a piece: h and x of row 0 -- the newest token -- and its logits if the prompt ends there; a piece in the middle still needs the
-    // combine of its last layer for nothing, but the kernel also returns the FFN's row counters to zero)
+    // (a piece: h and x of row 0 -- the newest token -- and its logits if the prompt ends there; where all rows went on, the kernel also returns
+    // the FFN's row counters to zero)
     enc_norm(e, b, hb, pending, e->final_norm, nb, e->L - 1);
     e->h_last = hb;
     if (piece) {

@@ -161,3 +161,27 @@ def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
         assert got == want
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("layers,every", [(4, 4), (5, 4), (1, 1), (3, 2)])
+def test_last_layer_of_a_prompt(gpu, layers, every):
+    """After the last layer's K, V and state only the prompt's last token goes on: Gated DeltaNet and attention as the last layer, one piece and several
+    (the last one of a single token too), then a step on the state left behind."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(layers=layers, attn_every=every, max_slots=2))
+    try:
+        lengths = {2, 64, 66, 200, 513}
+        text = np.random.default_rng(11).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+        both, _ = e.step([0, 1], [7, 7])
+        assert np.array_equal(both[0].view(np.uint32), both[1].view(np.uint32))
+    finally:
+        e.close()
