@@ -480,14 +480,15 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
 // reduction across warps.  MMA column g of a tile holds token (g / 2) + 4 (g % 2), so that the eight lanes of a 16-byte shared load fall into
 // eight different chunks of the swizzle.
 // TS = warps that share a row tile.  2: the tiles of a block are few (a projection has 3 to 6 per SM) and the warps are what hides
-// latency.  1 (Q8_0, 16 tiles per SM and more): a unit is decoded once for all tokens, because the kernel is then bound by the
-// shared-memory pipe.
+// latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S for several groups of 64 tokens, where a block has many tiles): a unit is decoded once for all
+// tokens, by fewer warps with more registers.  (12352 x 2048 IQ3_S, 419 tokens, TS 2 -> 1 on a B200: 121 -> 110 us; 2048 x 4096: 45 -> 42; prompts of 419
+// tokens, 48 layers, 37.5 -> 36.9 ms.)
 // Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
 // IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
 // 40 of its cycles per unit of 16 rows x 32 weights.
 template <int GF, int TS>
 struct WideCfg {
-    static constexpr int RG = TS == 2 ? 7 : 11;              // row tiles per round: 14 + 1 warps of 128 registers, or 11 + 1 of 168
+    static constexpr int RG = TS == 2 || GF == 21 ? 7 : 11;  // row tiles per round: 14 + 1 warps of 128 registers, 7 + 1 of up to 255 or 11 + 1 of 168
     static constexpr int UPW = GF == 21 ? 2 : 1;             // units per weight stage
     static constexpr int PITCH = GF == 21 ? 240 : 272;       // bytes between staged rows (eight rows: eight different groups of four banks)
     static constexpr int WS = GF == 21 || TS == 1 ? 2 : 3, XS = 3;  // stages
@@ -495,7 +496,7 @@ struct WideCfg {
     static constexpr int WBYTES = RG * 16 * PITCH;
     static constexpr size_t smem(int CT) { return 1024 + 256 + (size_t)TABB + (size_t)WS * WBYTES + (size_t)XS * CT * TS * 8 * 512; }
 };
-static_assert(WideCfg<21, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 1>::smem(8) <= 227 * 1024, "shared memory of the wide matvec");
+static_assert(WideCfg<21, 2>::smem(4) <= 227 * 1024 && WideCfg<21, 1>::smem(8) <= 227 * 1024 && WideCfg<8, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 1>::smem(8) <= 227 * 1024, "shared memory of the wide matvec");
 
 // q8_sub_h for rows 272 bytes apart, in half the shared-memory cycles: 32-bit loads only, and lanes t >= 2 take their words in another
 // order, so that rows g and g + 1 do not meet in a bank (only the third load of an even block has two lanes per bank).
@@ -706,9 +707,7 @@ static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     // one block per SM, shared evenly by the groups of 64 tokens
     const uint32_t groups = (p.nb + 63) / 64, most = (uint32_t)sm_count / groups > 0 ? (uint32_t)sm_count / groups : 1, bpg = p.items < most ? p.items : most;
     const uint32_t per = (p.items + bpg - 1) / bpg;
-    if constexpr (GF == 8) {
-        if (per >= 16) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
-    }
+    if (GF == 8 ? per >= 16 : groups > 1) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
     return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }
 
