@@ -101,7 +101,7 @@ struct qw_engine {
     // experts, so a wider piece reads and decodes fewer expert weights per token.
     int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
     qw_buf ctl_p{}, ffn_scr_w{};
-    qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_norm_cmb_rc_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
+    qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
               *k_group_w = nullptr, *k_ffn_w = nullptr, *k_qmv_in_w = nullptr, *k_qmv_oa_w = nullptr, *k_qmv_og_w = nullptr;
     qw_buf mlog{}, msel{}, Hhi{}, Hlo{}, Pg{}, rcnt{};
     size_t sel_bytes = 0;
@@ -399,13 +399,10 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
         mw.push_back({"WIDE", 1});
         mw.push_back({"IQ3X", e->ffn_iq3x ? 1 : 0});
         const std::vector<std::pair<const char *, long>> cw = {{"CMB", 1}, {"TOPK", e->TOPK}, {"ROWS", PROWS}, {"WIDE", 1}};
-        auto cr = cw;
-        cr.push_back({"ROWCNT", 1});
         ok = compile(e, "kb_embed", "kb_embed_wide", {{"ROWS", PROWS}}, &e->k_embed_w) &&
              compile(e, "add_rmsnorm", "rmsnorm_wide", {{"ADD", 0}, {"ROWS", PROWS}}, &e->k_norm0_w) &&
              compile(e, "add_rmsnorm", "add_rmsnorm_wide", {{"ADD", 1}, {"ROWS", PROWS}}, &e->k_norm_w) &&
              compile(e, "add_rmsnorm", "cmb_add_rmsnorm_wide", cw, &e->k_norm_cmb_w) &&
-             (!e->k_norm_cmb_rc || compile(e, "add_rmsnorm", "cmb_add_rmsnorm_rows_wide", cr, &e->k_norm_cmb_rc_w)) &&
              compile(e, "moe_route", "moe_logits_wide", mw, &e->k_logits_w) && compile(e, "moe_topk_wide", "moe_topk_wide", mw, &e->k_topk_w) &&
              (c.fma || (e->KA != 2048 && e->KA != 4096) || (e->KG != 2048 && e->KG != 4096) ||  // (else the matvecs go by 64 rows)
               (compile(e, "qmv_mma", "qmv_in_wide", {{"GF", 21}, {"KD", (long)e->D}, {"ROWS", PROWS}, {"YT_F32", 0}}, &e->k_qmv_in_w) &&
@@ -629,9 +626,9 @@ void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *h, const qw_buf *delta, s
     const uint32_t a[2] = {nb, (uint32_t)e->D};
     const bool cmb = delta == &e->Pg;
     const bool gathered = delta == &e->epx;  // slot sharding: the rows were stored by the ranks that own the slots
-    const bool rows = cmb && e->k_norm_cmb_rc && e->ffn_fused && !e->ep_fused && !e->moe_probe;  // the FFN counts its output rows in
     const bool wide = nb > ROWS;
-    if (wide) qw_batch_kernel(b, cmb ? (rows ? e->k_norm_cmb_rc_w : e->k_norm_cmb_w) : delta ? e->k_norm_w : e->k_norm0_w);
+    const bool rows = cmb && !wide && e->k_norm_cmb_rc && e->ffn_fused && !e->ep_fused && !e->moe_probe;  // the FFN counts its output rows in
+    if (wide) qw_batch_kernel(b, cmb ? e->k_norm_cmb_w : delta ? e->k_norm_w : e->k_norm0_w);
     else qw_batch_kernel(b, cmb ? (e->ep_fused ? e->k_norm_cmb_x : rows ? e->k_norm_cmb_rc : e->k_norm_cmb) : gathered ? e->k_norm_x : delta ? e->k_norm : e->k_norm0);
     qw_batch_buf(b, 0, h, 0);
     if (cmb) {
@@ -641,7 +638,7 @@ void enc_norm(qw_engine *e, qw_batch *b, const qw_buf *h, const qw_buf *delta, s
             qw_batch_buf(b, 7, &e->epx, 2 * e->pg_bytes);
             qw_batch_buf(b, 8, &e->rcnt, 64);
         } else qw_batch_buf(b, 6, &e->Pg, 0);
-        if (rows) qw_batch_buf(b, 9, wide ? &e->ffn_scr_w : &e->ffn_scr, 0);
+        if (rows) qw_batch_buf(b, 9, &e->ffn_scr, 0);
     } else if (delta) {
         qw_batch_buf(b, 1, delta, delta_off);
         if (gathered) {

@@ -43,12 +43,6 @@ namespace {
 
 constexpr int FFN_CW = 16;                       // consumer warps
 constexpr int FFN_THREADS = (FFN_CW + 1) * 32;   // + the producer warp
-// see moe_sel.h: the selection record and the scratch buffer of a step (WIDE 0) and of a piece of a prompt (WIDE 1)
-template <int WIDE>
-struct FfnRec {
-    typedef moe_sel_t<WIDE ? MOE_MAXB_WIDE : MOE_MAXB> sel;
-    static constexpr uint32_t MAXITEMS = WIDE ? MOE_FFN_MAXITEMS_WIDE : MOE_FFN_MAXITEMS, ROWCNT = WIDE ? MOE_FFN_ROWCNT_WIDE : MOE_FFN_ROWCNT;
-};
 constexpr int FFN_PITCH = 240;                   // IQ3_S: bytes between staged gate/up rows
 constexpr int FFN_D = 2048, FFN_I = 512;         // the shapes this kernel is built for (the launcher refuses others)
 constexpr int FFN_MAXG = 520;                    // groups kept in shared memory: E <= 512 experts (+ end markers)
@@ -96,8 +90,7 @@ struct __align__(16) FfnItem {
 };
 // item number w -> (group, pass): routed groups first (pre[] = passes before each group, in shared memory), then the shared
 // expert's passes.  The group's entries and expert come from the selection record in global memory.
-template <class SEL>
-__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const SEL *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
+__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const moe_sel *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
     FfnItem it{};
     const uint32_t routed = pre[U];
     uint32_t cnt;
@@ -265,6 +258,12 @@ __device__ __forceinline__ void iq3x_word_s(uint32_t q, const uint4 &c, uint32_t
     w[2] = *(const uint32_t *)&v2;
     w[3] = *(const uint32_t *)&v3;
 }
+// constants of the decode multiply-adds for scale field s: (S, -1040 S, S / 16, -80 S) as fp16 pairs, S = 1 + 2 s
+__device__ __forceinline__ void x_scale_entry(uint8_t *tab, int s) {
+    const float S = (float)(1 + 2 * s);
+    const __half2 m0 = __float2half2_rn(S), a0 = __float2half2_rn(-1040.0f * S), m1 = __float2half2_rn(S * 0.0625f), a1 = __float2half2_rn(-80.0f * S);
+    *(uint4 *)(tab + 16 * s) = make_uint4(*(const uint32_t *)&m0, *(const uint32_t *)&a0, *(const uint32_t *)&m1, *(const uint32_t *)&a1);
+}
 // Software-pipelined over the sub-blocks: the MMAs of sub-block i are issued, then the loads and the decode of sub-block
 // i + 1 -- the MMA results are not waited for.  (The predicated B loads keep zeros in lanes whose column is absent.)
 struct XDec {
@@ -328,11 +327,10 @@ __device__ __forceinline__ void x_unit(uint32_t rec0, uint32_t rec1, int kh, int
 // TMA boxes and bulk copies through the same ring, but the consumers only read every staged byte once (16-byte loads) and
 // compute nothing -- the role of the reference's pure-read probes (bench/moe_bw.c:1-3, bench/qmv.c:357-382).
 // (17 warps put five on one scheduler, whose 16 K registers then allow 96 per thread)
-template <bool PROBE, int FMT, int WIDE, bool HALF = false>
+template <bool PROBE, int FMT, bool HALF = false>
 __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(const __grid_constant__ CUtensorMap mG, const __grid_constant__ CUtensorMap mU,
                                                            const __grid_constant__ CUtensorMap mSG, const __grid_constant__ CUtensorMap mSU, const FfnP p) {
     using C = FfnCfg<FMT>;
-    using Rec = FfnRec<WIDE>;
     constexpr int FFN_STG = C::STG, FFN_SLOT = C::SLOT;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *bars = (uint64_t *)smem;
@@ -364,19 +362,15 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
             bulk_g2s(smem + C::OFF_TAB, p.tab->grid_u32x32, C::TAB, tab_bar);
         }
     }
-    if (FMT == 1 && tid < 16) {  // constants of the decode multiply-adds for scale field s = tid: (S, -1040 S, S / 16, -80 S) as fp16 pairs, S = 1 + 2 s
-        const float S = (float)(1 + 2 * tid);
-        const __half2 m0 = __float2half2_rn(S), a0 = __float2half2_rn(-1040.0f * S), m1 = __float2half2_rn(S * 0.0625f), a1 = __float2half2_rn(-80.0f * S);
-        *(uint4 *)(smem + C::OFF_TAB + 16 * tid) = make_uint4(*(const uint32_t *)&m0, *(const uint32_t *)&a0, *(const uint32_t *)&m1, *(const uint32_t *)&a1);
-    }
+    if (FMT == 1 && tid < 16) x_scale_entry(smem + C::OFF_TAB, tid);
     pdl_wait();  // the selection record, the tokens and Pg belong to earlier kernels
-    const typename Rec::sel *ms = (const typename Rec::sel *)p.ms;
+    const moe_sel *ms = (const moe_sel *)p.ms;
     // passes before every group: independent loads, so the table is in shared memory after one latency
     for (uint32_t i = tid; i < FFN_MAXG; i += FFN_THREADS) pre[i] = ms->pre[i];
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
     uint32_t items = pre[U] + (p.Sd ? (nb + 7) / 8 : 0);
-    if (items > Rec::MAXITEMS) {  // cannot happen with E <= 512 and 64 (512) tokens; never index past the flags
+    if (items > MOE_FFN_MAXITEMS) {  // cannot happen with E <= 512 and 64 tokens; never index past the flags
         if (tid == 0) set_status(p.status, ST_BAD_ARG | 5);
         items = 0;
     }
@@ -707,8 +701,8 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                     __syncwarp();
                     if (g == 0) {
                         __threadfence();  // the warp's stores (cumulative over the warp barrier) before the counts
-                        if (oo[0] != 0xffffffffu) atomicAdd(p.sync + Rec::ROWCNT + oo[0] / D, 1u);
-                        if (oo[1] != 0xffffffffu) atomicAdd(p.sync + Rec::ROWCNT + oo[1] / D, 1u);
+                        if (oo[0] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[0] / D, 1u);
+                        if (oo[1] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[1] / D, 1u);
                     }
                 }
             }
@@ -720,12 +714,408 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     __syncthreads();
     if (tid == 0 && !PROBE) {
         __threadfence();
-        if (atomicAdd(p.sync + Rec::MAXITEMS, 1u) == gridDim.x - 1) {
+        if (atomicAdd(p.sync + MOE_FFN_MAXITEMS, 1u) == gridDim.x - 1) {
             for (uint32_t i = 0; i < items; i++) p.sync[i] = 0;
-            p.sync[Rec::MAXITEMS] = 0;
+            p.sync[MOE_FFN_MAXITEMS] = 0;
         }
     }
     if (p.ep.nranks > 1) ep_publish(p.ep);
+}
+
+// ---- A piece of a prompt.  Its tokens choose nearly every expert, eight tokens and more each, so the decode of a stage is shared by more columns: an
+// item is up to WFFN_COLS columns (MMA column tiles of 8) of an expert, and a warp runs the decoded fragments of a sub-block against as many tiles as
+// the item has.  A column's MMAs and sums are those of moe_ffn_k, in the same order.
+// One block per SM (16 token rows are 65 KB, and four stages keep the copies ahead of the decode) of 16 + 1 warps with up to 96 registers: the tiles'
+// independent MMA chains take the place of the second block.  Shares of the work are cut by cost, not by piece: an item weighs a decode and its tiles
+// (WffnCost), because experts with one tile and the shared expert's full items lie apart in the list.  The two K halves of a row group exchange
+// tiles: even ones are finished by the low half, odd ones by the high half.  The combine + norm that follows waits for the whole launch, so no
+// output row is counted in.
+// One layer on a B200, against items of eight columns in moe_ffn_k: 419 tokens 372 -> 328 us, 512 tokens 423 -> 358; prompts of 419 tokens, 48 layers, 36.8 ->
+// 35.2 ms, of 1700 tokens, 12 layers, 34.2 -> 32.6.  Bound by the decode still (all 513 experts are 857 MB, 131 us).  With 32 columns two stages are
+// left in shared memory and the copies' latency shows: 355 us.
+constexpr int WFFN_RECS = 16;
+constexpr uint32_t WFFN_STG = 4, WFFN_COLS = MOE_FFN_COLS_WIDE, WFFN_CT = WFFN_COLS / 8;
+struct WffnCost {  // of a gate/up piece and of a down piece: a decode of the stage, and the MMAs and the epilogue of a column tile
+    uint32_t dec, tile;
+};
+__device__ constexpr WffnCost WFFN_GU{6, 1}, WFFN_DN{5, 2};
+constexpr uint32_t WFFN_XP = FFN_D * 2 + 64, WFFN_HP = FFN_I * 4 + 64;  // distance of the token rows, and of the H rows (both planes), in shared memory
+constexpr uint32_t WFFN_OFF_TAB = 128, WFFN_OFF_PRE = WFFN_OFF_TAB + 256, WFFN_OFF_REC = WFFN_OFF_PRE + 2 * FFN_MAXG * 4, WFFN_OFF_RED = WFFN_OFF_REC + 2 * WFFN_RECS * 32 + 128,
+                   WFFN_RED = 8 * WFFN_CT * 32 * 16, WFFN_OFF_XS = (WFFN_OFF_RED + 2 * WFFN_RED + 127) / 128 * 128, WFFN_OFF_STG = WFFN_OFF_XS + WFFN_COLS * WFFN_XP,
+                   WFFN_SMEM = WFFN_OFF_STG + WFFN_STG * IQ3X_STAGE;
+static_assert(WFFN_SMEM <= 227 * 1024 && WFFN_HP <= WFFN_XP && WFFN_COLS <= 32, "shared memory of the wide expert FFN");
+static_assert(WFFN_CT == 2, "column tiles that xw_tiles distinguishes");
+
+// one super-block of rows g / g + 8 against NT column tiles; xb[i] = address of this lane's 16 bytes of tile i
+template <int PLANES, int NT>
+__device__ __forceinline__ void xw_unit(uint32_t rec0, uint32_t rec1, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[WFFN_CT], uint32_t xo,
+                                        float (&acc)[WFFN_CT][4]) {
+    const uint32_t c0 = rec0 + kh * 128 + t * 4, c1 = rec1 + kh * 128 + t * 4;
+    const XHdr h0 = x_hdr(rec0, kh), h1 = x_hdr(rec1, kh);
+    float p[NT][4];
+    uint32_t q[2] = {lds_u32_off<0>(c0), lds_u32_off<0>(c1)};
+    XDec dec;
+    x_decode<0>(q, h0, h1, stab, dec);
+#define XW_SUB(IB)                                                                                                             \
+    {                                                                                                                          \
+        uint4 xv[NT], xl[NT];                                                                                                  \
+        _Pragma("unroll") for (int i = 0; i < NT; i++) {                                                                       \
+            xv[i] = lds_v4(xb[i] + xo + IB * 64);                                                                              \
+            if (PLANES == 2) xl[i] = lds_v4(xb[i] + xo + FFN_I * 2 + IB * 64);                                                 \
+        }                                                                                                                      \
+        if (IB < 7) {                                                                                                          \
+            q[0] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c0);                                                                \
+            q[1] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c1);                                                                \
+        }                                                                                                                      \
+        _Pragma("unroll") for (int i = 0; i < NT; i++) {                                                                       \
+            if (IB == 0) mma_f16(p[i], dec.a0, xv[i].x, xv[i].y, zr.z);                                                        \
+            else mma_f16(p[i], dec.a0, xv[i].x, xv[i].y, p[i]);                                                                \
+        }                                                                                                                      \
+        _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a1, xv[i].z, xv[i].w, p[i]);                          \
+        if (PLANES == 2) {                                                                                                     \
+            _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a0, xl[i].x, xl[i].y, p[i]);                      \
+            _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a1, xl[i].z, xl[i].w, p[i]);                      \
+        }                                                                                                                      \
+        if (IB < 7) x_decode<(IB < 7 ? IB + 1 : 0)>(q, h0, h1, stab, dec);                                                     \
+    }
+    XW_SUB(0) XW_SUB(1) XW_SUB(2) XW_SUB(3) XW_SUB(4) XW_SUB(5) XW_SUB(6) XW_SUB(7)
+#undef XW_SUB
+#pragma unroll
+    for (int i = 0; i < NT; i++) {
+        acc[i][0] = fmaf(h0.d, p[i][0], acc[i][0]);
+        acc[i][1] = fmaf(h0.d, p[i][1], acc[i][1]);
+        acc[i][2] = fmaf(h1.d, p[i][2], acc[i][2]);
+        acc[i][3] = fmaf(h1.d, p[i][3], acc[i][3]);
+    }
+}
+template <int PLANES>
+__device__ __forceinline__ void xw_tiles(uint32_t nt, uint32_t rec0, uint32_t rec1, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[WFFN_CT], uint32_t xo,
+                                         float (&acc)[WFFN_CT][4]) {
+    if (nt == 1) xw_unit<PLANES, 1>(rec0, rec1, kh, t, stab, zr, xb, xo, acc);
+    else xw_unit<PLANES, 2>(rec0, rec1, kh, t, stab, zr, xb, xo, acc);
+}
+
+// item -> its columns.  prw = items before a group (of the selection record, in shared memory)
+__device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_wide *ms, uint32_t U, uint32_t nb, uint32_t w) {
+    FfnItem it{};
+    const uint32_t routed = prw[U];
+    uint32_t cnt;
+    if (w >= routed) {
+        it.shared = 1;
+        it.e0 = ms->off[U];  // (the shared expert's H rows follow the entries')
+        cnt = nb;
+        it.c0 = (w - routed) * WFFN_COLS;
+    } else {
+        uint32_t lo = 0, hi = U;  // largest u with prw[u] <= w
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (prw[mid] <= w) lo = mid;
+            else hi = mid;
+        }
+        it.e0 = ms->off[lo];
+        cnt = ms->off[lo + 1] - it.e0;
+        it.c0 = (w - prw[lo]) * WFFN_COLS;
+        it.erow = ms->ue[lo];
+    }
+    it.ncols = cnt - it.c0 < WFFN_COLS ? cnt - it.c0 : WFFN_COLS;
+    return it;
+}
+// first piece (item * P + piece of the item) of block b of G: where b / G of the list's cost is reached.  pre = tiles of 8 before a group
+__device__ __forceinline__ uint32_t wffn_edge(const uint32_t *pre, const uint32_t *prw, uint32_t U, uint32_t nb, bool shared, uint32_t b, uint32_t G, uint32_t P, WffnCost c) {
+    const uint32_t st = shared ? (nb + 7) / 8 : 0, si = shared ? (nb + WFFN_COLS - 1) / WFFN_COLS : 0, items = prw[U] + si;
+    if (b == G) return items * P;
+    const uint32_t x = (uint32_t)((uint64_t)P * (c.dec * items + c.tile * (pre[U] + st)) * b / G);
+    auto at = [&](uint32_t u) { return P * (c.dec * prw[u] + c.tile * pre[u]); };  // cost before group u
+    uint32_t lo = 0, hi = U + 1;  // largest u <= U with at(u) <= x; group U is the shared expert
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (at(mid) <= x) lo = mid;
+        else hi = mid;
+    }
+    uint32_t rest = x - at(lo);
+    const uint32_t tiles = lo < U ? pre[lo + 1] - pre[lo] : st, full = P * (c.dec + c.tile * WFFN_CT);
+    const uint32_t q = rest / full;  // whole items of this group before x
+    rest -= q * full;
+    const uint32_t left = tiles - q * WFFN_CT, nt = left < WFFN_CT ? left : WFFN_CT;
+    return (prw[lo] + q) * P + rest / (c.dec + c.tile * nt);
+}
+
+__global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t *full = (uint64_t *)smem, *empty = full + WFFN_STG, *actfull = empty + WFFN_STG, *actfree = actfull + 2;
+    uint32_t *pre = (uint32_t *)(smem + WFFN_OFF_PRE), *prw = pre + FFN_MAXG;
+    FfnItem *recs = (FfnItem *)(smem + WFFN_OFF_REC);
+    uint32_t *edge = (uint32_t *)(smem + WFFN_OFF_REC + 2 * WFFN_RECS * 32);
+    constexpr uint32_t D = FFN_D, I = FFN_I, KP = D / 512, GT = I / 64, DT = D / 128;
+    const uint32_t act0 = smem_u32(smem + WFFN_OFF_XS), slot0 = smem_u32(smem + WFFN_OFF_STG);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    pdl_launch();
+    if (tid == 0) {
+        for (uint32_t s = 0; s < WFFN_STG; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], FFN_CW);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&actfull[s], 1);
+            mbar_init(&actfree[s], FFN_CW);
+        }
+        mbar_init_fence();
+    }
+    if (tid < 16) x_scale_entry(smem + WFFN_OFF_TAB, tid);
+    pdl_wait();
+    const moe_sel_wide *ms = (const moe_sel_wide *)p.ms;
+    for (uint32_t i = tid; i < FFN_MAXG; i += FFN_THREADS) {
+        pre[i] = ms->pre[i];
+        prw[i] = ms->prw[i];
+    }
+    const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
+    __syncthreads();
+    uint32_t items = prw[U] + (p.Sd ? (nb + WFFN_COLS - 1) / WFFN_COLS : 0);
+    const bool bad = items > MOE_FFN_MAXITEMS_WIDE;  // cannot happen with E <= 512 and MOE_MAXB_WIDE tokens; never index past the counters
+    if (bad && tid == 0) set_status(p.status, ST_BAD_ARG | 5);
+    if (bad) items = 0;
+    if (tid < 4) edge[tid] = bad ? 0 : wffn_edge(pre, prw, U, nb, p.Sd != nullptr, blockIdx.x + (tid & 1), gridDim.x, tid < 2 ? GT : DT, tid < 2 ? WFFN_GU : WFFN_DN);
+    __syncthreads();
+    uint32_t a_lo = edge[0], a_hi = edge[1], b_lo = edge[2], b_hi = edge[3];
+    const uint32_t wa0 = a_lo / GT, wb0 = b_lo / DT;
+    if ((a_hi > a_lo && (a_hi - 1) / GT - wa0 >= WFFN_RECS) || (b_hi > b_lo && (b_hi - 1) / DT - wb0 >= WFFN_RECS)) {  // a grid far smaller than the device's
+        if (tid == 0) set_status(p.status, ST_BAD_ARG | 6);
+        a_hi = a_lo;
+        b_hi = b_lo;
+    }
+    if (tid < 2 * WFFN_RECS) {
+        const uint32_t k = tid % WFFN_RECS, w = (tid < WFFN_RECS ? wa0 : wb0) + k;
+        const bool need = tid < WFFN_RECS ? (a_hi > a_lo && w <= (a_hi - 1) / GT) : (b_hi > b_lo && w <= (b_hi - 1) / DT);
+        if (need) recs[tid] = wffn_item(prw, ms, U, nb, w);
+    }
+    __syncthreads();
+    const FfnItem *rec_a = recs - wa0, *rec_b = recs + WFFN_RECS - wb0;  // rec_a[w], rec_b[w]
+
+    if (warp == FFN_CW) {
+        // ---- producer warp: lane 0 keeps the stages full; lane c fetches column c of a new item
+        bool ok = true;
+        uint32_t j = 0, k = 0, rowbase = 0, prev_n = WFFN_COLS;
+        auto stage = [&](const uint8_t *src) {
+            const uint32_t s = j % WFFN_STG;
+            if (j >= WFFN_STG && ok && !mbar_wait(&empty[s], (j / WFFN_STG - 1) & 1)) {
+                ok = false;
+                if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 6);
+            }
+            if (lane == 0) {
+                fence_proxy_async();  // the consumers' reads of the stage are ordered before the copy engine's writes
+                mbar_expect_tx(&full[s], IQ3X_STAGE);
+                bulk_s(slot0 + s * IQ3X_STAGE, src, IQ3X_STAGE, &full[s]);
+            }
+            j++;
+        };
+        // the ring of activation rows, as in moe_ffn_k: returns this lane's row for the item's column `lane`
+        auto act_for = [&](uint32_t ncols, uint32_t bytes, bool fresh) {
+            const uint32_t s = k & 1, n = k >> 1;
+            bool good = n < 1 || !ok || mbar_wait(&actfree[s], (n - 1) & 1);
+            if (k >= 1 && (fresh || prev_n + ncols > WFFN_COLS)) good = (!ok || mbar_wait(&actfree[(k - 1) & 1], ((k - 1) >> 1) & 1)) && good;
+            if (!good) {
+                ok = false;
+                if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 7);
+            }
+            if (fresh) rowbase = 0;
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_expect_tx(&actfull[s], bytes);
+            __syncwarp();
+            const uint32_t r0 = rowbase;
+            rowbase = (rowbase + ncols) % WFFN_COLS;
+            prev_n = ncols;
+            return (r0 + lane) % WFFN_COLS;
+        };
+        uint32_t cur = 0xffffffffu;
+        for (uint32_t a = a_lo; a < a_hi; a++) {
+            const uint32_t w = a / GT, gt = a - w * GT;
+            const FfnItem it = rec_a[w];
+            const uint8_t *src = (it.shared ? p.Sg : p.Wg) + ((size_t)it.erow * GT + gt) * KP * IQ3X_STAGE;
+            for (uint32_t kp = 0; kp < KP; kp++) {
+                stage(src + (size_t)kp * IQ3X_STAGE);
+                if (w != cur && kp == 0) {
+                    cur = w;
+                    uint32_t tok = 0, rank;
+                    if ((uint32_t)lane < it.ncols) ffn_entry(ms, it, topk, lane, tok, rank);
+                    const uint32_t row = act_for(it.ncols, it.ncols * D * 2, false);
+                    if ((uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_XP, p.x + (size_t)tok * D, D * 2, &actfull[k & 1]);
+                    k++;
+                }
+            }
+        }
+        cur = 0xffffffffu;
+        bool first_dn = true;
+        for (uint32_t bi = b_lo; bi < b_hi; bi++) {
+            const uint32_t w = bi / DT, dt = bi - w * DT;
+            const FfnItem it = rec_b[w];
+            stage((it.shared ? p.Sd : p.Wd) + ((size_t)it.erow * DT + dt) * IQ3X_STAGE);
+            if (w != cur) {  // H of a new item: complete when both K halves of all its row groups have counted in
+                cur = w;
+                if (ok && ld_acquire_gpu(p.sync + w) < GT * FFN_CW) {
+                    const uint64_t t0 = global_ns();
+                    while (ld_acquire_gpu(p.sync + w) < GT * FFN_CW)
+                        if (global_ns() - t0 > 2000000000ull) {
+                            ok = false;
+                            if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 11);
+                            break;
+                        }
+                }
+                __syncwarp();
+                asm volatile("fence.proxy.async.global;" ::: "memory");  // the H rows were written by ordinary stores; the copy engine reads them
+                const uint32_t row = act_for(it.ncols, it.ncols * I * 4, first_dn);
+                first_dn = false;
+                if ((uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_HP, p.H + (size_t)(it.e0 + it.c0 + lane) * 2 * I, I * 4, &actfull[k & 1]);
+                k++;
+            }
+        }
+    } else {
+        const int r = warp & 7, kh = warp >> 3;
+        bool ok = true;
+        const uint32_t stab = smem_u32(smem + WFFN_OFF_TAB);
+        const ZeroRegs zr = zero_regs();
+        uint32_t j = 0, k = 0, rowbase = 0, rc = 0, xb[WFFN_CT];
+        auto wait_full = [&]() {
+            if (ok && !mbar_wait(&full[j % WFFN_STG], (j / WFFN_STG) & 1)) {
+                ok = false;
+                if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 9);
+            }
+            return slot0 + (j % WFFN_STG) * IQ3X_STAGE;
+        };
+        auto release = [&]() {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[j % WFFN_STG]);
+            j++;
+        };
+        auto act_wait = [&](uint32_t ncols, uint32_t pitch) {  // columns past the item's read whatever the row holds: nobody looks at their results
+            if (ok && !mbar_wait(&actfull[k & 1], (k >> 1) & 1)) {
+                ok = false;
+                if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 10);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++) xb[i] = act0 + ((rowbase + 8 * i + g) % WFFN_COLS) * pitch + t * 16;
+            rowbase = (rowbase + ncols) % WFFN_COLS;
+        };
+        auto act_release = [&]() {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&actfree[k & 1]);
+            k++;
+        };
+        // The two K halves of a row group: odd tiles go to the high half, even ones to the low half; low + high either way.  Two buffers alternate.
+        auto exchange = [&](float (&acc)[WFFN_CT][4], uint32_t nt) {
+            float4 *rd = (float4 *)(smem + WFFN_OFF_RED + (rc & 1) * WFFN_RED) + r * WFFN_CT * 32 + lane;
+            rc++;
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++)
+                if (i < nt && (int)(i & 1) != kh) rd[i * 32] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            bar_sync_n(1 + r, 64);
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++)
+                if (i < nt && (int)(i & 1) == kh) {
+                    const float4 v = rd[i * 32];
+                    acc[i][0] += v.x;
+                    acc[i][1] += v.y;
+                    acc[i][2] += v.z;
+                    acc[i][3] += v.w;
+                }
+        };
+        uint32_t cur = 0xffffffffu, ncols = 0, nt = 0, hrow = 0;
+        for (uint32_t a = a_lo; a < a_hi; a++) {
+            const uint32_t w = a / GT, gt = a - w * GT;
+            if (w != cur) {
+                if (cur != 0xffffffffu) act_release();
+                cur = w;
+                const FfnItem it = rec_a[w];
+                ncols = it.ncols;
+                nt = (ncols + 7) / 8;
+                hrow = it.e0 + it.c0;
+                act_wait(ncols, WFFN_XP);
+            }
+            float acc[WFFN_CT][4];
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+            for (uint32_t kp = 0; kp < KP; kp++) {
+                const uint32_t st = wait_full(), rec0 = st + (8 * r + g) * IQ3X_REC;
+                xw_tiles<1>(nt, rec0, rec0 + 64 * IQ3X_REC, kh, t, stab, zr, xb, (2 * kp + kh) * 512, acc);
+                release();
+            }
+            exchange(acc, nt);
+            __half *Hw = p.H + (size_t)hrow * 2 * I + gt * 64 + 8 * r + g;  // H [row][plane][I]
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++) {
+                if (i >= nt || (int)(i & 1) != kh) continue;
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const float gs = acc[i][c], us = acc[i][2 + c];
+                    float h = gs / (1.0f + expf(-gs)) * us;
+                    h = fminf(fmaxf(h, -65504.0f), 65504.0f);
+                    const __half hi = __float2half_rn(h);
+                    const __half lo = __float2half_rn(h - __half2float(hi));
+                    const uint32_t n = 8 * i + 2 * t + c;
+                    if (n < ncols) {
+                        Hw[(size_t)n * 2 * I] = hi;
+                        Hw[(size_t)n * 2 * I + I] = lo;
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) {
+                if ((uint32_t)kh < nt) __threadfence();  // the warp's H values (cumulative over the warp barrier) before the count
+                atomicAdd(p.sync + w, 1u);
+            }
+        }
+        if (cur != 0xffffffffu) act_release();
+        // ---- down pieces
+        cur = 0xffffffffu;
+        rowbase = 0;
+        uint32_t oo[(WFFN_CT + 1) / 2][2];  // element offsets of the output rows of columns 2t and 2t + 1 of this half's tiles
+        for (uint32_t bi = b_lo; bi < b_hi; bi++) {
+            const uint32_t w = bi / DT, dt = bi - w * DT;
+            if (w != cur) {
+                if (cur != 0xffffffffu) act_release();
+                cur = w;
+                const FfnItem it = rec_b[w];
+                nt = (it.ncols + 7) / 8;
+#pragma unroll
+                for (uint32_t i = 0; i < (WFFN_CT + 1) / 2; i++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        const uint32_t n = 8 * (2 * i + kh) + 2 * t + c;
+                        oo[i][c] = 0xffffffffu;
+                        if (n < it.ncols) {
+                            uint32_t tok, rank;
+                            ffn_entry(ms, it, topk, n, tok, rank);
+                            oo[i][c] = (tok * (topk + 1) + rank) * D;
+                        }
+                    }
+                act_wait(it.ncols, WFFN_HP);
+            }
+            float acc[WFFN_CT][4];
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+            const uint32_t st = wait_full(), rec0 = st + (16 * r + g) * IQ3X_REC;
+            xw_tiles<2>(nt, rec0, rec0 + 8 * IQ3X_REC, kh, t, stab, zr, xb, kh * 512, acc);
+            release();
+            exchange(acc, nt);
+            const uint32_t row = dt * 128 + 16 * r + 2 * g;
+#pragma unroll
+            for (uint32_t i = 0; i < WFFN_CT; i++) {
+                if (i >= nt || (int)(i & 1) != kh) continue;
+                if (oo[i / 2][0] != 0xffffffffu) *(float2 *)(p.Pg + oo[i / 2][0] + row) = make_float2(acc[i][0], acc[i][2]);
+                if (oo[i / 2][1] != 0xffffffffu) *(float2 *)(p.Pg + oo[i / 2][1] + row) = make_float2(acc[i][1], acc[i][3]);
+            }
+        }
+        if (cur != 0xffffffffu) act_release();
+    }
+    // the last block to finish clears the items' counters for the next launch (every block has read what it needed by then)
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(p.sync + MOE_FFN_MAXITEMS_WIDE, 1u) == gridDim.x - 1) {
+            for (uint32_t i = 0; i < items; i++) p.sync[i] = 0;
+            p.sync[MOE_FFN_MAXITEMS_WIDE] = 0;
+        }
+    }
 }
 
 // ---- tensor maps: an expert tensor [rows][pitch bytes] seen as a 2-D byte array, box = 240 bytes x 64 rows, no swizzle
@@ -772,11 +1162,10 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     p.Wd = L.buf<uint8_t>(6);
     p.Wg = Wg;
     p.Sg = Sg;
-    // WIDE defined 1: a piece of a prompt -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has 512 rows of tokens; one GPU only
+    // WIDE defined 1: a piece of a prompt (moe_ffn_wide_k) -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has MOE_MAXB_WIDE rows of tokens; one GPU only
     const bool wide = L.def("WIDE", 0) != 0;
     p.sync = L.buf<unsigned>(8);
     QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I) : MOE_FFN_SCRATCH_BYTES(I)));
-    // and only IQ3X: with one block per SM a share of its items would not fit FFN_RECS.
     QW_CHECK_ARG(!wide || (x4 && L.def("EPX", 0) <= 1 && L.def("PROBE", 0) == 0));
     p.H = (__half *)((uint8_t *)p.sync + (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
     p.Sd = shared ? L.buf<uint8_t>(7) : nullptr;
@@ -828,8 +1217,18 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     const uint32_t nb = L.has_bytes(13, 4) ? L.bytes<uint32_t>(13) : 0, grid = (uint32_t)(L.sm_count * per_sm);
     const double items = E * (1 - pow(1 - (double)topk / E, (double)nb)) + (nb + 7) / 8;
     const bool half = x4 && !wide && !probe && p.ep.nranks == 1 && nb >= 1 && 2 * items * (I / 64) <= grid * (33.0 / 32);
-    auto kern = wide ? moe_ffn_k<false, 1, 1> : half ? moe_ffn_k<false, 1, 0, true>
-                : x4 ? (probe ? moe_ffn_k<true, 1, 0> : moe_ffn_k<false, 1, 0>) : (probe ? moe_ffn_k<true, 0, 0> : moe_ffn_k<false, 0, 0>);
+    if (wide) {
+        QW_CHECK_ARG(EL == E && p.ebase == 0);
+        cudaError_t e = cudaFuncSetAttribute(moe_ffn_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WFFN_SMEM);
+        if (e != cudaSuccess) return e;
+        int occ = 0;  // the blocks wait for one another's H
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, moe_ffn_wide_k, FFN_THREADS, WFFN_SMEM);
+        if (e != cudaSuccess) return e;
+        QW_CHECK_ARG(occ >= 1);
+        qw_launch(moe_ffn_wide_k, (uint32_t)L.sm_count, FFN_THREADS, WFFN_SMEM, L.stream, p);
+        return cudaGetLastError();
+    }
+    auto kern = half ? moe_ffn_k<false, 1, true> : x4 ? (probe ? moe_ffn_k<true, 1> : moe_ffn_k<false, 1>) : (probe ? moe_ffn_k<true, 0> : moe_ffn_k<false, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;  // the blocks wait for one another's H: all of them must be resident together

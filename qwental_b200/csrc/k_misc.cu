@@ -199,8 +199,8 @@ static cudaError_t launch_add_rmsnorm(const QwLaunch &L) {
             // ROWCNT defined 1 (one GPU, after moe_ffn): 9 = the FFN's scratch buffer, whose per-row counters replace the wait for the launch
             unsigned *rowcnt = nullptr;
             if (L.def("ROWCNT", 0)) {
-                QW_CHECK_ARG(nranks == 1 && L.buf<unsigned>(9) && L.avail(9) >= (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
-                rowcnt = L.buf<unsigned>(9) + (wide ? MOE_FFN_ROWCNT_WIDE : MOE_FFN_ROWCNT);
+                QW_CHECK_ARG(nranks == 1 && !wide && L.buf<unsigned>(9) && L.avail(9) >= MOE_FFN_SYNC_BYTES);
+                rowcnt = L.buf<unsigned>(9) + MOE_FFN_ROWCNT;
             }
             qw_launch(cmb_rmsnorm_cl_k, a.nb * 8, 256, 0, L.stream, L.buf<float>(0), L.buf<float>(2), L.buf<__half>(3), L.buf<moe_sel>(5), L.buf<float>(6), topk,
                       nranks > 1 ? L.buf<unsigned>(7) : nullptr, nranks > 1 ? L.buf<unsigned>(8) : nullptr, nranks, rowcnt, (unsigned *)L.status);

@@ -192,8 +192,9 @@ __device__ __forceinline__ void moe_topk_row(const float *lg, uint32_t E, uint32
 }
 
 // Grouping of nb tokens' chosen experts (sid [token][MOE_MAXK]) by one block of NTH >= E threads: thread e owns expert e in the scans.
+// prw: items of MOE_FFN_COLS_WIDE entries in the groups before u, or nullptr
 template <int NTH, class SEL, int W, int ME>
-__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][ME]) {
+__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][ME], uint32_t *prw) {
     __shared__ uint32_t pos[MOE_MAXE];
     __shared__ uint32_t wsum[2][32];
     constexpr uint32_t NW = NTH / 32;
@@ -207,12 +208,12 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
     }
     __syncthreads();
     {   // exclusive scans over experts (thread e = expert e): entries (low 16 bits of one word) and passes of 8 entries
-        // (high 16 bits: what the gate/up and down kernels enumerate their work units by), and non-empty flags
+        // (high 16 bits: what the gate/up and down kernels enumerate their work units by), and non-empty flags (with the wide items above)
         uint32_t c0 = 0;
         if (tid < E)
 #pragma unroll
             for (int q = 0; q < W; q++) c0 += __popc(mask[q][tid]);
-        const uint32_t f = c0 ? 1u : 0u, c = c0 | (((c0 + 7) / 8) << 16);
+        const uint32_t f = c0 ? 1u | ((c0 + MOE_FFN_COLS_WIDE - 1) / MOE_FFN_COLS_WIDE) << 16 : 0u, c = c0 | (((c0 + 7) / 8) << 16);
         uint32_t sc = c, sf = f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -236,16 +237,20 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
         const uint32_t ex = bc + sc - c;  // exclusive prefix: entries | passes << 16
         pos[tid] = ex & 0xffffu;          // first entry of expert tid
         if (c0) {
-            ms->ue[bf + sf - f] = tid;
-            ms->off[bf + sf - f] = ex & 0xffffu;
-            ms->pre[bf + sf - f] = ex >> 16;
+            const uint32_t fx = bf + sf - f, u = fx & 0xffffu;
+            ms->ue[u] = tid;
+            ms->off[u] = ex & 0xffffu;
+            ms->pre[u] = ex >> 16;
+            if (prw) prw[u] = fx >> 16;
         }
         if (tid == NTH - 1) {
-            ms->U = bf + sf;
+            const uint32_t U = (bf + sf) & 0xffffu;
+            ms->U = U;
             ms->nb = a.nb;
             ms->topk = topk;
-            ms->off[bf + sf] = (bc + sc) & 0xffffu;
-            ms->pre[bf + sf] = (bc + sc) >> 16;
+            ms->off[U] = (bc + sc) & 0xffffu;
+            ms->pre[U] = (bc + sc) >> 16;
+            if (prw) prw[U] = (bf + sf) >> 16;
         }
     }
     __syncthreads();
@@ -270,7 +275,7 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
     for (uint32_t t = warp; t < a.nb; t += NTH / 32)
         moe_topk_row(logits + (size_t)t * (E + 1), E, topk, tid & 31, cand_s[warp], ms->ids[t], sid + t * MOE_MAXK, ms->w[t]);
     __syncthreads();
-    moe_group_body<NTH>(sid, ms, E, topk, a, mask);
+    moe_group_body<NTH>(sid, ms, E, topk, a, mask, nullptr);
 }
 
 // ---- a piece of a prompt (up to 512 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(512) moe_group_wide_k(moe_sel_wide *ms, uint32
     for (int q = 0; q < MOE_MAXB_WIDE / 32; q++) mask[q][threadIdx.x] = 0;
     __syncthreads();
     pdl_wait();
-    moe_group_body<512>(&ms->sid[0][0], (moe_sel_t<MOE_MAXB_WIDE> *)ms, E, topk, a, mask);
+    moe_group_body<512>(&ms->sid[0][0], (moe_sel_t<MOE_MAXB_WIDE> *)ms, E, topk, a, mask, ms->prw);
 }
 static bool moe_wide_check(const QwLaunch &L, const sel_args &a, uint32_t E, uint32_t topk) {
     return L.buf<void>(1) && L.has_bytes(2, 12) && E % 32 == 0 && (E == 512 || E <= 256) && topk >= 1 && topk < MOE_MAXK && topk <= E && a.nb >= 1 &&

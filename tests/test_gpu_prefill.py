@@ -163,6 +163,26 @@ def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
         e.close()
 
 
+@pytest.mark.parametrize("experts,topk", [(32, 15), (512, 1), (64, 2)])
+def test_expert_items_of_a_piece(gpu, experts, topk):
+    """The expert FFN of a piece takes items of up to 16 columns: experts with hundreds of tokens (full items, a remainder of one column and of one
+    tile), with one token or none, and a work list shorter than the number of blocks."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(experts=experts, topk=topk, layers=2, attn_every=2, max_slots=2))
+    try:
+        lengths = {66, 129, 145, 400, 512}
+        text = np.random.default_rng(13).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+    finally:
+        e.close()
+
+
 @pytest.mark.parametrize("layers,every", [(4, 4), (5, 4), (1, 1), (3, 2)])
 def test_last_layer_of_a_prompt(gpu, layers, every):
     """After the last layer's K, V and state only the prompt's last token goes on: Gated DeltaNet and attention as the last layer, one piece and several
