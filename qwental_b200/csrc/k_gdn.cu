@@ -25,6 +25,19 @@ struct dn_epi_args {
     uint32_t nb, layer, nlayers, proj_stride;
 };
 
+// The epilogue of a channel, shared by the forms below so that they give the same bits.  (The multiply-adds of the convolution are spelt out: left to
+// the compiler, the sum may be contracted in one way in one kernel and in another way in the next.)  s3 = the newest of the channel's last four inputs
+__device__ __forceinline__ __half dn_conv(const float4 &w, float s0, float s1, float s2, float s3) {
+    const float y = __fmaf_rn(w.w, s3, __fmaf_rn(w.z, s2, __fmaf_rn(w.x, s0, __fmul_rn(w.y, s1))));
+    return __float2half_rn(y / (1.0f + expf(-y)));
+}
+__device__ __forceinline__ float dn_decay(float a, float dtb, float An) {
+    const float xa = a + dtb;
+    const float sp = xa > 20.0f ? xa : logf(1.0f + expf(xa));
+    return An * sp;
+}
+__device__ __forceinline__ float dn_beta(float b) { return 1.0f / (1.0f + expf(-b)); }
+
 // binds: 0 = proj fp16 [nb][proj_stride], 1 = conv weights fp32 [C][4], 2 = conv state pool fp32
 // [slot][nlayers][3][C], 3 = A_neg fp32 [HV], 4 = dt_bias fp32 [HV], 5 = cv out fp16 [nb][C],
 // 6 = la fp32 [nb][HV], 7 = beta fp32 [nb][HV], 8 = slot ids int32 [nb], 9 = dn_epi_args.
@@ -43,21 +56,18 @@ __global__ void __launch_bounds__(256) dn_epi_k(const __half *proj, const float 
         const float4 w = *(const float4 *)(cw + 4 * (size_t)g);
         if (early) pdl_wait();
         const float s3 = __half2float(pr[g]);
-        const float y = w.x * s0 + w.y * s1 + w.z * s2 + w.w * s3;
-        cv[(size_t)t * C + g] = __float2half_rn(y / (1.0f + expf(-y)));
+        cv[(size_t)t * C + g] = dn_conv(w, s0, s1, s2, s3);
         st[g] = s1;
         st[C + g] = s2;
         st[2 * C + g] = s3;
     } else if (g < C + HV) {
         if (early) pdl_wait();
         const uint32_t j = g - C;
-        const float xa = __half2float(pr[C + HV * 128 + j]) + dtb[j];
-        const float sp = xa > 20.0f ? xa : logf(1.0f + expf(xa));
-        la[t * HV + j] = An[j] * sp;
+        la[t * HV + j] = dn_decay(__half2float(pr[C + HV * 128 + j]), dtb[j], An[j]);
     } else if (g < C + 2 * HV) {
         if (early) pdl_wait();
         const uint32_t j = g - C - HV;
-        be[t * HV + j] = 1.0f / (1.0f + expf(-__half2float(pr[C + HV * 128 + HV + j])));
+        be[t * HV + j] = dn_beta(__half2float(pr[C + HV * 128 + HV + j]));
     }
 }
 
@@ -82,28 +92,77 @@ QW_FAMILY(dn_epi, launch_dn_epi, 256)
 // sequence position nb - 1 - r of the piece.  A token's three predecessors are rows of the same projection (the state holds
 // exactly those fp16 values as fp32) or, for the first three tokens, the slot's conv state, which this kernel only reads:
 // gdn_seq, the next launch, writes the piece's last three inputs into it.
-// binds as dn_epi (2 is not written).  grid (ceil((C + 2 HV)/256), nb) x 256
-__global__ void __launch_bounds__(256) dn_epi_seq_k(const __half *proj, const float *cw, const float *pool, const float *An, const float *dtb, __half *cv,
+// A thread takes V channels of RUN consecutive tokens.  More than 64 tokens: eight channels as 16 bytes of two tokens, whose inputs slide through the window
+// (419 tokens on a B200: 21.9 -> 15.9 us); fewer want every channel of a token on a thread of its own (45 tokens: 5.9, the other form 6.7).  The last block of a row
+// of blocks does decay and beta.
+// binds as dn_epi (2 is not written).  grid (ceil(C / (128 V)) + 1, ceil(nb / RUN)) x 128
+template <int V>
+__device__ __forceinline__ void load_halves(const __half *p, float (&f)[V]) {
+    if constexpr (V == 8) {
+        const uint4 v = *(const uint4 *)p;
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float2 x = __half22float2(*(const __half2 *)&w[i]);
+            f[2 * i] = x.x;
+            f[2 * i + 1] = x.y;
+        }
+    } else f[0] = __half2float(p[0]);
+}
+template <int V, uint32_t RUN>
+__global__ void __launch_bounds__(128) dn_epi_seq_k(const __half *proj, const float *cw, const float *pool, const float *An, const float *dtb, __half *cv,
                                                     float *la, float *be, const int32_t *sids, dn_epi_args a, uint32_t C, uint32_t HV) {
-    pdl_sync();
-    const uint32_t g = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
-    const int tau = (int)(a.nb - 1 - t);  // position in the piece
-    const __half *pr = proj + (size_t)t * a.proj_stride;
-    if (g < C) {
-        const float *st = pool + ((size_t)sids[0] * a.nlayers + a.layer) * 3 * C + g;
-        auto at = [&](int k) { return k >= 0 ? __half2float(pr[(size_t)(tau - k) * a.proj_stride + g]) : st[(size_t)(3 + k) * C]; };
-        const float s0 = at(tau - 3), s1 = at(tau - 2), s2 = at(tau - 1), s3 = __half2float(pr[g]);
-        const float4 w = *(const float4 *)(cw + 4 * (size_t)g);
-        const float y = w.x * s0 + w.y * s1 + w.z * s2 + w.w * s3;
-        cv[(size_t)t * C + g] = __float2half_rn(y / (1.0f + expf(-y)));
-    } else if (g < C + HV) {
-        const uint32_t j = g - C;
-        const float xa = __half2float(pr[C + HV * 128 + j]) + dtb[j];
-        const float sp = xa > 20.0f ? xa : logf(1.0f + expf(xa));
-        la[t * HV + j] = An[j] * sp;
-    } else if (g < C + 2 * HV) {
-        const uint32_t j = g - C - HV;
-        be[t * HV + j] = 1.0f / (1.0f + expf(-__half2float(pr[C + HV * 128 + HV + j])));
+    pdl_launch();
+    const uint32_t tau0 = blockIdx.y * RUN, tau1 = tau0 + RUN < a.nb ? tau0 + RUN : a.nb;  // positions in the piece: row nb - 1 - tau
+    if (blockIdx.x == gridDim.x - 1) {
+        pdl_wait();
+        for (uint32_t i = threadIdx.x; i < (tau1 - tau0) * 2 * HV; i += 128) {
+            const uint32_t t = a.nb - 1 - (tau0 + i / (2 * HV)), j = i % (2 * HV);
+            const float v = __half2float(proj[(size_t)t * a.proj_stride + C + HV * 128 + j]);
+            if (j < HV) la[t * HV + j] = dn_decay(v, dtb[j], An[j]);
+            else be[t * HV + j - HV] = dn_beta(v);
+        }
+        return;
+    }
+    const uint32_t g = (blockIdx.x * 128 + threadIdx.x) * V;
+    float4 w[V];
+    if (g < C)
+#pragma unroll
+        for (int i = 0; i < V; i++) w[i] = *(const float4 *)(cw + 4 * (size_t)(g + i));
+    pdl_wait();
+    if (g >= C) return;
+    const float *st = pool + ((size_t)sids[0] * a.nlayers + a.layer) * 3 * C + g;
+    const __half *last = proj + (size_t)(a.nb - 1) * a.proj_stride + g;  // position 0; position tau is tau rows before it
+    float s[3][V];  // the three inputs before the run
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int tau = (int)tau0 - 3 + k;
+        if (tau >= 0) load_halves<V>(last - (size_t)tau * a.proj_stride, s[k]);
+        else
+#pragma unroll
+            for (int i = 0; i < V; i++) s[k][i] = st[(size_t)(3 + tau) * C + i];
+    }
+#pragma unroll
+    for (uint32_t n = 0; n < RUN; n++) {
+        const uint32_t tau = tau0 + n;
+        if (tau >= tau1) break;
+        float x[V];
+        load_halves<V>(last - (size_t)tau * a.proj_stride, x);
+        __half o[V];
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+            o[i] = dn_conv(w[i], s[0][i], s[1][i], s[2][i], x[i]);
+            s[0][i] = s[1][i];
+            s[1][i] = s[2][i];
+            s[2][i] = x[i];
+        }
+        __half *out = cv + (size_t)(a.nb - 1 - tau) * C + g;
+        if constexpr (V == 8) {
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) u[i] = (uint32_t)__half_as_ushort(o[2 * i]) | (uint32_t)__half_as_ushort(o[2 * i + 1]) << 16;
+            *(uint4 *)out = make_uint4(u[0], u[1], u[2], u[3]);
+        } else out[0] = o[0];
     }
 }
 
@@ -116,8 +175,10 @@ static cudaError_t launch_dn_epi_seq(const QwLaunch &L) {
     for (int i = 0; i <= 8; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
     QW_CHECK_ARG(L.avail(0) >= ((size_t)(a.nb - 1) * a.proj_stride + C + HV * DV + 2 * HV) * 2 && L.avail(1) >= (size_t)C * 16 &&
                  L.avail(5) >= (size_t)a.nb * C * 2 && L.avail(6) >= (size_t)a.nb * HV * 4 && L.avail(7) >= (size_t)a.nb * HV * 4 && L.avail(8) >= 4);
-    qw_launch(dn_epi_seq_k, dim3((C + 2 * HV + 255) / 256, a.nb), 256, 0, L.stream, L.buf<__half>(0), L.buf<float>(1), L.buf<float>(2), L.buf<float>(3),
-              L.buf<float>(4), L.buf<__half>(5), L.buf<float>(6), L.buf<float>(7), L.buf<int32_t>(8), a, C, HV);
+    // (C is a multiple of 128)
+    const bool vec = a.nb > 64 && a.proj_stride % 8 == 0 && (((uintptr_t)L.buf<void>(0) | (uintptr_t)L.buf<void>(5)) & 15) == 0;
+    qw_launch(vec ? dn_epi_seq_k<8, 2> : dn_epi_seq_k<1, 1>, dim3((C + (vec ? 1023 : 127)) / (vec ? 1024 : 128) + 1, vec ? (a.nb + 1) / 2 : a.nb), 128, 0, L.stream, L.buf<__half>(0),
+              L.buf<float>(1), L.buf<float>(2), L.buf<float>(3), L.buf<float>(4), L.buf<__half>(5), L.buf<float>(6), L.buf<float>(7), L.buf<int32_t>(8), a, C, HV);
     return cudaGetLastError();
 }
 QW_FAMILY(dn_epi_seq, launch_dn_epi_seq, 256)
@@ -494,8 +555,38 @@ static cudaError_t launch_gdn_seq(const QwLaunch &L) {
 QW_FAMILY(gdn_seq, launch_gdn_seq, 256)
 
 // Gated RMSNorm of gdn_seq's output, in the expressions of gdn_fstep: y = o * rsqrt(mean o^2 + eps) * w * sigmoid(z), in place.
-// binds: 0 = o fp16 [nb][HV*DV] (becomes y), 4 = z fp16 (row stride z_stride), 5 = norm weight fp32 [DV], 8 = gdn_args.  grid (HV, nb) x 128
+// A warp takes a head of a token, four columns per lane 32 apart; its four sums of 32 squares are the four warps' of gdn_fstep.  (A block of four warps per head and token
+// met once in shared memory for 128 values: 419 tokens 15.9 -> 6.3 us on a B200.)
+// binds: 0 = o fp16 [nb][HV*DV] (becomes y), 4 = z fp16 (row stride z_stride), 5 = norm weight fp32 [DV], 8 = gdn_args.  grid ceil(HV nb / 4) x 128
 __global__ void __launch_bounds__(128) gdn_gate_k(__half *o, const __half *z, const float *nw, gdn_args a, uint32_t HV) {
+    constexpr int DV = 128;
+    pdl_launch();
+    const uint32_t lane = threadIdx.x & 31, n = blockIdx.x * 4 + (threadIdx.x >> 5);
+    float wv[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) wv[i] = nw[32 * i + lane];
+    pdl_wait();
+    if (n >= a.nb * HV) return;
+    const uint32_t t = n / HV, hv = n % HV;
+    __half *p = o + (size_t)n * DV + lane;
+    const __half *zp = z + (size_t)t * a.z_stride + hv * DV + lane;
+    float x[4], zz[4], ss[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        zz[i] = __half2float(zp[32 * i]);
+        x[i] = __half2float(p[32 * i]);
+        ss[i] = x[i] * x[i];
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1)
+#pragma unroll
+        for (int i = 0; i < 4; i++) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], off);
+    const float r = rsqrtf((((ss[0] + ss[1]) + ss[2]) + ss[3]) / DV + GDN_EPS);
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[32 * i] = __float2half_rn(x[i] * r * wv[i] * (1.0f / (1.0f + expf(-zz[i]))));
+}
+// Up to 64 rows: a block of four warps per head and token (prompts of 45 tokens, 12 layers: 2.42 ms, with the other form 2.47)
+__global__ void __launch_bounds__(128) gdn_gate_few_k(__half *o, const __half *z, const float *nw, gdn_args a, uint32_t HV) {
     constexpr int DV = 128;
     __shared__ float red[4];
     pdl_sync();
@@ -515,7 +606,8 @@ static cudaError_t launch_gdn_gate(const QwLaunch &L) {
     QW_CHECK_ARG(DV == 128 && L.has_bytes(8, 16) && a.nb >= 1 && a.nb <= GDN_SEQ_MAX && a.z_stride >= HV * DV);
     QW_CHECK_ARG(L.buf<void>(0) && L.buf<void>(4) && L.buf<void>(5) && L.avail(0) >= (size_t)a.nb * HV * DV * 2 &&
                  L.avail(4) >= ((size_t)(a.nb - 1) * a.z_stride + HV * DV) * 2 && L.avail(5) >= DV * 4);
-    qw_launch(gdn_gate_k, dim3(HV, a.nb), 128, 0, L.stream, L.buf<__half>(0), L.buf<__half>(4), L.buf<float>(5), a, HV);
+    if (a.nb <= 64) qw_launch(gdn_gate_few_k, dim3(HV, a.nb), 128, 0, L.stream, L.buf<__half>(0), L.buf<__half>(4), L.buf<float>(5), a, HV);
+    else qw_launch(gdn_gate_k, (a.nb * HV + 3) / 4, 128, 0, L.stream, L.buf<__half>(0), L.buf<__half>(4), L.buf<float>(5), a, HV);
     return cudaGetLastError();
 }
 QW_FAMILY(gdn_gate, launch_gdn_gate, 128)
