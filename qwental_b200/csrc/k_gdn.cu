@@ -341,27 +341,6 @@ QW_FAMILY(gdn_fstep, launch_gdn_fstep, 512)
 // v, then {decay, decay, beta}.  Sums of 16 row groups: a column's 16 floats, 20 apart.
 constexpr uint32_t SEQ_Q = 160, SEQ_V = 320, SEQ_GB = 352, SEQ_TOK = 356, SEQ_COL = 20, SEQ_OUT = 32 * SEQ_COL;
 constexpr size_t SEQ_SMEM = (2 * GDN_SEQ_CHUNK * (SEQ_TOK + SEQ_OUT) + 2 * SEQ_OUT) * 4;  // tokens, sums of S^T q, sums of S^T k of two tokens
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 halves_of(f32x2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 template <bool TILED>
 __global__ void __launch_bounds__(256, 1) gdn_seq_k(const __half *cv, const float *la, const float *beta, float *pool, const __half *proj, float *conv,
                                                  __half *oo, const int32_t *sids, gdn_args a, uint32_t HK, uint32_t HV) {
