@@ -54,7 +54,7 @@ int qw_engine_par_pick(qw_engine *e, const int32_t *prompt, int np, unsigned lon
  * pages, GDN state and conv state are seeded synthetic values (K, V ~ N(0,1); S ~ N(0, 0.01)).  0, or -1 (the slot is then free). */
 int qw_engine_par_seed(qw_engine *e, int sid, int ctx_len, unsigned long long seed);
 /* src/engine.h:81.  Processes a prompt into slot sid (released first if it was in use) and returns the logits of its last
- * position ([vocab], valid until the next step that succeeds), NULL on failure (the slot is then free).  The prompt runs in pieces of up to 512 tokens, each one
+ * position ([vocab], valid until the next step that succeeds), NULL on failure (the slot is then free).  The prompt runs in pieces of up to 1024 tokens, each one
  * pass over the weights in the arithmetic of the decode step: the result equals stepping every token.  No prefix cache (*cached = 0). */
 const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32_t *prompt, int np, int *cached);
 /* src/engine.h:91.  One decode step for B slots (sids distinct, 1 <= B <= QW_PAR_MAX): returns [B][vocab] fp32

@@ -1239,9 +1239,8 @@ extern "C" int qw_engine_par_step_sample(qw_engine *e, const int *sids, const in
 // Prompt processing for one slot (src/engine.h:81), from an empty slot -- recurrent and conv state zero, no KV.  The prompt runs in
 // pieces of up to piece_rows tokens, each one pass over the weights, submitted back to back; a token's arithmetic is that of the decode
 // step, so "prefill then step" equals stepping every token, bit for bit.  (There is no prefix cache: *cached = 0.)
-// Measured on a B200 for pieces of up to 1, 64, 256 and 512 tokens: 48 layers, 419 tokens 1206, 81.2, 50.0 and 43.3 ms; 12 layers, 1700 tokens
-// 1362, 80.0, 46.7 and 41.9 ms.  64 tokens choose about 370 of 512 experts, 256 nearly all; from there on fuller passes of eight
-// tokens per expert are what a wider piece still gains.
+// Wider pieces read and decode fewer weights per token: 64 tokens choose about 370 of 512 experts, 256 nearly all; from there on it is fuller items of an
+// expert.  On a B200, 12 layers, pieces of up to 512 and of up to 1024 tokens: 600 tokens 12.2 and 9.9 ms, 1024 17.1 and 15.2, 1700 30.4 and 26.0, 2500 42.4 and 38.7.
 extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32_t *prompt, int np, int *cached) {
     if (cached) *cached = 0;
     if (!e || sid < 0 || sid >= (int)e->slots.size() || !prompt || np < 1 || np >= e->c.max_ctx) return e ? (e->fail("par_prefill: bad arguments"), nullptr) : nullptr;
@@ -1280,6 +1279,7 @@ extern "C" const float *qw_engine_par_prefill(qw_engine *e, int sid, const int32
     int n = 0;
     for (int p0 = 0; p0 < np && ok; p0 += n) {
         n = std::min(e->moe_probe ? ROWS : e->piece_rows, np - p0);
+        if (n > PROWS / 2 && n <= PROWS / 2 + ROWS) n = PROWS / 2;  // a rest of up to 64 tokens goes by itself, on the kernels of a step
         int perm[PROWS], sids[PROWS], lo, hi;
         std::fill(sids, sids + n, sid);
         qw_ep_row_order(sids, n, e->slot_shard ? e->c.ep_size : 1, e->slot_shard ? e->c.ep_rank : 0, perm, &lo, &hi);  // one slot: all rows are this rank's, or none

@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
 // One layer on a B200, against items of eight columns in moe_ffn_k: 419 tokens 372 -> 328 us, 512 tokens 423 -> 358; prompts of 419 tokens, 48 layers, 36.8 ->
 // 35.2 ms, of 1700 tokens, 12 layers, 34.2 -> 32.6.  Bound by the decode still (all 513 experts are 857 MB, 131 us).  With 32 columns two stages are
 // left in shared memory and the copies' latency shows: 355 us.
-constexpr int WFFN_RECS = 16;
+constexpr int WFFN_RECS = 24;  // items a block's share can touch: 15 with 148 blocks, 1024 tokens and 15 choices each
 constexpr uint32_t WFFN_STG = 4, WFFN_COLS = MOE_FFN_COLS_WIDE, WFFN_CT = WFFN_COLS / 8;
 struct WffnCost {  // of a gate/up piece and of a down piece: a decode of the stage, and the MMAs and the epilogue of a column tile
     uint32_t dec, tile;

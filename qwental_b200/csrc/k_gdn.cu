@@ -17,7 +17,7 @@
 using namespace qw;
 
 #define GDN_EPS 1e-6f
-#define GDN_SEQ_MAX 512   // tokens of one launch of the sequence kernels
+#define GDN_SEQ_MAX 1024  // tokens of one launch of the sequence kernels
 #define GDN_SEQ_CHUNK 16  // tokens of one of gdn_seq's two staging buffers
 
 // proj row layout (fp16, stride PS): [q: HK*DK | k: HK*DK | v: HV*DV | z: HV*DV | a: HV | b: HV]

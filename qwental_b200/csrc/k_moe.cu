@@ -278,8 +278,8 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
     moe_group_body<NTH>(sid, ms, E, topk, a, mask, nullptr);
 }
 
-// ---- a piece of a prompt (up to 512 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
-// part is moe_route with SELECT defined 0.  (In moe_route's one last block 512 tokens would be 32 rounds of top-k.)
+// ---- a piece of a prompt (up to 1024 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
+// part is moe_route with SELECT defined 0.  (In moe_route's one last block 1024 tokens would be 64 rounds of top-k.)
 // moe_topk_wide binds: 0 = logits [nb][E+1], 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid ceil(nb/4) x 128
 __global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_sel_wide *ms, uint32_t E, uint32_t topk, uint32_t nb) {
     __shared__ uint64_t cand_s[4][32 + MOE_MAXK];
@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_
 }
 // moe_group_wide binds: 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid 1 x 512
 __global__ void __launch_bounds__(512) moe_group_wide_k(moe_sel_wide *ms, uint32_t E, uint32_t topk, sel_args a) {
-    __shared__ uint32_t mask[MOE_MAXB_WIDE / 32][512];  // (E <= 512)
+    extern __shared__ uint32_t group_smem[];
+    uint32_t (&mask)[MOE_MAXB_WIDE / 32][512] = *(uint32_t (*)[MOE_MAXB_WIDE / 32][512])group_smem;  // (E <= 512)
     pdl_launch();
 #pragma unroll
     for (int q = 0; q < MOE_MAXB_WIDE / 32; q++) mask[q][threadIdx.x] = 0;
@@ -314,7 +315,10 @@ static cudaError_t launch_moe_group_wide(const QwLaunch &L) {
     sel_args a = L.bytes<sel_args>(2);
     QW_CHECK_ARG(moe_wide_check(L, a, E, topk));
     if (a.e_hi > E) a.e_hi = E;
-    qw_launch(moe_group_wide_k, 1, 512, 0, L.stream, L.buf<moe_sel_wide>(1), E, topk, a);
+    const size_t smem = MOE_MAXB_WIDE / 32 * 512 * 4;
+    const cudaError_t e = cudaFuncSetAttribute(moe_group_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    qw_launch(moe_group_wide_k, 1, 512, smem, L.stream, L.buf<moe_sel_wide>(1), E, topk, a);
     return cudaGetLastError();
 }
 QW_FAMILY(moe_group_wide, launch_moe_group_wide, 512)
@@ -346,7 +350,7 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // Up to four tokens -- one per warp at most -- are read straight from L2: staging them costs a copy's latency and saves nothing.
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
 // 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.  With SELECT defined 0 only the
-// logits are computed, of up to 512 tokens (binds 4 and 5 are not used).
+// logits are computed, of up to 1024 tokens (binds 4 and 5 are not used).
 // With NORM defined 1 (D = 2048, up to four tokens) the launch begins with the residual add + RMSNorm before the router, in the order of
 // add_rmsnorm: 6 = h fp32 [nb][D], 7 = delta fp16 [nb][D], 8 = w fp32 [D], 9 = h out (another buffer: every block reads h), 2 = x out.
 // Every block normalises all tokens for itself -- 12 KB of L2 reads per token and block -- and the first one stores h and x; that is

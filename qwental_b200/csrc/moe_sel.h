@@ -8,7 +8,7 @@
 
 // Result of the selection, read by the gate/up, down and combine kernels (role of struct gg_sel,
 // kernels/moe_gg.metal:110-116).  Groups are in expert-id order; a group's entries are in token order.
-// MAXB = 64: a step.  MAXB = 512: a piece of a prompt; the fields up to w sit at the same offsets in both.
+// MAXB = 64: a step.  MAXB = 1024: a piece of a prompt; the fields up to w sit at the same offsets in both.
 template <int MAXB>
 struct moe_sel_t {
     uint32_t U;                               // groups (distinct experts in [e_lo, e_hi) that were chosen)
@@ -22,7 +22,7 @@ struct moe_sel_t {
     uint32_t pre[MOE_MAXE + 2];               // passes of 8 entries in the groups before u (pre[U] = all routed passes)
 };
 typedef moe_sel_t<MOE_MAXB> moe_sel;
-#define MOE_MAXB_WIDE 512
+#define MOE_MAXB_WIDE 1024
 struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
     uint16_t sid[MOE_MAXB_WIDE][MOE_MAXK];    // chosen experts of every token: from the top-k to the grouping
     uint32_t prw[MOE_MAXE + 2];               // items of the expert FFN (MOE_FFN_COLS_WIDE entries each) in the groups before u

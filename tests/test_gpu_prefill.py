@@ -163,6 +163,26 @@ def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
         e.close()
 
 
+def test_pieces_of_up_to_1024_tokens(gpu):
+    """One piece of 577 to 1024 tokens, and what is left after 1024: one token, one of the rests that go by themselves, more."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(experts=512, topk=10, layers=4, max_slots=2))
+    try:
+        lengths = {578, 1023, 1024, 1025, 1100, 1560}
+        text = np.random.default_rng(15).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
+
+
 @pytest.mark.parametrize("experts,topk", [(32, 15), (512, 1), (64, 2)])
 def test_expert_items_of_a_piece(gpu, experts, topk):
     """The expert FFN of a piece takes items of up to 16 columns: experts with hundreds of tokens (full items, a remainder of one column and of one
