@@ -35,6 +35,7 @@ namespace {
 
 constexpr int PAGE = 256;
 constexpr int ROWS = QW_PAR_MAX;      // rows of the control block of a step
+constexpr int PART_WIDE = 2048;       // (row, page) partials of the attention over a prompt's piece that have room at once, at least: 34 MB
 constexpr int PROWS = MOE_MAXB_WIDE;  // ... and of a piece of a prompt: its tokens
 std::string g_open_error;
 
@@ -102,7 +103,8 @@ struct qw_engine {
     int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
     qw_buf ctl_p{}, ffn_scr_w{};
     qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
-              *k_group_w = nullptr, *k_ffn_w = nullptr, *k_qmv_in_w = nullptr, *k_qmv_oa_w = nullptr, *k_qmv_og_w = nullptr;
+              *k_group_w = nullptr, *k_ffn_w = nullptr, *k_qmv_in_w = nullptr, *k_qmv_oa_w = nullptr, *k_qmv_og_w = nullptr, *k_prep_w = nullptr,
+              *k_attn_w = nullptr, *k_merge_w = nullptr;
     qw_buf mlog{}, msel{}, Hhi{}, Hlo{}, Pg{}, rcnt{};
     size_t sel_bytes = 0;
     // kernels
@@ -399,7 +401,11 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
         mw.push_back({"WIDE", 1});
         mw.push_back({"IQ3X", e->ffn_iq3x ? 1 : 0});
         const std::vector<std::pair<const char *, long>> cw = {{"CMB", 1}, {"TOPK", e->TOPK}, {"ROWS", PROWS}, {"WIDE", 1}};
-        ok = compile(e, "kb_embed", "kb_embed_wide", {{"ROWS", PROWS}}, &e->k_embed_w) &&
+        auto aw = ad;
+        aw.push_back({"ROWS", PROWS});
+        ok = compile(e, "qsa_prep", "qsa_prep_wide", aw, &e->k_prep_w) && compile(e, "qsa_attn_piece", "qsa_attn_piece", aw, &e->k_attn_w) &&
+             compile(e, "qsa_merge", "qsa_merge_wide", aw, &e->k_merge_w) &&
+             compile(e, "kb_embed", "kb_embed_wide", {{"ROWS", PROWS}}, &e->k_embed_w) &&
              compile(e, "add_rmsnorm", "rmsnorm_wide", {{"ADD", 0}, {"ROWS", PROWS}}, &e->k_norm0_w) &&
              compile(e, "add_rmsnorm", "add_rmsnorm_wide", {{"ADD", 1}, {"ROWS", PROWS}}, &e->k_norm_w) &&
              compile(e, "add_rmsnorm", "cmb_add_rmsnorm_wide", cw, &e->k_norm_cmb_w) &&
@@ -431,7 +437,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->shu, (size_t)e->L * gu_bytes) && new_buf(e, &e->shd, (size_t)e->L * gu_bytes) &&
          new_buf(e, &e->kvpool, (size_t)kvp * page_bytes) && new_buf(e, &e->ptab, (size_t)c.max_slots * e->max_pages * 4) &&
          new_buf(e, &e->sstate, (size_t)c.max_slots * ng * c.hv * 128 * 128 * 4) && new_buf(e, &e->cstate, (size_t)c.max_slots * ng * 3 * e->C * 4) &&
-         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->part, B * (size_t)e->max_pages * c.qh * (c.hd + 2) * 4) &&
+         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->part, std::max(B * (size_t)e->max_pages, e->k_attn_w ? (size_t)PART_WIDE : 0) * c.qh * (c.hd + 2) * 4) &&
          new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids_h, 2 * B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
          new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO);
     // The rest of the scratch memory in one allocation.  With wide pieces it is some 100 MB more; where they are not to be had, prompts run in
@@ -740,29 +746,31 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
             qw_batch_dispatch(b, 1, 1, 1, 32, 1, 1);
         } else if (w.attn) {
             enc_qmv(b, e->k_qmv_in_a, e->k_qmv_in_w, &e->dense, w.w_in, e->qkv_rows, D, &e->x, &e->proj, nbl, e->qkv_rows, xo);
-            // the attention kernels take up to 64 rows: one group of rows for a step, several for a wide piece -- all of its K and V first
-            auto group = [&](uint32_t r0) {
-                return qsa_args{std::min<uint32_t>(ROWS, nbl - r0), (uint32_t)w.idx, (uint32_t)e->n_attn, e->qkv_rows, (uint32_t)e->max_pages, max_chunks, 0, 0};
+            // A step's rows, or a piece's up to 64, go as one; a wide piece's rows all together into the cache, then through the core as many at a time as
+            // have room for their partials.
+            auto group = [&](uint32_t r0, uint32_t rows) {
+                return qsa_args{std::min<uint32_t>(rows, nbl - r0), (uint32_t)w.idx, (uint32_t)e->n_attn, e->qkv_rows, (uint32_t)e->max_pages, max_chunks, 0, 0};
             };
             const size_t QR = (size_t)e->QH * e->HD * 2;  // bytes of a row of q
-            for (uint32_t r0 = 0; r0 < nbl; r0 += ROWS) {
-                const qsa_args qa = group(r0);
-                qw_batch_kernel(b, e->k_prep);
-                qw_batch_buf(b, 0, &e->proj, (size_t)r0 * e->qkv_rows * 2);
+            {
+                const qsa_args qa = group(0, nbl);
+                qw_batch_kernel(b, wide ? e->k_prep_w : e->k_prep);
+                qw_batch_buf(b, 0, &e->proj, 0);
                 qw_batch_buf(b, 1, &e->small, (w.small + 2 * D) * 4);
                 qw_batch_buf(b, 2, &e->small, (w.small + 2 * D + 256) * 4);
-                qw_batch_buf(b, 3, &e->qb, r0 * QR);
+                qw_batch_buf(b, 3, &e->qb, 0);
                 qw_batch_buf(b, 4, &e->kvpool, 0);
                 qw_batch_buf(b, 5, &e->ptab, 0);
-                qw_batch_buf(b, 6, ctl, (2 * CR + r0) * 4 + co);
-                qw_batch_buf(b, 7, ctl, (CR + r0) * 4 + co);
+                qw_batch_buf(b, 6, ctl, 2 * CR * 4 + co);
+                qw_batch_buf(b, 7, ctl, CR * 4 + co);
                 qw_batch_bytes(b, 8, &qa, sizeof qa);
                 qw_batch_dispatch(b, e->QH + e->KVH, qa.nb, 1, 256, 1, 1);
             }
             if (state_only && !row0_goes_on()) return;
-            for (uint32_t r0 = 0; r0 < nbl; r0 += ROWS) {
-                const qsa_args qa = group(r0);
-                qw_batch_kernel(b, e->k_attn);
+            const uint32_t room = (uint32_t)(e->part.size / ((size_t)max_chunks * e->QH * (e->HD + 2) * 4)), rows = wide ? std::max<uint32_t>(ROWS, room / 16 * 16) : ROWS;
+            for (uint32_t r0 = 0; r0 < nbl; r0 += rows) {
+                const qsa_args qa = group(r0, rows);
+                qw_batch_kernel(b, wide ? e->k_attn_w : e->k_attn);
                 qw_batch_buf(b, 0, &e->qb, r0 * QR);
                 qw_batch_buf(b, 1, &e->kvpool, 0);
                 qw_batch_buf(b, 2, &e->ptab, 0);
@@ -771,7 +779,7 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
                 qw_batch_buf(b, 5, &e->part, 0);
                 qw_batch_bytes(b, 6, &qa, sizeof qa);
                 qw_batch_dispatch(b, max_chunks, e->KVH, qa.nb, 128, 1, 1);
-                qw_batch_kernel(b, e->k_merge);
+                qw_batch_kernel(b, wide ? e->k_merge_w : e->k_merge);
                 qw_batch_buf(b, 0, &e->part, 0);
                 qw_batch_buf(b, 1, &e->proj, (size_t)r0 * e->qkv_rows * 2);
                 qw_batch_buf(b, 2, &e->ya, (size_t)r0 * e->KA * 2);

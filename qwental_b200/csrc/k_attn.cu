@@ -91,7 +91,7 @@ static cudaError_t launch_qsa_prep(const QwLaunch &L) {
     uint32_t QH, KVH, HD;
     QW_CHECK_ARG(qsa_dims(L, QH, KVH, HD));
     qsa_args a = L.bytes<qsa_args>(8);
-    QW_CHECK_ARG(L.has_bytes(8, 24) && a.nb >= 1 && a.nb <= 64 && a.layer < a.nlayers && a.qkv_stride >= QH * 2 * HD + 2 * KVH * HD);
+    QW_CHECK_ARG(L.has_bytes(8, 24) && a.nb >= 1 && a.nb <= (uint32_t)L.def("ROWS", 64) && a.layer < a.nlayers && a.qkv_stride >= QH * 2 * HD + 2 * KVH * HD);
     for (int i = 0; i <= 7; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
     QW_CHECK_ARG(L.avail(0) >= ((size_t)(a.nb - 1) * a.qkv_stride + QH * 2 * HD + 2 * KVH * HD) * 2 && L.avail(3) >= (size_t)a.nb * QH * HD * 2 &&
                  L.avail(6) >= (size_t)a.nb * 4 && L.avail(7) >= (size_t)a.nb * 4 && L.tx == 256);
@@ -472,6 +472,211 @@ __global__ void __launch_bounds__(128) qsa_attn_mma_k(const __grid_constant__ CU
     if (!ok && lane == 0) set_status(status, ST_MBAR_TIMEOUT | 4);
 }
 
+// ---- The rows of a prompt's piece: up to a thousand queries of ONE slot.  Going by 64 rows, qsa_attn loads every page once per row and kv head -- 256 KB each,
+// 20 us per launch -- although neighbouring rows read the same tiles.  Here a block is 16 rows of one (page, kv head): its tiles come once for all of them
+// through a ring of four, and a warp runs two rows, so a fragment of K feeds two products and, below the rows' ends, a fragment of V too.
+// A row's operations are those of qsa_attn_mma_k in the same order.  With the cache writes and the merges of all rows in one launch each, prompts of 12 layers on
+// a B200: 419 tokens 7.58 -> 7.31 ms, 1024 15.2 -> 14.6, 1700 26.1 -> 25.0, 3000 45.3 -> 43.6.
+// binds and partials as qsa_attn, sids[0] for all rows; ROWS = the most rows.  grid ceil(nb / 16) * max_chunks * KVH x 256
+constexpr int AP_STG = 4, AP_WARPS = 8, AP_ROWS = 16;
+constexpr int AP_SMEM = 1024 + AP_STG * AT_TILE_BYTES + AT_ZERO_BYTES + 2 * AP_STG * 8;
+__global__ void __launch_bounds__(AP_WARPS * 32, 1) qsa_attn_piece_k(const __grid_constant__ CUtensorMap tm, const __half *q, const int32_t *pt, const int32_t *posv,
+                                                                     const int32_t *sids, float *part, qsa_args a, uint32_t QH, uint32_t KVH, unsigned *status) {
+    constexpr uint32_t HD = 256;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    uint8_t *zrow = smem + AP_STG * AT_TILE_BYTES;
+    uint64_t *full = (uint64_t *)(zrow + AT_ZERO_BYTES), *empty = full + AP_STG;
+    const uint32_t base = smem_u32(smem), zeros = smem_u32(zrow);
+    if (warp < 4) ((uint32_t *)zrow)[warp * 512 + lane] = 0;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < AP_STG; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], AP_WARPS);
+        }
+        mbar_init_fence();
+    }
+    pdl_sync();
+    const uint32_t rb = blockIdx.x / (a.max_chunks * KVH), rem = blockIdx.x % (a.max_chunks * KVH), ch = rem / KVH, kvh = rem % KVH;
+    // tokens of the page that a row attends to; the block walks as far as its longest row
+    auto tokens_of = [&](uint32_t r) {
+        const int n = r < a.nb ? posv[r] + 1 - (int)(ch * QSA_PAGE) : 0;
+        return (uint32_t)(n < 0 ? 0 : n > QSA_PAGE ? QSA_PAGE : n);
+    };
+    const uint32_t r0 = rb * AP_ROWS + warp * 2;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, tokens_of(lane < AP_ROWS ? rb * AP_ROWS + lane : a.nb)), steps = (most + 15) / 16;
+    const uint32_t n[2] = {tokens_of(r0), tokens_of(r0 + 1)};
+    __syncthreads();
+    if (steps == 0) return;
+    const uint32_t page = (uint32_t)pt[(size_t)sids[0] * a.max_pages + ch];
+    const int rowK = (int)(((page * a.nlayers + a.layer) * 2) * KVH * QSA_PAGE + kvh * QSA_PAGE), rowV = rowK + (int)(KVH * QSA_PAGE);
+    auto put = [&](uint32_t j) {  // tile pair j; by one thread
+        const uint32_t st = j % AP_STG;
+        if (j >= AP_STG && !mbar_wait(&empty[st], (j / AP_STG - 1) & 1)) return false;
+        fence_proxy_async();  // the warps' reads of the stage before the async-proxy writes
+        mbar_expect_tx(&full[st], AT_TILE_BYTES);
+#pragma unroll
+        for (int db = 0; db < 4; db++) {
+            tma_load_2d(base + st * AT_TILE_BYTES + db * 2048, &tm, db * 64, rowK + (int)j * 16, &full[st]);
+            tma_load_2d(base + st * AT_TILE_BYTES + 8192 + db * 2048, &tm, db * 64, rowV + (int)j * 16, &full[st]);
+        }
+        return true;
+    };
+    if (threadIdx.x == 0)
+        for (uint32_t j = 0; j < AP_STG - 1 && j < steps; j++) put(j);
+    // Q of both rows as B fragments (k = dim, n = head g), pre-scaled by HD^-1/2 = 1/16 (exact in fp16)
+    uint32_t qf[2][16][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const __half *qp = q + ((size_t)(r0 + i < a.nb ? r0 + i : a.nb - 1) * QH + kvh * 8 + g) * HD + 2 * t;
+        const __half2 sc = __floats2half2_rn(0.0625f, 0.0625f);
+#pragma unroll
+        for (int ks = 0; ks < 16; ks++) {
+            const __half2 v0 = __hmul2(*(const __half2 *)(qp + 16 * ks), sc), v1 = __hmul2(*(const __half2 *)(qp + 16 * ks + 8), sc);
+            qf[i][ks][0] = *(const uint32_t *)&v0;
+            qf[i][ks][1] = *(const uint32_t *)&v1;
+        }
+    }
+    const uint32_t mi = lane >> 3, r8 = lane & 7, vrow = (mi >> 1) * 8 + r8;
+    const uint32_t kbase = base + ((mi & 1) * 8 + r8) * 128, vbase = base + 8192 + vrow * 128;
+    float o[2][16][4], m[2][2], l[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+#pragma unroll
+        for (int dt = 0; dt < 16; dt++) o[i][dt][0] = o[i][dt][1] = o[i][dt][2] = o[i][dt][3] = 0.f;
+        m[i][0] = m[i][1] = -INFINITY;
+        l[i][0] = l[i][1] = 0.f;
+    }
+    bool ok = true;
+#pragma unroll 1
+    for (uint32_t step = 0; step < steps; step++) {
+        if (warp == 0) {  // two steps ahead, into the stage that every warp has left by now or leaves soon
+            if (lane == 0 && step + AP_STG - 1 < steps) ok = put(step + AP_STG - 1);
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0);
+        }
+        const uint32_t st = step % AP_STG, so = st * AT_TILE_BYTES;
+        ok = ok && mbar_wait(&full[st], (step / AP_STG) & 1);
+        if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+        }
+        const bool on0 = step * 16 < n[0], on1 = step * 16 < n[1];  // (the same in all lanes)
+        if (on0 || on1) {
+            float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+            for (int ks = 0; ks < 16; ks++) {
+                uint32_t af[4];
+                ldsm_x4(af, kbase + so + (ks >> 2) * 2048 + ((((ks & 3) * 2 + (mi >> 1)) ^ r8) << 4));
+                mma_f16(s[0], af, qf[0][ks][0], qf[0][ks][1], s[0]);
+                mma_f16(s[1], af, qf[1][ks][0], qf[1][ks][1], s[1]);
+            }
+            uint32_t pb[2][4];  // probabilities as B operands: high parts, remainders
+            const uint32_t ta = step * 16 + g;
+            auto softmax = [&](int i) {
+                if (ta >= n[i]) s[i][0] = s[i][1] = -INFINITY;
+                if (ta + 8 >= n[i]) s[i][2] = s[i][3] = -INFINITY;
+                float x0 = fmaxf(s[i][0], s[i][2]), x1 = fmaxf(s[i][1], s[i][3]);
+#pragma unroll
+                for (int off = 4; off < 32; off <<= 1) {
+                    x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
+                    x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
+                }
+                const float n0 = fmaxf(m[i][0], x0), n1 = fmaxf(m[i][1], x1);
+                const float a0 = expf(m[i][0] - n0), a1 = expf(m[i][1] - n1);
+                const float p0 = expf(s[i][0] - n0), p1 = expf(s[i][1] - n1), p2 = expf(s[i][2] - n0), p3 = expf(s[i][3] - n1);
+                l[i][0] = l[i][0] * a0 + (p0 + p2);
+                l[i][1] = l[i][1] * a1 + (p1 + p3);
+                m[i][0] = n0;
+                m[i][1] = n1;
+#pragma unroll
+                for (int dt = 0; dt < 16; dt++) {
+                    o[i][dt][0] *= a0;
+                    o[i][dt][1] *= a1;
+                    o[i][dt][2] *= a0;
+                    o[i][dt][3] *= a1;
+                }
+                const __half2 h01 = __floats2half2_rn(p0, p1), h23 = __floats2half2_rn(p2, p3);
+                const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
+                const __half2 e01 = __floats2half2_rn(p0 - f01.x, p1 - f01.y), e23 = __floats2half2_rn(p2 - f23.x, p3 - f23.y);
+                const int srcA = (2 * t) * 4 + (g >> 1), srcB = srcA + 4;
+                const uint32_t sel = (g & 1) ? 0x7632u : 0x5410u;
+                auto to_b = [&](const __half2 &h) {
+                    const uint32_t u = *(const uint32_t *)&h;
+                    return __byte_perm(__shfl_sync(0xffffffffu, u, srcA), __shfl_sync(0xffffffffu, u, srcB), sel);
+                };
+                pb[i][0] = to_b(h01);
+                pb[i][1] = to_b(h23);
+                pb[i][2] = to_b(e01);
+                pb[i][3] = to_b(e23);
+            };
+            auto value_of = [&](int i, int dq, const uint32_t (&af)[4][4]) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f16(o[i][4 * dq + j], af[j], pb[i][0], pb[i][1], o[i][4 * dq + j]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f16(o[i][4 * dq + j], af[j], pb[i][2], pb[i][3], o[i][4 * dq + j]);
+            };
+            auto v_frag = [&](uint32_t (&af)[4][4], uint32_t va, int dq) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) ldsm_x4_t(af[j], va + dq * 2048 + (((j * 2 + (mi & 1)) ^ r8) << 4));
+            };
+            if (step * 16 + 16 <= n[0] && step * 16 + 16 <= n[1]) {  // both rows see the whole tile
+                softmax(0);
+                softmax(1);
+#pragma unroll
+                for (int dq = 0; dq < 4; dq++) {
+                    uint32_t af[4][4];
+                    v_frag(af, vbase + so, dq);
+                    value_of(0, dq, af);
+                    value_of(1, dq, af);
+                }
+            } else {  // the tile in which a row ends: rows of V past it are read as zeros, whatever the page holds there
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    if (!(i ? on1 : on0)) continue;
+                    softmax(i);
+                    const uint32_t va = step * 16 + vrow < n[i] ? vbase + so : zeros;
+#pragma unroll
+                    for (int dq = 0; dq < 4; dq++) {
+                        uint32_t af[4][4];
+                        v_frag(af, va, dq);
+                        value_of(i, dq, af);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[st]);
+    }
+    if (!ok) {
+        if (lane == 0) set_status(status, ST_MBAR_TIMEOUT | 17);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        if (n[i] == 0) continue;
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+            l[i][0] += __shfl_xor_sync(0xffffffffu, l[i][0], off);
+            l[i][1] += __shfl_xor_sync(0xffffffffu, l[i][1], off);
+        }
+        float *po0 = part + (((size_t)(r0 + i) * a.max_chunks + ch) * QH + kvh * 8 + 2 * t) * (HD + 2), *po1 = po0 + (HD + 2);
+#pragma unroll
+        for (int dt = 0; dt < 16; dt++) {
+            po0[16 * dt + g] = o[i][dt][0];
+            po1[16 * dt + g] = o[i][dt][1];
+            po0[16 * dt + g + 8] = o[i][dt][2];
+            po1[16 * dt + g + 8] = o[i][dt][3];
+        }
+        if (g == 0) {
+            po0[HD] = m[i][0];
+            po0[HD + 1] = l[i][0];
+            po1[HD] = m[i][1];
+            po1[HD + 1] = l[i][1];
+        }
+    }
+}
+
 // The pool seen as [rows of one token of one kv head][256 halves]
 static bool attn_encode_map(CUtensorMap *tm, const void *pool, size_t bytes) {
     return tmap_2d(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, pool, 256, bytes / 512, 512, 64, 16, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
@@ -502,6 +707,25 @@ static AttnLaunch attn_launch(uint32_t most, uint32_t sms) {
     const uint32_t blocks = (most + 3) / 4, cap = sms * at_blocks_per_sm(1);
     return {qsa_attn_mma_k<1>, blocks < cap ? blocks : cap, at_smem(1)};
 }
+
+static cudaError_t launch_qsa_attn_piece(const QwLaunch &L) {
+    uint32_t QH, KVH, HD;
+    QW_CHECK_ARG(qsa_dims(L, QH, KVH, HD));
+    qsa_args a = L.bytes<qsa_args>(6);
+    QW_CHECK_ARG(L.has_bytes(6, 24) && a.nb >= 1 && a.nb <= (uint32_t)L.def("ROWS", 64) && a.layer < a.nlayers && a.max_chunks >= 1 && a.max_chunks <= a.max_pages);
+    for (int i = 0; i <= 5; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
+    QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * QH * HD * 2 && L.avail(3) >= (size_t)a.nb * 4 && L.avail(4) >= 4 &&
+                 L.avail(5) >= (size_t)a.nb * a.max_chunks * QH * (HD + 2) * 4);
+    QW_CHECK_ARG(((uintptr_t)L.buf<void>(1) & 15) == 0 && L.avail(1) >= 512 && L.avail(1) / 512 < 0x7fffffffull);
+    const CUtensorMap *tm = attn_tensor_map(L.buf<void>(1), L.avail(1) / 512 * 512);
+    QW_CHECK_ARG(tm != nullptr);
+    const cudaError_t e = cudaFuncSetAttribute(qsa_attn_piece_k, cudaFuncAttributeMaxDynamicSharedMemorySize, AP_SMEM);
+    if (e != cudaSuccess) return e;
+    qw_launch(qsa_attn_piece_k, (a.nb + AP_ROWS - 1) / AP_ROWS * a.max_chunks * KVH, AP_WARPS * 32, AP_SMEM, L.stream, *tm, L.buf<__half>(0), L.buf<int32_t>(2), L.buf<int32_t>(3),
+              L.buf<int32_t>(4), L.buf<float>(5), a, QH, KVH, L.status);
+    return cudaGetLastError();
+}
+QW_FAMILY(qsa_attn_piece, launch_qsa_attn_piece, 256)
 
 static cudaError_t launch_qsa_attn_mma(const QwLaunch &L) {
     uint32_t QH, KVH, HD;
@@ -584,14 +808,62 @@ __global__ void __launch_bounds__(512) qsa_merge_k(const float *part, const __ha
     }
 }
 
+// Many rows of few chunks (a prompt's piece, at most 16 pages): a warp per head and row, eight dims per lane.  The 16 groups of qsa_merge_k are then the chunks
+// themselves, added in order; absent ones add zero, as there.  grid ceil(QH nb / 8) x 256
+__global__ void __launch_bounds__(256) qsa_merge_rows_k(const float *part, const __half *qkv, __half *y, const int32_t *posv, qsa_args a, uint32_t QH) {
+    constexpr uint32_t HD = 256;
+    pdl_sync();
+    const uint32_t n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, t = n / QH, qh = n % QH;
+    if (t >= a.nb) return;
+    const uint32_t ntok = (uint32_t)posv[t] + 1, nch = min((ntok + QSA_PAGE - 1) / QSA_PAGE, a.max_chunks);
+    const float *base = part + ((size_t)t * a.max_chunks * QH + qh) * (HD + 2);
+    const size_t cstride = (size_t)QH * (HD + 2);
+    const float pm = lane < nch ? base[lane * cstride + HD] : 0.f, pl = lane < nch ? base[lane * cstride + HD + 1] : 0.f;
+    const float M = warp_max(pl > 0.f ? pm : -INFINITY);
+    const float w = pl > 0.f ? expf(pm - M) : 0.f;
+    float lt = 0.f, at[8];
+#pragma unroll
+    for (uint32_t c = 0; c < 16; c++) {
+        const float wc = __shfl_sync(0xffffffffu, w, c), lc = __shfl_sync(0xffffffffu, pl, c);
+        float x[8], lx = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = 0.f;
+        if (c < nch) {  // (the same in all lanes)
+            const float2 *pv = (const float2 *)(base + c * cstride) + 4 * lane;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float2 v = pv[i];
+                x[2 * i] = fmaf(v.x, wc, 0.f);
+                x[2 * i + 1] = fmaf(v.y, wc, 0.f);
+            }
+            lx = fmaf(lc, wc, 0.f);
+        }
+        lt = c ? lt + lx : lx;
+#pragma unroll
+        for (int i = 0; i < 8; i++) at[i] = c ? at[i] + x[i] : x[i];
+    }
+    const __half *gp = qkv + (size_t)t * a.qkv_stride + qh * 2 * HD + HD + 8 * lane;
+    __half *yp = y + ((size_t)t * QH + qh) * HD + 8 * lane;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const float g = __half2float(gp[i]);
+        const float o = __half2float(__float2half_rn(at[i] / lt));
+        yp[i] = __float2half_rn(o * (1.0f / (1.0f + expf(-g))));
+    }
+}
+
 static cudaError_t launch_qsa_merge(const QwLaunch &L) {
     uint32_t QH, KVH, HD;
     QW_CHECK_ARG(qsa_dims(L, QH, KVH, HD));
     qsa_args a = L.bytes<qsa_args>(4);
-    QW_CHECK_ARG(L.has_bytes(4, 24) && a.nb >= 1 && a.nb <= 64 && a.max_chunks >= 1 && a.max_chunks <= QSA_MAXCH);
+    QW_CHECK_ARG(L.has_bytes(4, 24) && a.nb >= 1 && a.nb <= (uint32_t)L.def("ROWS", 64) && a.max_chunks >= 1 && a.max_chunks <= QSA_MAXCH);
     for (int i = 0; i <= 3; i++) QW_CHECK_ARG(L.buf<void>(i) != nullptr);
     QW_CHECK_ARG(L.avail(0) >= (size_t)a.nb * a.max_chunks * QH * (HD + 2) * 4 && L.avail(2) >= (size_t)a.nb * QH * HD * 2 &&
                  L.avail(1) >= ((size_t)(a.nb - 1) * a.qkv_stride + QH * 2 * HD) * 2);
+    if (a.nb > 64 && a.max_chunks <= 16) {
+        qw_launch(qsa_merge_rows_k, (QH * a.nb + 7) / 8, 256, 0, L.stream, L.buf<float>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<int32_t>(3), a, QH);
+        return cudaGetLastError();
+    }
     qw_launch(qsa_merge_k, dim3(QH, a.nb), 512, 0, L.stream, L.buf<float>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<int32_t>(3), a, QH);
     return cudaGetLastError();
 }

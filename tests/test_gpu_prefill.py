@@ -163,6 +163,27 @@ def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
         e.close()
 
 
+def test_attention_over_the_rows_of_a_piece(gpu):
+    """The attention core takes 16 rows of a piece per (page, kv head): pieces around multiples of 16 rows, rows that end in every part of a tile, pages that some
+    rows of a block reach and others do not, pieces behind earlier ones, and (4300 tokens) more than 16 pages, which go through the general merge."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(layers=3, attn_every=2, max_slots=2, max_ctx=4608))
+    try:
+        lengths = {65, 79, 80, 81, 127, 255, 256, 257, 263, 271, 272, 300, 511, 590, 777, 1024, 1100, 1301, 2000, 4300}
+        text = np.random.default_rng(17).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
+
+
 def test_pieces_of_up_to_1024_tokens(gpu):
     """One piece of 577 to 1024 tokens, and what is left after 1024: one token, one of the rests that go by themselves, more."""
     from qwental_b200.engine import Engine, wide_cfg
