@@ -480,9 +480,10 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
 // reduction across warps.  MMA column g of a tile holds token (g / 2) + 4 (g % 2), so that the eight lanes of a 16-byte shared load fall into
 // eight different chunks of the swizzle.
 // TS = warps that share a row tile.  2: the tiles of a block are few (a projection has 3 to 6 per SM) and the warps are what hides
-// latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S for several groups of 64 tokens, where a block has many tiles): a unit is decoded once for all
+// latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S for three and more groups of 64 tokens, where a block has many tiles): a unit is decoded once for all
 // tokens, by fewer warps with more registers.  (12352 x 2048 IQ3_S, 419 tokens, TS 2 -> 1 on a B200: 121 -> 110 us; 2048 x 4096: 45 -> 42; prompts of 419
-// tokens, 48 layers, 37.5 -> 36.9 ms.)
+// tokens, 48 layers, 37.5 -> 36.9 ms.  Two groups are better off with 2: prompts of 65, 100 and 128 tokens, 12 layers, 3.37 -> 3.26, 3.69 -> 3.61 and
+// 4.11 -> 4.03 ms.)
 // Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
 // IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
 // 40 of its cycles per unit of 16 rows x 32 weights.
@@ -707,7 +708,7 @@ static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     // one block per SM, shared evenly by the groups of 64 tokens
     const uint32_t groups = (p.nb + 63) / 64, most = (uint32_t)sm_count / groups > 0 ? (uint32_t)sm_count / groups : 1, bpg = p.items < most ? p.items : most;
     const uint32_t per = (p.items + bpg - 1) / bpg;
-    if (GF == 8 ? per >= 16 : groups > 1) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
+    if (GF == 8 ? per >= 16 : groups > 2) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
     return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }
 
