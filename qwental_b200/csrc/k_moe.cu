@@ -525,12 +525,14 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
 }
 
 // Logits alone, of the many tokens of a prompt's piece.  moe_route_k reads every token in every block of four rows (1.7 MB x 129 at 419 tokens) and converts it
-// once per row; here a warp takes four rows x eight tokens, so a converted value serves eight (weights) or four (tokens) chains, two tokens to a packed
-// multiply-add, and a block is 16 rows x 32 tokens.  Rows and tokens come through L1, which its warps share.  A dot product is the same single-lane chain and the
-// same butterfly (over 32 values at once: every step halves them).  512 experts, 419 tokens on a B200: 61 -> 40 us.  grid (ceil((E + 1) / 16), ceil(nb / 32)) x 512
-__global__ void __launch_bounds__(512) moe_logits_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, uint32_t E, uint32_t nb) {
-    constexpr int D = 2048, CH = D / 8 / 32, R = 4, T = 8;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * 16 + (warp & 3) * R, t0 = blockIdx.y * 32 + (warp >> 2) * T;
+// once per row; here a warp takes four rows x four tokens, so a converted value serves four chains, two tokens to a packed multiply-add, and a block is
+// 16 rows x 8 tokens.  Rows and tokens come through L1, which its warps share.  A dot product is the same single-lane chain and the same butterfly (over 16
+// values at once: every step but the first halves them).  512 experts, 419 tokens on a B200: 61 -> 40 us with eight tokens per warp, 32 per block and every
+// chunk waited for; four tokens leave registers to fetch the next chunk ahead, and smaller blocks fill the last wave: prompts of 70, 164 and 419 tokens, 12
+// layers, 3.556 -> 3.531, 4.800 -> 4.757 and 7.237 -> 7.211 ms.  (Fetching ahead with eight tokens per warp: 7.298.)  grid (ceil((E + 1) / 16), ceil(nb / 8)) x 256
+__global__ void __launch_bounds__(256) moe_logits_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, uint32_t E, uint32_t nb) {
+    constexpr int D = 2048, CH = D / 8 / 32, R = 4, T = 4;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * 16 + (warp & 3) * R, t0 = blockIdx.y * 8 + (warp >> 2) * T;
     pdl_sync();
     if (r0 > E || t0 >= nb) return;  // (whole warps)
     const uint4 *wp[R], *xp[T];
@@ -543,13 +545,18 @@ __global__ void __launch_bounds__(512) moe_logits_k(const __half *Wr, const __ha
     for (int r = 0; r < R; r++)
 #pragma unroll
         for (int t = 0; t < T / 2; t++) acc[r][t] = 0;
+    uint4 w[R], v[T];
+    auto load = [&](uint4 (&ww)[R], uint4 (&vv)[T], int c) {
+#pragma unroll
+        for (int t = 0; t < T; t++) vv[t] = xp[t][32 * c];
+#pragma unroll
+        for (int r = 0; r < R; r++) ww[r] = __ldg(wp[r] + 32 * c);
+    };
+    load(w, v, 0);
 #pragma unroll 1
     for (int c = 0; c < CH; c++) {
-        uint4 w[R], v[T];
-#pragma unroll
-        for (int t = 0; t < T; t++) v[t] = xp[t][32 * c];
-#pragma unroll
-        for (int r = 0; r < R; r++) w[r] = __ldg(wp[r] + 32 * c);
+        uint4 wn[R], vn[T];
+        load(wn, vn, c + 1 < CH ? c + 1 : c);  // the next chunk is on its way while this one is multiplied (the last one again)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             auto two = [&](const uint4 &q) { return __half22float2(*(const __half2 *)((const uint32_t *)&q + j)); };
@@ -566,6 +573,10 @@ __global__ void __launch_bounds__(512) moe_logits_k(const __half *Wr, const __ha
                 for (int t = 0; t < T / 2; t++) acc[r][t] = fma2(m1, pair_of(f[2 * t].y, f[2 * t + 1].y), acc[r][t]);
             }
         }
+#pragma unroll
+        for (int r = 0; r < R; r++) w[r] = wn[r];
+#pragma unroll
+        for (int t = 0; t < T; t++) v[t] = vn[t];
     }
     float s[R * T];
 #pragma unroll
@@ -576,8 +587,11 @@ __global__ void __launch_bounds__(512) moe_logits_k(const __half *Wr, const __ha
             s[r * T + 2 * t] = h.x;
             s[r * T + 2 * t + 1] = h.y;
         }
+    // 16 values over 32 lanes: the first step adds the half-warps (both keep all values), every further one halves the values
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
+    for (int i = 0; i < R * T; i++) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], 16));
+#pragma unroll
+    for (int off = 8; off; off >>= 1) {
         const bool up = lane & off;
 #pragma unroll
         for (int i = 0; i < off; i++) {
@@ -585,7 +599,8 @@ __global__ void __launch_bounds__(512) moe_logits_k(const __half *Wr, const __ha
             s[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, off));
         }
     }
-    const uint32_t row = r0 + lane / T, tok = t0 + lane % T;  // lane l has value l
+    const uint32_t row = r0 + (lane & 15) / T, tok = t0 + lane % T;  // lanes l and l + 16 have value l
+    if (lane >= 16) return;
     if (row <= E && tok < nb) logits[(size_t)tok * (E + 1) + row] = s[0];
 }
 
@@ -619,7 +634,7 @@ static cudaError_t launch_moe_route(const QwLaunch &L) {
                  L.avail(3) >= (size_t)a.nb * (E + 1) * 4 && (!select || (L.avail(4) >= 4 && L.avail(5) >= sizeof(moe_sel))));
     if (a.e_hi > E) a.e_hi = E;
     if (!select && D == 2048 && a.nb > MOE_MAXB && !L.def("NORM", 0)) {
-        qw_launch(moe_logits_k, dim3((E + 1 + 15) / 16, (a.nb + 31) / 32), 512, 0, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), E, a.nb);
+        qw_launch(moe_logits_k, dim3((E + 1 + 15) / 16, (a.nb + 7) / 8), 256, 0, L.stream, L.buf<__half>(0), L.buf<__half>(1), L.buf<__half>(2), L.buf<float>(3), E, a.nb);
         return cudaGetLastError();
     }
     const unsigned grid = (E + 1 + 3) / 4;  // (the grid given by the host is ignored)
