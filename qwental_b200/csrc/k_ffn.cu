@@ -90,8 +90,7 @@ struct __align__(16) FfnItem {
 };
 // item number w -> (group, pass): routed groups first (pre[] = passes before each group, in shared memory), then the shared
 // expert's passes.  The group's entries and expert come from the selection record in global memory.
-template <class SEL>
-__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const SEL *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
+__device__ __forceinline__ FfnItem ffn_item(const uint32_t *pre, const moe_sel *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
     FfnItem it{};
     const uint32_t routed = pre[U];
     uint32_t cnt;
@@ -328,8 +327,7 @@ __device__ __forceinline__ void x_unit(uint32_t rec0, uint32_t rec1, int kh, int
 // TMA boxes and bulk copies through the same ring, but the consumers only read every staged byte once (16-byte loads) and
 // compute nothing -- the role of the reference's pure-read probes (bench/moe_bw.c:1-3, bench/qmv.c:357-382).
 // (17 warps put five on one scheduler, whose 16 K registers then allow 96 per thread)
-// WIDE: a piece of a prompt whose tokens are too few for moe_ffn_wide_k; its output rows are not counted in
-template <bool PROBE, int FMT, bool HALF = false, bool WIDE = false>
+template <bool PROBE, int FMT, bool HALF = false>
 __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(const __grid_constant__ CUtensorMap mG, const __grid_constant__ CUtensorMap mU,
                                                            const __grid_constant__ CUtensorMap mSG, const __grid_constant__ CUtensorMap mSU, const FfnP p) {
     using C = FfnCfg<FMT>;
@@ -366,15 +364,13 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     }
     if (FMT == 1 && tid < 16) x_scale_entry(smem + C::OFF_TAB, tid);
     pdl_wait();  // the selection record, the tokens and Pg belong to earlier kernels
-    typedef moe_sel_t<WIDE ? MOE_MAXB_WIDE : MOE_MAXB> sel_t;
-    constexpr uint32_t MAXITEMS = WIDE ? MOE_FFN_MAXITEMS_WIDE : MOE_FFN_MAXITEMS;
-    const sel_t *ms = (const sel_t *)p.ms;
+    const moe_sel *ms = (const moe_sel *)p.ms;
     // passes before every group: independent loads, so the table is in shared memory after one latency
     for (uint32_t i = tid; i < FFN_MAXG; i += FFN_THREADS) pre[i] = ms->pre[i];
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
     uint32_t items = pre[U] + (p.Sd ? (nb + 7) / 8 : 0);
-    if (items > MAXITEMS) {  // cannot happen with E <= 512 and 64 tokens; never index past the flags
+    if (items > MOE_FFN_MAXITEMS) {  // cannot happen with E <= 512 and 64 tokens; never index past the flags
         if (tid == 0) set_status(p.status, ST_BAD_ARG | 5);
         items = 0;
     }
@@ -703,7 +699,7 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
                     // this warp's 16 rows of the tile are stored for every column: count it in on the columns' output rows (lanes
                     // t = 0 .. 3 of row g = 0 know two columns each), so that the combine + norm of a token can start when its rows are complete
                     __syncwarp();
-                    if (!WIDE && g == 0) {
+                    if (g == 0) {
                         __threadfence();  // the warp's stores (cumulative over the warp barrier) before the counts
                         if (oo[0] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[0] / D, 1u);
                         if (oo[1] != 0xffffffffu) atomicAdd(p.sync + MOE_FFN_ROWCNT + oo[1] / D, 1u);
@@ -718,51 +714,57 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
     __syncthreads();
     if (tid == 0 && !PROBE) {
         __threadfence();
-        if (atomicAdd(p.sync + MAXITEMS, 1u) == gridDim.x - 1) {
+        if (atomicAdd(p.sync + MOE_FFN_MAXITEMS, 1u) == gridDim.x - 1) {
             for (uint32_t i = 0; i < items; i++) p.sync[i] = 0;
-            p.sync[MAXITEMS] = 0;
+            p.sync[MOE_FFN_MAXITEMS] = 0;
         }
     }
     if (p.ep.nranks > 1) ep_publish(p.ep);
 }
 
 // ---- A piece of a prompt.  Its tokens choose nearly every expert, eight tokens and more each, so the decode of a stage is shared by more columns: an
-// item is up to 16 or 24 columns (CT = 2 or 3 MMA column tiles of 8) of an expert, and a warp runs the decoded fragments of a sub-block against as many tiles as
+// item is up to WFFN_COLS columns (MMA column tiles of 8) of an expert, and a warp runs the decoded fragments of a sub-block against as many tiles as
 // the item has.  A column's MMAs and sums are those of moe_ffn_k, in the same order.
-// One block per SM (16 token rows are 65 KB beside four stages, 24 are 98 KB beside three: the copies have to stay ahead of the decode) of 16 + 1 warps with up to 96 registers: the tiles'
-// independent MMA chains take the place of the second block.  Shares of the work are cut by cost, not by piece: an item weighs a decode and its tiles
-// (WffnCost), because experts with one tile and the shared expert's full items lie apart in the list.  The two K halves of a row group exchange
-// tiles: even ones are finished by the low half, odd ones by the high half.  The combine + norm that follows waits for the whole launch, so no
-// output row is counted in.
-// One layer on a B200, against items of eight columns in moe_ffn_k: 419 tokens 372 -> 328 us, 512 tokens 423 -> 358; prompts of 419 tokens, 48 layers, 36.8 ->
-// 35.2 ms, of 1700 tokens, 12 layers, 34.2 -> 32.6.  Bound by the decode still (all 513 experts are 857 MB, 131 us).  With 32 columns two stages are
-// left in shared memory and the copies' latency shows: 355 us.  What counts is the number of items, about 0.6 us each whatever their columns:
-// 24 columns pay from about nine entries per expert (launch_moe_ffn has the prompts' times).
+// One block per SM (16 token rows are 65 KB, and four stages keep the copies ahead of the decode) of 16 + 1 warps with up to 96 registers.  Two stages are
+// worked on side by side, each by half of the warps: a warp takes two row tiles x one K half of its stage, so every 16 bytes of activations it loads serve
+// both, and the tiles' independent MMA chains take the place of the second block.  (One row tile per warp and all warps on one stage: activations were most of
+// the shared-memory pipe's work, 66 % busy, with 51 % of the issue slots used.)  The two K halves of a pair of row tiles exchange one tile each.
+// Shares of the work are cut by cost, not by piece: an item weighs a decode and its tiles (WffnCost), because experts with one tile and the shared
+// expert's full items lie apart in the list.  The combine + norm that follows waits for the whole launch, so no output row is counted in.
+// One layer on a B200, items of eight columns in moe_ffn_k / one row tile per warp / two: 419 tokens 372 / 328 / 297 us.  Prompts, 12 layers, one row tile / two: 200
+// tokens 5.07 -> 4.78 ms, 419 7.20 -> 6.83, 512 8.26 -> 7.79, 1024 14.32 -> 13.59.  Bound by the decode still (all 513 experts are 857 MB, 131 us).
+// Items of 24 columns leave room for three stages: with one row tile per warp 13.67 ms at 1024 tokens, with two (276 bytes of spills) 14.06; 32 columns leave
+// two.  Short prompts on moe_ffn_k's eight columns and two blocks per SM: 65 tokens 3.26 against 3.23 to 3.34 ms here, 100 3.59 / 3.66, 128 4.02 / 3.97.
 constexpr int WFFN_RECS = 24;  // items a block's share can touch: 15 with 148 blocks, 1024 tokens and 15 choices each
 struct WffnCost {  // of a gate/up piece and of a down piece: a decode of the stage, and the MMAs and the epilogue of a column tile
     uint32_t dec, tile;
 };
 __device__ constexpr WffnCost WFFN_GU{6, 1}, WFFN_DN{5, 2};
+constexpr uint32_t WFFN_COLS = MOE_FFN_COLS_WIDE, WFFN_CT = WFFN_COLS / 8, WFFN_STG = 4;
 constexpr uint32_t WFFN_XP = FFN_D * 2 + 64, WFFN_HP = FFN_I * 4 + 64;  // distance of the token rows, and of the H rows (both planes), in shared memory
-template <int CT>
-struct WffnCfg {
-    static constexpr uint32_t COLS = 8 * CT, STG = CT == 2 ? 4 : 3, SEL = CT == 2 ? 0 : 1;  // SEL: which prw
-    static constexpr uint32_t OFF_TAB = 128, OFF_PRE = OFF_TAB + 256, OFF_REC = OFF_PRE + 2 * FFN_MAXG * 4, OFF_RED = OFF_REC + 2 * WFFN_RECS * 32 + 128, RED = 8 * CT * 32 * 16,
-                              REDS = STG == 4 ? 2 : 1, OFF_XS = (OFF_RED + REDS * RED + 127) / 128 * 128, OFF_STG = OFF_XS + COLS * WFFN_XP, SMEM = OFF_STG + STG * IQ3X_STAGE;
-    static_assert(SMEM <= 227 * 1024 && COLS <= 32 && COLS * WFFN_HP + RED <= COLS * WFFN_XP, "shared memory of the wide expert FFN");
-};
-static_assert(WffnCfg<2>::COLS == MOE_FFN_COLS_WIDE && WffnCfg<3>::COLS == MOE_FFN_COLS_WIDER, "columns of an item");
+constexpr uint32_t WFFN_OFF_TAB = 128, WFFN_OFF_PRE = WFFN_OFF_TAB + 256, WFFN_OFF_REC = WFFN_OFF_PRE + 2 * FFN_MAXG * 4, WFFN_OFF_RED = WFFN_OFF_REC + 2 * WFFN_RECS * 32 + 128,
+                   WFFN_RED = 16 * WFFN_CT * 32 * 16, WFFN_OFF_XS = (WFFN_OFF_RED + WFFN_RED + 127) / 128 * 128, WFFN_OFF_STG = WFFN_OFF_XS + WFFN_COLS * WFFN_XP,
+                   WFFN_SMEM = WFFN_OFF_STG + WFFN_STG * IQ3X_STAGE;
+static_assert(WFFN_SMEM <= 227 * 1024 && WFFN_COLS * WFFN_HP + WFFN_RED <= WFFN_COLS * WFFN_XP, "shared memory of the wide expert FFN");
+static_assert(WFFN_CT == 2 && WFFN_STG % 2 == 0, "column tiles that xw_tiles distinguishes; a stage for each half of the warps");
 
-// one super-block of rows g / g + 8 against NT column tiles; xb[i] = address of this lane's 16 bytes of tile i
-template <int PLANES, int NT, int CT>
-__device__ __forceinline__ void xw_unit(uint32_t rec0, uint32_t rec1, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[CT], uint32_t xo,
-                                        float (&acc)[CT][4]) {
+// one super-block of rows g / g + 8 of two row tiles (records rdist apart) against NT column tiles; xb[i] = address of this lane's 16 bytes of tile i
+template <int PLANES, int NT>
+__device__ __forceinline__ void xw_unit(uint32_t rec0, uint32_t rec1, uint32_t rdist, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[WFFN_CT], uint32_t xo,
+                                        float (&acc)[2][WFFN_CT][4]) {
     const uint32_t c0 = rec0 + kh * 128 + t * 4, c1 = rec1 + kh * 128 + t * 4;
-    const XHdr h0 = x_hdr(rec0, kh), h1 = x_hdr(rec1, kh);
-    float p[NT][4];
-    uint32_t q[2] = {lds_u32_off<0>(c0), lds_u32_off<0>(c1)};
-    XDec dec;
-    x_decode<0>(q, h0, h1, stab, dec);
+    XHdr h0[2], h1[2];
+    float p[2][NT][4];
+    uint32_t q[2][2];
+    XDec dec[2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        h0[r] = x_hdr(rec0 + r * rdist, kh);
+        h1[r] = x_hdr(rec1 + r * rdist, kh);
+        q[r][0] = lds_u32_off<0>(c0 + r * rdist);
+        q[r][1] = lds_u32_off<0>(c1 + r * rdist);
+        x_decode<0>(q[r], h0[r], h1[r], stab, dec[r]);
+    }
 #define XW_SUB(IB)                                                                                                             \
     {                                                                                                                          \
         uint4 xv[NT], xl[NT];                                                                                                  \
@@ -770,41 +772,43 @@ __device__ __forceinline__ void xw_unit(uint32_t rec0, uint32_t rec1, int kh, in
             xv[i] = lds_v4(xb[i] + xo + IB * 64);                                                                              \
             if (PLANES == 2) xl[i] = lds_v4(xb[i] + xo + FFN_I * 2 + IB * 64);                                                 \
         }                                                                                                                      \
-        if (IB < 7) {                                                                                                          \
-            q[0] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c0);                                                                \
-            q[1] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c1);                                                                \
+        _Pragma("unroll") for (int r = 0; r < 2; r++) {                                                                       \
+            if (IB < 7) {                                                                                                      \
+                q[r][0] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c0 + r * rdist);                                             \
+                q[r][1] = lds_u32_off<(IB < 7 ? IB + 1 : 0) * 16>(c1 + r * rdist);                                             \
+            }                                                                                                                  \
+            _Pragma("unroll") for (int i = 0; i < NT; i++) {                                                                   \
+                if (IB == 0) mma_f16(p[r][i], dec[r].a0, xv[i].x, xv[i].y, zr.z);                                              \
+                else mma_f16(p[r][i], dec[r].a0, xv[i].x, xv[i].y, p[r][i]);                                                   \
+            }                                                                                                                  \
+            _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[r][i], dec[r].a1, xv[i].z, xv[i].w, p[r][i]);             \
+            if (PLANES == 2) {                                                                                                 \
+                _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[r][i], dec[r].a0, xl[i].x, xl[i].y, p[r][i]);         \
+                _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[r][i], dec[r].a1, xl[i].z, xl[i].w, p[r][i]);         \
+            }                                                                                                                  \
+            if (IB < 7) x_decode<(IB < 7 ? IB + 1 : 0)>(q[r], h0[r], h1[r], stab, dec[r]);                                     \
         }                                                                                                                      \
-        _Pragma("unroll") for (int i = 0; i < NT; i++) {                                                                       \
-            if (IB == 0) mma_f16(p[i], dec.a0, xv[i].x, xv[i].y, zr.z);                                                        \
-            else mma_f16(p[i], dec.a0, xv[i].x, xv[i].y, p[i]);                                                                \
-        }                                                                                                                      \
-        _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a1, xv[i].z, xv[i].w, p[i]);                          \
-        if (PLANES == 2) {                                                                                                     \
-            _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a0, xl[i].x, xl[i].y, p[i]);                      \
-            _Pragma("unroll") for (int i = 0; i < NT; i++) mma_f16(p[i], dec.a1, xl[i].z, xl[i].w, p[i]);                      \
-        }                                                                                                                      \
-        if (IB < 7) x_decode<(IB < 7 ? IB + 1 : 0)>(q, h0, h1, stab, dec);                                                     \
     }
     XW_SUB(0) XW_SUB(1) XW_SUB(2) XW_SUB(3) XW_SUB(4) XW_SUB(5) XW_SUB(6) XW_SUB(7)
 #undef XW_SUB
 #pragma unroll
-    for (int i = 0; i < NT; i++) {
-        acc[i][0] = fmaf(h0.d, p[i][0], acc[i][0]);
-        acc[i][1] = fmaf(h0.d, p[i][1], acc[i][1]);
-        acc[i][2] = fmaf(h1.d, p[i][2], acc[i][2]);
-        acc[i][3] = fmaf(h1.d, p[i][3], acc[i][3]);
-    }
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            acc[r][i][0] = fmaf(h0[r].d, p[r][i][0], acc[r][i][0]);
+            acc[r][i][1] = fmaf(h0[r].d, p[r][i][1], acc[r][i][1]);
+            acc[r][i][2] = fmaf(h1[r].d, p[r][i][2], acc[r][i][2]);
+            acc[r][i][3] = fmaf(h1[r].d, p[r][i][3], acc[r][i][3]);
+        }
 }
-template <int PLANES, int CT>
-__device__ __forceinline__ void xw_tiles(uint32_t nt, uint32_t rec0, uint32_t rec1, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[CT], uint32_t xo,
-                                         float (&acc)[CT][4]) {
-    if (nt == 1) xw_unit<PLANES, 1, CT>(rec0, rec1, kh, t, stab, zr, xb, xo, acc);
-    else if (CT == 2 || nt == 2) xw_unit<PLANES, 2, CT>(rec0, rec1, kh, t, stab, zr, xb, xo, acc);
-    else xw_unit<PLANES, CT, CT>(rec0, rec1, kh, t, stab, zr, xb, xo, acc);
+template <int PLANES>
+__device__ __forceinline__ void xw_tiles(uint32_t nt, uint32_t rec0, uint32_t rec1, uint32_t rdist, int kh, int t, uint32_t stab, const ZeroRegs &zr, const uint32_t (&xb)[WFFN_CT],
+                                         uint32_t xo, float (&acc)[2][WFFN_CT][4]) {
+    if (nt == 1) xw_unit<PLANES, 1>(rec0, rec1, rdist, kh, t, stab, zr, xb, xo, acc);
+    else xw_unit<PLANES, 2>(rec0, rec1, rdist, kh, t, stab, zr, xb, xo, acc);
 }
 
 // item -> its columns.  prw = items before a group (of the selection record, in shared memory)
-template <uint32_t COLS>
 __device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_wide *ms, uint32_t U, uint32_t nb, uint32_t w) {
     FfnItem it{};
     const uint32_t routed = prw[U];
@@ -813,7 +817,7 @@ __device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_
         it.shared = 1;
         it.e0 = ms->off[U];  // (the shared expert's H rows follow the entries')
         cnt = nb;
-        it.c0 = (w - routed) * COLS;
+        it.c0 = (w - routed) * WFFN_COLS;
     } else {
         uint32_t lo = 0, hi = U;  // largest u with prw[u] <= w
         while (hi - lo > 1) {
@@ -823,16 +827,15 @@ __device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_
         }
         it.e0 = ms->off[lo];
         cnt = ms->off[lo + 1] - it.e0;
-        it.c0 = (w - prw[lo]) * COLS;
+        it.c0 = (w - prw[lo]) * WFFN_COLS;
         it.erow = ms->ue[lo];
     }
-    it.ncols = cnt - it.c0 < COLS ? cnt - it.c0 : COLS;
+    it.ncols = cnt - it.c0 < WFFN_COLS ? cnt - it.c0 : WFFN_COLS;
     return it;
 }
 // first piece (item * P + piece of the item) of block b of G: where b / G of the list's cost is reached.  pre = tiles of 8 before a group
-template <uint32_t COLS>
 __device__ __forceinline__ uint32_t wffn_edge(const uint32_t *pre, const uint32_t *prw, uint32_t U, uint32_t nb, bool shared, uint32_t b, uint32_t G, uint32_t P, WffnCost c) {
-    const uint32_t st = shared ? (nb + 7) / 8 : 0, si = shared ? (nb + COLS - 1) / COLS : 0, items = prw[U] + si;
+    const uint32_t st = shared ? (nb + 7) / 8 : 0, si = shared ? (nb + WFFN_COLS - 1) / WFFN_COLS : 0, items = prw[U] + si;
     if (b == G) return items * P;
     const uint32_t x = (uint32_t)((uint64_t)P * (c.dec * items + c.tile * (pre[U] + st)) * b / G);
     auto at = [&](uint32_t u) { return P * (c.dec * prw[u] + c.tile * pre[u]); };  // cost before group u
@@ -843,30 +846,27 @@ __device__ __forceinline__ uint32_t wffn_edge(const uint32_t *pre, const uint32_
         else hi = mid;
     }
     uint32_t rest = x - at(lo);
-    const uint32_t tiles = lo < U ? pre[lo + 1] - pre[lo] : st, full = P * (c.dec + c.tile * (COLS / 8));
+    const uint32_t tiles = lo < U ? pre[lo + 1] - pre[lo] : st, full = P * (c.dec + c.tile * (WFFN_COLS / 8));
     const uint32_t q = rest / full;  // whole items of this group before x
     rest -= q * full;
-    const uint32_t left = tiles - q * (COLS / 8), nt = left < (COLS / 8) ? left : (COLS / 8);
+    const uint32_t left = tiles - q * (WFFN_COLS / 8), nt = left < (WFFN_COLS / 8) ? left : (WFFN_COLS / 8);
     return (prw[lo] + q) * P + rest / (c.dec + c.tile * nt);
 }
 
-template <int CT>
 __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
-    using C = WffnCfg<CT>;
-    constexpr uint32_t WFFN_STG = C::STG, WFFN_COLS = C::COLS;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = (uint64_t *)smem, *empty = full + WFFN_STG, *actfull = empty + WFFN_STG, *actfree = actfull + 2;
-    uint32_t *pre = (uint32_t *)(smem + C::OFF_PRE), *prw = pre + FFN_MAXG;
-    FfnItem *recs = (FfnItem *)(smem + C::OFF_REC);
-    uint32_t *edge = (uint32_t *)(smem + C::OFF_REC + 2 * WFFN_RECS * 32);
-    constexpr uint32_t D = FFN_D, I = FFN_I, KP = D / 512, GT = I / 64, DT = D / 128;
-    const uint32_t act0 = smem_u32(smem + C::OFF_XS), slot0 = smem_u32(smem + C::OFF_STG);
+    uint32_t *pre = (uint32_t *)(smem + WFFN_OFF_PRE), *prw = pre + FFN_MAXG;
+    FfnItem *recs = (FfnItem *)(smem + WFFN_OFF_REC);
+    uint32_t *edge = (uint32_t *)(smem + WFFN_OFF_REC + 2 * WFFN_RECS * 32);
+    constexpr uint32_t D = FFN_D, I = FFN_I, KP = D / 512, GT = I / 128, DT = D / 256;  // GT, DT: pieces of an item, two stages side by side
+    const uint32_t act0 = smem_u32(smem + WFFN_OFF_XS), slot0 = smem_u32(smem + WFFN_OFF_STG);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     pdl_launch();
     if (tid == 0) {
         for (uint32_t s = 0; s < WFFN_STG; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], FFN_CW);
+            mbar_init(&empty[s], FFN_CW / 2);
         }
         for (int s = 0; s < 2; s++) {
             mbar_init(&actfull[s], 1);
@@ -874,12 +874,12 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
         }
         mbar_init_fence();
     }
-    if (tid < 16) x_scale_entry(smem + C::OFF_TAB, tid);
+    if (tid < 16) x_scale_entry(smem + WFFN_OFF_TAB, tid);
     pdl_wait();
     const moe_sel_wide *ms = (const moe_sel_wide *)p.ms;
     for (uint32_t i = tid; i < FFN_MAXG; i += FFN_THREADS) {
         pre[i] = ms->pre[i];
-        prw[i] = ms->prw[C::SEL][i];
+        prw[i] = ms->prw[i];
     }
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
@@ -887,7 +887,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     const bool bad = items > MOE_FFN_MAXITEMS_WIDE;  // cannot happen with E <= 512 and MOE_MAXB_WIDE tokens; never index past the counters
     if (bad && tid == 0) set_status(p.status, ST_BAD_ARG | 5);
     if (bad) items = 0;
-    if (tid < 4) edge[tid] = bad ? 0 : wffn_edge<WFFN_COLS>(pre, prw, U, nb, p.Sd != nullptr, blockIdx.x + (tid & 1), gridDim.x, tid < 2 ? GT : DT, tid < 2 ? WFFN_GU : WFFN_DN);
+    if (tid < 4) edge[tid] = bad ? 0 : wffn_edge(pre, prw, U, nb, p.Sd != nullptr, blockIdx.x + (tid & 1), gridDim.x, tid < 2 ? GT : DT, tid < 2 ? WFFN_GU : WFFN_DN);
     __syncthreads();
     uint32_t a_lo = edge[0], a_hi = edge[1], b_lo = edge[2], b_hi = edge[3];
     const uint32_t wa0 = a_lo / GT, wb0 = b_lo / DT;
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     if (tid < 2 * WFFN_RECS) {
         const uint32_t k = tid % WFFN_RECS, w = (tid < WFFN_RECS ? wa0 : wb0) + k;
         const bool need = tid < WFFN_RECS ? (a_hi > a_lo && w <= (a_hi - 1) / GT) : (b_hi > b_lo && w <= (b_hi - 1) / DT);
-        if (need) recs[tid] = wffn_item<WFFN_COLS>(prw, ms, U, nb, w);
+        if (need) recs[tid] = wffn_item(prw, ms, U, nb, w);
     }
     __syncthreads();
     const FfnItem *rec_a = recs - wa0, *rec_b = recs + WFFN_RECS - wb0;  // rec_a[w], rec_b[w]
@@ -944,9 +944,9 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
         for (uint32_t a = a_lo; a < a_hi; a++) {
             const uint32_t w = a / GT, gt = a - w * GT;
             const FfnItem it = rec_a[w];
-            const uint8_t *src = (it.shared ? p.Sg : p.Wg) + ((size_t)it.erow * GT + gt) * KP * IQ3X_STAGE;
+            const uint8_t *src = (it.shared ? p.Sg : p.Wg) + ((size_t)it.erow * GT + gt) * 2 * KP * IQ3X_STAGE;
             for (uint32_t kp = 0; kp < KP; kp++) {
-                stage(src + (size_t)kp * IQ3X_STAGE);
+                for (uint32_t h = 0; h < 2; h++) stage(src + ((size_t)h * KP + kp) * IQ3X_STAGE);
                 if (w != cur && kp == 0) {
                     cur = w;
                     uint32_t tok = 0, rank;
@@ -962,7 +962,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
         for (uint32_t bi = b_lo; bi < b_hi; bi++) {
             const uint32_t w = bi / DT, dt = bi - w * DT;
             const FfnItem it = rec_b[w];
-            stage((it.shared ? p.Sd : p.Wd) + ((size_t)it.erow * DT + dt) * IQ3X_STAGE);
+            for (uint32_t h = 0; h < 2; h++) stage((it.shared ? p.Sd : p.Wd) + (((size_t)it.erow * DT + dt) * 2 + h) * IQ3X_STAGE);
             if (w != cur) {  // H of a new item: complete when both K halves of all its row groups have counted in
                 cur = w;
                 if (ok && ld_acquire_gpu(p.sync + w) < GT * FFN_CW) {
@@ -983,21 +983,22 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
             }
         }
     } else {
-        const int r = warp & 7, kh = warp >> 3;
+        const int sh = warp >> 3, r = 2 * (warp & 3), kh = (warp >> 2) & 1, pr = sh * 4 + (warp & 3);  // stage of the two, first row tile, K half, pair of warps
         bool ok = true;
-        const uint32_t stab = smem_u32(smem + C::OFF_TAB);
+        const uint32_t stab = smem_u32(smem + WFFN_OFF_TAB);
         const ZeroRegs zr = zero_regs();
-        uint32_t j = 0, k = 0, rowbase = 0, rc = 0, xb[CT];
+        uint32_t j = 0, k = 0, rowbase = 0, rc = 0, xb[WFFN_CT];
         auto wait_full = [&]() {
-            if (ok && !mbar_wait(&full[j % WFFN_STG], (j / WFFN_STG) & 1)) {
+            const uint32_t js = 2 * j + sh;
+            if (ok && !mbar_wait(&full[js % WFFN_STG], (js / WFFN_STG) & 1)) {
                 ok = false;
                 if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 9);
             }
-            return slot0 + (j % WFFN_STG) * IQ3X_STAGE;
+            return slot0 + (js % WFFN_STG) * IQ3X_STAGE;
         };
         auto release = [&]() {
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[j % WFFN_STG]);
+            if (lane == 0) mbar_arrive(&empty[(2 * j + sh) % WFFN_STG]);
             j++;
         };
         auto act_wait = [&](uint32_t ncols, uint32_t pitch) {  // columns past the item's read whatever the row holds: nobody looks at their results
@@ -1006,7 +1007,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                 if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 10);
             }
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++) xb[i] = act0 + ((rowbase + 8 * i + g) % WFFN_COLS) * pitch + t * 16;
+            for (uint32_t i = 0; i < WFFN_CT; i++) xb[i] = act0 + ((rowbase + 8 * i + g) % WFFN_COLS) * pitch + t * 16;
             rowbase = (rowbase + ncols) % WFFN_COLS;
         };
         auto act_release = [&]() {
@@ -1014,25 +1015,28 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
             if (lane == 0) mbar_arrive(&actfree[k & 1]);
             k++;
         };
-        // The two K halves of a row group: odd tiles go to the high half, even ones to the low half; low + high either way.  Two buffers alternate.  With three
-        // stages there is room for one: gate/up has four stages between two exchanges, and a stage comes round only when the partner has released it after its
-        // own reads; down pieces, one stage each, alternate with a second buffer behind the H rows.
-        auto exchange = [&](float (&acc)[CT][4], uint32_t nt, bool down) {
-            const bool second = C::REDS == 2 || down ? rc & 1 : false;
-            rc = C::REDS == 2 || down ? rc + 1 : 0;
-            float4 *rd = (float4 *)(smem + (second ? (C::REDS == 2 ? C::OFF_RED + C::RED : C::OFF_XS + WFFN_COLS * WFFN_HP) : C::OFF_RED)) + r * CT * 32 + lane;
+        // The two K halves of a pair of row tiles: the low half finishes the first, the high half the second; low + high either way.  Down pieces, one stage
+        // each, alternate between two buffers, the second behind the H rows (the X rows are longer).  Gate/up has four stages between two exchanges, and this
+        // half's two stages come round only when the partner has released them after its own reads: one buffer is enough.
+        auto exchange = [&](float (&acc)[2][WFFN_CT][4], uint32_t nt, bool down) {
+            const bool second = down && (rc & 1);
+            rc = down ? rc + 1 : 0;
+            float4 *rd = (float4 *)(smem + (second ? WFFN_OFF_XS + WFFN_COLS * WFFN_HP : WFFN_OFF_RED)) + pr * 2 * WFFN_CT * 32 + lane;
+            auto of = [&](int tile, uint32_t i) {
+                return make_float4(tile ? acc[1][i][0] : acc[0][i][0], tile ? acc[1][i][1] : acc[0][i][1], tile ? acc[1][i][2] : acc[0][i][2], tile ? acc[1][i][3] : acc[0][i][3]);
+            };
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++)
-                if (i < nt && (int)(i & 1) != kh) rd[i * 32] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-            bar_sync_n(1 + r, 64);
+            for (uint32_t i = 0; i < WFFN_CT; i++)
+                if (i < nt) rd[(kh * WFFN_CT + i) * 32] = of(kh ^ 1, i);
+            bar_sync_n(1 + pr, 64);
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++)
-                if (i < nt && (int)(i & 1) == kh) {
-                    const float4 v = rd[i * 32];
-                    acc[i][0] += v.x;
-                    acc[i][1] += v.y;
-                    acc[i][2] += v.z;
-                    acc[i][3] += v.w;
+            for (uint32_t i = 0; i < WFFN_CT; i++)
+                if (i < nt) {
+                    const float4 m = of(kh, i), v = rd[((kh ^ 1) * WFFN_CT + i) * 32];
+                    acc[0][i][0] = m.x + v.x;
+                    acc[0][i][1] = m.y + v.y;
+                    acc[0][i][2] = m.z + v.z;
+                    acc[0][i][3] = m.w + v.w;
                 }
         };
         uint32_t cur = 0xffffffffu, ncols = 0, nt = 0, hrow = 0;
@@ -1047,22 +1051,22 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                 hrow = it.e0 + it.c0;
                 act_wait(ncols, WFFN_XP);
             }
-            float acc[CT][4];
+            float acc[2][WFFN_CT][4];
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+            for (uint32_t i = 0; i < 2 * WFFN_CT; i++) acc[i / WFFN_CT][i % WFFN_CT][0] = acc[i / WFFN_CT][i % WFFN_CT][1] = acc[i / WFFN_CT][i % WFFN_CT][2] = acc[i / WFFN_CT][i % WFFN_CT][3] = 0.f;
             for (uint32_t kp = 0; kp < KP; kp++) {
                 const uint32_t st = wait_full(), rec0 = st + (8 * r + g) * IQ3X_REC;
-                xw_tiles<1, CT>(nt, rec0, rec0 + 64 * IQ3X_REC, kh, t, stab, zr, xb, (2 * kp + kh) * 512, acc);
+                xw_tiles<1>(nt, rec0, rec0 + 64 * IQ3X_REC, 8 * IQ3X_REC, kh, t, stab, zr, xb, (2 * kp + kh) * 512, acc);
                 release();
             }
             exchange(acc, nt, false);
-            __half *Hw = p.H + (size_t)hrow * 2 * I + gt * 64 + 8 * r + g;  // H [row][plane][I]
+            __half *Hw = p.H + (size_t)hrow * 2 * I + (gt * 2 + sh) * 64 + 8 * (r + kh) + g;  // H [row][plane][I]
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++) {
-                if (i >= nt || (int)(i & 1) != kh) continue;
+            for (uint32_t i = 0; i < WFFN_CT; i++) {
+                if (i >= nt) continue;
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
-                    const float gs = acc[i][c], us = acc[i][2 + c];
+                    const float gs = acc[0][i][c], us = acc[0][i][2 + c];
                     float h = gs / (1.0f + expf(-gs)) * us;
                     h = fminf(fmaxf(h, -65504.0f), 65504.0f);
                     const __half hi = __float2half_rn(h);
@@ -1076,7 +1080,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
             }
             __syncwarp();
             if (lane == 0) {
-                if ((uint32_t)kh < nt) __threadfence();  // the warp's H values (cumulative over the warp barrier) before the count
+                __threadfence();  // the warp's H values (cumulative over the warp barrier) before the count
                 atomicAdd(p.sync + w, 1u);
             }
         }
@@ -1084,7 +1088,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
         // ---- down pieces
         cur = 0xffffffffu;
         rowbase = 0;
-        uint32_t oo[(CT + 1) / 2][2];  // element offsets of the output rows of columns 2t and 2t + 1 of this half's tiles
+        uint32_t oo[WFFN_CT][2];  // element offsets of the output rows of columns 2t and 2t + 1 of the tiles
         for (uint32_t bi = b_lo; bi < b_hi; bi++) {
             const uint32_t w = bi / DT, dt = bi - w * DT;
             if (w != cur) {
@@ -1093,10 +1097,10 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                 const FfnItem it = rec_b[w];
                 nt = (it.ncols + 7) / 8;
 #pragma unroll
-                for (uint32_t i = 0; i < (CT + 1) / 2; i++)
+                for (uint32_t i = 0; i < WFFN_CT; i++)
 #pragma unroll
                     for (int c = 0; c < 2; c++) {
-                        const uint32_t n = 8 * (2 * i + kh) + 2 * t + c;
+                        const uint32_t n = 8 * i + 2 * t + c;
                         oo[i][c] = 0xffffffffu;
                         if (n < it.ncols) {
                             uint32_t tok, rank;
@@ -1106,19 +1110,19 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                     }
                 act_wait(it.ncols, WFFN_HP);
             }
-            float acc[CT][4];
+            float acc[2][WFFN_CT][4];
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+            for (uint32_t i = 0; i < 2 * WFFN_CT; i++) acc[i / WFFN_CT][i % WFFN_CT][0] = acc[i / WFFN_CT][i % WFFN_CT][1] = acc[i / WFFN_CT][i % WFFN_CT][2] = acc[i / WFFN_CT][i % WFFN_CT][3] = 0.f;
             const uint32_t st = wait_full(), rec0 = st + (16 * r + g) * IQ3X_REC;
-            xw_tiles<2, CT>(nt, rec0, rec0 + 8 * IQ3X_REC, kh, t, stab, zr, xb, kh * 512, acc);
+            xw_tiles<2>(nt, rec0, rec0 + 8 * IQ3X_REC, 16 * IQ3X_REC, kh, t, stab, zr, xb, kh * 512, acc);
             release();
             exchange(acc, nt, true);
-            const uint32_t row = dt * 128 + 16 * r + 2 * g;
+            const uint32_t row = (dt * 2 + sh) * 128 + 16 * (r + kh) + 2 * g;
 #pragma unroll
-            for (uint32_t i = 0; i < (uint32_t)CT; i++) {
-                if (i >= nt || (int)(i & 1) != kh) continue;
-                if (oo[i / 2][0] != 0xffffffffu) *(float2 *)(p.Pg + oo[i / 2][0] + row) = make_float2(acc[i][0], acc[i][2]);
-                if (oo[i / 2][1] != 0xffffffffu) *(float2 *)(p.Pg + oo[i / 2][1] + row) = make_float2(acc[i][1], acc[i][3]);
+            for (uint32_t i = 0; i < WFFN_CT; i++) {
+                if (i >= nt) continue;
+                if (oo[i][0] != 0xffffffffu) *(float2 *)(p.Pg + oo[i][0] + row) = make_float2(acc[0][i][0], acc[0][i][2]);
+                if (oo[i][1] != 0xffffffffu) *(float2 *)(p.Pg + oo[i][1] + row) = make_float2(acc[0][i][1], acc[0][i][3]);
             }
         }
         if (cur != 0xffffffffu) act_release();
@@ -1233,27 +1237,18 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     const uint32_t nb = L.has_bytes(13, 4) ? L.bytes<uint32_t>(13) : 0, grid = (uint32_t)(L.sm_count * per_sm);
     const double items = E * (1 - pow(1 - (double)topk / E, (double)nb)) + (nb + 7) / 8;
     const bool half = x4 && !wide && !probe && p.ep.nranks == 1 && nb >= 1 && 2 * items * (I / 64) <= grid * (33.0 / 32);
-    // A piece of a prompt: the columns of an item, by the entries that nb tokens (bind 13) leave an expert on average.  Few entries: eight columns and two
-    // blocks per SM (moe_ffn_k, without the row counts); many: 24, so that fewer experts are decoded twice.  Prompts on a B200, 12 layers, 512 experts, top-10,
-    // with 8, 16 and 24 columns (ms): 65 tokens 3.37, 3.51, 3.70; 128 4.11, 4.28, 4.42; 164 4.67, 4.77, 5.00; 200 5.08, 5.07, 5.27; 256 5.55, 5.46, 5.61;
-    // 419 7.85, 7.21, 7.25; 512 -, 8.26, 8.19; 600 -, 9.40, 9.23; 1024 -, 14.32, 13.68.  (Up to 3.75 E entries in items of eight columns are at most
-    // 512 + 240 items, beside up to 128 of the shared expert: inside the counters, the H of the wide scratch and FFN_RECS.)
-    const uint32_t entries = nb * topk;
-    const bool eight = wide && nb && entries <= E * 15 / 4, wider = entries >= E * 9;
-    QW_CHECK_ARG(!wide || (EL == E && p.ebase == 0));
-    if (wide && !eight) {
-        auto kw = wider ? moe_ffn_wide_k<3> : moe_ffn_wide_k<2>;
-        const uint32_t sm = wider ? WffnCfg<3>::SMEM : WffnCfg<2>::SMEM;
-        cudaError_t e = cudaFuncSetAttribute(kw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (wide) {
+        QW_CHECK_ARG(EL == E && p.ebase == 0);
+        cudaError_t e = cudaFuncSetAttribute(moe_ffn_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WFFN_SMEM);
         if (e != cudaSuccess) return e;
         int occ = 0;  // the blocks wait for one another's H
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kw, FFN_THREADS, sm);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, moe_ffn_wide_k, FFN_THREADS, WFFN_SMEM);
         if (e != cudaSuccess) return e;
         QW_CHECK_ARG(occ >= 1);
-        qw_launch(kw, (uint32_t)L.sm_count, FFN_THREADS, sm, L.stream, p);
+        qw_launch(moe_ffn_wide_k, (uint32_t)L.sm_count, FFN_THREADS, WFFN_SMEM, L.stream, p);
         return cudaGetLastError();
     }
-    auto kern = eight ? moe_ffn_k<false, 1, false, true> : half ? moe_ffn_k<false, 1, true> : x4 ? (probe ? moe_ffn_k<true, 1> : moe_ffn_k<false, 1>) : (probe ? moe_ffn_k<true, 0> : moe_ffn_k<false, 0>);
+    auto kern = half ? moe_ffn_k<false, 1, true> : x4 ? (probe ? moe_ffn_k<true, 1> : moe_ffn_k<false, 1>) : (probe ? moe_ffn_k<true, 0> : moe_ffn_k<false, 0>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;  // the blocks wait for one another's H: all of them must be resident together

@@ -192,12 +192,12 @@ __device__ __forceinline__ void moe_topk_row(const float *lg, uint32_t E, uint32
 }
 
 // Grouping of nb tokens' chosen experts (sid [token][MOE_MAXK]) by one block of NTH >= E threads: thread e owns expert e in the scans.
-// prw: items of MOE_FFN_COLS_WIDE and of MOE_FFN_COLS_WIDER entries in the groups before u, or nullptr.  before: with many token words, room for the entries of an expert ahead of each
+// prw: items of MOE_FFN_COLS_WIDE entries in the groups before u, or nullptr.  before: with many token words, room for the entries of an expert ahead of each
 // of them -- an entry then finds its place by one look-up instead of walking up to 31 words (1024 tokens: 26.8 -> 18.7 us), or nullptr
 template <int NTH, class SEL, int W, int ME>
-__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][ME], uint32_t (*prw)[MOE_MAXE + 2], uint16_t (*before)[ME]) {
+__device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uint32_t E, uint32_t topk, sel_args a, uint32_t (&mask)[W][ME], uint32_t *prw, uint16_t (*before)[ME]) {
     __shared__ uint32_t pos[MOE_MAXE];
-    __shared__ uint32_t wsum[3][32];
+    __shared__ uint32_t wsum[2][32];
     constexpr uint32_t NW = NTH / 32;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // group by expert.  mask[e] = tokens that chose e; an entry's place inside its group is the number of
@@ -218,36 +218,26 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
                 c0 += __popc(mask[q][tid]);
             }
         const uint32_t f = c0 ? 1u | ((c0 + MOE_FFN_COLS_WIDE - 1) / MOE_FFN_COLS_WIDE) << 16 : 0u, c = c0 | (((c0 + 7) / 8) << 16);
-        const uint32_t f2 = (c0 + MOE_FFN_COLS_WIDER - 1) / MOE_FFN_COLS_WIDER;
-        uint32_t sc = c, sf = f, s2 = f2;
+        uint32_t sc = c, sf = f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t tc = __shfl_up_sync(0xffffffffu, sc, o), tf = __shfl_up_sync(0xffffffffu, sf, o);
             if (lane >= (uint32_t)o) { sc += tc; sf += tf; }
-            if (prw) {
-                const uint32_t t2 = __shfl_up_sync(0xffffffffu, s2, o);
-                if (lane >= (uint32_t)o) s2 += t2;
-            }
         }
-        if (lane == 31) { wsum[0][warp] = sc; wsum[1][warp] = sf; wsum[2][warp] = s2; }
+        if (lane == 31) { wsum[0][warp] = sc; wsum[1][warp] = sf; }
         __syncthreads();
         if (warp == 0) {
-            uint32_t xc = lane < NW ? wsum[0][lane] : 0, xf = lane < NW ? wsum[1][lane] : 0, x2 = lane < NW ? wsum[2][lane] : 0;
+            uint32_t xc = lane < NW ? wsum[0][lane] : 0, xf = lane < NW ? wsum[1][lane] : 0;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t tc = __shfl_up_sync(0xffffffffu, xc, o), tf = __shfl_up_sync(0xffffffffu, xf, o);
                 if (lane >= (uint32_t)o) { xc += tc; xf += tf; }
-                if (prw) {
-                    const uint32_t t2 = __shfl_up_sync(0xffffffffu, x2, o);
-                    if (lane >= (uint32_t)o) x2 += t2;
-                }
             }
             wsum[0][lane] = xc;
             wsum[1][lane] = xf;
-            wsum[2][lane] = x2;
         }
         __syncthreads();
-        const uint32_t bc = warp ? wsum[0][warp - 1] : 0, bf = warp ? wsum[1][warp - 1] : 0, b2 = warp ? wsum[2][warp - 1] : 0;
+        const uint32_t bc = warp ? wsum[0][warp - 1] : 0, bf = warp ? wsum[1][warp - 1] : 0;
         const uint32_t ex = bc + sc - c;  // exclusive prefix: entries | passes << 16
         pos[tid] = ex & 0xffffu;          // first entry of expert tid
         if (c0) {
@@ -255,10 +245,7 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
             ms->ue[u] = tid;
             ms->off[u] = ex & 0xffffu;
             ms->pre[u] = ex >> 16;
-            if (prw) {
-                prw[0][u] = fx >> 16;
-                prw[1][u] = b2 + s2 - f2;
-            }
+            if (prw) prw[u] = fx >> 16;
         }
         if (tid == NTH - 1) {
             const uint32_t U = (bf + sf) & 0xffffu;
@@ -267,10 +254,7 @@ __device__ __forceinline__ void moe_group_body(const uint16_t *sid, SEL *ms, uin
             ms->topk = topk;
             ms->off[U] = (bc + sc) & 0xffffu;
             ms->pre[U] = (bc + sc) >> 16;
-            if (prw) {
-                prw[0][U] = (bf + sf) >> 16;
-                prw[1][U] = b2 + s2;
-            }
+            if (prw) prw[U] = (bf + sf) >> 16;
         }
     }
     __syncthreads();

@@ -25,7 +25,7 @@ typedef moe_sel_t<MOE_MAXB> moe_sel;
 #define MOE_MAXB_WIDE 1024
 struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
     uint16_t sid[MOE_MAXB_WIDE][MOE_MAXK];    // chosen experts of every token: from the top-k to the grouping
-    uint32_t prw[2][MOE_MAXE + 2];            // items of the expert FFN in the groups before u: of MOE_FFN_COLS_WIDE entries, of MOE_FFN_COLS_WIDER
+    uint32_t prw[MOE_MAXE + 2];               // items of the expert FFN (MOE_FFN_COLS_WIDE entries each) in the groups before u
 };
 
 // Scratch buffer of the fused expert-FFN kernel (k_ffn.cu): the items' counters and the finished-block counter in the first
@@ -40,10 +40,9 @@ struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
 #define MOE_FFN_ROWCNT 1024
 #define MOE_FFN_ROW_DONE(D) ((D) / 128 * 8)
 #define MOE_FFN_SCRATCH_BYTES(I) ((size_t)MOE_FFN_SYNC_BYTES + (size_t)MOE_FFN_MAXITEMS * 16 * (I) * 2)
-// The same for a piece of a prompt, in a buffer of its own.  An item has up to MOE_FFN_COLS_WIDE or MOE_FFN_COLS_WIDER columns.  H is [entry, then the shared expert's
+// The same for a piece of a prompt, in a buffer of its own.  An item has up to MOE_FFN_COLS_WIDE columns.  H is [entry, then the shared expert's
 // tokens][2 planes][I].  No output row is counted in.
 #define MOE_FFN_COLS_WIDE 16
-#define MOE_FFN_COLS_WIDER 24
 #define MOE_FFN_MAXITEMS_WIDE (512 + MOE_MAXB_WIDE * MOE_MAXK / MOE_FFN_COLS_WIDE)
 #define MOE_FFN_SYNC_BYTES_WIDE 8192
 #define MOE_FFN_SCRATCH_BYTES_WIDE(I) ((size_t)MOE_FFN_SYNC_BYTES_WIDE + (size_t)MOE_MAXB_WIDE * MOE_MAXK * 2 * (I) * 2)
