@@ -484,20 +484,21 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
 // tokens, by fewer warps with more registers.  (12352 x 2048 IQ3_S, 419 tokens, TS 2 -> 1 on a B200: 121 -> 110 us; 2048 x 4096: 45 -> 42; prompts of 419
 // tokens, 48 layers, 37.5 -> 36.9 ms.  Two groups are better off with 2: prompts of 65, 100 and 128 tokens, 12 layers, 3.37 -> 3.26, 3.69 -> 3.61 and
 // 4.11 -> 4.03 ms.)
+// RT = row tiles per warp.  2 (IQ3_S): the activations are read once for both; the weight stages are then one unit long (shared memory).
 // Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
 // IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
 // 40 of its cycles per unit of 16 rows x 32 weights.
-template <int GF, int TS>
+template <int GF, int TS, int RT = 1>
 struct WideCfg {
-    static constexpr int RG = TS == 2 || GF == 21 ? 7 : 11;  // row tiles per round: 14 + 1 warps of 128 registers, 7 + 1 of up to 255 or 11 + 1 of 168
-    static constexpr int UPW = GF == 21 ? 2 : 1;             // units per weight stage
-    static constexpr int PITCH = GF == 21 ? 240 : 272;       // bytes between staged rows (eight rows: eight different groups of four banks)
+    static constexpr int RG = RT * (TS == 2 || GF == 21 ? 7 : 11);  // row tiles per round: 14 + 1 warps of 128 registers, 7 + 1 of up to 255 (with one or two tiles each) or 11 + 1 of 168
+    static constexpr int UPW = GF == 21 && RT == 1 ? 2 : 1;             // units per weight stage
+    static constexpr int PITCH = GF == 8 ? 272 : UPW == 2 ? 240 : 144;  // bytes between staged rows (eight rows: eight different groups of four banks)
     static constexpr int WS = GF == 21 || TS == 1 ? 2 : 3, XS = 3;  // stages
     static constexpr int TABB = GF == 21 ? 65536 : 0;
     static constexpr int WBYTES = RG * 16 * PITCH;
     static constexpr size_t smem(int CT) { return 1024 + 256 + (size_t)TABB + (size_t)WS * WBYTES + (size_t)XS * CT * TS * 8 * 512; }
 };
-static_assert(WideCfg<21, 2>::smem(4) <= 227 * 1024 && WideCfg<21, 1>::smem(8) <= 227 * 1024 && WideCfg<8, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 1>::smem(8) <= 227 * 1024, "shared memory of the wide matvec");
+static_assert(WideCfg<21, 2>::smem(4) <= 227 * 1024 && WideCfg<21, 1>::smem(8) <= 227 * 1024 && WideCfg<21, 1, 2>::smem(8) <= 227 * 1024 && WideCfg<8, 2>::smem(4) <= 227 * 1024 && WideCfg<8, 1>::smem(8) <= 227 * 1024, "shared memory of the wide matvec");
 
 // q8_sub_h for rows 272 bytes apart, in half the shared-memory cycles: 32-bit loads only, and lanes t >= 2 take their words in another
 // order, so that rows g and g + 1 do not meet in a bank (only the third load of an even block has two lanes per bank).
@@ -544,10 +545,10 @@ __device__ __forceinline__ void wide_decode(uint32_t u0, uint32_t u1, int t, con
 // the grid: blocks_per_group blocks each, so that a group's blocks have many row tiles and run them side by side.  One launch for all groups
 // instead of one per 64 tokens, and K = 4096 here instead of in qmv_mma2: a prompt of 419 tokens, 48 layers, 42.5 -> 39.6 ms, 1700 tokens, 12
 // layers, 41.2 -> 38.9 ms on a B200.  UNITS = K / 256.  grid: at most one block per SM
-template <int GF, bool F32OUT, int TS, int CT, int UNITS>
-__global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wide_k(const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx,
+template <int GF, bool F32OUT, int TS, int CT, int UNITS, int RT = 1>
+__global__ void __launch_bounds__((TS * WideCfg<GF, TS, RT>::RG / RT + 1) * 32, 1) qmv_wide_k(const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx,
                                                                                     const QmvMmaP p, uint32_t rg, uint32_t blocks_per_group) {
-    using C = WideCfg<GF, TS>;
+    using C = WideCfg<GF, TS, RT>;
     constexpr int WS = C::WS, XS = C::XS, UPW = C::UPW, R = 8 * CT * TS, XBYTES = R * 512, CH = CT <= 4 ? CT : CT / 2;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;  // the swizzle pattern repeats every 1024 bytes
@@ -555,7 +556,7 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
     uint64_t *bars = (uint64_t *)(smem_raw + (tab0 + C::TABB - smem_u32(smem_raw)));
     uint64_t *wfull = bars, *wempty = wfull + WS, *xfull = wempty + WS, *xempty = xfull + XS, *tbar = xempty + XS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const uint32_t ncw = TS * rg;  // consumer warps; warp ncw is the producer
+    const uint32_t ncw = TS * rg / RT;  // consumer warps; warp ncw is the producer
     pdl_launch();
     if (tid == 0) {
         for (int s = 0; s < WS; s++) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], ncw); }
@@ -584,7 +585,7 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
                 if (jw >= WS && !mbar_wait(&wempty[s], (jw / WS - 1) & 1)) return false;
                 const uint32_t lo = cnt * r / rounds, n = cnt * (r + 1) / rounds - lo;
                 mbar_expect_tx(&wfull[s], n * 16 * C::PITCH);
-                const int xc = GF == 21 ? (int)((220 * kp) & ~15u) : (int)(136 * kp);  // bytes, or pairs of bytes
+                const int xc = GF == 21 ? (int)((110 * UPW * kp) & ~15u) : (int)(136 * kp);  // bytes, or pairs of bytes
                 for (uint32_t i = 0; i < n; i++) tma_load_2d(ws0 + s * C::WBYTES + i * 16 * C::PITCH, &mw, xc, (int)((t0 + lo + i) * 16), &wfull[s]);
                 jw++;
                 return true;
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
         return;
     }
     pdl_wait();
-    const uint32_t r = (uint32_t)warp % rg, th = (uint32_t)warp / rg;
+    const uint32_t r = (uint32_t)warp % (rg / RT) * RT, th = (uint32_t)warp / (rg / RT);
     // (this warp's column tiles: th, th + TS, ...; rows past the last token read as zero)
     const uint32_t tokr = (uint32_t)(g >> 1) | ((uint32_t)(g & 1) << 2);                      // token of MMA column g within a tile
     const uint32_t xoff = th * 1024 + tokr * 128 + ((uint32_t)t ^ tokr) * 16, tabc = tab0 + (lane & 15) * 8;
@@ -613,54 +614,64 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
     uint32_t jw = 0, jx = 0;
     for (uint32_t rd = 0; rd < rounds && ok; rd++) {
         const uint32_t lo = cnt * rd / rounds, n = cnt * (rd + 1) / rounds - lo;
-        float tot[CT][4];
+        float tot[RT][CT][4];
 #pragma unroll
-        for (int i = 0; i < CT; i++) tot[i][0] = tot[i][1] = tot[i][2] = tot[i][3] = 0.f;
+        for (int i = 0; i < RT * CT; i++) tot[i / CT][i % CT][0] = tot[i / CT][i % CT][1] = tot[i / CT][i % CT][2] = tot[i / CT][i % CT][3] = 0.f;
 #pragma unroll 1
         for (uint32_t u = 0; u < UNITS; u++, jx++) {
             if (u % UPW == 0 && !mbar_wait(&wfull[jw % WS], (jw / WS) & 1)) { ok = false; break; }
             if (!mbar_wait(&xfull[jx % XS], (jx / XS) & 1)) { ok = false; break; }
-            if (r < n) {
-                const uint32_t u0 = ws0 + (jw % WS) * C::WBYTES + (r * 16 + g) * C::PITCH + (GF == 21 ? ((220 * (u / 2)) & 15) + (u & 1) * 110 : 0);
+            if (r < n) {  // (a second row tile past the round's last one is computed from whatever the stage holds, and not stored)
+                const uint32_t u0 = ws0 + (jw % WS) * C::WBYTES + (r * 16 + g) * C::PITCH + (GF == 21 ? ((110 * UPW * (u / UPW)) & 15) + (u % UPW) * 110 : 0);
                 const uint32_t u1 = u0 + 8 * C::PITCH, xa = xs0 + (jx % XS) * XBYTES + xoff;
-                Iq3sHdr h0{}, h1{};
-                if (GF == 21) {
-                    h0 = iq3s_hdr(u0, t);
-                    h1 = iq3s_hdr(u1, t);
-                }
-                float acc[CT][4];
+                Iq3sHdr h0[RT]{}, h1[RT]{};
+                float acc[RT][CT][4];
 #pragma unroll
-                for (int i = 0; i < CT; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+                for (int i = 0; i < RT * CT; i++) acc[i / CT][i % CT][0] = acc[i / CT][i % CT][1] = acc[i / CT][i % CT][2] = acc[i / CT][i % CT][3] = 0.f;
                 // The MMAs of the column tiles are issued back to back, first halves then second halves, and the next sub-block is decoded before
                 // their results are used: in program order one tile after the other, every tile waited for its load and for two dependent MMAs.
-                uint32_t a0[4], a1[4];
-                float da, db;
-                wide_decode<GF, 0>(u0, u1, t, h0, h1, tabc, a0, a1, da, db);
+                uint32_t a0[RT][4], a1[RT][4];
+                float da[RT], db[RT];
+#pragma unroll
+                for (int m = 0; m < RT; m++) {
+                    if (GF == 21) {
+                        h0[m] = iq3s_hdr(u0 + m * 16 * C::PITCH, t);
+                        h1[m] = iq3s_hdr(u1 + m * 16 * C::PITCH, t);
+                    }
+                    wide_decode<GF, 0>(u0 + m * 16 * C::PITCH, u1 + m * 16 * C::PITCH, t, h0[m], h1[m], tabc, a0[m], a1[m], da[m], db[m]);
+                }
 #define WIDE_SUB(IB)                                                                                                              \
     {                                                                                                                             \
         const uint32_t xb = (IB & 1 ? xa ^ 64u : xa) + (IB / 2) * R * 128;                                                        \
-        const float ea = da, eb = db;                                                                                             \
+        float ea[RT], eb[RT];                                                                                                     \
+        _Pragma("unroll") for (int m = 0; m < RT; m++) {                                                                          \
+            ea[m] = da[m];                                                                                                        \
+            eb[m] = db[m];                                                                                                        \
+        }                                                                                                                         \
         _Pragma("unroll") for (int c = 0; c < CT; c += CH) { /* CH column tiles at a time: registers */                           \
             uint4 xv[CH];                                                                                                         \
-            float q[CH][4];                                                                                                       \
             _Pragma("unroll") for (int i = 0; i < CH; i++) xv[i] = lds_v4(xb + (c + i) * TS * 1024);                              \
-            _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a0, xv[i].x, xv[i].y, zr.z);                             \
-            _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a1, xv[i].z, xv[i].w, q[i]);                             \
-            if (IB < 7 && c + CH == CT) wide_decode<GF, (IB < 7 ? IB + 1 : 7)>(u0, u1, t, h0, h1, tabc, a0, a1, da, db);          \
-            _Pragma("unroll") for (int i = 0; i < CH; i++) {                                                                      \
-                acc[c + i][0] = fmaf(ea, q[i][0], acc[c + i][0]);                                                                 \
-                acc[c + i][1] = fmaf(ea, q[i][1], acc[c + i][1]);                                                                 \
-                acc[c + i][2] = fmaf(eb, q[i][2], acc[c + i][2]);                                                                 \
-                acc[c + i][3] = fmaf(eb, q[i][3], acc[c + i][3]);                                                                 \
+            _Pragma("unroll") for (int m = 0; m < RT; m++) {                                                                      \
+                float q[CH][4];                                                                                                   \
+                _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a0[m], xv[i].x, xv[i].y, zr.z);                      \
+                _Pragma("unroll") for (int i = 0; i < CH; i++) mma_f16(q[i], a1[m], xv[i].z, xv[i].w, q[i]);                      \
+                if (IB < 7 && c + CH == CT)                                                                                       \
+                    wide_decode<GF, (IB < 7 ? IB + 1 : 7)>(u0 + m * 16 * C::PITCH, u1 + m * 16 * C::PITCH, t, h0[m], h1[m], tabc, a0[m], a1[m], da[m], db[m]); \
+                _Pragma("unroll") for (int i = 0; i < CH; i++) {                                                                  \
+                    acc[m][c + i][0] = fmaf(ea[m], q[i][0], acc[m][c + i][0]);                                                    \
+                    acc[m][c + i][1] = fmaf(ea[m], q[i][1], acc[m][c + i][1]);                                                    \
+                    acc[m][c + i][2] = fmaf(eb[m], q[i][2], acc[m][c + i][2]);                                                    \
+                    acc[m][c + i][3] = fmaf(eb[m], q[i][3], acc[m][c + i][3]);                                                    \
+                }                                                                                                                 \
             }                                                                                                                     \
         }                                                                                                                         \
     }
                 WIDE_SUB(0) WIDE_SUB(1) WIDE_SUB(2) WIDE_SUB(3) WIDE_SUB(4) WIDE_SUB(5) WIDE_SUB(6) WIDE_SUB(7)
 #undef WIDE_SUB
 #pragma unroll
-                for (int i = 0; i < CT; i++)
+                for (int i = 0; i < RT * CT; i++)
 #pragma unroll
-                    for (int k = 0; k < 4; k++) tot[i][k] += acc[i][k];
+                    for (int k = 0; k < 4; k++) tot[i / CT][i % CT][k] += acc[i / CT][i % CT][k];
             }
             __syncwarp();
             if (lane == 0) {
@@ -670,37 +681,41 @@ __global__ void __launch_bounds__((TS * WideCfg<GF, TS>::RG + 1) * 32, 1) qmv_wi
             if (u % UPW == UPW - 1) jw++;
         }
         if (!ok || r >= n) continue;
-        const uint32_t row = (t0 + lo + r) * 16 + g;
 #pragma unroll
-        for (int i = 0; i < CT; i++)
+        for (int m = 0; m < RT; m++) {
+            if (RT > 1 && r + m >= n) break;
+            const uint32_t row = (t0 + lo + r + m) * 16 + g;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t col = c0 + (TS * i + th) * 8 + t + 4 * (k & 1), rw = row + 8 * (k >> 1);
-                if (col >= p.nb) continue;
-                if (F32OUT) ((float *)p.y)[(size_t)col * p.ystride + rw] = tot[i][k];
-                else ((__half *)p.y)[(size_t)col * p.ystride + rw] = __float2half_rn(tot[i][k]);
-            }
+            for (int i = 0; i < CT; i++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t col = c0 + (TS * i + th) * 8 + t + 4 * (k & 1), rw = row + 8 * (k >> 1);
+                    if (col >= p.nb) continue;
+                    if (F32OUT) ((float *)p.y)[(size_t)col * p.ystride + rw] = tot[m][i][k];
+                    else ((__half *)p.y)[(size_t)col * p.ystride + rw] = __float2half_rn(tot[m][i][k]);
+                }
+        }
     }
     if (!ok && lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 13);
 }
 
-template <int GF, bool F32OUT, int TS, int UNITS>
+template <int GF, bool F32OUT, int TS, int UNITS, int RT = 1>
 static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t groups, uint32_t bpg, uint32_t per, cudaStream_t st) {
-    using C = WideCfg<GF, TS>;
+    using C = WideCfg<GF, TS, RT>;
     CUtensorMap mw, mx;
     constexpr int B = 2 / TS;  // column tiles per 16 tokens of a warp
     const int n = p.nb <= 32 ? 2 : p.nb <= 48 ? 3 : 4, ct = n * B;
-    const bool mok = GF == 21 ? tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, p.rb, p.N, p.rb, 240, 16, CU_TENSOR_MAP_SWIZZLE_NONE)
+    const bool mok = GF == 21 ? tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, p.rb, p.N, p.rb, C::PITCH, 16, CU_TENSOR_MAP_SWIZZLE_NONE)
                               : tmap_2d(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT16, p.W, p.rb / 2, p.N, p.rb, 136, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (!mok || !tmap_2d(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x, p.K, p.nb, (uint64_t)p.xstride * 2, 64, 16 * n, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
-    auto k = n == 2 ? qmv_wide_k<GF, F32OUT, TS, 2 * B, UNITS> : n == 3 ? qmv_wide_k<GF, F32OUT, TS, 3 * B, UNITS> : qmv_wide_k<GF, F32OUT, TS, 4 * B, UNITS>;
+    auto k = n == 2 ? qmv_wide_k<GF, F32OUT, TS, 2 * B, UNITS, RT> : n == 3 ? qmv_wide_k<GF, F32OUT, TS, 3 * B, UNITS, RT> : qmv_wide_k<GF, F32OUT, TS, 4 * B, UNITS, RT>;
     const size_t smem = C::smem(ct);
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     // as many row tiles per round as split the block's tiles into equal rounds of at most RG
-    const uint32_t rounds = (per + C::RG - 1) / C::RG, rg = (per + rounds - 1) / rounds;
-    qw_launch(k, groups * bpg, (TS * rg + 1) * 32, smem, st, mw, mx, p, rg, bpg);
+    const uint32_t rounds = (per + C::RG - 1) / C::RG, rg = ((per + rounds - 1) / rounds + RT - 1) / RT * RT;
+    qw_launch(k, groups * bpg, (TS * rg / RT + 1) * 32, smem, st, mw, mx, p, rg, bpg);
     return cudaGetLastError();
 }
 template <int GF, bool F32OUT, int UNITS = 8>
@@ -708,6 +723,13 @@ static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
     // one block per SM, shared evenly by the groups of 64 tokens
     const uint32_t groups = (p.nb + 63) / 64, most = (uint32_t)sm_count / groups > 0 ? (uint32_t)sm_count / groups : 1, bpg = p.items < most ? p.items : most;
     const uint32_t per = (p.items + bpg - 1) / bpg;
+    if constexpr (GF == 21) {
+        // Two row tiles per warp where that halves the rounds, or nearly: a round of 14 tiles takes 1.86 times one of 7 (12352 x 2048, 419 tokens: 3 x 36.6 against
+        // 6 x 19.7 us).  Prompts of 419, 600 and 1024 tokens, 12 layers, on a B200: 6.81 -> 6.71, 8.92 -> 8.74 and 13.56 -> 13.49 ms; where the rounds do not
+        // come down so far (200 and 512 tokens) pairs throughout were 1 to 1.5 % slower.
+        const uint32_t one = (per + 6) / 7, two = (per + 13) / 14;
+        if (groups > 2 && 13 * two <= 7 * one) return qmv_wide_ts<GF, F32OUT, 1, UNITS, 2>(p, groups, bpg, per, st);
+    }
     if (GF == 8 ? per >= 16 : groups > 2) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
     return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }

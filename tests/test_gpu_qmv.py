@@ -146,6 +146,21 @@ def test_matvec_of_a_prompt_piece_equals_groups_of_64(gpu, N, K, B):
             run(kern, rows)
 
 
+# Two row tiles per warp (on 148 SMs): rounds of 8 and of 14 tiles, of 13 (one warp has a single tile), of 12 and 13 in turn, and the last tile count before pairs
+@pytest.mark.parametrize("tiles,K,B", [(168, 2048, 419), (294, 2048, 419), (273, 4096, 419), (772, 2048, 448), (147, 2048, 419), (49 * 13 - 1, 2048, 130)])
+def test_matvec_of_a_piece_with_pairs_of_row_tiles(gpu, tiles, K, B):
+    rng = np.random.default_rng(tiles)
+    N = 16 * tiles
+    W = synth.iq3s_rows(rng, N, K)
+    x = synth.acts_fp16(rng, B, K)
+    k = gpu.compile("qmv_mma", "qmv_piece32_%d" % K, GF=21, KD=K, ROWS=512, YT_F32=1)
+    wb, xb, yb = gpu.buf_from(W), gpu.buf_from(x), gpu.buf(B * N * 4).zero()
+    gpu.batch().kernel(k).buf(0, wb).buf(3, xb).buf(4, yb).bytes(5, np.array([N, K, N, B], np.uint32)).dispatch(((N + 7) // 8,), (256,)).end()
+    y = yb.download(np.float32, B * N).reshape(B, N)
+    for r in range(0, B, 64):  # each group of 64 the bits of a launch of its own
+        assert np.array_equal(bits(y[r:r + 64]), bits(run_qmv(gpu, "qmv_mma", 21, W, K, x[r:r + 64]))), r
+
+
 # Around the row-tile counts (on 148 SMs) where 17 to 21, 22 to 42 and more tokens change from one form to the other.
 @pytest.mark.parametrize("qtype", [21, 8])
 @pytest.mark.parametrize("tiles", [166, 167, 314, 315, 610, 611])
