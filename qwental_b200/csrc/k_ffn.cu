@@ -733,10 +733,10 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
 // expert's full items lie apart in the list.
 // Prompts of 65, 164, 419, 1024 tokens, 12 layers, ms, with gate/up 6 : 1 and down 5 : 2 as with one row tile per warp: 3.21, 4.46, 6.70, 13.47; 3 : 1 and 5 : 4 (here): 3.12, 4.33,
 // 6.61, 13.43; 2 : 1 and 1 : 1: 3.09, 4.30, 6.62, 13.48; 1 : 1 and 1 : 2: 3.10, 4.35, 6.77, 13.66.  The combine + norm that follows waits for the whole launch, so no output row is counted in.
-// One layer on a B200, items of eight columns in moe_ffn_k / one row tile per warp / two: 419 tokens 372 / 328 / 297 us.  Prompts, 12 layers, one row tile / two: 200
+// One layer on a B200, items of eight columns in moe_ffn_k / one row tile per warp / two: 419 tokens 372 / 328 / 297 us, 287 with the shares below.  Prompts, 12 layers, one row tile / two: 200
 // tokens 5.07 -> 4.78 ms, 419 7.20 -> 6.83, 512 8.26 -> 7.79, 1024 14.32 -> 13.59.  Bound by the decode still (all 513 experts are 857 MB, 131 us).
 // Items of 24 columns leave room for three stages: with one row tile per warp 13.67 ms at 1024 tokens, with two (276 bytes of spills) 14.06; 32 columns leave
-// two.  Short prompts on moe_ffn_k's eight columns and two blocks per SM: 65 tokens 3.26 against 3.23 to 3.34 ms here, 100 3.59 / 3.66, 128 4.02 / 3.97.
+// two.  Short prompts on moe_ffn_k's eight columns and two blocks per SM: 65 tokens 3.26 against 3.12 ms here, 100 3.59 / 3.50.
 constexpr int WFFN_RECS = 24;  // items a block's share can touch: at most 17 with 148 blocks, 1024 tokens and 15 choices each
 struct WffnCost {  // of a gate/up piece and of a down piece: a decode of the stage, and the MMAs and the epilogue of a column tile
     uint32_t dec, tile;
