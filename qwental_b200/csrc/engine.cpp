@@ -452,7 +452,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
             {&e->gy, RB * e->KG * 2}, {&e->qb, RB * c.qh * c.hd * 2}, {&e->ya, RB * e->KA * 2}, {&e->ob, RB * e->D * 2}, {&e->mo, B * e->D * 2}, {&e->ids, B * 4},
             {&e->mlog, RB * (e->E + 1) * 4}, {&e->msel, (size_t)e->L * e->sel_bytes}, {&e->Hhi, B * (e->TOPK + 1) * e->I * 2},
             {&e->Hlo, B * (e->TOPK + 1) * e->I * 2}, {&e->Pg, RB * (e->TOPK + 1) * e->D * 4}, {&e->rcnt, 256},
-            {&e->ffn_scr, e->ffn_fused ? MOE_FFN_SCRATCH_BYTES(e->I) : 0}, {&e->ctl_p, wide ? 3 * PROWS * 4 : 0}, {&e->ffn_scr_w, wide ? MOE_FFN_SCRATCH_BYTES_WIDE(e->I) : 0}};
+            {&e->ffn_scr, e->ffn_fused ? MOE_FFN_SCRATCH_BYTES(e->I) : 0}, {&e->ctl_p, wide ? 3 * PROWS * 4 : 0}, {&e->ffn_scr_w, wide ? MOE_FFN_SCRATCH_BYTES_WIDE(e->I, RB) : 0}};
         // Buffers of a megabyte and more begin at 2 MB boundaries, as if allocated one by one; the others follow, packed.  (All packed, a step of 16
         // slots takes 0.6 % longer.)  256 spare bytes behind each, see qw_buf_new_kind.
         size_t at[std::size(cut)], total = 0;

@@ -71,7 +71,7 @@ struct FfnP {
     const void *ms;           // moe_sel, or moe_sel_wide
     const QwTables *tab;
     unsigned *status;
-    uint32_t ebase;
+    uint32_t ebase, rows;     // rows: a piece's tokens that H and Pg have room for
     unsigned *sync;           // [0 .. MAXITEMS) per-item counters of finished gate/up warps, [MAXITEMS] finished blocks; all zero between launches
     __half *H;                // [item][2][8][I]
     float *PgR[8];            // expert-parallel exchange: Pg of every rank (see moe_dn in k_moe.cu)
@@ -811,7 +811,7 @@ __device__ __forceinline__ void xw_tiles(uint32_t nt, uint32_t rec0, uint32_t re
 }
 
 // item -> its columns.  prw = items before a group (of the selection record, in shared memory)
-__device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_wide *ms, uint32_t U, uint32_t nb, uint32_t w) {
+__device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_wide *ms, uint32_t U, uint32_t nb, uint32_t ebase, uint32_t w) {
     FfnItem it{};
     const uint32_t routed = prw[U];
     uint32_t cnt;
@@ -830,7 +830,7 @@ __device__ __forceinline__ FfnItem wffn_item(const uint32_t *prw, const moe_sel_
         it.e0 = ms->off[lo];
         cnt = ms->off[lo + 1] - it.e0;
         it.c0 = (w - prw[lo]) * WFFN_COLS;
-        it.erow = ms->ue[lo];
+        it.erow = ms->ue[lo] - ebase;
     }
     it.ncols = cnt - it.c0 < WFFN_COLS ? cnt - it.c0 : WFFN_COLS;
     return it;
@@ -886,7 +886,8 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     const uint32_t U = ms->U, nb = ms->nb, topk = ms->topk;
     __syncthreads();
     uint32_t items = prw[U] + (p.Sd ? (nb + WFFN_COLS - 1) / WFFN_COLS : 0);
-    const bool bad = items > MOE_FFN_MAXITEMS_WIDE;  // cannot happen with E <= 512 and MOE_MAXB_WIDE tokens; never index past the counters
+    // items: cannot happen with E <= 512 and MOE_MAXB_WIDE tokens; never index past the counters.  Tokens: the record may hold more than the buffers have room for
+    const bool bad = items > MOE_FFN_MAXITEMS_WIDE || nb > p.rows;
     if (bad && tid == 0) set_status(p.status, ST_BAD_ARG | 5);
     if (bad) items = 0;
     if (tid < 4) edge[tid] = bad ? 0 : wffn_edge(pre, prw, U, nb, p.Sd != nullptr, blockIdx.x + (tid & 1), gridDim.x, tid < 2 ? GT : DT, tid < 2 ? WFFN_GU : WFFN_DN);
@@ -901,7 +902,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     if (tid < 2 * WFFN_RECS) {
         const uint32_t k = tid % WFFN_RECS, w = (tid < WFFN_RECS ? wa0 : wb0) + k;
         const bool need = tid < WFFN_RECS ? (a_hi > a_lo && w <= (a_hi - 1) / GT) : (b_hi > b_lo && w <= (b_hi - 1) / DT);
-        if (need) recs[tid] = wffn_item(prw, ms, U, nb, w);
+        if (need) recs[tid] = wffn_item(prw, ms, U, nb, p.ebase, w);
     }
     __syncthreads();
     const FfnItem *rec_a = recs - wa0, *rec_b = recs + WFFN_RECS - wb0;  // rec_a[w], rec_b[w]
@@ -1164,6 +1165,8 @@ const CUtensorMap *ffn_tensor_map(const void *base, uint64_t pitch, uint64_t row
 // With IQ3X defined 1 the weights are the re-coded form of iq3x.cuh (made by iq3x_pack): 0 = routed gate + up
 // [EL][I/64][D/512] stages, 2 = the shared expert's, 6 = routed down [EL][D/128][I/512] stages, 7 = the shared expert's;
 // binds 1 and 3 are not used.
+// With WIDE defined 1 (IQ3X; a piece of a prompt, moe_ffn_wide_k) 5 is a moe_sel_wide; 8 (MOE_FFN_SCRATCH_BYTES_WIDE) and 9 have room for 1024
+// tokens, or for 512 and pieces of no more.
 static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     FfnP p{};
     const uint32_t E = (uint32_t)L.def("E", 512), topk = (uint32_t)L.def("TOPK", 10);
@@ -1184,10 +1187,14 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     p.Wd = L.buf<uint8_t>(6);
     p.Wg = Wg;
     p.Sg = Sg;
-    // WIDE defined 1: a piece of a prompt (moe_ffn_wide_k) -- bind 5 is a moe_sel_wide, 8 the wide scratch, Pg has MOE_MAXB_WIDE rows of tokens; one GPU only
     const bool wide = L.def("WIDE", 0) != 0;
+    auto room = [&](uint32_t r) {
+        return L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I, r) : MOE_FFN_SCRATCH_BYTES(I)) && L.avail(9) >= (size_t)r * (topk + 1) * D * 4;
+    };
+    p.rows = !wide ? MOE_MAXB : room(MOE_MAXB_WIDE) ? MOE_MAXB_WIDE : MOE_MAXB_WIDE / 2;
+    const uint32_t nb = L.has_bytes(13, 4) ? L.bytes<uint32_t>(13) : 0;
     p.sync = L.buf<unsigned>(8);
-    QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && L.avail(8) >= (wide ? MOE_FFN_SCRATCH_BYTES_WIDE(I) : MOE_FFN_SCRATCH_BYTES(I)));
+    QW_CHECK_ARG(p.sync && ((uintptr_t)p.sync & 15) == 0 && room(p.rows) && (!wide || nb <= p.rows));
     QW_CHECK_ARG(!wide || (x4 && L.def("EPX", 0) <= 1 && L.def("PROBE", 0) == 0));
     p.H = (__half *)((uint8_t *)p.sync + (wide ? MOE_FFN_SYNC_BYTES_WIDE : MOE_FFN_SYNC_BYTES));
     p.Sd = shared ? L.buf<uint8_t>(7) : nullptr;
@@ -1206,7 +1213,7 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
         QW_CHECK_ARG(L.avail(0) >= wsz && L.avail(1) >= wsz && L.avail(6) >= wsz && (!shared || (L.avail(2) >= ssz && L.avail(3) >= ssz && L.avail(7) >= ssz)));
     }
     QW_CHECK_ARG((((uintptr_t)Wg | (uintptr_t)Wu | (uintptr_t)p.Wd | (uintptr_t)Sg | (uintptr_t)Su | (uintptr_t)p.Sd | (uintptr_t)p.x) & 15) == 0);
-    QW_CHECK_ARG(L.avail(9) >= (size_t)(wide ? MOE_MAXB_WIDE : MOE_MAXB) * (topk + 1) * D * 4 && L.avail(4) >= (size_t)D * 2);
+    QW_CHECK_ARG(L.avail(4) >= (size_t)D * 2);
     p.ep = EpPeers{};
     p.ep.nranks = 1;
     if (L.def("EPX", 0) > 1) {
@@ -1236,11 +1243,10 @@ static cudaError_t launch_moe_ffn(const QwLaunch &L) {
     // 19 on 148 SMs.  Beyond that some blocks run two, and the variant itself costs 1 to 2 %.  Step time with whole pieces over step time with half
     // pieces on a B200 (items): 512 experts, top-10, 1 to 4 slots 1.057 (11), 0.994 (20.8), 0.986 (30), 0.997 (39); 32 experts, top-4, 5 to 8 slots
     // 1.038 (17), 1.015 (18.8), 0.999 (20.2), 0.990 (21.5); 256 experts, top-2, 8 and 10 slots 1.044 (16.5), 0.986 (21).
-    const uint32_t nb = L.has_bytes(13, 4) ? L.bytes<uint32_t>(13) : 0, grid = (uint32_t)(L.sm_count * per_sm);
+    const uint32_t grid = (uint32_t)(L.sm_count * per_sm);
     const double items = E * (1 - pow(1 - (double)topk / E, (double)nb)) + (nb + 7) / 8;
     const bool half = x4 && !wide && !probe && p.ep.nranks == 1 && nb >= 1 && 2 * items * (I / 64) <= grid * (33.0 / 32);
     if (wide) {
-        QW_CHECK_ARG(EL == E && p.ebase == 0);
         cudaError_t e = cudaFuncSetAttribute(moe_ffn_wide_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WFFN_SMEM);
         if (e != cudaSuccess) return e;
         int occ = 0;  // the blocks wait for one another's H

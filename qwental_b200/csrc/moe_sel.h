@@ -40,9 +40,9 @@ struct moe_sel_wide : moe_sel_t<MOE_MAXB_WIDE> {
 #define MOE_FFN_ROWCNT 1024
 #define MOE_FFN_ROW_DONE(D) ((D) / 128 * 8)
 #define MOE_FFN_SCRATCH_BYTES(I) ((size_t)MOE_FFN_SYNC_BYTES + (size_t)MOE_FFN_MAXITEMS * 16 * (I) * 2)
-// The same for a piece of a prompt, in a buffer of its own.  An item has up to MOE_FFN_COLS_WIDE columns.  H is [entry, then the shared expert's
-// tokens][2 planes][I].  No output row is counted in.
+// The same for a piece of a prompt of up to ROWS tokens, in a buffer of its own.  An item has up to MOE_FFN_COLS_WIDE columns.  H is [entry, then the
+// shared expert's tokens][2 planes][I].  No output row is counted in.
 #define MOE_FFN_COLS_WIDE 16
 #define MOE_FFN_MAXITEMS_WIDE (512 + MOE_MAXB_WIDE * MOE_MAXK / MOE_FFN_COLS_WIDE)
 #define MOE_FFN_SYNC_BYTES_WIDE 8192
-#define MOE_FFN_SCRATCH_BYTES_WIDE(I) ((size_t)MOE_FFN_SYNC_BYTES_WIDE + (size_t)MOE_MAXB_WIDE * MOE_MAXK * 2 * (I) * 2)
+#define MOE_FFN_SCRATCH_BYTES_WIDE(I, ROWS) ((size_t)MOE_FFN_SYNC_BYTES_WIDE + (size_t)(ROWS) * MOE_MAXK * 2 * (I) * 2)

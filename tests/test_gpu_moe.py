@@ -224,3 +224,69 @@ def test_half_pieces_of_few_items_give_the_same_rows(gpu, topk, edge):
     assert np.array_equal(few.view(np.uint16), whole[:edge].view(np.uint16))
     ref, _, _ = orc.moe_ref(x, h["Wr"], h["wsg"], h["gate"], h["up"], h["down"], h["sg"], h["su"], h["sd"], D, I, topk, ids=ids)
     assert np.abs(few.astype(np.float64) - ref[:edge]).max() < 2e-3 * np.abs(ref).max()  # the bound of the layer test above
+
+
+def wide_ffn(gpu, h, x, E, topk, lo=0, hi=None, rows=1024, say=True):
+    """Pg [tokens][topk + 1][D] and the chosen experts of a prompt's piece: logits, top-k, grouping and the one-launch FFN on records of their own, with
+    the weights of experts [lo, hi) alone.  rows = tokens that Pg and the scratch have room for; say: the launcher is told the number of tokens"""
+    import ctypes as C
+    from qwental_b200.layers import iq3x_pack, u32
+    D, I, nb, hi = 2048, 512, len(x), E if hi is None else hi
+    gpu.L.qw_moe_sel_wide_bytes.restype = C.c_size_t
+    d = dict(E=E, EL=hi - lo, D=D, I=I, TOPK=topk, SHARED=1, WIDE=1, IQ3X=1, SELECT=0)
+    k = {f: gpu.compile(f, "t_%s_%d_%d_%d" % (f, E, topk, lo), **d) for f in ("moe_route", "moe_topk_wide", "moe_group_wide", "moe_ffn")}
+    up = lambda a: gpu.buf_from(a)
+    gu, dn = iq3x_pack(gpu, up(h["gate"][lo:hi]), up(h["up"][lo:hi]), up(h["down"][lo:hi]), hi - lo, D, I)
+    sgu, sdn = iq3x_pack(gpu, up(h["sg"]), up(h["su"]), up(h["sd"]), 1, D, I)
+    sel, lg, xb = gpu.buf(gpu.L.qw_moe_sel_wide_bytes()).zero(), gpu.buf(nb * (E + 1) * 4), up(x)
+    Wr, wsg = up(h["Wr"]), up(h["wsg"])
+    scr, Pg = gpu.buf(8192 + rows * 16 * 2 * I * 2).zero(), gpu.buf(rows * (topk + 1) * D * 4).zero()
+    b = gpu.batch()
+    b.kernel(k["moe_route"]).buf(0, Wr).buf(1, wsg).buf(2, xb).buf(3, lg).bytes(14, u32(nb, lo, hi)).dispatch((1,), (1024,))
+    b.kernel(k["moe_topk_wide"]).buf(0, lg).buf(1, sel).bytes(2, u32(nb, lo, hi)).dispatch((1,), (128,))
+    b.kernel(k["moe_group_wide"]).buf(1, sel).bytes(2, u32(nb, lo, hi)).dispatch((1,), (512,))
+    b.kernel(k["moe_ffn"]).buf(0, gu).buf(2, sgu).buf(4, xb).buf(5, sel).buf(6, dn).buf(7, sdn).buf(8, scr).buf(9, Pg).bytes(10, u32(lo))
+    if say:
+        b.bytes(13, u32(nb))
+    b.dispatch((1,), (256,)).end()
+    ids, _ = orc.topk(lg.download(np.float32, nb * (E + 1)).reshape(nb, E + 1)[:, :E], topk)
+    return Pg.download(np.float32, nb * (topk + 1) * D).reshape(nb, topk + 1, D), ids
+
+
+def test_wide_ffn_of_a_range_of_experts(gpu):
+    """The expert FFN of a piece on a slice of the experts writes the rows of those experts (and the shared one's) and no others; the slices' rows together are
+    the step kernel's, bit for bit."""
+    E, topk, B = 64, 10, 150
+    layer, h, _ = make_layer(gpu, E, 2048, 512, topk, seed=6, ffn="iq3x")
+    x = synth.acts_fp16(np.random.default_rng(12), B, 2048)
+    want = []
+    for t in range(0, B, 64):
+        run_layer(gpu, layer, x[t:t + 64])
+        n = len(x[t:t + 64])
+        want.append(layer.Pg.download(np.float32, n * (topk + 1) * 2048).reshape(n, topk + 1, 2048))
+    want = np.concatenate(want)
+    whole, ids = wide_ffn(gpu, h, x, E, topk)
+    assert np.array_equal(whole.view(np.uint32), want.view(np.uint32))
+    for lo, hi in ((0, 32), (32, 64)):
+        part, _ = wide_ffn(gpu, h, x, E, topk, lo, hi)
+        mine = (ids >= lo) & (ids < hi)
+        assert np.all(part[:, :topk][~mine] == 0)
+        assert np.array_equal(part[:, :topk][mine].view(np.uint32), want[:, :topk][mine].view(np.uint32))
+        assert np.array_equal(part[:, topk].view(np.uint32), want[:, topk].view(np.uint32))
+
+
+def test_wide_ffn_with_room_for_half_a_piece(gpu):
+    """Pg and scratch for 512 tokens do for pieces of up to 512; more are refused, by the launcher or (where it is not told their number) by the kernel."""
+    from qwental_b200.gpu import GpuError
+    E, topk = 64, 2
+    _, h, _ = make_layer(gpu, E, 2048, 512, topk, seed=7, ffn="iq3x")
+    x = synth.acts_fp16(np.random.default_rng(3), 513, 2048)
+    want, _ = wide_ffn(gpu, h, x, E, topk)
+    for say in (True, False):
+        got, _ = wide_ffn(gpu, h, x[:512], E, topk, rows=512, say=say)
+        assert np.array_equal(got.view(np.uint32), want[:512].view(np.uint32))
+    for say in (True, False):
+        with pytest.raises(GpuError):
+            wide_ffn(gpu, h, x, E, topk, rows=513, say=say)
+    with pytest.raises(GpuError):
+        wide_ffn(gpu, h, x[:100], E, topk, rows=511)
