@@ -35,8 +35,8 @@ namespace {
 
 constexpr int PAGE = 256;
 constexpr int ROWS = QW_PAR_MAX;      // rows of the control block of a step
-constexpr int PART_WIDE = 2048;       // (row, page) partials of the attention over a prompt's piece that have room at once, at least: 34 MB
 constexpr int PROWS = MOE_MAXB_WIDE;  // ... and of a piece of a prompt: its tokens
+constexpr int PART_WIDE = 2048;       // (row, page) partials of attention that have room at once with pieces of PROWS tokens, at least: 34 MB
 std::string g_open_error;
 
 struct Slot {
@@ -100,7 +100,7 @@ struct qw_engine {
     qw_buf prompt_d{};  // par_prefill: the prompt's token ids
     // Pieces of more than 64 tokens: one GPU with the one-launch expert FFN on IQ3X.  Eight times the tokens choose far fewer than eight times the
     // experts, so a wider piece reads and decodes fewer expert weights per token.
-    int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it
+    int piece_rows = ROWS;  // the most tokens of a piece: PROWS where the shapes allow it, half of them or ROWS where its rows' memory is not there
     qw_buf ctl_p{}, ffn_scr_w{};
     qw_kernel *k_embed_w = nullptr, *k_norm0_w = nullptr, *k_norm_w = nullptr, *k_norm_cmb_w = nullptr, *k_logits_w = nullptr, *k_topk_w = nullptr,
               *k_group_w = nullptr, *k_ffn_w = nullptr, *k_qmv_in_w = nullptr, *k_qmv_oa_w = nullptr, *k_qmv_og_w = nullptr, *k_prep_w = nullptr,
@@ -437,11 +437,28 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
          new_buf(e, &e->shu, (size_t)e->L * gu_bytes) && new_buf(e, &e->shd, (size_t)e->L * gu_bytes) &&
          new_buf(e, &e->kvpool, (size_t)kvp * page_bytes) && new_buf(e, &e->ptab, (size_t)c.max_slots * e->max_pages * 4) &&
          new_buf(e, &e->sstate, (size_t)c.max_slots * ng * c.hv * 128 * 128 * 4) && new_buf(e, &e->cstate, (size_t)c.max_slots * ng * 3 * e->C * 4) &&
-         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->part, std::max(B * (size_t)e->max_pages, e->k_attn_w ? (size_t)PART_WIDE : 0) * c.qh * (c.hd + 2) * 4) &&
-         new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids_h, 2 * B * 4, QW_BUF_HOSTIO) && new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) &&
-         new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO);
-    // The rest of the scratch memory in one allocation.  With wide pieces it is some 100 MB more; where they are not to be had, prompts run in
-    // pieces of 64 tokens instead.
+         new_buf(e, &e->ctl_h, 3 * ROWS * 4, QW_BUF_HOSTIO) && new_buf(e, &e->logits, B * (size_t)e->V * 4) && new_buf(e, &e->ids_h, 2 * B * 4, QW_BUF_HOSTIO) &&
+         new_buf(e, &e->cand_h, B * 256 * 8, QW_BUF_HOSTIO) && new_buf(e, &e->logits_h, (size_t)e->V * 4, QW_BUF_HOSTIO);
+    if (ok) ok = qw_buf_zero(g, &e->ptab, 0, e->ptab.size) && qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size);
+    if (ok && e->ffn_iq3x) {
+        e->x_gus = (size_t)(e->I / 64) * (e->D / 512) * 128 * 272;
+        e->x_dns = (size_t)(e->D / 128) * (e->I / 512) * 128 * 272;
+        ok = new_buf(e, &e->xq_gu, (size_t)e->L * e->EL * e->x_gus) && new_buf(e, &e->xq_d, (size_t)e->L * e->EL * e->x_dns) &&
+             new_buf(e, &e->xs_gu, (size_t)e->L * e->x_gus) && new_buf(e, &e->xs_d, (size_t)e->L * e->x_dns);
+    }
+    if (ok) ok = init_weights(e);
+    if (ok && e->ffn_iq3x) ok = pack_experts(e);
+    // The step reads only the re-coded experts from here on.  A model of real size gives the raw IQ3_S blocks back (33 GB at
+    // the benchmark shape: room for KV pages); small models keep them, so that tests can read the tensors they were built from.
+    if (ok && e->ffn_iq3x && (size_t)e->L * e->EL * 3 * gu_bytes > ((size_t)4 << 30)) {
+        qw_buf *raw[] = {&e->exg, &e->exu, &e->exd, &e->shg, &e->shu, &e->shd};
+        for (qw_buf *b : raw) {
+            qw_buf_free(b);
+            *b = qw_buf{};
+        }
+    }
+    // The rest of the scratch memory in one allocation, and attention's partials.  With pieces of 1024 tokens it is some 250 MB, with 512 half of that; it comes
+    // last, behind all that an engine cannot do without, and where it is not to be had, prompts run in pieces of 512 tokens or of 64 (20 MB).
     while (ok) {
         const size_t RB = (size_t)e->piece_rows;  // the most rows of a pass
         const bool wide = RB > ROWS;
@@ -462,9 +479,11 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
                 at[i] = total = align_up(total, big ? 2u << 20 : 256);
                 total += cut[i].second + 256;
             }
-        if (!new_buf(e, &e->scratch, total)) {
+        const size_t partials = std::max(B * (size_t)e->max_pages, RB == PROWS ? (size_t)PART_WIDE : 0) * c.qh * (c.hd + 2) * 4;
+        if (!new_buf(e, &e->part, partials) || !new_buf(e, &e->scratch, total)) {
+            qw_buf_free(&e->part);
             ok = wide;
-            e->piece_rows = ROWS;
+            e->piece_rows = RB == PROWS ? PROWS / 2 : ROWS;
             if (ok) e->err.clear();
             continue;
         }
@@ -472,24 +491,7 @@ extern "C" qw_engine *qw_engine_open_synth(qw_gpu *g, const qw_model_cfg *cfg) {
             if (cut[i].second) ok = ok && qw_buf_slice(&e->scratch, at[i], cut[i].second, cut[i].first);
         break;
     }
-    if (ok) ok = qw_buf_zero(g, &e->scratch, 0, e->scratch.size) && qw_buf_zero(g, &e->ptab, 0, e->ptab.size) && qw_buf_zero(g, &e->kvpool, 0, e->kvpool.size);
-    if (ok && e->ffn_iq3x) {
-        e->x_gus = (size_t)(e->I / 64) * (e->D / 512) * 128 * 272;
-        e->x_dns = (size_t)(e->D / 128) * (e->I / 512) * 128 * 272;
-        ok = new_buf(e, &e->xq_gu, (size_t)e->L * e->EL * e->x_gus) && new_buf(e, &e->xq_d, (size_t)e->L * e->EL * e->x_dns) &&
-             new_buf(e, &e->xs_gu, (size_t)e->L * e->x_gus) && new_buf(e, &e->xs_d, (size_t)e->L * e->x_dns);
-    }
-    if (ok) ok = init_weights(e);
-    if (ok && e->ffn_iq3x) ok = pack_experts(e);
-    // The step reads only the re-coded experts from here on.  A model of real size gives the raw IQ3_S blocks back (33 GB at
-    // the benchmark shape: room for KV pages); small models keep them, so that tests can read the tensors they were built from.
-    if (ok && e->ffn_iq3x && (size_t)e->L * e->EL * 3 * gu_bytes > ((size_t)4 << 30)) {
-        qw_buf *raw[] = {&e->exg, &e->exu, &e->exd, &e->shg, &e->shu, &e->shd};
-        for (qw_buf *b : raw) {
-            qw_buf_free(b);
-            *b = qw_buf{};
-        }
-    }
+    if (ok) ok = qw_buf_zero(g, &e->scratch, 0, e->scratch.size);
     if (!ok) {
         g_open_error = e->err.empty() ? "engine open failed" : e->err;
         qw_engine_close(e);

@@ -418,3 +418,46 @@ def test_replayed_steps_and_their_ids(gpu, start):
         gpu.L.qw_gpu_set_graphs(gpu.g, False)
         a.close()
         b.close()
+
+
+def test_engines_open_with_less_memory_for_prompts(gpu):
+    """What an engine cannot do without is allocated first, then the rows of a prompt's piece: 1024, or 512, or 64 where the memory is not there.  With ever less free
+    memory the same prompt runs in 1, 2 and 16 pieces, to the same logits, before the engine no longer opens; and that happens no sooner than 64 rows need."""
+    import torch
+    from qwental_b200.engine import Engine, wide_cfg
+    from qwental_b200.gpu import GpuError
+    MB = 1 << 20
+    free = lambda: torch.cuda.mem_get_info()[0]
+    text = np.random.default_rng(2).integers(0, 512, 1024).astype(np.int32)
+
+    def prompt():  # launches of the whole prompt, its logits, memory taken by the engine
+        before = free()
+        e = Engine(gpu, wide_cfg(max_slots=1))
+        try:
+            taken, n = before - free(), gpu.launches()
+            lg = e.prefill(0, text)
+            return gpu.launches() - n, lg, taken
+        finally:
+            e.close()
+
+    prompt()  # (loads the kernels: what that takes is not the engine's)
+    one, want, most = prompt()
+    seen, left, least = [], most + 8 * MB, None
+    while left > 0:
+        filler = gpu.buf(free() - left)
+        try:
+            n, lg, _ = prompt()
+        except GpuError as err:
+            assert "allocation of" in str(err)
+            break
+        finally:
+            filler.free()
+        assert np.array_equal(lg.view(np.uint32), want.view(np.uint32)), left // MB
+        if not seen or seen[-1] != n:
+            seen.append(n)
+        least = left
+        left -= 20 * MB
+    assert len(seen) == 3 and seen[0] == one and seen[1] < 3 * one and seen[2] > 10 * one, (one, seen)
+    # 64 rows instead of 1024: 39 MB less of Pg (topk + 1 = 5 rows of 2048 fp32 per token), 33 of the FFN's scratch, 24 of projections, 25 of attention's partials, and so on
+    assert most - least > 130 * MB, (most // MB, least // MB)
+
