@@ -108,7 +108,7 @@ struct qw_gpu {
         std::vector<uint64_t> key;
         unsigned long long ticket, launches;
         cudaStream_t stream;
-        std::string pdl_off;
+        int pdl;  // g_pdl at its capture: a switch of the process, so another device handle may have turned it since
     };
     std::unordered_map<uint64_t, GraphEnt> graph_cache;
     std::unordered_map<unsigned long long, GraphEnt *> tickets;
@@ -566,10 +566,6 @@ static uint64_t hash_words(const uint64_t *w, size_t n) {  // four chains, so th
     for (uint64_t c : h) r = (r ^ c) * 0x100000001B3ull;
     return r ^ (r >> 32);
 }
-static const char *pdl_off_env() {
-    const char *p = getenv("QW_PDL_OFF");
-    return p ? p : "";
-}
 static cudaError_t replay(qw_gpu *g, const qw_gpu::GraphEnt &e) {
     g->launches += e.launches;
     const cudaError_t r = cudaGraphLaunch(e.exec, e.stream);
@@ -683,7 +679,7 @@ extern "C" void qw_batch_submit(qw_batch *b) {
                 b->failed = true;
                 return;
             }
-            it = g->graph_cache.emplace(h, qw_gpu::GraphEnt{exec, std::move(key), ++g->last_ticket, b->recs.size(), b->stream, pdl_off_env()}).first;
+            it = g->graph_cache.emplace(h, qw_gpu::GraphEnt{exec, std::move(key), ++g->last_ticket, b->recs.size(), b->stream, g_pdl}).first;
             g->tickets[it->second.ticket] = &it->second;  // (entries do not move)
         }
         b->ticket = it->second.ticket;
@@ -697,7 +693,7 @@ extern "C" unsigned long long qw_batch_ticket(const qw_batch *b) { return b && b
 extern "C" qw_batch *qw_batch_replay(qw_gpu *g, unsigned long long ticket) {
     if (!g || !g->graphs || g->profile) return nullptr;
     const auto it = g->tickets.find(ticket);
-    if (it == g->tickets.end() || it->second->stream != g->stream[g->cur] || it->second->pdl_off != pdl_off_env()) return nullptr;
+    if (it == g->tickets.end() || it->second->stream != g->stream[g->cur] || it->second->pdl != g_pdl) return nullptr;
     cudaSetDevice(g->dev);
     qw_batch *b = new qw_batch();
     b->g = g;

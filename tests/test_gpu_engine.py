@@ -461,3 +461,79 @@ def test_engines_open_with_less_memory_for_prompts(gpu):
     # 64 rows instead of 1024: 39 MB less of Pg (topk + 1 = 5 rows of 2048 fp32 per token), 33 of the FFN's scratch, 24 of projections, 25 of attention's partials, and so on
     assert most - least > 130 * MB, (most // MB, least // MB)
 
+
+
+def ticket_calls(gpu):
+    import ctypes as C
+    L = gpu.L
+    L.qw_batch_ticket.restype, L.qw_batch_ticket.argtypes = C.c_ulonglong, [C.c_void_p]
+    L.qw_batch_replay.restype, L.qw_batch_replay.argtypes = C.c_void_p, [C.c_void_p, C.c_ulonglong]
+    L.qw_gpu_set_pdl.restype, L.qw_gpu_set_pdl.argtypes = None, [C.c_void_p, C.c_bool]
+    return L
+
+
+def test_tickets_are_void_where_the_batch_would_be_another(gpu, monkeypatch):
+    """A ticket replays its batch, and only while the recorded graph is what a new recording would give: not with graphs off, with profiling on, on another
+    stream, in another launch mode (set through any device handle: the mode is the process's), after a kernel was registered anew, or once the graphs were dropped for
+    others.  What is read from the environment once does not void it later."""
+    from qwental_b200.gpu import Gpu
+    L = ticket_calls(gpu)
+    k = gpu.compile("qw_fill", "ticket_fill")
+    buf = gpu.buf(1024)
+    n = 256
+
+    def fill(value, kind=5, keep=False):  # fills the buffer with a constant, then with its double
+        b = gpu.batch()
+        for v in (value, 2 * value):
+            a = np.zeros(1, np.dtype([("seed", "<u8"), ("n", "<u8"), ("base", "<u8"), ("mode", "<u4"), ("p0", "<f4"), ("p1", "<f4"), ("pad", "<u4")]))
+            a["n"], a["mode"], a["p0"] = n, kind, v
+            b.kernel(k).buf(0, buf).bytes(1, a).dispatch((1,), (256,))
+        L.qw_batch_submit(b.b)
+        t = L.qw_batch_ticket(b.b)
+        assert L.qw_batch_wait(b.b) >= 0
+        b.b = None
+        return t
+
+    def replays(t):
+        buf.zero()
+        b = L.qw_batch_replay(gpu.g, t)
+        if not b:
+            return False
+        assert L.qw_batch_wait(b) >= 0
+        assert np.all(buf.download(np.float32, n) == 6.0)
+        return True
+
+    assert fill(3.0) == 0  # graphs are off: no ticket
+    gpu.L.qw_gpu_set_graphs(gpu.g, True)
+    other = Gpu()
+    try:
+        t = fill(3.0)
+        assert t and replays(t) and replays(t) and not replays(t + 1) and not replays(0)
+        for off, on in ((lambda: L.qw_gpu_set_graphs(gpu.g, False), lambda: L.qw_gpu_set_graphs(gpu.g, True)),
+                        (lambda: L.qw_profile_enable(gpu.g, True), lambda: L.qw_profile_enable(gpu.g, False)),
+                        (lambda: L.qw_gpu_set_stream(gpu.g, 1), lambda: L.qw_gpu_set_stream(gpu.g, 0)),
+                        (lambda: L.qw_gpu_set_pdl(other.g, False), lambda: L.qw_gpu_set_pdl(other.g, True)),
+                        (lambda: L.qw_gpu_set_pdl(None, False), lambda: L.qw_gpu_set_pdl(None, True))):
+            off()
+            try:
+                assert not replays(t)
+            finally:
+                on()
+            assert replays(t)
+        monkeypatch.setenv("QW_PDL_OFF", "qw_fill")
+        assert replays(t) and fill(3.0) == t
+        L.qw_gpu_set_pdl(gpu.g, True)  # drops this device's graphs
+        assert not replays(t)
+        u = fill(3.0)
+        assert u and u != t and replays(u)
+        k = gpu.compile("qw_fill", "ticket_fill")
+        assert not replays(u)
+        u = fill(3.0)
+        for i in range(256):
+            assert replays(u)
+            fill(100.0 + i)
+        assert not replays(u) and fill(3.0) not in (0, t, u)
+    finally:
+        gpu.L.qw_gpu_set_graphs(gpu.g, False)
+        other.close()
+
