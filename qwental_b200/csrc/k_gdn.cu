@@ -354,10 +354,12 @@ __global__ void __launch_bounds__(256, 1) gdn_seq_k(const __half *cv, const floa
     const uint32_t slot = (uint32_t)sids[0];
     const bool runs = warp < 4;  // warps 0 .. 3 hold the state: rows 8 j + i and 8 (j + 8) + i of columns col and col + 1
     float *S = pool + (((size_t)slot * a.nlayers + a.layer) * HV + hv) * DK * DV + (size_t)(8 * j) * DV + col;
+    const bool pairs = ((uintptr_t)pool & 7) == 0;  // else the two columns one by one: the state is read and written once
+    auto get = [&](const float *p) { return pairs ? *(const float2 *)p : make_float2(p[0], p[1]); };
     f32x2 s0[8], s1[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const float2 x = runs ? *(const float2 *)(S + (size_t)i * DV) : make_float2(0.f, 0.f), y = runs ? *(const float2 *)(S + (size_t)(64 + i) * DV) : x;
+        const float2 x = runs ? get(S + (size_t)i * DV) : make_float2(0.f, 0.f), y = runs ? get(S + (size_t)(64 + i) * DV) : x;
         s0[i] = pair_of(x.x, y.x);
         s1[i] = pair_of(x.y, y.y);
     }
@@ -502,13 +504,20 @@ __global__ void __launch_bounds__(256, 1) gdn_seq_k(const __half *cv, const floa
         }
         __syncthreads();
     }
+    auto put_state = [&](float *p, float a0, float a1) {
+        if (pairs) *(float2 *)p = make_float2(a0, a1);
+        else {
+            p[0] = a0;
+            p[1] = a1;
+        }
+    };
     if (runs) {
         out_sums(nb);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const float2 x = halves_of(s0[i]), y = halves_of(s1[i]);
-            *(float2 *)(S + (size_t)i * DV) = make_float2(x.x, y.x);
-            *(float2 *)(S + (size_t)(64 + i) * DV) = make_float2(x.y, y.y);
+            put_state(S + (size_t)i * DV, x.x, y.x);
+            put_state(S + (size_t)(64 + i) * DV, x.y, y.y);
         }
     }
     __syncthreads();

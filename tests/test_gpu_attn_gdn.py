@@ -221,3 +221,29 @@ def test_what_lies_behind_a_slots_length_does_not_matter(gpu, family, lens):
         rest[:] = [np.inf, -np.inf, np.nan][r % 3]
     core.pool.upload(pool)
     assert np.array_equal(attn_run(gpu, core, d, range(len(lens))).view(np.uint16), clean.view(np.uint16))
+
+
+@pytest.mark.parametrize("shift", [4, 8])
+def test_recurrence_over_a_prompt_wherever_its_state_lies(gpu, shift):
+    """gdn_seq moves two columns of the state at a time where they lie at 8-byte boundaries, and one by one elsewhere: the same bits, and the floats around the
+    state are left alone."""
+    from qwental_b200.layers import u32
+    HK, HV, nb = 2, 4, 21
+    rng = np.random.default_rng(shift)
+    C = 2 * HK * 128 + HV * 128
+    k = gpu.compile("gdn_seq", "gdn_seq_shift", HK=HK, HV=HV, DK=128, DV=128, GDN_TILED=1)
+    cv, proj = (gpu.buf_from(rng.standard_normal((nb, C)).astype(np.float16)) for _ in range(2))
+    la, be = gpu.buf_from(-rng.random((nb, HV)).astype(np.float32)), gpu.buf_from(rng.random((nb, HV)).astype(np.float32))
+    S = (rng.standard_normal(HV * 128 * 128) * 0.1).astype(np.float32)
+    conv, sid, out = gpu.buf(3 * C * 4).zero(), gpu.buf_from(np.zeros(1, np.int32)), gpu.buf(nb * HV * 128 * 2)
+
+    def run(off):
+        pool = gpu.buf(S.nbytes + 16).zero().upload(S, off)
+        b = gpu.batch()
+        b.kernel(k).buf(0, cv).buf(1, la).buf(2, be).buf(3, pool, off).buf(4, proj).buf(5, conv).buf(6, out).buf(7, sid).bytes(8, u32(nb, 0, 1, C)).dispatch((4, HV), (256,)).end()
+        got = pool.download(np.uint32, S.size + 4)
+        assert not got[:off // 4].any() and not got[off // 4 + S.size:].any()
+        return got[off // 4:off // 4 + S.size], out.download(np.uint16, nb * HV * 128)
+
+    for a, b in zip(run(0), run(shift)):
+        assert np.array_equal(a, b)
