@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 1) qsa_attn_piece_k(const __gri
     bool ok = true;
 #pragma unroll 1
     for (uint32_t step = 0; step < steps; step++) {
-        if (warp == 0) {  // two steps ahead, into the stage that every warp has left by now or leaves soon
+        if (warp == 0) {  // three steps ahead, into the stage that every warp has left by now or leaves soon
             if (lane == 0 && step + AP_STG - 1 < steps) ok = put(step + AP_STG - 1);
             ok = __shfl_sync(0xffffffffu, (int)ok, 0);
         }
@@ -559,6 +559,9 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 1) qsa_attn_piece_k(const __gri
         ok = ok && mbar_wait(&full[st], (step / AP_STG) & 1);
         if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
+            // no block ends with copies of its own in flight: those that may be are waited for, with a limit again
+            if (threadIdx.x == 0)
+                for (uint32_t j = step; j < steps && j < step + AP_STG; j++) mbar_wait(&full[j % AP_STG], (j / AP_STG) & 1);
             break;
         }
         const bool on0 = step * 16 < n[0], on1 = step * 16 < n[1];  // (the same in all lanes)

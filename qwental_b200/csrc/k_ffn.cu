@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     const FfnItem *rec_a = recs - wa0, *rec_b = recs + WFFN_RECS - wb0;  // rec_a[w], rec_b[w]
 
     if (warp == FFN_CW) {
-        // ---- producer warp: lane 0 keeps the stages full; lane c fetches column c of a new item
+        // ---- producer warp: lane 0 keeps the stages full; lane c fetches column c of a new item.  After a wait that ran out it requests nothing more.
         bool ok = true;
         uint32_t j = 0, k = 0, rowbase = 0, prev_n = WFFN_COLS;
         auto stage = [&](const uint8_t *src) {
@@ -917,12 +917,12 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                 ok = false;
                 if (lane == 0) set_status(p.status, ST_MBAR_TIMEOUT | 6);
             }
-            if (lane == 0) {
+            if (lane == 0 && ok) {
                 fence_proxy_async();  // the consumers' reads of the stage are ordered before the copy engine's writes
                 mbar_expect_tx(&full[s], IQ3X_STAGE);
                 bulk_s(slot0 + s * IQ3X_STAGE, src, IQ3X_STAGE, &full[s]);
             }
-            j++;
+            j += ok ? 1 : 0;
         };
         // the ring of activation rows, as in moe_ffn_k: returns this lane's row for the item's column `lane`
         auto act_for = [&](uint32_t ncols, uint32_t bytes, bool fresh) {
@@ -935,8 +935,8 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
             }
             if (fresh) rowbase = 0;
             fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_expect_tx(&actfull[s], bytes);
+            ok = __all_sync(0xffffffffu, ok);
+            if (lane == 0 && ok) mbar_expect_tx(&actfull[s], bytes);
             __syncwarp();
             const uint32_t r0 = rowbase;
             rowbase = (rowbase + ncols) % WFFN_COLS;
@@ -955,8 +955,8 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                     uint32_t tok = 0, rank;
                     if ((uint32_t)lane < it.ncols) ffn_entry(ms, it, topk, lane, tok, rank);
                     const uint32_t row = act_for(it.ncols, it.ncols * D * 2, false);
-                    if ((uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_XP, p.x + (size_t)tok * D, D * 2, &actfull[k & 1]);
-                    k++;
+                    if (ok && (uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_XP, p.x + (size_t)tok * D, D * 2, &actfull[k & 1]);
+                    k += ok ? 1 : 0;
                 }
             }
         }
@@ -981,9 +981,13 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
                 asm volatile("fence.proxy.async.global;" ::: "memory");  // the H rows were written by ordinary stores; the copy engine reads them
                 const uint32_t row = act_for(it.ncols, it.ncols * I * 4, first_dn);
                 first_dn = false;
-                if ((uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_HP, p.H + (size_t)(it.e0 + it.c0 + lane) * 2 * I, I * 4, &actfull[k & 1]);
-                k++;
+                if (ok && (uint32_t)lane < it.ncols) bulk_s(act0 + row * WFFN_HP, p.H + (size_t)(it.e0 + it.c0 + lane) * 2 * I, I * 4, &actfull[k & 1]);
+                k += ok ? 1 : 0;
             }
+        }
+        if (lane == 0) {  // requested stages and items
+            edge[0] = j;
+            edge[1] = k;
         }
     } else {
         const int sh = warp >> 3, r = 2 * (warp & 3), kh = (warp >> 2) & 1, pr = sh * 4 + (warp & 3);  // stage of the two, first row tile, K half, pair of warps
@@ -1132,6 +1136,11 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     }
     // the last block to finish clears the items' counters for the next launch (every block has read what it needed by then)
     __syncthreads();
+    if (tid == FFN_CW * 32) {
+        // No block ends with copies of its own in flight: the last ones have landed by now, unless a wait for them ran out; then they are waited for again, with a limit.
+        for (uint32_t n = edge[0] > WFFN_STG ? edge[0] - WFFN_STG : 0; n < edge[0]; n++) mbar_wait(&full[n % WFFN_STG], (n / WFFN_STG) & 1);
+        for (uint32_t n = edge[1] > 2 ? edge[1] - 2 : 0; n < edge[1]; n++) mbar_wait(&actfull[n & 1], (n >> 1) & 1);
+    }
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(p.sync + MOE_FFN_MAXITEMS_WIDE, 1u) == gridDim.x - 1) {
