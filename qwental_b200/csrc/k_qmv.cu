@@ -480,10 +480,7 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
 // reduction across warps.  MMA column g of a tile holds token (g / 2) + 4 (g % 2), so that the eight lanes of a 16-byte shared load fall into
 // eight different chunks of the swizzle.
 // TS = warps that share a row tile.  2: the tiles of a block are few (a projection has 3 to 6 per SM) and the warps are what hides
-// latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S for three and more groups of 64 tokens, where a block has many tiles): a unit is decoded once for all
-// tokens, by fewer warps with more registers.  (12352 x 2048 IQ3_S, 419 tokens, TS 2 -> 1 on a B200: 121 -> 110 us; 2048 x 4096: 45 -> 42; prompts of 419
-// tokens, 48 layers, 37.5 -> 36.9 ms.  Two groups are better off with 2: prompts of 65, 100 and 128 tokens, 12 layers, 3.37 -> 3.26, 3.69 -> 3.61 and
-// 4.11 -> 4.03 ms.)
+// latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S by qmv_wide_form): a unit is decoded once for all tokens, by fewer warps with more registers.
 // RT = row tiles per warp.  2 (IQ3_S): the activations are read once for both; the weight stages are then one unit long (shared memory).
 // Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
 // IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
@@ -718,19 +715,32 @@ static cudaError_t qmv_wide_ts(const QmvMmaP &p, uint32_t groups, uint32_t bpg, 
     qw_launch(k, groups * bpg, (TS * rg / RT + 1) * 32, smem, st, mw, mx, p, rg, bpg);
     return cudaGetLastError();
 }
+// IQ3_S, more than 64 tokens: two warps per row tile (0), one (1), or one per pair of row tiles (2)?  What a block's `per` row tiles cost in each is rounds times the time of
+// a round, and that goes by the busiest of the SM's four schedulers: decode and MMAs of half the tokens of a tile, of a tile, or of two.  Tables: times of a round of 1 to 7 tiles
+// (0, 1; a warp idle in a shorter round frees no other scheduler), of up to 8 and of up to 14 tiles (2), in half microseconds at K = 2048.  Measured on a B200 (L2
+// flushed) with 1 to 32 tiles per block, 2 to 16 groups of 64 tokens, K = 2048 and 4096: the ratios depend on the tiles alone.  Time of 0 at K = 2048, us; ratios of 1 and 2 to it:
+//   tiles  0    1    2         tiles  0    1    2         tiles  0    1    2          tiles  0    1    2
+//     1   18  1.11 1.68         6    26  1.03 1.17         14   50  0.94 0.87          21   72  0.91 1.05
+//     3   22  1.01 1.40         7    30  0.95 1.10         15   59  1.08 0.96          24   79  1.06 0.97
+//     4   22  0.96 1.33         8    36  0.96 0.93         16   60  1.06 0.95          28   93  0.91 0.85
+//     5   26  1.06 1.20        12    44  1.05 0.99         18   61  1.06 1.23          30   95  1.07 1.16
+// With 1 for three and more groups, and 2 where the rounds nearly halve, whatever the tiles: 12352 x 2048, 129 to 192 tokens, 66 us, now 58 to 60; 9216 x 2048, 193 to
+// 256, 66 -> 60; 5120 x 2048, 385 to 448, 64 -> 57; 4800 x 4096, 385 to 448, 116 -> 102.  Prompts of 160, 192 and 1024 tokens, 12 layers: 4.30 -> 4.22, 4.51 -> 4.40 and 13.47 -> 13.32 ms.
+static int qmv_wide_form(uint32_t per) {
+    constexpr uint32_t T0[7] = {19, 20, 26, 27, 33, 34, 42}, T1[7] = {22, 23, 25, 25, 37, 37, 38};
+    const uint32_t r7 = (per + 6) / 7, t7 = (per + r7 - 1) / r7, r14 = (per + 13) / 14, t14 = (per + r14 - 1) / r14;
+    const uint32_t c0 = r7 * T0[t7 - 1], c1 = r7 * T1[t7 - 1], c2 = r14 * (t14 <= 8 ? 49 : 68);
+    return c2 <= c0 && c2 <= c1 ? 2 : c1 < c0 ? 1 : 0;
+}
 template <int GF, bool F32OUT, int UNITS = 8>
 static cudaError_t qmv_wide_go(const QmvMmaP &p, int sm_count, cudaStream_t st) {
     // one block per SM, shared evenly by the groups of 64 tokens
     const uint32_t groups = (p.nb + 63) / 64, most = (uint32_t)sm_count / groups > 0 ? (uint32_t)sm_count / groups : 1, bpg = p.items < most ? p.items : most;
     const uint32_t per = (p.items + bpg - 1) / bpg;
-    if constexpr (GF == 21) {
-        // Two row tiles per warp where that halves the rounds, or nearly: a round of 14 tiles takes 1.86 times one of 7 (12352 x 2048, 419 tokens: 3 x 36.6 against
-        // 6 x 19.7 us).  Prompts of 419, 600 and 1024 tokens, 12 layers, on a B200: 6.81 -> 6.71, 8.92 -> 8.74 and 13.56 -> 13.49 ms; where the rounds do not
-        // come down so far (200 and 512 tokens) pairs throughout were 1 to 1.5 % slower.
-        const uint32_t one = (per + 6) / 7, two = (per + 13) / 14;
-        if (groups > 2 && 13 * two <= 7 * one) return qmv_wide_ts<GF, F32OUT, 1, UNITS, 2>(p, groups, bpg, per, st);
-    }
-    if (GF == 8 ? per >= 16 : groups > 2) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
+    const int form = GF == 8 ? per >= 16 : groups > 1 ? qmv_wide_form(per) : 0;
+    if constexpr (GF == 21)
+        if (form == 2) return qmv_wide_ts<GF, F32OUT, 1, UNITS, 2>(p, groups, bpg, per, st);
+    if (form == 1) return qmv_wide_ts<GF, F32OUT, 1, UNITS>(p, groups, bpg, per, st);
     return qmv_wide_ts<GF, F32OUT, 2, UNITS>(p, groups, bpg, per, st);
 }
 

@@ -173,3 +173,20 @@ def test_both_forms_of_more_than_16_tokens_agree_with_the_row_alone(gpu, qtype, 
         y = run_qmv(gpu, "qmv_mma", qtype, W, 2048, x[:B])
         for b, want in alone.items():
             assert b >= B or np.array_equal(bits(y[b]), bits(want)), (B, b)
+
+
+# The three forms of a piece (on 148 SMs): row tiles per block on both sides of every line, at two groups of 64 tokens, three, five and seven; and up to 16 groups (9 blocks each).
+@pytest.mark.parametrize("K", [2048, 4096])
+@pytest.mark.parametrize("per,B", [(2, 65), (3, 129), (4, 130), (5, 320), (7, 128), (8, 100), (9, 192), (10, 257), (11, 70), (12, 449), (13, 448), (15, 577), (17, 385),
+                                   (18, 1000), (19, 512), (22, 1024), (25, 577), (29, 1000), (31, 1024)])
+def test_the_forms_of_a_piece_agree_with_groups_of_64(gpu, K, per, B):
+    rng = np.random.default_rng(per)
+    N = 16 * (per * (148 // ((B + 63) // 64)) - per // 2)  # (the last block has fewer tiles)
+    W = synth.iq3s_rows(rng, N, K)
+    x = synth.acts_fp16(rng, B, K)
+    k = gpu.compile("qmv_mma", "qmv_forms_%d" % K, GF=21, KD=K, ROWS=1024, YT_F32=1)
+    wb, xb, yb = gpu.buf_from(W), gpu.buf_from(x), gpu.buf(B * N * 4).zero()
+    gpu.batch().kernel(k).buf(0, wb).buf(3, xb).buf(4, yb).bytes(5, np.array([N, K, N, B], np.uint32)).dispatch(((N + 7) // 8,), (256,)).end()
+    y = yb.download(np.float32, B * N).reshape(B, N)
+    for r in range(0, B, 64):  # each group of 64 the bits of a launch of its own
+        assert np.array_equal(bits(y[r:r + 64]), bits(run_qmv(gpu, "qmv_mma", 21, W, K, x[r:r + 64]))), r
