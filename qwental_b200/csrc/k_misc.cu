@@ -249,6 +249,7 @@ static cudaError_t launch_add_rmsnorm(const QwLaunch &L) {
                 QW_CHECK_ARG(nranks == 1 && !wide && L.buf<unsigned>(9) && L.avail(9) >= MOE_FFN_SYNC_BYTES);
                 rowcnt = L.buf<unsigned>(9) + MOE_FFN_ROWCNT;
             }
+            // many rows by 16-byte loads; buffers that do not lie at such boundaries (the engine's do) go through the cluster form, whose loads are of 4 bytes
             if (wide && a.nb > MOE_MAXB && nranks == 1 && (((uintptr_t)L.buf<void>(0) | (uintptr_t)L.buf<void>(2) | (uintptr_t)L.buf<void>(3) | (uintptr_t)L.buf<void>(6)) & 15) == 0) {
                 qw_launch(cmb_rmsnorm_rows_k, a.nb, 512, 0, L.stream, L.buf<float>(0), L.buf<float>(2), L.buf<__half>(3), L.buf<moe_sel>(5), L.buf<float>(6), topk);
                 return cudaGetLastError();

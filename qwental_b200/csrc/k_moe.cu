@@ -285,7 +285,7 @@ __device__ __forceinline__ void moe_select_body(const float *logits, moe_sel *ms
 }
 
 // ---- a piece of a prompt (up to 1024 tokens): top-k with a warp per token over many blocks, then the grouping by one block; the router
-// part is moe_route with SELECT defined 0.  (In moe_route's one last block 1024 tokens would be 64 rounds of top-k.)
+// logits are moe_route's with SELECT defined 0 (moe_logits_k).  (In moe_route's one last block 1024 tokens would be 64 rounds of top-k.)
 // moe_topk_wide binds: 0 = logits [nb][E+1], 1 = moe_sel_wide, 2 = {nb, e_lo, e_hi}.  grid ceil(nb/4) x 128
 __global__ void __launch_bounds__(128) moe_topk_wide_k(const float *logits, moe_sel_wide *ms, uint32_t E, uint32_t topk, uint32_t nb) {
     __shared__ uint64_t cand_s[4][32 + MOE_MAXK];
@@ -357,7 +357,7 @@ QW_FAMILY(moe_select, launch_moe_select, 1024)
 // Up to four tokens -- one per warp at most -- are read straight from L2: staging them costs a copy's latency and saves nothing.
 // binds: 0 = Wr, 1 = Wsg, 2 = x, 3 = logits, 4 = counter (uint32, zero before the first launch; left zero), 5 = moe_sel,
 // 14 = {nb, e_lo, e_hi}.  The launcher sets the grid itself: ceil((E+1)/4) blocks of 512 threads.  With SELECT defined 0 only the
-// logits are computed, of up to 1024 tokens (binds 4 and 5 are not used).
+// logits are computed, of up to 1024 tokens (binds 4 and 5 are not used): by moe_logits_k at D = 2048 and more than 64 tokens -- the engine's pieces of a prompt --, else here.
 // With NORM defined 1 (D = 2048, up to four tokens) the launch begins with the residual add + RMSNorm before the router, in the order of
 // add_rmsnorm: 6 = h fp32 [nb][D], 7 = delta fp16 [nb][D], 8 = w fp32 [D], 9 = h out (another buffer: every block reads h), 2 = x out.
 // Every block normalises all tokens for itself -- 12 KB of L2 reads per token and block -- and the first one stores h and x; that is

@@ -290,3 +290,41 @@ def test_wide_ffn_with_room_for_half_a_piece(gpu):
             wide_ffn(gpu, h, x, E, topk, rows=513, say=say)
     with pytest.raises(GpuError):
         wide_ffn(gpu, h, x[:100], E, topk, rows=511)
+
+
+@pytest.mark.parametrize("D,nb", [(2048, 3), (2048, 64), (2048, 65), (2048, 143), (256, 4), (256, 65), (256, 200)])
+def test_logits_alone_are_those_of_the_router(gpu, D, nb):
+    """moe_route with SELECT defined 0, in the form for many tokens and in the other one: the canonical-order logits, bit for bit."""
+    from qwental_b200.layers import u32
+    E = 64
+    rng = np.random.default_rng(nb)
+    Wr, wsg = (rng.standard_normal((E, D)) * 0.02).astype(np.float16), (rng.standard_normal(D) * 0.02).astype(np.float16)
+    x = synth.acts_fp16(rng, nb, D)
+    k = gpu.compile("moe_route", "t_logits_%d" % D, E=E, D=D, TOPK=4, SELECT=0)
+    b = [gpu.buf_from(a) for a in (Wr, wsg, x)] + [gpu.buf(nb * (E + 1) * 4)]
+    gpu.batch().kernel(k).buf(0, b[0]).buf(1, b[1]).buf(2, b[2]).buf(3, b[3]).bytes(14, u32(nb, 0, E)).dispatch((1,), (1024,)).end()
+    got = b[3].download(np.uint32, nb * (E + 1)).reshape(nb, E + 1)
+    assert np.array_equal(got, orc.router_canon(np.concatenate([Wr, wsg[None]]), x).view(np.uint32))
+
+
+@pytest.mark.parametrize("nb", [65, 131])
+def test_combine_and_norm_of_many_rows_wherever_the_buffers_lie(gpu, nb):
+    """More than 64 rows of the combine + norm go by 16-byte loads where all buffers lie at such boundaries, and column by column where one does not: the same bits."""
+    import ctypes as C
+    from qwental_b200.layers import u32
+    D, topk = 2048, 10
+    rng = np.random.default_rng(nb)
+    gpu.L.qw_moe_sel_wide_bytes.restype = C.c_size_t
+    k = gpu.compile("add_rmsnorm", "t_cmb_wide", CMB=1, TOPK=topk, WIDE=1, ROWS=1024)
+    sel = gpu.buf(gpu.L.qw_moe_sel_wide_bytes()).zero()
+    sel.upload(rng.random((nb, 17)).astype(np.float32), 16 + 64 * 16 * 4)
+    h, Pg = rng.standard_normal((nb, D)).astype(np.float32), rng.standard_normal((nb, topk + 1, D)).astype(np.float32)
+    w, pg = gpu.buf_from((1 + 0.1 * rng.standard_normal(D)).astype(np.float32)), gpu.buf_from(Pg)
+
+    def run(off):
+        hb, x = gpu.buf(h.nbytes + 16).upload(h, off), gpu.buf(nb * D * 2)
+        gpu.batch().kernel(k).buf(0, hb, off).buf(2, w).buf(3, x).buf(5, sel).buf(6, pg).bytes(4, u32(nb, D)).dispatch((nb,), (256,)).end()
+        return hb.download(np.uint32, nb * D, off), x.download(np.uint16, nb * D)
+
+    for a, b in zip(run(0), run(4)):
+        assert np.array_equal(a, b)
