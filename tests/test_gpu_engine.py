@@ -537,3 +537,37 @@ def test_tickets_are_void_where_the_batch_would_be_another(gpu, monkeypatch):
         gpu.L.qw_gpu_set_graphs(gpu.g, False)
         other.close()
 
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_a_chain_whose_second_step_fails(gpu, graphs):
+    """The step that is fed by the one before uses kernels the first one does not (the Gated DeltaNet forms that read ahead, in layers 0 and 1); one of them made to
+    fail at launch, it fails while the first step runs: the call fails, the first step's ids are there, and the engine works on."""
+    import ctypes as C
+    from qwental_b200.engine import Engine, wide_cfg
+    from qwental_b200.gpu import GpuError
+    e = Engine(gpu, wide_cfg(layers=3, attn_every=3))
+    gd = dict(HK=16, HV=32, DV=128, GDN_TILED=1, EARLY=1)
+
+    def seed():
+        for s in (0, 2):
+            e.seed_slot(s, 70 + s, 9 + s)
+    try:
+        seed()
+        want, _ = e.decode_greedy([0, 2], [5, 6], 3)
+        gpu.L.qw_gpu_set_graphs(gpu.g, graphs)
+        seed()
+        out = np.full((3, 2), -7, np.int32)
+        s, t = np.array([0, 2], np.int32), np.array([5, 6], np.int32)
+        p = lambda a, ty: a.ctypes.data_as(C.POINTER(ty))
+        gpu.compile("gdn_fstep", "gdn_fstep_early", **dict(gd, DV=64))
+        assert e.L.qw_engine_par_decode_greedy(e.e, p(s, C.c_int), p(t, C.c_int32), 2, 3, p(out, C.c_int32), None) == -1
+        assert "at step 1" in e.error() and np.array_equal(out[0], want[0]) and np.all(out[1:] == -7)
+        with pytest.raises(GpuError):
+            e.decode_greedy([0, 2], [5, 6], 2)
+        gpu.compile("gdn_fstep", "gdn_fstep_early", **gd)
+        seed()
+        assert np.array_equal(e.decode_greedy([0, 2], [5, 6], 3)[0], want)
+    finally:
+        gpu.L.qw_gpu_set_graphs(gpu.g, False)
+        e.close()

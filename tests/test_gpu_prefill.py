@@ -246,3 +246,46 @@ def test_last_layer_of_a_prompt(gpu, layers, every):
         assert np.array_equal(both[0].view(np.uint32), both[1].view(np.uint32))
     finally:
         e.close()
+
+
+@pytest.mark.parametrize("experts", [32, 512])
+def test_a_full_piece_with_the_most_choices(gpu, experts):
+    """1023 and 1024 tokens with 15 experts each: every row of the FFN's H (15360 entries and the shared expert's 1024), the most items a block's share can touch (512
+    experts) and experts with some 480 entries (32)."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(experts=experts, topk=15, layers=2, attn_every=2, max_slots=2))
+    try:
+        text = np.random.default_rng(experts).integers(0, e.cfg.vocab, 1024).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, 1025):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n < 1023:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
+
+
+@pytest.mark.parametrize("hk,hv", [(16, 16), (16, 48), (8, 64)])
+def test_prompts_with_other_numbers_of_value_heads(gpu, hk, hv):
+    """Other numbers of Gated DeltaNet heads than 16 and 32: the recurrence in more than one wave of blocks (48 and 64 value heads on 148 SMs), channels that fill the
+    epilogue's blocks in part, output projections without a form for wide pieces."""
+    from qwental_b200.engine import Engine, wide_cfg
+    e = Engine(gpu, wide_cfg(layers=3, attn_every=2, hk=hk, hv=hv, max_slots=2))
+    try:
+        lengths = {2, 17, 64, 65, 130, 300}
+        text = np.random.default_rng(hv).integers(0, e.cfg.vocab, max(lengths)).astype(np.int32)
+        e.prefill(0, text[:1])  # slot 0 steps every token
+        for n in range(2, max(lengths) + 1):
+            lg, _ = e.step([0], text[n - 1:n])
+            if n not in lengths:
+                continue
+            got = e.prefill(1, text[:n])
+            assert np.array_equal(got.view(np.uint32), lg[0].view(np.uint32)), n
+            for a, b in zip(state_of(e, 1), state_of(e, 0)):
+                assert np.array_equal(a, b), n
+    finally:
+        e.close()
