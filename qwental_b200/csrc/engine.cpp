@@ -148,8 +148,8 @@ struct qw_engine {
     long long last_ctx = 0;
     int last_own = 0;  // rows of the last step whose token mixers ran on this rank
     // Graphs of the steps recorded so far, by what encode_step's work depends on.  Recording 350 to 400 launches again and looking their graph up by
-    // its key kept the device waiting 0.39 ms in every step: with this, and a greedy step submitted before its predecessor is waited for, steps of 1, 3
-    // (small model), 16 and 23 slots take 1.17, 1.13, 1.08 and 1.06 times less on a B200.
+    // its key kept the device waiting 0.39 ms in every step: with this, and a greedy step submitted before its predecessor is waited for, a step of one
+    // slot takes 1.17 times less on a B200; of 3 (small model), 16 and 23 slots 1.13, 1.07 and 1.06, about what two runs of those differ by.
     struct StepPlan {
         unsigned long long ticket;
         const qw_buf *h_last;
@@ -733,8 +733,8 @@ void encode_step(qw_engine *e, qw_batch *b, uint32_t nb, uint32_t max_chunks, bo
         const LayerW &w = e->layers[l];
         // Of a piece, the last layer only has to bring the KV cache and the recurrent state forward; what follows it is wanted for the prompt's
         // last token alone -- row 0 of the last piece, which goes on as a step of one row.  (Ranks that share the experts keep all rows: their
-        // exchange is built for one row count per pass.)  Prompts of 45 and 419 tokens, 48 layers: 1.013x, 1.017x; of 1700 tokens, 12 layers: 36.3 ->
-        // 33.7 ms on a B200.
+        // exchange is built for one row count per pass.)  Prompts of 45 and 419 tokens, 48 layers, on a B200: 9.57 -> 9.43 and 27.5 -> 27.1 ms; of 1700 tokens, 12
+        // layers: 24.5 -> 23.0.
         const bool state_only = piece && l == e->L - 1 && e->c.ep_size == 1;
         auto row0_goes_on = [&] {
             nb = nbl = 1;

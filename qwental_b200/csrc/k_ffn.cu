@@ -550,7 +550,6 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
             if (lane == 0) mbar_arrive(&empty[j % FFN_STG]);
             j++;
         };
-        // activation slot of the next item: waits for its copy, returns its shared address
         // activation rows of the next item (see the producer's act_for): waits for their copy; returns the address of column g's row
         uint32_t rowbase = 0;
         auto act_wait = [&](uint32_t ncols, uint32_t pitch) {
@@ -736,7 +735,8 @@ __global__ void __launch_bounds__(FFN_THREADS, FfnCfg<FMT>::PER_SM) moe_ffn_k(co
 // One layer on a B200, items of eight columns in moe_ffn_k / one row tile per warp / two: 419 tokens 372 / 328 / 297 us, 287 with the shares below.  Prompts, 12 layers, one row tile / two: 200
 // tokens 5.07 -> 4.78 ms, 419 7.20 -> 6.83, 512 8.26 -> 7.79, 1024 14.32 -> 13.59.  Bound by the decode still (all 513 experts are 857 MB, 131 us).
 // Items of 24 columns leave room for three stages: with one row tile per warp 13.67 ms at 1024 tokens, with two (276 bytes of spills) 14.06; 32 columns leave
-// two.  Short prompts on moe_ffn_k's eight columns and two blocks per SM: 65 tokens 3.26 against 3.12 ms here, 100 3.59 / 3.50.
+// two.  Short prompts on moe_ffn_k's eight columns and two blocks per SM: 65 tokens 3.26 against 3.12 ms here, 100 3.59 / 3.50.  Pieces and steps of up to 64 rows
+// run moe_ffn_k all the same: their selection record is the smaller one and the norm behind it starts by rows.  Which form is the faster there has not been measured.
 constexpr int WFFN_RECS = 24;  // items a block's share can touch: at most 17 with 148 blocks, 1024 tokens and 15 choices each
 struct WffnCost {  // of a gate/up piece and of a down piece: a decode of the stage, and the MMAs and the epilogue of a column tile
     uint32_t dec, tile;
@@ -1137,7 +1137,8 @@ __global__ void __launch_bounds__(FFN_THREADS, 1) moe_ffn_wide_k(const FfnP p) {
     // the last block to finish clears the items' counters for the next launch (every block has read what it needed by then)
     __syncthreads();
     if (tid == FFN_CW * 32) {
-        // No block ends with copies of its own in flight: the last ones have landed by now, unless a wait for them ran out; then they are waited for again, with a limit.
+        // No block ends with copies of its own in flight: the last ones have landed by now, unless a wait for them ran out; then they are waited for again, with
+        // a limit.  (By the producer before the barrier above: prompts 0.3 % longer.)
         for (uint32_t n = edge[0] > WFFN_STG ? edge[0] - WFFN_STG : 0; n < edge[0]; n++) mbar_wait(&full[n % WFFN_STG], (n / WFFN_STG) & 1);
         for (uint32_t n = edge[1] > 2 ? edge[1] - 2 : 0; n < edge[1]; n++) mbar_wait(&actfull[n & 1], (n >> 1) & 1);
     }

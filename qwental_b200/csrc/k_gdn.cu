@@ -211,11 +211,11 @@ __global__ void __launch_bounds__(512, 2) gdn_fstep_k(const __half *cv, const fl
     float4 *S = (float4 *)(pool + (((size_t)sids[t] * a.nlayers + a.layer) * HV + hv) * DK * DV) + c4;
 
     // State rows into registers: the long-latency part.  With EARLY defined 1 they, and the slot id they are found by, are requested before the
-    // wait for the previous kernel.  The state was last written in an earlier batch, which the host has waited for; the slot table by
+    // wait for the previous kernel.  The state was last written a step earlier, which may still be running; the slot table by
     // par_begin at the start of this step, possibly.  A launch cannot begin before every block of its predecessor has started, but that alone says
     // little: the small launches of a layer can all be resident while par_begin still reads the host's memory.  So the host runs this form
-    // only behind two launches that fill every SM (moe_ffn: as many blocks as fit the device) after par_begin: the later one cannot have
-    // started all its blocks before the earlier one has left, and that one has waited for everything before it.
+    // only behind two launches that fill every SM (moe_ffn: as many blocks as fit the device) after either writer -- a step has at least three --: the later
+    // one cannot have started all its blocks before the earlier one has left, and that one has waited for everything before it.
     float4 s[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) s[i] = S[(size_t)(8 * rq + i) * (DV / 4)];

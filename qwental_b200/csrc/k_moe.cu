@@ -529,7 +529,9 @@ __global__ void __launch_bounds__(512) moe_route_k(const __half *Wr, const __hal
 // 16 rows x 8 tokens.  Rows and tokens come through L1, which its warps share.  A dot product is the same single-lane chain and the same butterfly (over 16
 // values at once: every step but the first halves them).  512 experts, 419 tokens on a B200: 61 -> 40 us with eight tokens per warp, 32 per block and every
 // chunk waited for; four tokens leave registers to fetch the next chunk ahead, and smaller blocks fill the last wave: prompts of 70, 164 and 419 tokens, 12
-// layers, 3.556 -> 3.531, 4.800 -> 4.757 and 7.237 -> 7.211 ms.  (Fetching ahead with eight tokens per warp: 7.298.)  grid (ceil((E + 1) / 16), ceil(nb / 8)) x 256
+// layers, 3.556 -> 3.531, 4.800 -> 4.757 and 7.237 -> 7.211 ms.  (Fetching ahead with eight tokens per warp: 7.298.)
+// At 1024 tokens the blocks read 405 MB through L2 in 87 us, 4.7 TB/s, about what L2 gives (419 tokens: 168 MB in 38): larger blocks would be what is left.
+// grid (ceil((E + 1) / 16), ceil(nb / 8)) x 256
 __global__ void __launch_bounds__(256) moe_logits_k(const __half *Wr, const __half *Wsg, const __half *x, float *logits, uint32_t E, uint32_t nb) {
     constexpr int D = 2048, CH = D / 8 / 32, R = 4, T = 4;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * 16 + (warp & 3) * R, t0 = blockIdx.y * 8 + (warp >> 2) * T;

@@ -483,8 +483,9 @@ static cudaError_t qmv_mma2_go(const QmvMmaP &p, int sm_count, cudaStream_t st) 
 // latency.  1 (Q8_0, 16 tiles per SM and more; IQ3_S by qmv_wide_form): a unit is decoded once for all tokens, by fewer warps with more registers.
 // RT = row tiles per warp.  2 (IQ3_S): the activations are read once for both; the weight stages are then one unit long (shared memory).
 // Measured on a B200, before -> now, L2 flushed: Q8_0 151936 x 2048, 17 tokens 138 -> 110 us, 61 tokens 253 -> 165 us (TS = 2: 144 and 192);
-// IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us; 61 tokens are bound by the shared-memory pipe, about
-// 40 of its cycles per unit of 16 rows x 32 weights.
+// IQ3_S 5120 x 2048, 61 tokens 27.2 -> 22.5 us.  330 MB of weights take 50 us.  The head at 61 tokens fills no pipe: shared memory is busy 61 % of the time, the
+// tensor pipe 47 %, issue slots 43 %, DRAM 26 % (ncu); with three warps per scheduler a warp issues every 7 cycles, 2.2 of them the latency of its own last
+// instruction, 1.9 waiting for loads, 0.8 for the tensor pipe.
 template <int GF, int TS, int RT = 1>
 struct WideCfg {
     static constexpr int RG = RT * (TS == 2 || GF == 21 ? 7 : 11);  // row tiles per round: 14 + 1 warps of 128 registers, 7 + 1 of up to 255 (with one or two tiles each) or 11 + 1 of 168

@@ -227,7 +227,7 @@ class Engine:
         return out
 
     def prefill(self, sid: int, prompt) -> np.ndarray:
-        """Feeds a prompt into an empty slot (in pieces of up to 512 tokens; equal to stepping every token); returns the last position's logits."""
+        """Feeds a prompt into an empty slot (in pieces of up to 1024 tokens; equal to stepping every token); returns the last position's logits."""
         p = np.ascontiguousarray(prompt, np.int32)
         ptr = self.L.qw_engine_par_prefill(self.e, sid, p.ctypes.data, len(p), None)
         if not ptr:

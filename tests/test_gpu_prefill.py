@@ -68,8 +68,8 @@ def test_recurrence_around_the_edges_of_its_buffers(gpu):
 
 
 def test_wide_pieces_equal_stepping_every_token(gpu):
-    """Pieces of 65 to 512 tokens (512 experts, ten per token: several passes per expert and most experts chosen), at the edges of a piece,
-    of the groups of 64 rows inside it and of what is left for a second and third piece."""
+    """Pieces of 65 to 577 tokens (512 experts, ten per token: several items per expert and most experts chosen), at the edges of the groups of 64 rows
+    inside them and of half a piece, whose rest of up to 64 tokens goes by itself."""
     from qwental_b200.engine import Engine, wide_cfg
     e = Engine(gpu, wide_cfg(experts=512, topk=10, max_slots=2))
     try:
@@ -134,7 +134,7 @@ def test_a_failed_prompt_frees_its_slot(gpu, n, kernel, family, broken, whole):
 
 @pytest.mark.parametrize("n", [2, 40, 130, 600])
 def test_records_after_a_prompt_are_those_of_its_last_token(gpu, n):
-    """The selection record and the step's byte counts after a prompt (pieces of up to 64 tokens and of up to 512 keep different records on the
+    """The selection record and the step's byte counts after a prompt (pieces of up to 64 tokens and wider ones keep different records on the
     device) equal those after stepping its last token; h, x and logits are that token's."""
     from qwental_b200.engine import Engine, wide_cfg
     e = Engine(gpu, wide_cfg(experts=256, topk=6, max_slots=2))
