@@ -331,7 +331,8 @@ QW_FAMILY(gdn_fstep, launch_gdn_fstep, 512)
 // Bound by the latency of one token's chain: decay, the fma chain of S^T k, the 16 group sums through shared memory, their ordered sum, the
 // update.  Everything else is off it: S^T q of a token runs beside the next token's sums, and its 16 group sums are left to the other warps.
 // 419 tokens on a B200: 146 -> 95 us (before, a lane held 32 rows of one column: every fma its own instruction and its own operand from shared
-// memory, the running sum handed on by four shuffles); prompts of 419 tokens, 48 layers, 40.3 -> 38.4 ms.
+// memory, the running sum handed on by four shuffles); prompts of 419 tokens, 48 layers, 40.3 -> 38.4 ms.  One block per SM, by registers and by shared memory (before, by
+// registers alone): 48 and 64 value heads are two waves of 148 blocks, as before; prompts of 1024 tokens, 3 layers, 9.6 -> 5.9 and 11.2 -> 7.0 ms with the rest of the path.
 // Bit-identical to nb launches of gdn_fstep: the 16 partial sums of eight rows each are the same fma chains and are added in the same order.
 // The gated RMSNorm needs all 128 columns of a head: gdn_gate does it afterwards.
 // binds: 0 = cv fp16 [nb][C], 1 = la [nb][HV], 2 = beta [nb][HV], 3 = state pool, 4 = proj fp16 (row stride z_stride), 5 = conv state
